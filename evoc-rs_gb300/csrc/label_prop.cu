@@ -16,13 +16,16 @@
 //
 // The vote sums are the same f32 additions in the same order as the
 // reference's loop, so labels match the CPU restatement exactly. Random draws
-// come from Philox4x32-10 (counters below) instead of rand::SmallRng. Each
-// node keeps its vote table in its own CSR row range of a scratch array
-// (a row has at most as many distinct labels as entries), so no node can
-// overflow it; rows longer than 64 also get a hash index (at most half full)
-// in four entries per row of two more scratch arrays.
+// come from Philox4x32-10 (counters below) instead of rand::SmallRng. With
+// labels below RG_LABELS (every call of the initialisation) a row's votes are
+// grouped on the SM (k_lp_iter_rows). With more labels each node keeps its vote
+// table in its own CSR row range of a scratch array (a row has at most as many
+// distinct labels as entries), so no node can overflow it; rows longer than 64
+// also get a hash index (at most half full) in four entries per row of two more
+// scratch arrays (k_lp_iter).
 #include "evoc_internal.h"
 #include "evoc_device.cuh"
+#include "row_groups.cuh"
 
 #include <algorithm>
 
@@ -141,6 +144,191 @@ __global__ void k_lp_hcap(const int64_t* __restrict__ indptr, int64_t n,
   cap_out[i] = cap;
 }
 
+// Marks the neighbours of newly labelled nodes for the round that comes next.
+__device__ __forceinline__ void lp_mark_row(const uint32_t* __restrict__ indices, int64_t b,
+                                            int64_t e, int first, int stride, uint8_t tag,
+                                            uint8_t* __restrict__ mark) {
+  for (int64_t q = b + first; q < e; q += stride) mark[indices[q]] = tag;
+}
+
+__global__ void k_lp_mark_seeds(const int64_t* __restrict__ indptr,
+                                const uint32_t* __restrict__ indices, int64_t n, int64_t parts,
+                                uint64_t seed, uint8_t* __restrict__ mark) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= parts) return;
+  const uint32_t v = lp_seed_draw(seed, (uint32_t)i, (uint32_t)n);
+  lp_mark_row(indices, indptr[v], indptr[v + 1], threadIdx.x & 31, 32, 0, mark);
+}
+
+// One conservative iteration for labels below RG_LABELS, a warp per 32 nodes:
+// labelled nodes pass their label on, and each unlabelled node's row is read by
+// the whole warp (coalesced, 32 label gathers in flight), its labelled entries
+// are compacted and grouped on the SM (row_groups.cuh). The winner is the
+// largest sum of at least 1.0, among equal sums the label whose first entry
+// comes last, as in k_lp_iter. Rows with more than RG_CAP labelled or RG_LONG_ROW
+// entries go to `longs`. A round after one that labelled nobody returns at once:
+// both label arrays are equal then, so no round needs the host.
+// With `mark` (symmetric graphs) only nodes with a neighbour labelled in the
+// round before are looked at: the others' votes, and so their outcome, are the
+// ones they had. A winner marks its neighbours with the next round's number in
+// the other of two arrays, so no mark that this round still reads is overwritten.
+__global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_lp_iter_rows(
+    const int64_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
+    const float* __restrict__ w, int64_t n, const int32_t* __restrict__ in,
+    int32_t* __restrict__ out, const int32_t* __restrict__ prev_changed,
+    int32_t* __restrict__ changed, uint32_t* __restrict__ longs, int32_t* __restrict__ n_long,
+    int32_t round, const uint8_t* __restrict__ mark, uint8_t* __restrict__ next_mark) {
+  __shared__ RgWarp<RG_CAP> sm_all[RG_WARPS];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (prev_changed && *prev_changed == 0) return;
+  const int64_t v0 = ((int64_t)blockIdx.x * RG_WARPS + wid) * 32;
+  if (v0 >= n) return;
+  RgWarp<RG_CAP>& sm = sm_all[wid];
+  const int64_t v = v0 + lane;
+  int32_t mine = v < n ? in[v] : 0;
+  const bool look = mine < 0 && (!mark || mark[v] == (uint8_t)round);
+  const int64_t pb = look ? indptr[v] : 0, pe = look ? indptr[v + 1] : 0;
+  const uint32_t lt = (1u << lane) - 1u;
+  bool won = false;
+  for (uint32_t todo = __ballot_sync(FULL, look); todo; todo &= todo - 1) {
+    const int src = __ffs(todo) - 1;
+    const int64_t b = __shfl_sync(FULL, pb, src), e = __shfl_sync(FULL, pe, src);
+    int m = 0;
+    float votes = 0.0f;  // the lane's share of the row's votes
+    bool fits = e - b <= RG_LONG_ROW;
+    __syncwarp();  // the previous node's readers are done
+    for (int64_t q0 = b; q0 < e && fits; q0 += 32) {
+      const int64_t q = q0 + lane;
+      const int32_t l = q < e ? in[indices[q]] : -1;
+      const uint32_t has = __ballot_sync(FULL, l >= 0);
+      const int at = m + __popc(has & lt);
+      m += __popc(has);
+      fits = m <= RG_CAP;
+      if (fits && l >= 0) {
+        const float wq = w[q];
+        sm.key[at] = ((uint32_t)l << RG_POS_BITS) | (uint32_t)at;
+        sm.val[at] = wq;
+        votes += fabsf(wq);
+      }
+    }
+    if (!fits) {
+      if (lane == 0) longs[atomicAdd(n_long, 1)] = (uint32_t)(v0 + src);
+      continue;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) votes += __shfl_xor_sync(FULL, votes, o);
+    // no label reaches 1.0 if all votes together, rounding included, do not
+    if (votes < 0.999f) continue;
+    const int runs = rg_group(sm, m, lane);
+    float best = 1.0f;  // threshold
+    int first = -1;     // position of the best label's first entry
+    uint32_t lab = 0;
+    for (int r = lane; r < runs; r += 32) {
+      const uint32_t k = sm.key[sm.start[r]];
+      const float s = sm.sum[r];
+      const int pos = (int)(k & RG_POS);
+      if (s > best || (s == best && pos > first)) {
+        best = s;
+        first = pos;
+        lab = k >> RG_POS_BITS;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float s = __shfl_xor_sync(FULL, best, o);
+      const int p = __shfl_xor_sync(FULL, first, o);
+      const uint32_t l = __shfl_xor_sync(FULL, lab, o);
+      if (s > best || (s == best && p > first)) {
+        best = s;
+        first = p;
+        lab = l;
+      }
+    }
+    if (first >= 0) {
+      if (lane == src) {
+        mine = (int32_t)lab;
+        won = true;
+      }
+      if (mark) lp_mark_row(indices, b, e, lane, 32, (uint8_t)(round + 1), next_mark);
+    }
+  }
+  if (v < n) out[v] = mine;
+  if (won) *changed = 1;
+}
+
+// The rows of `longs`, a block per row.
+__global__ void __launch_bounds__(RG_LONG_THREADS) k_lp_iter_long(
+    const int64_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
+    const float* __restrict__ w, const int32_t* __restrict__ in, int32_t* __restrict__ out,
+    int32_t* __restrict__ changed, const uint32_t* __restrict__ longs,
+    const int32_t* __restrict__ n_long, int32_t round, uint8_t* __restrict__ next_mark) {
+  extern __shared__ __align__(16) unsigned char rg_raw[];
+  RgLongVotes& sm = *reinterpret_cast<RgLongVotes*>(rg_raw);
+  __shared__ int any;
+  __shared__ float wb[RG_LONG_THREADS / 32];
+  __shared__ uint32_t wf[RG_LONG_THREADS / 32], wl[RG_LONG_THREADS / 32];
+  const unsigned FULL = 0xffffffffu;
+  const int nl = *n_long;
+  for (int item = blockIdx.x; item < nl; item += gridDim.x) {
+    const uint32_t i = longs[item];
+    const int64_t b = indptr[i], e = indptr[i + 1];
+    rg_long_clear(sm);
+    for (int64_t c = b; c < e; c += RG_CHUNK) {
+      for (int q = threadIdx.x; q < RG_CHUNK; q += RG_LONG_THREADS) {
+        const int32_t l = c + q < e ? in[indices[c + q]] : -1;
+        sm.key[q] = l >= 0 ? ((uint32_t)l << 10) | (uint32_t)q : 0xffffffffu;
+        sm.val[q] = l >= 0 ? w[c + q] : 0.0f;
+      }
+      rg_long_chunk(sm, sm.first, (uint32_t)(c - b));
+    }
+    float best = 1.0f;  // threshold; first + 1 of the best label, 0 for none
+    uint32_t first = 0, lab = 0;
+    for (int l = threadIdx.x; l < RG_LABELS; l += RG_LONG_THREADS) {
+      if (!((sm.bits[l >> 5] >> (l & 31)) & 1u)) continue;
+      const float s = sm.acc[l];
+      const uint32_t p = sm.first[l] + 1u;
+      if (s > best || (s == best && p > first)) {
+        best = s;
+        first = p;
+        lab = (uint32_t)l;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float s = __shfl_xor_sync(FULL, best, o);
+      const uint32_t p = __shfl_xor_sync(FULL, first, o), l = __shfl_xor_sync(FULL, lab, o);
+      if (s > best || (s == best && p > first)) {
+        best = s;
+        first = p;
+        lab = l;
+      }
+    }
+    if ((threadIdx.x & 31) == 0) {
+      wb[threadIdx.x >> 5] = best;
+      wf[threadIdx.x >> 5] = first;
+      wl[threadIdx.x >> 5] = lab;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int q = 1; q < RG_LONG_THREADS / 32; ++q)
+        if (wb[q] > best || (wb[q] == best && wf[q] > first)) {
+          best = wb[q];
+          first = wf[q];
+          lab = wl[q];
+        }
+      any = first > 0;
+      if (first > 0) {
+        out[i] = (int32_t)lab;
+        *changed = 1;
+      }
+    }
+    __syncthreads();
+    if (next_mark && any)
+      lp_mark_row(indices, b, e, threadIdx.x, RG_LONG_THREADS, (uint8_t)(round + 1), next_mark);
+  }
+}
+
 __global__ void k_lp_max(const int32_t* __restrict__ labels, int64_t n, int32_t* __restrict__ mx,
                          int32_t* __restrict__ unl) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -165,38 +353,53 @@ __global__ void k_lp_list(const int32_t* __restrict__ unl, const int64_t* __rest
 // resolves the pointers. A walk pops at most 64 nodes, so only the top 64
 // stack entries can ever be popped: the stack is a 64-entry ring that drops
 // its bottom entry when full.
-__global__ void k_lp_walk(const int64_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
-                          const int32_t* __restrict__ labels, const int32_t* __restrict__ unl,
-                          const int64_t* __restrict__ pos, const uint32_t* __restrict__ list,
-                          int64_t count, int32_t max_label, uint64_t seed,
-                          int32_t* __restrict__ res) {
-  const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per walk: it reads a popped node's row 32 entries at a time (one node's
+// row can hold thousands), stops at the first entry that ends the walk, and
+// pushes the others in row order.
+constexpr int LP_WALK_WARPS = 8;
+__global__ void __launch_bounds__(32 * LP_WALK_WARPS) k_lp_walk(
+    const int64_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
+    const int32_t* __restrict__ labels, const int64_t* __restrict__ pos,
+    const uint32_t* __restrict__ list, int64_t count, int32_t max_label, uint64_t seed,
+    int32_t* __restrict__ res) {
+  __shared__ uint32_t ring_all[LP_WALK_WARPS][64];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t u = (int64_t)blockIdx.x * LP_WALK_WARPS + wid;
   if (u >= count) return;
+  uint32_t* ring = ring_all[wid];
   const uint32_t i = list[u];
-  uint32_t ring[64];
-  int64_t top = 0, bottom = 0;  // entries [bottom, top), slot = index % 64
-  ring[0] = i;
-  top = 1;
+  int64_t top = 1, bottom = 0;  // entries [bottom, top), slot = index % 64
+  if (lane == 0) ring[0] = i;
+  __syncwarp();
   for (int step = 0; step < 64 && top > bottom; ++step) {
     --top;
     const uint32_t node = ring[top & 63];
-    for (int64_t q = indptr[node]; q < indptr[node + 1]; ++q) {
-      const uint32_t j = indices[q];
-      const int32_t l = labels[j];
-      if (l >= 0) {
-        res[u] = l;
+    __syncwarp();  // read before the slot is pushed over
+    const int64_t b = indptr[node], e = indptr[node + 1];
+    for (int64_t q0 = b; q0 < e; q0 += 32) {
+      const int64_t q = q0 + lane;
+      uint32_t j = 0;
+      int32_t l = -1;
+      if (q < e) {
+        j = indices[q];
+        l = labels[j];
+      }
+      // labelled, or an earlier outlier (unlabelled here): labelled by then
+      const uint32_t hit = __ballot_sync(FULL, q < e && (l >= 0 || j < i));
+      const int cnt = hit ? __ffs(hit) - 1 : (int)min((int64_t)32, e - q0);
+      if (hit) {
+        if (lane == cnt) res[u] = l >= 0 ? l : (int32_t)(-2 - pos[j]);
         return;
       }
-      if (unl[j] && j < i) {  // an earlier outlier: labelled by then
-        res[u] = (int32_t)(-2 - pos[j]);
-        return;
-      }
-      ring[top & 63] = j;
-      ++top;
-      if (top - bottom > 64) ++bottom;
+      __syncwarp();  // a long row's earlier pushes to these slots come first
+      if (lane < cnt) ring[(top + lane) & 63] = j;
+      top += cnt;
+      if (top - bottom > 64) bottom = top - 64;
     }
+    __syncwarp();
   }
-  res[u] = (int32_t)lp_outlier_draw(seed, i, (uint32_t)max_label + 1u);
+  if (lane == 0) res[u] = (int32_t)lp_outlier_draw(seed, i, (uint32_t)max_label + 1u);
 }
 
 // Pointer jumping over the walk results; pointers only go to earlier
@@ -237,17 +440,12 @@ __global__ void k_lp_remap(const int32_t* __restrict__ labels, int64_t n,
 
 inline unsigned grid_for(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
-}  // namespace
-
-int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_n_parts,
-                             int32_t n_iter, uint64_t seed, uint32_t* d_partition) {
-  cudaStream_t s = ctx->stream;
+// The rounds for labels of any size (k_lp_iter): thread per node, vote tables in
+// global memory; one look at the host per round.
+void lp_rounds_any_label(const evoc_graph* g, int32_t n_iter, DevBuf<int32_t>& la,
+                         DevBuf<int32_t>& lb, int32_t* flag, cudaStream_t s) {
   const int64_t n = g->n, nnz = g->nnz;
-  if (n == 0) return 0;
-  if (approx_n_parts < 0 || approx_n_parts >= (1LL << 31))
-    throw Error(EVOC_ERR_INVALID_ARGUMENT, "approx_n_parts outside [0, 2^31)");
-  if (n_iter < 0) throw Error(EVOC_ERR_INVALID_ARGUMENT, "n_iter < 0");
-  DevBuf<int32_t> la(n, s), lb(n, s), vlab(std::max<int64_t>(nnz, 1), s), flag(1, s);
+  DevBuf<int32_t> vlab(std::max<int64_t>(nnz, 1), s);
   DevBuf<float> vsum(std::max<int64_t>(nnz, 1), s);
   // hash tables only for the long rows, packed by a prefix sum of their sizes
   DevBuf<int64_t> hcap(n, s), hoff(n + 1, s);
@@ -259,25 +457,81 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
   EVOC_CUDA(cudaStreamSynchronize(s));
   hcap.release();
   DevBuf<int32_t> hkey(std::max<int64_t>(htot, 1), s), hpos(std::max<int64_t>(htot, 1), s);
+  // a round that labels no node is a fixed point: the rest would leave the
+  // labels unchanged and are skipped
+  for (int32_t it = 0; it < n_iter; ++it) {
+    EVOC_CUDA(cudaMemsetAsync(flag, 0, sizeof(int32_t), s));
+    k_lp_iter<<<grid_for(n, 128), 128, 0, s>>>(g->indptr.get(), g->indices.get(),
+                                               g->weights.get(), n, la.get(), lb.get(),
+                                               vlab.get(), vsum.get(), hoff.get(), hkey.get(),
+                                               hpos.get(), flag);
+    EVOC_CHECK_LAUNCH();
+    std::swap(la, lb);
+    int32_t h = 0;
+    EVOC_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    EVOC_CUDA(cudaStreamSynchronize(s));
+    if (!h) break;
+  }
+}
+
+}  // namespace
+
+int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_n_parts,
+                             int32_t n_iter, uint64_t seed, uint32_t* d_partition) {
+  cudaStream_t s = ctx->stream;
+  const int64_t n = g->n, nnz = g->nnz;
+  if (n == 0) return 0;
+  if (approx_n_parts < 0 || approx_n_parts >= (1LL << 31))
+    throw Error(EVOC_ERR_INVALID_ARGUMENT, "approx_n_parts outside [0, 2^31)");
+  if (n_iter < 0) throw Error(EVOC_ERR_INVALID_ARGUMENT, "n_iter < 0");
+  DevBuf<int32_t> la(n, s), lb(n, s), flag(std::max(n_iter, 1), s);
   k_lp_fill<<<grid_for(n), 256, 0, s>>>(la.get(), n);
   if (approx_n_parts > 0)
     k_lp_seed<<<grid_for(approx_n_parts), 256, 0, s>>>(la.get(), n, approx_n_parts, seed);
   EVOC_CHECK_LAUNCH();
-  // n_iter rounds; a round that labels no node is a fixed point, so the rest
-  // would leave the labels unchanged and are skipped.
-  for (int32_t it = 0; it < n_iter; ++it) {
-    EVOC_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int32_t), s));
-    k_lp_iter<<<grid_for(n, 128), 128, 0, s>>>(g->indptr.get(), g->indices.get(),
-                                               g->weights.get(), n, la.get(), lb.get(),
-                                               vlab.get(), vsum.get(), hoff.get(), hkey.get(),
-                                               hpos.get(),
-                                               flag.get());
-    EVOC_CHECK_LAUNCH();
-    std::swap(la, lb);
-    int32_t h = 0;
-    EVOC_CUDA(cudaMemcpyAsync(&h, flag.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    EVOC_CUDA(cudaStreamSynchronize(s));
-    if (!h) break;
+  if (approx_n_parts <= RG_LABELS) {
+    // n_iter rounds without the host: a round sees from the one before whether
+    // anything is left to do
+    DevBuf<uint32_t> longs(n, s);
+    DevBuf<int32_t> n_long(std::max(n_iter, 1), s);
+    EVOC_CUDA(cudaMemsetAsync(flag.get(), 0, flag.bytes(), s));
+    EVOC_CUDA(cudaMemsetAsync(n_long.get(), 0, n_long.bytes(), s));
+    EVOC_CUDA(cudaFuncSetAttribute((const void*)k_lp_iter_long,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(RgLongVotes)));
+    // rows of a symmetric graph list the nodes that see a new label; a round's
+    // number has to fit a mark
+    DevBuf<uint8_t> marks;
+    const bool use_marks = g->canonical && n_iter < 255;
+    if (use_marks) {
+      marks.alloc(2 * n, s);
+      EVOC_CUDA(cudaMemsetAsync(marks.get(), 0xff, marks.bytes(), s));
+      if (approx_n_parts > 0) {
+        k_lp_mark_seeds<<<grid_for(approx_n_parts * 32), 256, 0, s>>>(
+            g->indptr.get(), g->indices.get(), n, approx_n_parts, seed, marks.get());
+        EVOC_CHECK_LAUNCH();
+      }
+    }
+    const unsigned grid = (unsigned)((n + 32 * RG_WARPS - 1) / (32 * RG_WARPS));
+    const unsigned lgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms, nnz / RG_CAP));
+    for (int32_t it = 0; it < n_iter; ++it) {
+      uint8_t* mark = use_marks ? marks.get() + (it & 1) * n : nullptr;
+      uint8_t* next = use_marks ? marks.get() + (1 - (it & 1)) * n : nullptr;
+      k_lp_iter_rows<<<grid, 32 * RG_WARPS, 0, s>>>(
+          g->indptr.get(), g->indices.get(), g->weights.get(), n, la.get(), lb.get(),
+          it > 0 ? flag.get() + it - 1 : nullptr, flag.get() + it, longs.get(),
+          n_long.get() + it, it, mark, next);
+      EVOC_CHECK_LAUNCH();
+      if (nnz > RG_CAP) {
+        k_lp_iter_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLongVotes), s>>>(
+            g->indptr.get(), g->indices.get(), g->weights.get(), la.get(), lb.get(),
+            flag.get() + it, longs.get(), n_long.get() + it, it, next);
+        EVOC_CHECK_LAUNCH();
+      }
+      std::swap(la, lb);
+    }
+  } else {
+    lp_rounds_any_label(g, n_iter, la, lb, flag.get(), s);
   }
   // mop-up of the nodes still unlabelled, in node order
   DevBuf<int32_t> mx(1, s), unl(n, s);
@@ -296,9 +550,9 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
     DevBuf<uint32_t> list(count, s);
     DevBuf<int32_t> res(count, s);
     k_lp_list<<<grid_for(n), 256, 0, s>>>(unl.get(), pos.get(), n, list.get());
-    k_lp_walk<<<grid_for(count, 128), 128, 0, s>>>(g->indptr.get(), g->indices.get(), la.get(),
-                                                   unl.get(), pos.get(), list.get(), count,
-                                                   max_label, seed + 2000, res.get());
+    k_lp_walk<<<grid_for(count, LP_WALK_WARPS), 32 * LP_WALK_WARPS, 0, s>>>(
+        g->indptr.get(), g->indices.get(), la.get(), pos.get(), list.get(), count, max_label,
+        seed + 2000, res.get());
     EVOC_CHECK_LAUNCH();
     for (int pass = 0; pass < 64; ++pass) {  // chains halve per pass
       EVOC_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int32_t), s));

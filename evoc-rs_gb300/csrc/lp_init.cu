@@ -27,6 +27,9 @@
 // the small Gram matrix in double on the host, with a fixed sign convention.
 #include "evoc_device.cuh"
 #include "evoc_internal.h"
+#include "row_groups.cuh"
+
+#include <cuda_pipeline.h>
 
 #include <algorithm>
 #include <cmath>
@@ -143,18 +146,71 @@ __global__ void k_run_heads(const uint32_t* __restrict__ keys, const uint2* __re
   head[e] = (e == 0 || keys[e] != keys[e - 1] || vals[e].x != vals[e - 1].x) ? 1 : 0;
 }
 
-// Serial sum of each run into slot rid[e]: (key, (vals.x, sum bits)).
-__global__ void k_run_sums(const uint32_t* __restrict__ keys, const uint2* __restrict__ vals,
-                           int64_t m, const int32_t* __restrict__ head,
-                           const int64_t* __restrict__ rid, uint32_t* __restrict__ okeys,
-                           uint2* __restrict__ ovals) {
+// First entry of each run: start[rid[e]] = e for heads; start[runs] = m.
+__global__ void k_run_starts(const int32_t* __restrict__ head, const int64_t* __restrict__ rid,
+                             int64_t m, int64_t* __restrict__ start) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m || !head[e]) return;
-  float s = __uint_as_float(vals[e].y);
-  for (int64_t f = e + 1; f < m && !head[f]; ++f) s = fadd(s, __uint_as_float(vals[f].y));
-  const int64_t r = rid[e];
-  okeys[r] = keys[e];
-  ovals[r] = make_uint2(vals[e].x, __float_as_uint(s));
+  if (e >= m) return;
+  if (head[e]) start[rid[e]] = e;
+  if (e == m - 1) start[rid[m]] = m;
+}
+
+// Serial sum of each run: (key, (vals.x, sum bits)). A thread per run, the next
+// eight values loaded before the eight in hand are added: runs are a few entries
+// or, for a part's own weight in the coarse graph, thousands, and one dependent
+// load per addition made those the kernel's length.
+__global__ void k_run_sums(const uint32_t* __restrict__ keys, const uint2* __restrict__ vals,
+                           const int64_t* __restrict__ start, int64_t runs,
+                           uint32_t* __restrict__ okeys, uint2* __restrict__ ovals) {
+  constexpr int U = 8;
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= runs) return;
+  const int64_t a = start[r], b = start[r + 1];
+  const uint2 v0 = vals[a];
+  float s = __uint_as_float(v0.y);
+  int64_t f = a + 1;
+  if (f + U <= b) {
+    float t[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = __uint_as_float(vals[f + u].y);
+    for (f += U; f + U <= b; f += U) {
+      float x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = __uint_as_float(vals[f + u].y);
+#pragma unroll
+      for (int u = 0; u < U; ++u) s = fadd(s, t[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) t[u] = x[u];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) s = fadd(s, t[u]);
+  }
+  for (; f < b; ++f) s = fadd(s, __uint_as_float(vals[f].y));
+  okeys[r] = keys[a];
+  ovals[r] = make_uint2(v0.x, __float_as_uint(s));
+}
+
+// Sums the equal-(keys, vals.x) runs of a sorted list serially into (ok, ov);
+// returns their count.
+int64_t sum_runs(const uint32_t* keys, const uint2* vals, int64_t m, DevBuf<uint32_t>& ok,
+                 DevBuf<uint2>& ov, cudaStream_t s) {
+  DevBuf<int32_t> head(m, s);
+  DevBuf<int64_t> rid(m + 1, s);
+  k_run_heads<<<grid_of(m), 256, 0, s>>>(keys, vals, m, head.get());
+  EVOC_CHECK_LAUNCH();
+  exclusive_scan_i32_to_i64(head.get(), rid.get(), m, s);
+  int64_t runs = 0;
+  EVOC_CUDA(cudaMemcpyAsync(&runs, rid.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  EVOC_CUDA(cudaStreamSynchronize(s));
+  DevBuf<int64_t> start(runs + 1, s);
+  k_run_starts<<<grid_of(m), 256, 0, s>>>(head.get(), rid.get(), m, start.get());
+  EVOC_CHECK_LAUNCH();
+  ok.alloc(runs, s);
+  ov.alloc(runs, s);
+  k_run_sums<<<grid_of(runs, 128), 128, 0, s>>>(keys, vals, start.get(), runs, ok.get(),
+                                                ov.get());
+  EVOC_CHECK_LAUNCH();
+  return runs;
 }
 
 // Sorts (keys, vals) by (keys major, vals.x minor), stably, then sums the
@@ -170,22 +226,11 @@ int64_t sort_and_sum(uint32_t* keys, uint2* vals, int64_t m, int major_bits, int
   k_swap_keys<<<grid_of(m), 256, 0, s>>>(keys, vals, m);
   EVOC_CHECK_LAUNCH();
   radix_sort_pairs(keys, vals, m, major_bits, s);
-  DevBuf<int32_t> head(m, s);
-  DevBuf<int64_t> rid(m + 1, s);
-  k_run_heads<<<grid_of(m), 256, 0, s>>>(keys, vals, m, head.get());
-  EVOC_CHECK_LAUNCH();
-  exclusive_scan_i32_to_i64(head.get(), rid.get(), m, s);
-  int64_t runs = 0;
-  EVOC_CUDA(cudaMemcpyAsync(&runs, rid.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaStreamSynchronize(s));
-  DevBuf<uint32_t> ok(runs, s);
-  DevBuf<uint2> ov(runs, s);
-  k_run_sums<<<grid_of(m), 256, 0, s>>>(keys, vals, m, head.get(), rid.get(), ok.get(),
-                                        ov.get());
-  EVOC_CHECK_LAUNCH();
+  DevBuf<uint32_t> ok;
+  DevBuf<uint2> ov;
+  const int64_t runs = sum_runs(keys, vals, m, ok, ov, s);
   EVOC_CUDA(cudaMemcpyAsync(keys, ok.get(), runs * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   EVOC_CUDA(cudaMemcpyAsync(vals, ov.get(), runs * sizeof(uint2), cudaMemcpyDeviceToDevice, s));
-  EVOC_CUDA(cudaStreamSynchronize(s));
   return runs;
 }
 
@@ -208,6 +253,219 @@ __global__ void k_runs_to_csr(const uint2* __restrict__ vals, int64_t m, float l
     v = hi;
   idx[e] = vals[e].x;
   w[e] = v;
+}
+
+// ---------------------------------------------------------------------------
+// Canonical graphs (symmetric, sorted rows, equal weights both ways): row j of G
+// lists column j's entries too, so both products of a level are sums over one
+// row, grouped by the part of the neighbour (row_groups.cuh), and no entry has
+// to be sorted across rows. Needs at most RG_LABELS parts.
+// ---------------------------------------------------------------------------
+struct RowGraph {
+  const int64_t* indptr;
+  const uint32_t* indices;
+  const float* w;
+  const uint32_t* part;
+  const float* inv;
+};
+
+// Entry q's label and product: inv_P * w of the coarse graph, or (SYM) the
+// expansion's (w * w) * inv_Q (the symmetric part of an equal pair).
+template <bool SYM>
+__device__ __forceinline__ uint32_t row_entry(const RowGraph& g, int64_t q, float* v) {
+  const uint32_t l = g.part[g.indices[q]];
+  const float w = g.w[q];
+  *v = SYM ? fmul(fmul(w, w), g.inv[l]) : fmul(g.inv[l], w);
+  return l;
+}
+
+template <bool SYM, int CAP>
+__device__ __forceinline__ int row_groups(const RowGraph& g, RgWarp<CAP>& sm, int64_t b, int len,
+                                          int lane) {
+  for (int p = lane; p < len; p += 32) {
+    float v;
+    const uint32_t l = row_entry<SYM>(g, b + p, &v);
+    sm.key[p] = (l << RG_POS_BITS) | (uint32_t)p;
+    sm.val[p] = v;
+  }
+  return rg_group(sm, len, lane);
+}
+
+template <bool SYM>
+__device__ __forceinline__ int long_row_groups(const RowGraph& g, RgLong& sm, int64_t b, int64_t e) {
+  rg_long_clear(sm);
+  for (int64_t c = b; c < e; c += RG_CHUNK) {
+    for (int q = threadIdx.x; q < RG_CHUNK; q += RG_LONG_THREADS) {
+      uint32_t key = 0xffffffffu;
+      float v = 0.0f;
+      if (c + q < e) key = (row_entry<SYM>(g, c + q, &v) << 10) | (uint32_t)q;
+      sm.key[q] = key;
+      sm.val[q] = v;
+    }
+    rg_long_chunk(sm, nullptr, 0u);
+  }
+  return rg_long_list(sm);
+}
+
+// Coarse graph, first product: row j's (P, sum of inv_P w_ij over i in P), P
+// ascending, at the head of the row's CSR range in tmp; cnt[j] of them.
+template <int CAP>
+__device__ __forceinline__ void coarse_row(const RowGraph& g, RgWarp<CAP>& sm, int64_t j, int64_t b,
+                                           int len, int lane, uint2* __restrict__ tmp,
+                                           int32_t* __restrict__ cnt) {
+  const int runs = row_groups<false>(g, sm, b, len, lane);
+  for (int r = lane; r < runs; r += 32)
+    tmp[b + r] = make_uint2(sm.key[sm.start[r]] >> RG_POS_BITS, __float_as_uint(sm.sum[r]));
+  if (lane == 0) cnt[j] = runs;
+}
+
+__global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_coarse_rows(RowGraph g, int64_t n,
+                                                               uint2* __restrict__ tmp,
+                                                               int32_t* __restrict__ cnt,
+                                                               RgLists lists) {
+  __shared__ RgWarp<RG_CAP> sm_all[RG_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t j = (int64_t)blockIdx.x * RG_WARPS + wid;
+  if (j >= n) return;
+  const int64_t b = g.indptr[j], len = g.indptr[j + 1] - b;
+  if (rg_defer(lists, j, len, lane)) return;
+  coarse_row(g, sm_all[wid], j, b, (int)len, lane, tmp, cnt);
+}
+
+__global__ void __launch_bounds__(32 * RG_MID_WARPS) k_coarse_rows_mid(RowGraph g,
+                                                                       uint2* __restrict__ tmp,
+                                                                       int32_t* __restrict__ cnt,
+                                                                       RgLists lists) {
+  extern __shared__ __align__(16) unsigned char rg_raw[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  RgWarp<RG_MID>& sm = reinterpret_cast<RgWarp<RG_MID>*>(rg_raw)[wid];
+  for (int64_t j; (j = rg_next_mid(lists, lane)) >= 0;) {
+    __syncwarp();  // the previous row's readers are done
+    coarse_row(g, sm, j, g.indptr[j], (int)(g.indptr[j + 1] - g.indptr[j]), lane, tmp, cnt);
+  }
+}
+
+__global__ void __launch_bounds__(RG_LONG_THREADS) k_coarse_rows_long(
+    RowGraph g, uint2* __restrict__ tmp, int32_t* __restrict__ cnt, RgLists lists) {
+  extern __shared__ __align__(16) unsigned char rg_raw[];
+  RgLong& sm = *reinterpret_cast<RgLong*>(rg_raw);
+  const int nl = lists.count[1];
+  for (int item = blockIdx.x; item < nl; item += gridDim.x) {
+    const uint32_t j = lists.longs[item];
+    const int64_t b = g.indptr[j];
+    const int runs = long_row_groups<false>(g, sm, b, g.indptr[j + 1]);
+    for (int r = threadIdx.x; r < runs; r += RG_LONG_THREADS) {
+      const uint32_t l = sm.list[r];
+      tmp[b + r] = make_uint2(l, __float_as_uint(sm.acc[l]));
+    }
+    if (threadIdx.x == 0) cnt[j] = runs;
+  }
+}
+
+// cnt of the nodes in part order.
+__global__ void k_perm_counts(const uint2* __restrict__ nodes, int64_t n,
+                              const int32_t* __restrict__ cnt, int32_t* __restrict__ out) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) out[t] = cnt[nodes[t].x];
+}
+
+// The rows' sums in (Q = part(j), j) order: key P, value (Q, sum). Eight lanes
+// per row (a row has about ten parts).
+__global__ void k_coarse_gather(const uint2* __restrict__ nodes, int64_t n,
+                                const int64_t* __restrict__ indptr,
+                                const uint32_t* __restrict__ part, const uint2* __restrict__ tmp,
+                                const int64_t* __restrict__ off, uint32_t* __restrict__ keys,
+                                uint2* __restrict__ vals) {
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  if (t >= n) return;
+  const uint32_t j = nodes[t].x, Q = part[j];
+  const uint2* src = tmp + indptr[j];
+  const int64_t o = off[t];
+  const int c = (int)(off[t + 1] - o);
+  for (int r = threadIdx.x & 7; r < c; r += 8) {
+    const uint2 v = src[r];
+    keys[o + r] = v.x;
+    vals[o + r] = make_uint2(Q, v.y);
+  }
+}
+
+// Expansion: row i's (Q, e) groups, L1-normalised (serial over Q), times the
+// coarse layout (serial over Q, a lane per dimension), plus the direct term,
+// halved: res[i][k]. Label and sum of run r come from the two accessors.
+template <class Label, class Sum>
+__device__ __forceinline__ void expand_row(int64_t i, int runs, int lane, int32_t dim,
+                                           const float* __restrict__ layout,
+                                           const uint32_t* __restrict__ part,
+                                           const float* __restrict__ u, float* __restrict__ res,
+                                           Label label, Sum sum) {
+  float nrm = 0.0f;
+  for (int r = 0; r < runs; ++r) nrm = fadd(nrm, fabsf(sum(r)));
+  const bool scale = nrm > 0.0f;
+  const float sc = scale ? fdiv(1.0f, nrm) : 1.0f;
+  if (lane >= dim) return;
+  float acc = 0.0f;
+#pragma unroll 4
+  for (int r = 0; r < runs; ++r) {
+    const float e = sum(r);
+    const float v = scale ? fmul(e, sc) : e;
+    acc = fadd(acc, fmul(v, layout[(int64_t)label(r) * dim + lane]));
+  }
+  const uint32_t P = part[i];
+  const float direct = fadd(0.0f, fmul(u[P], layout[(int64_t)P * dim + lane]));
+  res[i * dim + lane] = fmul(fadd(acc, direct), 0.5f);
+}
+
+template <int CAP>
+__device__ __forceinline__ void expand_warp_row(const RowGraph& g, RgWarp<CAP>& sm, int64_t i,
+                                                int64_t b, int len, int lane, int32_t dim,
+                                                const float* __restrict__ layout,
+                                                const float* __restrict__ u,
+                                                float* __restrict__ res) {
+  const int runs = row_groups<true>(g, sm, b, len, lane);
+  expand_row(
+      i, runs, lane, dim, layout, g.part, u, res,
+      [&](int r) { return sm.key[sm.start[r]] >> RG_POS_BITS; }, [&](int r) { return sm.sum[r]; });
+}
+
+__global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_expand_groups(
+    RowGraph g, int64_t n, int32_t dim, const float* __restrict__ layout,
+    const float* __restrict__ u, float* __restrict__ res, RgLists lists) {
+  __shared__ RgWarp<RG_CAP> sm_all[RG_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t i = (int64_t)blockIdx.x * RG_WARPS + wid;
+  if (i >= n) return;
+  const int64_t b = g.indptr[i], len = g.indptr[i + 1] - b;
+  if (rg_defer(lists, i, len, lane)) return;
+  expand_warp_row(g, sm_all[wid], i, b, (int)len, lane, dim, layout, u, res);
+}
+
+__global__ void __launch_bounds__(32 * RG_MID_WARPS) k_expand_groups_mid(
+    RowGraph g, int32_t dim, const float* __restrict__ layout, const float* __restrict__ u,
+    float* __restrict__ res, RgLists lists) {
+  extern __shared__ __align__(16) unsigned char rg_raw[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  RgWarp<RG_MID>& sm = reinterpret_cast<RgWarp<RG_MID>*>(rg_raw)[wid];
+  for (int64_t i; (i = rg_next_mid(lists, lane)) >= 0;) {
+    __syncwarp();  // the previous row's readers are done
+    expand_warp_row(g, sm, i, g.indptr[i], (int)(g.indptr[i + 1] - g.indptr[i]), lane, dim, layout,
+                    u, res);
+  }
+}
+
+__global__ void __launch_bounds__(RG_LONG_THREADS) k_expand_groups_long(
+    RowGraph g, int32_t dim, const float* __restrict__ layout, const float* __restrict__ u,
+    float* __restrict__ res, RgLists lists) {
+  extern __shared__ __align__(16) unsigned char rg_raw[];
+  RgLong& sm = *reinterpret_cast<RgLong*>(rg_raw);
+  const int nl = lists.count[1];
+  for (int item = blockIdx.x; item < nl; item += gridDim.x) {
+    const uint32_t i = lists.longs[item];
+    const int runs = long_row_groups<true>(g, sm, g.indptr[i], g.indptr[i + 1]);
+    if (threadIdx.x < 32)
+      expand_row(
+          (int64_t)i, runs, (int)threadIdx.x, dim, layout, g.part, u, res,
+          [&](int r) { return (uint32_t)sm.list[r]; }, [&](int r) { return sm.acc[sm.list[r]]; });
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -332,53 +590,73 @@ __global__ void k_expand_rows(const int64_t* __restrict__ eptr, const uint2* __r
   }
 }
 
-// Runs keyed by row i carry (Q, e) in vals; the row index of run e is keys[e].
 // Column centring (serial column sums over all rows), then scaling.
-// One block: the rows stream through shared memory in chunks of
-// COLMEAN_FLOATS values (double buffered, all threads loading) while thread
-// j < dim adds column j's values serially in row order, the next eight values
-// read while the current eight are added.
-constexpr int COLMEAN_THREADS = 1024;
-constexpr int COLMEAN_FLOATS = 5120;  // per chunk: 5120 / dim rows
+// One block: warps 1.. bring the rows into shared memory in chunks (a ring of
+// three filled by cp.async, rows padded to DIMP) while lane j < dim of warp 0
+// adds column j's values serially in row order. The chain of additions (4 cycles
+// each) is the bound, so the adding warp loads nothing from global memory, its
+// addresses are constant offsets and 16 values are read ahead of their additions.
+constexpr int COLMEAN_THREADS = 512;
+constexpr int COLMEAN_FLOATS = 4096;  // per chunk: 4096 / DIMP rows, a multiple of 16
+template <int DIMP>
 __global__ void __launch_bounds__(COLMEAN_THREADS) k_col_mean(const float* __restrict__ res,
                                                              int64_t n, int32_t dim, float inv_n,
                                                              float* __restrict__ mean) {
-  __shared__ float buf[2][COLMEAN_FLOATS];
+  __shared__ __align__(16) float buf[3][COLMEAN_FLOATS];
+  constexpr int ROWS = COLMEAN_FLOATS / DIMP, U = 16, LOADERS = COLMEAN_THREADS - 32;
   const int j = threadIdx.x;
-  const int64_t rows_per = COLMEAN_FLOATS / dim;
-  const int64_t nch = (n + rows_per - 1) / rows_per;
-  auto load = [&](int64_t c, int b) {
-    const int64_t r0 = c * rows_per;
-    const int64_t cnt = min(rows_per, n - r0) * dim;
-    for (int64_t q = j; q < cnt; q += COLMEAN_THREADS) buf[b][q] = __ldg(res + r0 * dim + q);
+  const int64_t nch = (n + ROWS - 1) / ROWS;
+  const bool wide = dim == DIMP && (reinterpret_cast<uintptr_t>(res) & 15u) == 0;
+  auto load = [&](int64_t c) {
+    if (c < nch) {
+      float* dst = buf[c % 3];
+      const int64_t r0 = c * ROWS;
+      const int rows = (int)min((int64_t)ROWS, n - r0);
+      const float* src = res + r0 * dim;
+      if (wide) {
+        for (int q = j - 32; q < rows * (DIMP / 4); q += LOADERS)
+          __pipeline_memcpy_async(dst + 4 * q, src + 4 * q, 16);
+      } else {
+        for (int q = j - 32; q < rows * dim; q += LOADERS) {
+          const int r = q / dim;
+          __pipeline_memcpy_async(dst + r * DIMP + (q - r * dim), src + q, 4);
+        }
+      }
+    }
+    __pipeline_commit();
   };
   float s = 0.0f;
-  if (nch > 0) load(0, 0);
+  if (j >= 32) {
+    load(0);
+    load(1);
+    __pipeline_wait_prior(1);
+  }
   __syncthreads();
   for (int64_t c = 0; c < nch; ++c) {
-    const int b = (int)(c & 1);
-    if (c + 1 < nch) load(c + 1, b ^ 1);  // the next chunk loads during this one's adds
-    if (j < dim) {
-      const float* col = buf[b] + j;
-      const int rows = (int)min(rows_per, n - c * rows_per);
+    if (j >= 32) {
+      load(c + 2);
+      __pipeline_wait_prior(1);  // chunk c + 1 has landed
+    } else if (j < dim) {
+      const float* col = buf[c % 3] + j;
+      const int rows = (int)min((int64_t)ROWS, n - c * ROWS);
       int r = 0;
-      if (rows >= 8) {
-        float t[8];
+      if (rows >= U) {
+        float t[U];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) t[u] = col[u * dim];
-        for (r = 8; r + 8 <= rows; r += 8) {
-          float nx[8];
+        for (int u = 0; u < U; ++u) t[u] = col[u * DIMP];
+        for (r = U; r + U <= rows; r += U) {
+          float nx[U];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) nx[u] = col[(r + u) * dim];
+          for (int u = 0; u < U; ++u) nx[u] = col[(r + u) * DIMP];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) s = fadd(s, t[u]);
+          for (int u = 0; u < U; ++u) s = fadd(s, t[u]);
 #pragma unroll
-          for (int u = 0; u < 8; ++u) t[u] = nx[u];
+          for (int u = 0; u < U; ++u) t[u] = nx[u];
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) s = fadd(s, t[u]);  // rows r - 8 .. r - 1
+        for (int u = 0; u < U; ++u) s = fadd(s, t[u]);  // rows r - U .. r - 1
       }
-      for (; r < rows; ++r) s = fadd(s, col[r * dim]);
+      for (; r < rows; ++r) s = fadd(s, col[r * DIMP]);
     }
     __syncthreads();
   }
@@ -564,6 +842,40 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
   EVOC_CHECK_LAUNCH();
   const int pbits = bits_for((uint64_t)std::max<int64_t>(np - 1, 1));
   const int nbits = bits_for((uint64_t)std::max<int64_t>(n - 1, 1));
+  // the nodes in part order (stable sort of node ids by part)
+  DevBuf<uint2> nodes(n, s);
+  {
+    DevBuf<uint32_t> pk(n, s);
+    EVOC_CUDA(cudaMemcpyAsync(pk.get(), part.get(), n * sizeof(uint32_t),
+                              cudaMemcpyDeviceToDevice, s));
+    k_iota_pairs<<<grid_of(n), 256, 0, s>>>(nodes.get(), n);
+    EVOC_CHECK_LAUNCH();
+    radix_sort_pairs(pk.get(), nodes.get(), n, pbits, s);
+  }
+  // canonical graphs sum within their rows; others by sorting all entries
+  const bool by_rows = g->canonical && np <= RG_LABELS && g->nnz > 0;
+  const RowGraph rg{g->indptr.get(), g->indices.get(), g->weights.get(), part.get(), inv.get()};
+  DevBuf<uint32_t> row_lists;  // rows above RG_CAP: middle, long
+  DevBuf<int32_t> row_counts;  // their counters: coarse graph, expansion
+  RgLists lists{}, lists2{};
+  const unsigned rgrid = (unsigned)((n + RG_WARPS - 1) / RG_WARPS);
+  // no row is above RG_CAP (RG_MID) when the graph has no more entries than that
+  const unsigned mgrid = g->nnz <= RG_CAP ? 0u : (unsigned)std::min<int64_t>(
+      4 * (int64_t)ctx->num_sms, (g->nnz / RG_CAP + RG_MID_WARPS - 1) / RG_MID_WARPS);
+  const unsigned lgrid = (unsigned)std::min<int64_t>(2 * (int64_t)ctx->num_sms, g->nnz / RG_MID);
+  const size_t msmem = RG_MID_WARPS * sizeof(RgWarp<RG_MID>);
+  if (by_rows) {
+    row_lists.alloc(2 * n, s);
+    row_counts.alloc(6, s);
+    EVOC_CUDA(cudaMemsetAsync(row_counts.get(), 0, row_counts.bytes(), s));
+    lists = RgLists{row_lists.get(), row_lists.get() + n, row_counts.get()};
+    lists2 = RgLists{row_lists.get(), row_lists.get() + n, row_counts.get() + 3};
+    for (const void* f : {(const void*)k_coarse_rows_long, (const void*)k_expand_groups_long})
+      EVOC_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(RgLong)));
+    for (const void* f : {(const void*)k_coarse_rows_mid, (const void*)k_expand_groups_mid})
+      EVOC_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem));
+  }
   // 3. coarse graph clip(N^T G B)
   evoc_graph coarse;
   coarse.ctx = ctx;
@@ -572,10 +884,41 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
   coarse.indptr.alloc(np + 1, s);
   {
     const int64_t m = g->nnz;
-    DevBuf<uint32_t> keys(std::max<int64_t>(m, 1), s);
-    DevBuf<uint2> vals(std::max<int64_t>(m, 1), s);
+    DevBuf<uint32_t> keys, ok;
+    DevBuf<uint2> vals, ov;
     int64_t runs = 0;
-    if (m > 0) {
+    if (by_rows) {
+      // (P, a) per row j, gathered in (Q, j) order and sorted by P: (P, Q, j)
+      DevBuf<uint2> tmp(m, s);
+      DevBuf<int32_t> rcnt(n, s), pcnt(n, s);
+      k_coarse_rows<<<rgrid, 32 * RG_WARPS, 0, s>>>(rg, n, tmp.get(), rcnt.get(), lists);
+      EVOC_CHECK_LAUNCH();
+      if (lgrid) {
+        k_coarse_rows_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLong), s>>>(rg, tmp.get(),
+                                                                          rcnt.get(), lists);
+        EVOC_CHECK_LAUNCH();
+      }
+      if (mgrid) {
+        k_coarse_rows_mid<<<mgrid, 32 * RG_MID_WARPS, msmem, s>>>(rg, tmp.get(), rcnt.get(),
+                                                                  lists);
+        EVOC_CHECK_LAUNCH();
+      }
+      k_perm_counts<<<grid_of(n), 256, 0, s>>>(nodes.get(), n, rcnt.get(), pcnt.get());
+      EVOC_CHECK_LAUNCH();
+      DevBuf<int64_t> off(n + 1, s);
+      exclusive_scan_i32_to_i64(pcnt.get(), off.get(), n, s);
+      EVOC_CUDA(cudaMemcpyAsync(&runs, off.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      EVOC_CUDA(cudaStreamSynchronize(s));
+      keys.alloc(runs, s);
+      vals.alloc(runs, s);
+      k_coarse_gather<<<grid_of(n * 8), 256, 0, s>>>(nodes.get(), n, g->indptr.get(), part.get(),
+                                                     tmp.get(), off.get(), keys.get(),
+                                                     vals.get());
+      EVOC_CHECK_LAUNCH();
+      radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
+    } else if (m > 0) {
+      keys.alloc(m, s);
+      vals.alloc(m, s);
       k_gen_products<<<grid_of(n * 32), 256, 0, s>>>(g->indptr.get(), g->indices.get(),
                                                      g->weights.get(), n, part.get(), inv.get(),
                                                      keys.get(), vals.get());
@@ -584,63 +927,41 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
       k_swap_keys<<<grid_of(m), 256, 0, s>>>(keys.get(), vals.get(), m);  // keys P, vals (j, .)
       EVOC_CHECK_LAUNCH();
       runs = sort_and_sum(keys.get(), vals.get(), m, pbits, nbits, s);
-      // (P, (j, a)) -> (P, Q = part(j), j order kept) -> runs (P, (Q, sum))
+      // (P, (j, a)) -> (P, Q = part(j), j order kept): stable sort by Q, then by P
       DevBuf<uint32_t> q(runs, s);
       k_map_keys<<<grid_of(runs), 256, 0, s>>>(q.get(), vals.get(), runs, part.get());
       EVOC_CHECK_LAUNCH();
-      // order (P, j) -> (P, Q, j): stable sort by Q, then by P
-      {
-        k_swap_keys<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs);  // keys j, vals (P, a)
-        EVOC_CHECK_LAUNCH();
-        EVOC_CUDA(cudaMemcpyAsync(keys.get(), q.get(), runs * sizeof(uint32_t),
-                                  cudaMemcpyDeviceToDevice, s));  // keys Q
-        radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
-        k_swap_keys<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs);  // keys P, vals (Q, a)
-        EVOC_CHECK_LAUNCH();
-        radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
-        DevBuf<int32_t> head(runs, s);
-        DevBuf<int64_t> rid(runs + 1, s);
-        k_run_heads<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs, head.get());
-        EVOC_CHECK_LAUNCH();
-        exclusive_scan_i32_to_i64(head.get(), rid.get(), runs, s);
-        int64_t r2 = 0;
-        EVOC_CUDA(cudaMemcpyAsync(&r2, rid.get() + runs, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        EVOC_CUDA(cudaStreamSynchronize(s));
-        DevBuf<uint32_t> ok(r2, s);
-        DevBuf<uint2> ov(r2, s);
-        k_run_sums<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs, head.get(),
-                                                 rid.get(), ok.get(), ov.get());
-        EVOC_CHECK_LAUNCH();
-        runs = r2;
-        DevBuf<int32_t> rc(np, s);
-        EVOC_CUDA(cudaMemsetAsync(rc.get(), 0, np * sizeof(int32_t), s));
-        k_row_hist<<<grid_of(runs), 256, 0, s>>>(ok.get(), runs, rc.get());
-        EVOC_CHECK_LAUNCH();
-        exclusive_scan_i32_to_i64(rc.get(), coarse.indptr.get(), np, s);
-        coarse.nnz = runs;
-        coarse.indices.alloc(std::max<int64_t>(runs, 1), s);
-        coarse.weights.alloc(std::max<int64_t>(runs, 1), s);
-        k_runs_to_csr<<<grid_of(runs), 256, 0, s>>>(ov.get(), runs, 0.0f, 1.0f,
-                                                    coarse.indices.get(), coarse.weights.get());
-        EVOC_CHECK_LAUNCH();
-        EVOC_CUDA(cudaStreamSynchronize(s));
-      }
+      k_swap_keys<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs);  // keys j, vals (P, a)
+      EVOC_CHECK_LAUNCH();
+      EVOC_CUDA(cudaMemcpyAsync(keys.get(), q.get(), runs * sizeof(uint32_t),
+                                cudaMemcpyDeviceToDevice, s));  // keys Q
+      radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
+      k_swap_keys<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs);  // keys P, vals (Q, a)
+      EVOC_CHECK_LAUNCH();
+      radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
+    }
+    if (m > 0) {
+      runs = sum_runs(keys.get(), vals.get(), runs, ok, ov, s);
+      DevBuf<int32_t> rc(np, s);
+      EVOC_CUDA(cudaMemsetAsync(rc.get(), 0, np * sizeof(int32_t), s));
+      k_row_hist<<<grid_of(runs), 256, 0, s>>>(ok.get(), runs, rc.get());
+      EVOC_CHECK_LAUNCH();
+      exclusive_scan_i32_to_i64(rc.get(), coarse.indptr.get(), np, s);
+      coarse.nnz = runs;
+      coarse.indices.alloc(std::max<int64_t>(runs, 1), s);
+      coarse.weights.alloc(std::max<int64_t>(runs, 1), s);
+      k_runs_to_csr<<<grid_of(runs), 256, 0, s>>>(ov.get(), runs, 0.0f, 1.0f,
+                                                  coarse.indices.get(), coarse.weights.get());
+      EVOC_CHECK_LAUNCH();
     } else {
       EVOC_CUDA(cudaMemsetAsync(coarse.indptr.get(), 0, (np + 1) * sizeof(int64_t), s));
       coarse.nnz = 0;
     }
   }
   mark("coarse graph");
-  // 4. coarse data: per part, its nodes in order (stable sort of node ids by part)
+  // 4. coarse data: per part, its nodes in order
   DevBuf<float> cdata;
   if (d_data) {
-    DevBuf<uint32_t> pk(n, s);
-    DevBuf<uint2> nodes(n, s);
-    EVOC_CUDA(cudaMemcpyAsync(pk.get(), part.get(), n * sizeof(uint32_t),
-                              cudaMemcpyDeviceToDevice, s));
-    k_iota_pairs<<<grid_of(n), 256, 0, s>>>(nodes.get(), n);
-    EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(pk.get(), nodes.get(), n, pbits, s);
     DevBuf<int64_t> poff(np + 1, s);
     exclusive_scan_i32_to_i64(cnt.get(), poff.get(), np, s);
     cdata.alloc(np * d, s);
@@ -676,75 +997,92 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
   mark("coarse embedding");
   // 7. expansion (label_prop.rs:500-534)
   {
-    // the transpose of g (rows of G^T, entries in row order)
-    DevBuf<int64_t> tptr;
-    DevBuf<uint32_t> tidx;
-    DevBuf<float> tw;
-    const int64_t *bp = g->indptr.get();
-    const uint32_t* bi = g->indices.get();
-    const float* bw = g->weights.get();
-    if (!g->canonical && g->nnz > 0) {
-      const int64_t m = g->nnz;
-      DevBuf<uint32_t> tk(m, s);
-      DevBuf<uint2> tv(m, s);
-      k_transpose_gen<<<grid_of(n * 32), 256, 0, s>>>(g->indptr.get(), g->indices.get(),
-                                                      g->weights.get(), n, tk.get(), tv.get());
+    if (by_rows) {
+      k_expand_groups<<<rgrid, 32 * RG_WARPS, 0, s>>>(rg, n, dim, layout.get(), u.get(), d_out,
+                                                      lists2);
       EVOC_CHECK_LAUNCH();
-      radix_sort_pairs(tk.get(), tv.get(), m, nbits, s);
-      DevBuf<int32_t> tc(n, s);
-      EVOC_CUDA(cudaMemsetAsync(tc.get(), 0, n * sizeof(int32_t), s));
-      k_row_hist<<<grid_of(m), 256, 0, s>>>(tk.get(), m, tc.get());
+      if (lgrid) {
+        k_expand_groups_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLong), s>>>(
+            rg, dim, layout.get(), u.get(), d_out, lists2);
+        EVOC_CHECK_LAUNCH();
+      }
+      if (mgrid) {
+        k_expand_groups_mid<<<mgrid, 32 * RG_MID_WARPS, msmem, s>>>(rg, dim, layout.get(),
+                                                                    u.get(), d_out, lists2);
+        EVOC_CHECK_LAUNCH();
+      }
+    } else {
+      // the transpose of g (rows of G^T, entries in row order)
+      DevBuf<int64_t> tptr;
+      DevBuf<uint32_t> tidx;
+      DevBuf<float> tw;
+      const int64_t *bp = g->indptr.get();
+      const uint32_t* bi = g->indices.get();
+      const float* bw = g->weights.get();
+      if (!g->canonical && g->nnz > 0) {
+        const int64_t m = g->nnz;
+        DevBuf<uint32_t> tk(m, s);
+        DevBuf<uint2> tv(m, s);
+        k_transpose_gen<<<grid_of(n * 32), 256, 0, s>>>(g->indptr.get(), g->indices.get(),
+                                                        g->weights.get(), n, tk.get(), tv.get());
+        EVOC_CHECK_LAUNCH();
+        radix_sort_pairs(tk.get(), tv.get(), m, nbits, s);
+        DevBuf<int32_t> tc(n, s);
+        EVOC_CUDA(cudaMemsetAsync(tc.get(), 0, n * sizeof(int32_t), s));
+        k_row_hist<<<grid_of(m), 256, 0, s>>>(tk.get(), m, tc.get());
+        EVOC_CHECK_LAUNCH();
+        tptr.alloc(n + 1, s);
+        exclusive_scan_i32_to_i64(tc.get(), tptr.get(), n, s);
+        tidx.alloc(m, s);
+        tw.alloc(m, s);
+        k_unpack_pairs<<<grid_of(m), 256, 0, s>>>(tv.get(), m, tidx.get(), tw.get());
+        EVOC_CHECK_LAUNCH();
+        bp = tptr.get();
+        bi = tidx.get();
+        bw = tw.get();
+      }
+      mark("expansion: transpose");
+      DevBuf<int32_t> sc(n, s);
+      DevBuf<int64_t> soff(n + 1, s);
+      k_sym_count<<<grid_of(n), 256, 0, s>>>(g->indptr.get(), g->indices.get(), bp, bi, n,
+                                             sc.get());
       EVOC_CHECK_LAUNCH();
-      tptr.alloc(n + 1, s);
-      exclusive_scan_i32_to_i64(tc.get(), tptr.get(), n, s);
-      tidx.alloc(m, s);
-      tw.alloc(m, s);
-      k_unpack_pairs<<<grid_of(m), 256, 0, s>>>(tv.get(), m, tidx.get(), tw.get());
+      exclusive_scan_i32_to_i64(sc.get(), soff.get(), n, s);
+      int64_t ms = 0;
+      EVOC_CUDA(cudaMemcpyAsync(&ms, soff.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      EVOC_CUDA(cudaStreamSynchronize(s));
+      DevBuf<uint32_t> keys(std::max<int64_t>(ms, 1), s);
+      DevBuf<uint2> vals(std::max<int64_t>(ms, 1), s);
+      DevBuf<int64_t> eptr(n + 1, s);
+      int64_t runs = 0;
+      if (ms > 0) {
+        k_sym_products<<<grid_of(n), 256, 0, s>>>(g->indptr.get(), g->indices.get(),
+                                                  g->weights.get(), bp, bi, bw, n, soff.get(),
+                                                  part.get(), inv.get(), keys.get(), vals.get());
+        EVOC_CHECK_LAUNCH();
+        // keys Q, vals (i, prod): order (i, Q, j) -> runs (i, (Q, e))
+        k_swap_keys<<<grid_of(ms), 256, 0, s>>>(keys.get(), vals.get(), ms);  // keys i, vals (Q, .)
+        EVOC_CHECK_LAUNCH();
+        mark("expansion: symmetric products");
+        runs = sort_and_sum(keys.get(), vals.get(), ms, nbits, pbits, s);
+      }
+      mark("expansion: sort and sum");
+      DevBuf<int32_t> rc(n, s);
+      EVOC_CUDA(cudaMemsetAsync(rc.get(), 0, n * sizeof(int32_t), s));
+      if (runs > 0) {
+        k_row_hist<<<grid_of(runs), 256, 0, s>>>(keys.get(), runs, rc.get());
+        EVOC_CHECK_LAUNCH();
+      }
+      exclusive_scan_i32_to_i64(rc.get(), eptr.get(), n, s);
+      k_expand_rows<<<grid_of(n, 128), 128, 0, s>>>(eptr.get(), vals.get(), n, dim, layout.get(),
+                                                    part.get(), u.get(), d_out);
       EVOC_CHECK_LAUNCH();
-      bp = tptr.get();
-      bi = tidx.get();
-      bw = tw.get();
     }
-    mark("expansion: transpose");
-    DevBuf<int32_t> sc(n, s);
-    DevBuf<int64_t> soff(n + 1, s);
-    k_sym_count<<<grid_of(n), 256, 0, s>>>(g->indptr.get(), g->indices.get(), bp, bi, n,
-                                           sc.get());
-    EVOC_CHECK_LAUNCH();
-    exclusive_scan_i32_to_i64(sc.get(), soff.get(), n, s);
-    int64_t ms = 0;
-    EVOC_CUDA(cudaMemcpyAsync(&ms, soff.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    EVOC_CUDA(cudaStreamSynchronize(s));
-    DevBuf<uint32_t> keys(std::max<int64_t>(ms, 1), s);
-    DevBuf<uint2> vals(std::max<int64_t>(ms, 1), s);
-    DevBuf<int64_t> eptr(n + 1, s);
-    int64_t runs = 0;
-    if (ms > 0) {
-      k_sym_products<<<grid_of(n), 256, 0, s>>>(g->indptr.get(), g->indices.get(),
-                                                g->weights.get(), bp, bi, bw, n, soff.get(),
-                                                part.get(), inv.get(), keys.get(), vals.get());
-      EVOC_CHECK_LAUNCH();
-      // keys Q, vals (i, prod): order (i, Q, j) -> runs (i, (Q, e))
-      k_swap_keys<<<grid_of(ms), 256, 0, s>>>(keys.get(), vals.get(), ms);  // keys i, vals (Q, .)
-      EVOC_CHECK_LAUNCH();
-      mark("expansion: symmetric products");
-      runs = sort_and_sum(keys.get(), vals.get(), ms, nbits, pbits, s);
-    }
-    mark("expansion: sort and sum");
-    DevBuf<int32_t> rc(n, s);
-    EVOC_CUDA(cudaMemsetAsync(rc.get(), 0, n * sizeof(int32_t), s));
-    if (runs > 0) {
-      k_row_hist<<<grid_of(runs), 256, 0, s>>>(keys.get(), runs, rc.get());
-      EVOC_CHECK_LAUNCH();
-    }
-    exclusive_scan_i32_to_i64(rc.get(), eptr.get(), n, s);
-    k_expand_rows<<<grid_of(n, 128), 128, 0, s>>>(eptr.get(), vals.get(), n, dim, layout.get(),
-                                                  part.get(), u.get(), d_out);
-    EVOC_CHECK_LAUNCH();
     mark("expansion: rows");
     DevBuf<float> mean(dim, s);
     const float inv_n = (float)(1.0 / (double)n);
-    k_col_mean<<<1, COLMEAN_THREADS, 0, s>>>(d_out, n, dim, inv_n, mean.get());
+    auto* col_mean = dim <= 4 ? k_col_mean<4> : dim <= 8 ? k_col_mean<8> : k_col_mean<16>;
+    col_mean<<<1, COLMEAN_THREADS, 0, s>>>(d_out, n, dim, inv_n, mean.get());
     EVOC_CHECK_LAUNCH();
     k_center_scale<<<grid_of(n * dim), 256, 0, s>>>(d_out, n, dim, mean.get(),
                                                     (float)lp.scaling);
