@@ -1889,7 +1889,7 @@ static bool build_slots(evoc_plan* pl, const float* inc_ps, const uint8_t* inc_u
   }
   trace.mark("count pass");
   DevBuf<int64_t> off(cells + 1, s);
-  exclusive_scan_i32_to_i64(counts.get(), off.get(), cells, s);
+  exclusive_scan_i32_to_i64(pl->ctx, counts.get(), off.get(), cells);
   int64_t total = 0;
   std::vector<unsigned long long> htot(2 * ne);
   EVOC_CUDA(cudaMemcpyAsync(&total, off.get() + cells, sizeof(int64_t),
@@ -1914,7 +1914,7 @@ static bool build_slots(evoc_plan* pl, const float* inc_ps, const uint8_t* inc_u
     k_tile_weight<<<blocks_for(pl->ntiles), 256, 0, s>>>(counts.get(), pl->ntiles, ne,
                                                           keys.get(), vals.get());
     EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(keys.get(), vals.get(), pl->ntiles, 32, s);
+    radix_sort_pairs(pl->ctx, keys, vals, pl->ntiles, 32);
     pl->tile_order.alloc(pl->ntiles, s);
     k_tile_order<<<blocks_for(pl->ntiles), 256, 0, s>>>(vals.get(), pl->ntiles,
                                                          pl->tile_order.get());
@@ -2357,7 +2357,7 @@ evoc_plan* plan_create(evoc_ctx* ctx, const std::vector<ProblemDesc>& probs,
                                                   lcnt.get());
   EVOC_CHECK_LAUNCH();
   DevBuf<int64_t> uptr(n + 1, s);
-  exclusive_scan_i32_to_i64(ucnt.get(), uptr.get(), n, s);
+  exclusive_scan_i32_to_i64(pl->ctx, ucnt.get(), uptr.get(), n);
   int64_t U = 0;
   EVOC_CUDA(cudaMemcpyAsync(&U, uptr.get() + n, sizeof(int64_t),
                             cudaMemcpyDeviceToHost, s));
@@ -2397,9 +2397,9 @@ evoc_plan* plan_create(evoc_ctx* ctx, const std::vector<ProblemDesc>& probs,
     EVOC_CUDA(cudaMemcpyAsync(keys.get(), e_dst.get(), U * sizeof(uint32_t),
                               cudaMemcpyDeviceToDevice, s));
     fill_eidx_src(lower.get(), e_src.get(), U, s);
-    radix_sort_pairs(keys.get(), lower.get(), U, bits_for((uint64_t)(n - 1)), s);
+    radix_sort_pairs(pl->ctx, keys, lower, U, bits_for((uint64_t)(n - 1)));
     lptr.alloc(n + 1, s);
-    exclusive_scan_i32_to_i64(lcnt.get(), lptr.get(), n, s);
+    exclusive_scan_i32_to_i64(pl->ctx, lcnt.get(), lptr.get(), n);
   }
   e_dst.release();
   e_src.release();
@@ -2409,7 +2409,7 @@ evoc_plan* plan_create(evoc_ctx* ctx, const std::vector<ProblemDesc>& probs,
   DevBuf<int32_t> deg(n, s);
   add_counts(ucnt.get(), lcnt.get(), deg.get(), n, s);
   pl->inc_ptr.alloc(n + 1, s);
-  exclusive_scan_i32_to_i64(deg.get(), pl->inc_ptr.get(), n, s);
+  exclusive_scan_i32_to_i64(pl->ctx, deg.get(), pl->inc_ptr.get(), n);
   deg.release();
   int64_t n_inc = 0;
   EVOC_CUDA(cudaMemcpyAsync(&n_inc, pl->inc_ptr.get() + n, sizeof(int64_t),

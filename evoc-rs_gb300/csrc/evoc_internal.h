@@ -166,15 +166,14 @@ struct evoc_graph {
 namespace evoc {
 
 // ---- primitives.cu ---------------------------------------------------------
-// out[0..n] = exclusive prefix sum of in[0..n-1]; out[n] = total.
-void exclusive_scan_i32_to_i64(const int32_t* in, int64_t* out, int64_t n,
-                               cudaStream_t s);
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n,
-                        cudaStream_t s);
-// Stable LSD radix sort of (key, value) pairs by key, keys < 2^key_bits.
-// Results are written back to keys/vals.
-void radix_sort_pairs(uint32_t* keys, uint2* vals, int64_t n, int key_bits,
-                      cudaStream_t s);
+// out[0..n] = exclusive prefix sum of in[0..n-1]; out[n] = total (below 2^62,
+// no negative terms).
+void exclusive_scan_i32_to_i64(evoc_ctx* ctx, const int32_t* in, int64_t* out, int64_t n);
+void exclusive_scan_i64(evoc_ctx* ctx, const int64_t* in, int64_t* out, int64_t n);
+// Stable LSD radix sort of the first n (key, value) pairs by key, keys <
+// 2^key_bits. keys and vals hold the result (their buffers may be exchanged).
+void radix_sort_pairs(evoc_ctx* ctx, DevBuf<uint32_t>& keys, DevBuf<uint2>& vals, int64_t n,
+                      int key_bits);
 int bits_for(uint64_t max_value);
 // Read the context's status word and reset it; throw on any set bit.
 void check_status(evoc_ctx* ctx, const char* where);

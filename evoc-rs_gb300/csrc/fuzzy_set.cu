@@ -545,7 +545,7 @@ void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
                                                   n, k, cnt.get(), nullptr,
                                                   nullptr, nullptr);
     EVOC_CHECK_LAUNCH();
-    exclusive_scan_i32_to_i64(cnt.get(), out->indptr.get(), n, s);
+    exclusive_scan_i32_to_i64(ctx, cnt.get(), out->indptr.get(), n);
     int64_t nnz = 0;
     EVOC_CUDA(cudaMemcpyAsync(&nnz, out->indptr.get() + n, sizeof(int64_t),
                               cudaMemcpyDeviceToHost, s));
@@ -581,8 +581,8 @@ void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
   trace.mark("forward rows");
 
   DevBuf<int64_t> fptr(n + 1, s), bptr(n + 1, s);
-  exclusive_scan_i32_to_i64(fcnt.get(), fptr.get(), n, s);
-  exclusive_scan_i32_to_i64(indeg.get(), bptr.get(), n, s);
+  exclusive_scan_i32_to_i64(ctx, fcnt.get(), fptr.get(), n);
+  exclusive_scan_i32_to_i64(ctx, indeg.get(), bptr.get(), n);
   int64_t nf = 0;
   EVOC_CUDA(cudaMemcpyAsync(&nf, fptr.get() + n, sizeof(int64_t),
                             cudaMemcpyDeviceToHost, s));
@@ -596,7 +596,7 @@ void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
     k_forward_compact<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
         fcol.get(), fw.get(), fptr.get(), n, k, keys.get(), vals.get());
     EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(keys.get(), vals.get(), nf, bits_for((uint64_t)(n - 1)), s);
+    radix_sort_pairs(ctx, keys, vals, nf, bits_for((uint64_t)(n - 1)));
   }
   keys.release();
   fptr.release();
@@ -611,7 +611,7 @@ void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
   k_union<<<(unsigned)((n * 32 + 255) / 256), 256, 0, s>>>(
       fcol.get(), fw.get(), fcnt.get(), bptr.get(), vals.get(), n, k, ucnt.get(), utmp.get());
   EVOC_CHECK_LAUNCH();
-  exclusive_scan_i32_to_i64(ucnt.get(), out->indptr.get(), n, s);
+  exclusive_scan_i32_to_i64(ctx, ucnt.get(), out->indptr.get(), n);
   int64_t nnz = 0;
   EVOC_CUDA(cudaMemcpyAsync(&nnz, out->indptr.get() + n, sizeof(int64_t),
                             cudaMemcpyDeviceToHost, s));

@@ -442,8 +442,9 @@ inline unsigned grid_for(int64_t n, int t = 256) { return (unsigned)((n + t - 1)
 
 // The rounds for labels of any size (k_lp_iter): thread per node, vote tables in
 // global memory; one look at the host per round.
-void lp_rounds_any_label(const evoc_graph* g, int32_t n_iter, DevBuf<int32_t>& la,
-                         DevBuf<int32_t>& lb, int32_t* flag, cudaStream_t s) {
+void lp_rounds_any_label(evoc_ctx* ctx, const evoc_graph* g, int32_t n_iter, DevBuf<int32_t>& la,
+                         DevBuf<int32_t>& lb, int32_t* flag) {
+  cudaStream_t s = ctx->stream;
   const int64_t n = g->n, nnz = g->nnz;
   DevBuf<int32_t> vlab(std::max<int64_t>(nnz, 1), s);
   DevBuf<float> vsum(std::max<int64_t>(nnz, 1), s);
@@ -451,7 +452,7 @@ void lp_rounds_any_label(const evoc_graph* g, int32_t n_iter, DevBuf<int32_t>& l
   DevBuf<int64_t> hcap(n, s), hoff(n + 1, s);
   k_lp_hcap<<<grid_for(n), 256, 0, s>>>(g->indptr.get(), n, hcap.get());
   EVOC_CHECK_LAUNCH();
-  exclusive_scan_i64(hcap.get(), hoff.get(), n, s);
+  exclusive_scan_i64(ctx, hcap.get(), hoff.get(), n);
   int64_t htot = 0;
   EVOC_CUDA(cudaMemcpyAsync(&htot, hoff.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   EVOC_CUDA(cudaStreamSynchronize(s));
@@ -531,7 +532,7 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
       std::swap(la, lb);
     }
   } else {
-    lp_rounds_any_label(g, n_iter, la, lb, flag.get(), s);
+    lp_rounds_any_label(ctx, g, n_iter, la, lb, flag.get());
   }
   // mop-up of the nodes still unlabelled, in node order
   DevBuf<int32_t> mx(1, s), unl(n, s);
@@ -539,7 +540,7 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
   EVOC_CUDA(cudaMemsetAsync(mx.get(), 0xff, sizeof(int32_t), s));  // -1
   k_lp_max<<<grid_for(n), 256, 0, s>>>(la.get(), n, mx.get(), unl.get());
   EVOC_CHECK_LAUNCH();
-  exclusive_scan_i32_to_i64(unl.get(), pos.get(), n, s);
+  exclusive_scan_i32_to_i64(ctx, unl.get(), pos.get(), n);
   int64_t count = 0;
   EVOC_CUDA(cudaMemcpyAsync(&count, pos.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   EVOC_CUDA(cudaStreamSynchronize(s));
@@ -573,8 +574,8 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
   EVOC_CUDA(cudaMemsetAsync(present.get(), 0, np * sizeof(int32_t), s));
   k_lp_present<<<grid_for(n), 256, 0, s>>>(la.get(), n, present.get(), neg.get());
   EVOC_CHECK_LAUNCH();
-  exclusive_scan_i32_to_i64(present.get(), newid.get(), np, s);
-  exclusive_scan_i32_to_i64(neg.get(), negrank.get(), n, s);
+  exclusive_scan_i32_to_i64(ctx, present.get(), newid.get(), np);
+  exclusive_scan_i32_to_i64(ctx, neg.get(), negrank.get(), n);
   int64_t n_unique = 0, n_neg = 0;
   EVOC_CUDA(cudaMemcpyAsync(&n_unique, newid.get() + np, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   EVOC_CUDA(cudaMemcpyAsync(&n_neg, negrank.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));

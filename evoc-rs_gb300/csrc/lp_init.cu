@@ -192,13 +192,14 @@ __global__ void k_run_sums(const uint32_t* __restrict__ keys, const uint2* __res
 
 // Sums the equal-(keys, vals.x) runs of a sorted list serially into (ok, ov);
 // returns their count.
-int64_t sum_runs(const uint32_t* keys, const uint2* vals, int64_t m, DevBuf<uint32_t>& ok,
-                 DevBuf<uint2>& ov, cudaStream_t s) {
+int64_t sum_runs(evoc_ctx* ctx, const uint32_t* keys, const uint2* vals, int64_t m,
+                 DevBuf<uint32_t>& ok, DevBuf<uint2>& ov) {
+  cudaStream_t s = ctx->stream;
   DevBuf<int32_t> head(m, s);
   DevBuf<int64_t> rid(m + 1, s);
   k_run_heads<<<grid_of(m), 256, 0, s>>>(keys, vals, m, head.get());
   EVOC_CHECK_LAUNCH();
-  exclusive_scan_i32_to_i64(head.get(), rid.get(), m, s);
+  exclusive_scan_i32_to_i64(ctx, head.get(), rid.get(), m);
   int64_t runs = 0;
   EVOC_CUDA(cudaMemcpyAsync(&runs, rid.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   EVOC_CUDA(cudaStreamSynchronize(s));
@@ -215,22 +216,23 @@ int64_t sum_runs(const uint32_t* keys, const uint2* vals, int64_t m, DevBuf<uint
 
 // Sorts (keys, vals) by (keys major, vals.x minor), stably, then sums the
 // equal-(key, minor) runs serially. Returns the run count; the runs replace
-// the list's head (keys, vals).
-int64_t sort_and_sum(uint32_t* keys, uint2* vals, int64_t m, int major_bits, int minor_bits,
-                     cudaStream_t s) {
+// the list.
+int64_t sort_and_sum(evoc_ctx* ctx, DevBuf<uint32_t>& keys, DevBuf<uint2>& vals, int64_t m,
+                     int major_bits, int minor_bits) {
+  cudaStream_t s = ctx->stream;
   if (m == 0) return 0;
   // minor first (keys <- vals.x), then major
-  k_swap_keys<<<grid_of(m), 256, 0, s>>>(keys, vals, m);
+  k_swap_keys<<<grid_of(m), 256, 0, s>>>(keys.get(), vals.get(), m);
   EVOC_CHECK_LAUNCH();
-  radix_sort_pairs(keys, vals, m, minor_bits, s);
-  k_swap_keys<<<grid_of(m), 256, 0, s>>>(keys, vals, m);
+  radix_sort_pairs(ctx, keys, vals, m, minor_bits);
+  k_swap_keys<<<grid_of(m), 256, 0, s>>>(keys.get(), vals.get(), m);
   EVOC_CHECK_LAUNCH();
-  radix_sort_pairs(keys, vals, m, major_bits, s);
+  radix_sort_pairs(ctx, keys, vals, m, major_bits);
   DevBuf<uint32_t> ok;
   DevBuf<uint2> ov;
-  const int64_t runs = sum_runs(keys, vals, m, ok, ov, s);
-  EVOC_CUDA(cudaMemcpyAsync(keys, ok.get(), runs * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-  EVOC_CUDA(cudaMemcpyAsync(vals, ov.get(), runs * sizeof(uint2), cudaMemcpyDeviceToDevice, s));
+  const int64_t runs = sum_runs(ctx, keys.get(), vals.get(), m, ok, ov);
+  keys = std::move(ok);
+  vals = std::move(ov);
   return runs;
 }
 
@@ -850,7 +852,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
                               cudaMemcpyDeviceToDevice, s));
     k_iota_pairs<<<grid_of(n), 256, 0, s>>>(nodes.get(), n);
     EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(pk.get(), nodes.get(), n, pbits, s);
+    radix_sort_pairs(ctx, pk, nodes, n, pbits);
   }
   // canonical graphs sum within their rows; others by sorting all entries
   const bool by_rows = g->canonical && np <= RG_LABELS && g->nnz > 0;
@@ -906,7 +908,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
       k_perm_counts<<<grid_of(n), 256, 0, s>>>(nodes.get(), n, rcnt.get(), pcnt.get());
       EVOC_CHECK_LAUNCH();
       DevBuf<int64_t> off(n + 1, s);
-      exclusive_scan_i32_to_i64(pcnt.get(), off.get(), n, s);
+      exclusive_scan_i32_to_i64(ctx, pcnt.get(), off.get(), n);
       EVOC_CUDA(cudaMemcpyAsync(&runs, off.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
       EVOC_CUDA(cudaStreamSynchronize(s));
       keys.alloc(runs, s);
@@ -915,7 +917,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
                                                      tmp.get(), off.get(), keys.get(),
                                                      vals.get());
       EVOC_CHECK_LAUNCH();
-      radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
+      radix_sort_pairs(ctx, keys, vals, runs, pbits);
     } else if (m > 0) {
       keys.alloc(m, s);
       vals.alloc(m, s);
@@ -926,27 +928,26 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
       // keys j, vals (P, prod): order (P, j, i) -> runs (P, (j, A_Pj))
       k_swap_keys<<<grid_of(m), 256, 0, s>>>(keys.get(), vals.get(), m);  // keys P, vals (j, .)
       EVOC_CHECK_LAUNCH();
-      runs = sort_and_sum(keys.get(), vals.get(), m, pbits, nbits, s);
+      runs = sort_and_sum(ctx, keys, vals, m, pbits, nbits);
       // (P, (j, a)) -> (P, Q = part(j), j order kept): stable sort by Q, then by P
       DevBuf<uint32_t> q(runs, s);
       k_map_keys<<<grid_of(runs), 256, 0, s>>>(q.get(), vals.get(), runs, part.get());
       EVOC_CHECK_LAUNCH();
       k_swap_keys<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs);  // keys j, vals (P, a)
       EVOC_CHECK_LAUNCH();
-      EVOC_CUDA(cudaMemcpyAsync(keys.get(), q.get(), runs * sizeof(uint32_t),
-                                cudaMemcpyDeviceToDevice, s));  // keys Q
-      radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
+      std::swap(keys, q);  // keys Q
+      radix_sort_pairs(ctx, keys, vals, runs, pbits);
       k_swap_keys<<<grid_of(runs), 256, 0, s>>>(keys.get(), vals.get(), runs);  // keys P, vals (Q, a)
       EVOC_CHECK_LAUNCH();
-      radix_sort_pairs(keys.get(), vals.get(), runs, pbits, s);
+      radix_sort_pairs(ctx, keys, vals, runs, pbits);
     }
     if (m > 0) {
-      runs = sum_runs(keys.get(), vals.get(), runs, ok, ov, s);
+      runs = sum_runs(ctx, keys.get(), vals.get(), runs, ok, ov);
       DevBuf<int32_t> rc(np, s);
       EVOC_CUDA(cudaMemsetAsync(rc.get(), 0, np * sizeof(int32_t), s));
       k_row_hist<<<grid_of(runs), 256, 0, s>>>(ok.get(), runs, rc.get());
       EVOC_CHECK_LAUNCH();
-      exclusive_scan_i32_to_i64(rc.get(), coarse.indptr.get(), np, s);
+      exclusive_scan_i32_to_i64(ctx, rc.get(), coarse.indptr.get(), np);
       coarse.nnz = runs;
       coarse.indices.alloc(std::max<int64_t>(runs, 1), s);
       coarse.weights.alloc(std::max<int64_t>(runs, 1), s);
@@ -963,7 +964,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
   DevBuf<float> cdata;
   if (d_data) {
     DevBuf<int64_t> poff(np + 1, s);
-    exclusive_scan_i32_to_i64(cnt.get(), poff.get(), np, s);
+    exclusive_scan_i32_to_i64(ctx, cnt.get(), poff.get(), np);
     cdata.alloc(np * d, s);
     k_reduce_data<<<dim3((unsigned)np, (unsigned)((d + RD_THREADS - 1) / RD_THREADS)),
                     RD_THREADS, 0, s>>>(d_data, d, poff.get(), nodes.get(), rv.get(),
@@ -1026,13 +1027,13 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
         k_transpose_gen<<<grid_of(n * 32), 256, 0, s>>>(g->indptr.get(), g->indices.get(),
                                                         g->weights.get(), n, tk.get(), tv.get());
         EVOC_CHECK_LAUNCH();
-        radix_sort_pairs(tk.get(), tv.get(), m, nbits, s);
+        radix_sort_pairs(ctx, tk, tv, m, nbits);
         DevBuf<int32_t> tc(n, s);
         EVOC_CUDA(cudaMemsetAsync(tc.get(), 0, n * sizeof(int32_t), s));
         k_row_hist<<<grid_of(m), 256, 0, s>>>(tk.get(), m, tc.get());
         EVOC_CHECK_LAUNCH();
         tptr.alloc(n + 1, s);
-        exclusive_scan_i32_to_i64(tc.get(), tptr.get(), n, s);
+        exclusive_scan_i32_to_i64(ctx, tc.get(), tptr.get(), n);
         tidx.alloc(m, s);
         tw.alloc(m, s);
         k_unpack_pairs<<<grid_of(m), 256, 0, s>>>(tv.get(), m, tidx.get(), tw.get());
@@ -1047,7 +1048,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
       k_sym_count<<<grid_of(n), 256, 0, s>>>(g->indptr.get(), g->indices.get(), bp, bi, n,
                                              sc.get());
       EVOC_CHECK_LAUNCH();
-      exclusive_scan_i32_to_i64(sc.get(), soff.get(), n, s);
+      exclusive_scan_i32_to_i64(ctx, sc.get(), soff.get(), n);
       int64_t ms = 0;
       EVOC_CUDA(cudaMemcpyAsync(&ms, soff.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
       EVOC_CUDA(cudaStreamSynchronize(s));
@@ -1064,7 +1065,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
         k_swap_keys<<<grid_of(ms), 256, 0, s>>>(keys.get(), vals.get(), ms);  // keys i, vals (Q, .)
         EVOC_CHECK_LAUNCH();
         mark("expansion: symmetric products");
-        runs = sort_and_sum(keys.get(), vals.get(), ms, nbits, pbits, s);
+        runs = sort_and_sum(ctx, keys, vals, ms, nbits, pbits);
       }
       mark("expansion: sort and sum");
       DevBuf<int32_t> rc(n, s);
@@ -1073,7 +1074,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
         k_row_hist<<<grid_of(runs), 256, 0, s>>>(keys.get(), runs, rc.get());
         EVOC_CHECK_LAUNCH();
       }
-      exclusive_scan_i32_to_i64(rc.get(), eptr.get(), n, s);
+      exclusive_scan_i32_to_i64(ctx, rc.get(), eptr.get(), n);
       k_expand_rows<<<grid_of(n, 128), 128, 0, s>>>(eptr.get(), vals.get(), n, dim, layout.get(),
                                                     part.get(), u.get(), d_out);
       EVOC_CHECK_LAUNCH();

@@ -749,11 +749,11 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
   k_mst_morton<<<grid_of(n), 256, 0, s>>>(d_data, n, dim, bits, bmin.get(), bmax.get(), key.get(),
                                           val.get());
   EVOC_CHECK_LAUNCH();
-  radix_sort_pairs(key.get(), val.get(), n, std::min(32, total_bits), s);
+  radix_sort_pairs(ctx, key, val, n, std::min(32, total_bits));
   if (total_bits > 32) {
     k_mst_hi_keys<<<grid_of(n), 256, 0, s>>>(val.get(), n, key.get());
     EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(key.get(), val.get(), n, total_bits - 32, s);
+    radix_sort_pairs(ctx, key, val, n, total_bits - 32);
   }
   DevBuf<float> xs(n * DIMP, s);
   DevBuf<uint32_t> orig(n, s), pos_of(n, s);
@@ -847,8 +847,8 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
     EVOC_CHECK_LAUNCH();
     k_mst_label<<<gm, 256, 0, s>>>(A.get(), m, pin, nid.get(), lab.get(), alive.get());
     EVOC_CHECK_LAUNCH();
-    exclusive_scan_i32_to_i64(keep.get(), off.get(), m, s);
-    exclusive_scan_i32_to_i64(alive.get(), off2.get(), m, s);
+    exclusive_scan_i32_to_i64(ctx, keep.get(), off.get(), m);
+    exclusive_scan_i32_to_i64(ctx, alive.get(), off2.get(), m);
     k_mst_emit<<<gm, 256, 0, s>>>(m, keep.get(), off.get(), eu.get(), ev.get(), ew.get(), len,
                                   d_u, d_v, d_w);
     EVOC_CHECK_LAUNCH();
