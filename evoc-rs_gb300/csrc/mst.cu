@@ -2,10 +2,14 @@
 // GPU: Boruvka's minimum spanning tree over mutual reachability distance, the
 // first step of the clustering stage that turns the embedding into labels.
 //
-// Spatial index. Points are sorted by a 64-bit Morton code of their
-// coordinates (quantised on the bounding box); an implicit complete binary
-// tree over leaves of 32 consecutive sorted points holds the bounding box of
-// each node (heap order: node v has children 2v and 2v + 1, leaves are P..2P-1).
+// Spatial index. An implicit complete binary tree over leaves of 32 points
+// (heap order: node v has children 2v and 2v + 1, leaves are P..2P-1), each node's
+// points split along the widest side of their bounding box: the points of every
+// node are ordered by that coordinate and the first half of the node's leaves
+// takes the first ones. Nodes above KD_BLOCK points are ordered by one radix sort
+// per level over (node, coordinate), the levels below by a block per node in
+// shared memory. Against Morton order (whose 8 bits per dimension cut clusters at
+// fixed planes) the boxes are tighter and a search meets far fewer of them.
 // It plays the part of the reference's KD-tree (kd_tree.rs:93-236): only
 // pruning bounds come from it, never a result.
 //
@@ -16,14 +20,17 @@
 // current k-th distance (knn_recurse, kd_tree.rs:489-535).
 //
 // Boruvka rounds (mst.rs:115-160):
-//   1. node components, bottom-up (update_node_components, kd_tree.rs:387-419);
+//   1. what each node holds of the components, bottom-up (k_mst_leaf_parts; the
+//      reference's update_node_components, kd_tree.rs:387-419, marks pure nodes);
 //   2. per point, the nearest point of another component under squared mutual
 //      reachability max(d^2, core_i, core_j) (nearest_other_component,
 //      kd_tree.rs:275-378), with the same three pruning rules; among equal
-//      values the smallest point index. A per-component bound starts each
+//      values the smallest point index. A point whose nearest foreign point is
+//      known from an earlier round or from the kNN lists is not searched for
+//      again (k_mst_near_init). A per-component bound starts each other
 //      query just above it and is lowered while the round runs: first the
-//      smallest value over the component's leaving kNN edges (kept from the
-//      core-distance pass), then the best value found so far by its points.
+//      smallest known value leaving the component (k_mst_bound), then the best
+//      value found so far by its points.
 //      Each is the value of a real edge leaving the component, so no
 //      component's pick changes;
 //   3. per component (its id is its smallest point index), the pick with the
@@ -51,8 +58,6 @@ namespace evoc {
 namespace {
 
 constexpr int MST_LEAF = 32;     // points per leaf
-constexpr uint32_t NC_MIXED = 0xffffffffu;  // node holds points of several components
-constexpr uint32_t NC_EMPTY = 0xfffffffeu;  // node holds no point
 constexpr uint32_t NO_POINT = 0xffffffffu;
 constexpr uint32_t FMAX_BITS = 0x7f7fffffu;  // FLT_MAX
 
@@ -67,57 +72,155 @@ __device__ __forceinline__ float of_ord(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-// Bounding box of dimension blockIdx.y; every coordinate must be finite.
-__global__ void k_mst_bbox(const float* __restrict__ x, int64_t n, int dim,
-                           uint32_t* __restrict__ omin, uint32_t* __restrict__ omax,
-                           int32_t* __restrict__ status) {
-  const int d = blockIdx.y;
-  float lo = FLT_MAX, hi = -FLT_MAX;
+// Every coordinate must be finite.
+__global__ void k_mst_finite(const float* __restrict__ x, int64_t count,
+                             int32_t* __restrict__ status) {
   bool bad = false;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const float v = x[i * dim + d];
-    bad |= !isfinite(v);
-    lo = fminf(lo, v);
-    hi = fmaxf(hi, v);
-  }
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
+       i += (int64_t)gridDim.x * blockDim.x)
+    bad |= !isfinite(x[i]);
   if (bad) set_status(status, ST_BAD_VALUE);
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMin(&omin[d], ord_of(lo));
-    atomicMax(&omax[d], ord_of(hi));
-  }
 }
 
-// Morton code: each coordinate quantised to `bits` bits on the box, bits
-// interleaved from the top (dimension 0 first). Low 32 bits as the sort key,
-// (point, high 32 bits) as the value.
-__global__ void k_mst_morton(const float* __restrict__ x, int64_t n, int dim, int bits,
-                             const uint32_t* __restrict__ omin, const uint32_t* __restrict__ omax,
-                             uint32_t* __restrict__ key, uint2* __restrict__ val) {
+__global__ void k_mst_iota_pairs(uint2* __restrict__ val, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t q[16];
-  const float maxq = (float)((1u << bits) - 1u);
+  if (i < n) val[i] = make_uint2((uint32_t)i, 0u);
+}
+
+// Bounding boxes of the nodes of `size` consecutive points (size a multiple of
+// 32 KD_RUN): a warp reduces KD_RUN runs of 32 points, then one atomic per side.
+constexpr int KD_RUN = 32;
+__global__ void k_kd_box(const float* __restrict__ x, int64_t n, int dim, int64_t size,
+                         const uint2* __restrict__ val, uint32_t* __restrict__ bmin,
+                         uint32_t* __restrict__ bmax) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t p0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * KD_RUN);
+  if (p0 >= n) return;
+  const int64_t node = p0 / size;
   for (int d = 0; d < dim; ++d) {
-    const float lo = of_ord(omin[d]), hi = of_ord(omax[d]);
-    const float span = hi - lo;
-    const float t = span > 0.0f ? (x[i * dim + d] - lo) / span * maxq : 0.0f;
-    q[d] = (uint32_t)fminf(fmaxf(t, 0.0f), maxq);
+    uint32_t lo = 0xffffffffu, hi = 0u;
+#pragma unroll 8
+    for (int r = 0; r < KD_RUN; ++r) {
+      const int64_t pos = p0 + 32 * r + lane;
+      if (pos < n) {
+        const uint32_t o = ord_of(x[(int64_t)val[pos].x * dim + d]);
+        lo = min(lo, o);
+        hi = max(hi, o);
+      }
+    }
+    lo = __reduce_min_sync(FULL, lo);
+    hi = __reduce_max_sync(FULL, hi);
+    if (lane == 0) {
+      atomicMin(&bmin[node * dim + d], lo);
+      atomicMax(&bmax[node * dim + d], hi);
+    }
   }
-  uint64_t code = 0;
-  for (int b = bits - 1; b >= 0; --b)
-    for (int d = 0; d < dim; ++d) code = (code << 1) | ((q[d] >> b) & 1u);
-  key[i] = (uint32_t)code;
-  val[i] = make_uint2((uint32_t)i, (uint32_t)(code >> 32));
 }
 
-__global__ void k_mst_hi_keys(const uint2* __restrict__ val, int64_t n, uint32_t* __restrict__ key) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) key[i] = val[i].y;
+// Widest side of a box.
+__device__ __forceinline__ int kd_side(const uint32_t* bmin, const uint32_t* bmax, int dim) {
+  int side = 0;
+  float wide = -1.0f;
+  for (int d = 0; d < dim; ++d) {
+    const float w = of_ord(bmax[d]) - of_ord(bmin[d]);
+    if (w > wide) {
+      wide = w;
+      side = d;
+    }
+  }
+  return side;
+}
+
+// Sort key of a level: node, then the coordinate along the node's widest side
+// on `bits` bits of its extent.
+__global__ void k_kd_key(const float* __restrict__ x, int64_t n, int dim, int64_t size, int bits,
+                         const uint2* __restrict__ val, const uint32_t* __restrict__ bmin,
+                         const uint32_t* __restrict__ bmax, uint32_t* __restrict__ key) {
+  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pos >= n) return;
+  const int64_t node = pos / size;
+  const int side = kd_side(bmin + node * dim, bmax + node * dim, dim);
+  const float lo = of_ord(bmin[node * dim + side]), hi = of_ord(bmax[node * dim + side]);
+  const float maxq = (float)((1u << bits) - 1u), span = hi - lo;
+  const float t = span > 0.0f ? (x[(int64_t)val[pos].x * dim + side] - lo) / span * maxq : 0.0f;
+  key[pos] = ((uint32_t)node << bits) | (uint32_t)fminf(fmaxf(t, 0.0f), maxq);
+}
+
+// All levels of the nodes of at most KD_BLOCK points, a block per such node: per
+// level the boxes of the nodes inside, then a bitonic sort of (coordinate, slot)
+// within each of them. Bound by shared memory; the coordinates come from L2.
+constexpr int KD_BLOCK = 4096;
+constexpr int KD_THREADS = 512;
+struct KdSmem {
+  unsigned long long key[KD_BLOCK];  // coordinate image << 32 | slot
+  uint32_t id[KD_BLOCK];             // point of each slot
+  uint32_t bmin[KD_BLOCK / 64][16], bmax[KD_BLOCK / 64][16];
+  uint8_t side[KD_BLOCK / 64];
+};
+__global__ void __launch_bounds__(KD_THREADS) k_kd_block(const float* __restrict__ x, int64_t n,
+                                                         int dim, int top,
+                                                         uint2* __restrict__ val) {
+  extern __shared__ __align__(16) unsigned char kd_raw[];
+  KdSmem& sm = *reinterpret_cast<KdSmem*>(kd_raw);
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t base = (int64_t)blockIdx.x * top;
+  const int cnt = (int)min((int64_t)top, n - base);
+  for (int e = threadIdx.x; e < top; e += KD_THREADS) {
+    sm.id[e] = e < cnt ? val[base + e].x : 0u;
+    sm.key[e] = (unsigned long long)e;  // slots past the end stay behind (all-ones coordinate)
+  }
+  for (int size = top; size >= 2 * MST_LEAF; size >>= 1) {
+    const int nodes = top / size;
+    for (int q = threadIdx.x; q < nodes * dim; q += KD_THREADS) {
+      sm.bmin[q / dim][q % dim] = 0xffffffffu;
+      sm.bmax[q / dim][q % dim] = 0u;
+    }
+    __syncthreads();
+    for (int c = warp; c < top / 32; c += KD_THREADS / 32) {
+      const int slot = (int)(uint32_t)sm.key[32 * c + lane];
+      const bool on = slot < cnt;
+      const float* p = x + (int64_t)sm.id[slot] * dim;
+      for (int d = 0; d < dim; ++d) {
+        const uint32_t o = on ? ord_of(p[d]) : 0u;
+        const uint32_t lo = __reduce_min_sync(FULL, on ? o : 0xffffffffu);
+        const uint32_t hi = __reduce_max_sync(FULL, o);
+        if (lane == 0) {
+          atomicMin(&sm.bmin[32 * c / size][d], lo);
+          atomicMax(&sm.bmax[32 * c / size][d], hi);
+        }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < nodes)
+      sm.side[threadIdx.x] = (uint8_t)kd_side(sm.bmin[threadIdx.x], sm.bmax[threadIdx.x], dim);
+    __syncthreads();
+    for (int e = threadIdx.x; e < top; e += KD_THREADS) {
+      const uint32_t slot = (uint32_t)sm.key[e];
+      const uint32_t o = (int)slot < cnt
+                             ? ord_of(x[(int64_t)sm.id[slot] * dim + sm.side[e / size]])
+                             : 0xffffffffu;
+      sm.key[e] = ((unsigned long long)o << 32) | slot;
+    }
+    for (int run = 2; run <= size; run <<= 1)
+      for (int stride = run >> 1; stride >= 1; stride >>= 1) {
+        __syncthreads();
+        for (int q = threadIdx.x; q < top / 2; q += KD_THREADS) {
+          const int i = 2 * q - (q & (stride - 1)), j = i + stride;
+          const unsigned long long a = sm.key[i], b = sm.key[j];
+          const bool up = run == size || (i & run) == 0;  // every node ascends
+          if ((a > b) == up) {
+            sm.key[i] = b;
+            sm.key[j] = a;
+          }
+        }
+      }
+    __syncthreads();
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < cnt; e += KD_THREADS)
+    val[base + e].x = sm.id[(uint32_t)sm.key[e]];
 }
 
 // Sorted copy of the points, padded with zeros to DIMP (a zero pad adds +0 to
@@ -149,14 +252,16 @@ __device__ __forceinline__ void mst_load(const float* __restrict__ xs, int64_t p
   }
 }
 
-// sum_d (a_d - b_d)^2, serial over the dimensions (mst.rs's squared metric).
+// sum_d (a_d - b_d)^2, serial over the dimensions (mst.rs's squared metric); the
+// differences and squares are packed pairs (the same roundings).
 template <int DIMP>
 __device__ __forceinline__ float mst_sqd(const float (&a)[DIMP], const float (&b)[DIMP]) {
   float s = 0.0f;
 #pragma unroll
-  for (int d = 0; d < DIMP; ++d) {
-    const float t = fsub(a[d], b[d]);
-    s = fadd(s, fmul(t, t));
+  for (int d = 0; d < DIMP; d += 2) {
+    const float2 t = fsub2(make_float2(a[d], a[d + 1]), make_float2(b[d], b[d + 1]));
+    const float2 t2 = fmul2(t, t);
+    s = fadd(fadd(s, t2.x), t2.y);
   }
   return s;
 }
@@ -174,13 +279,13 @@ __device__ __forceinline__ float mst_box_lb(const float* __restrict__ lo,
 #pragma unroll
   for (int q = 0; q < DIMP / 4; ++q) {
     const float4 a = __ldg(l4 + q), b = __ldg(h4 + q);
-    const float la[4] = {a.x, a.y, a.z, a.w}, hb[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float x = p[4 * q + e];
-      const float diff = x < la[e] ? fsub(la[e], x) : (x > hb[e] ? fsub(x, hb[e]) : 0.0f);
-      r = fadd(r, fmul(diff, diff));
-    }
+    const float2 p0 = make_float2(p[4 * q], p[4 * q + 1]), p1 = make_float2(p[4 * q + 2], p[4 * q + 3]);
+    const float2 l0 = fsub2(make_float2(a.x, a.y), p0), l1 = fsub2(make_float2(a.z, a.w), p1);
+    const float2 h0 = fsub2(p0, make_float2(b.x, b.y)), h1 = fsub2(p1, make_float2(b.z, b.w));
+    const float2 d0 = make_float2(fmaxf(fmaxf(l0.x, h0.x), 0.0f), fmaxf(fmaxf(l0.y, h0.y), 0.0f));
+    const float2 d1 = make_float2(fmaxf(fmaxf(l1.x, h1.x), 0.0f), fmaxf(fmaxf(l1.y, h1.y), 0.0f));
+    const float2 s0 = fmul2(d0, d0), s1 = fmul2(d1, d1);
+    r = fadd(fadd(fadd(fadd(r, s0.x), s0.y), s1.x), s1.y);
   }
   return r;
 }
@@ -218,229 +323,435 @@ __global__ void k_mst_leaf_boxes(const float* __restrict__ xs, int64_t n, int64_
   }
 }
 
-// Internal boxes of one level: nodes [first, first + count).
+// Internal boxes, up to eight levels per launch: a block takes 256 nodes of the
+// level that starts at `first` (of count = first nodes) and goes up while it has
+// two nodes left.
+constexpr int UP_NODES = 256;
 template <int DIMP>
-__global__ void k_mst_level_boxes(float* __restrict__ lo, float* __restrict__ hi, int64_t first,
-                                  int64_t count) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const int64_t v = first + k;
-  const float4* l4 = reinterpret_cast<const float4*>(lo);
-  const float4* h4 = reinterpret_cast<const float4*>(hi);
+__global__ void __launch_bounds__(UP_NODES / 2) k_mst_boxes_up(float* __restrict__ lo,
+                                                             float* __restrict__ hi,
+                                                             int64_t first) {
+  constexpr int Q = DIMP / 4;
   float4* lo4 = reinterpret_cast<float4*>(lo);
   float4* hi4 = reinterpret_cast<float4*>(hi);
-  constexpr int Q = DIMP / 4;
+  const int64_t n0 = first + (int64_t)blockIdx.x * UP_NODES;
+  int64_t base = n0 >> 1;
+  for (int cnt = (int)min((int64_t)UP_NODES, first) >> 1; cnt >= 1; cnt >>= 1, base >>= 1) {
+    if ((int)threadIdx.x < cnt) {
+      const int64_t v = base + threadIdx.x;
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const float4 a = l4[2 * v * Q + q], b = l4[(2 * v + 1) * Q + q];
-    const float4 c = h4[2 * v * Q + q], e = h4[(2 * v + 1) * Q + q];
-    lo4[v * Q + q] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), fminf(a.w, b.w));
-    hi4[v * Q + q] = make_float4(fmaxf(c.x, e.x), fmaxf(c.y, e.y), fmaxf(c.z, e.z), fmaxf(c.w, e.w));
+      for (int q = 0; q < Q; ++q) {
+        const float4 a = lo4[2 * v * Q + q], b = lo4[(2 * v + 1) * Q + q];
+        const float4 c = hi4[2 * v * Q + q], e = hi4[(2 * v + 1) * Q + q];
+        lo4[v * Q + q] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), fminf(a.w, b.w));
+        hi4[v * Q + q] = make_float4(fmaxf(c.x, e.x), fmaxf(c.y, e.y), fmaxf(c.z, e.z), fmaxf(c.w, e.w));
+      }
+    }
+    __syncthreads();  // the level is written (the block reads only its own nodes)
   }
 }
 
-// Warp-cooperative traversal. A warp serves 32 consecutive sorted points
-// (spatially close in Morton order) and walks the union of their searches in
-// lockstep: it enters a node when any lane's own pruning rule keeps it,
-// descends first into the child most lanes find nearer and pushes the other
-// (re-tested when popped); the stack is warp-uniform, entry i held by lane i
-// (the tree is at most 28 levels deep). A leaf's points are staged once in
-// shared memory and every lane that needs the leaf scans them.
-constexpr int MST_WARPS = 4;  // warps per block
+// Searches. A warp serves one point and walks the tree 32 nodes at a time: the
+// descendants five levels below a node are consecutive in heap order, so each
+// lane tests one of them, the nearest that can still matter is entered first, and
+// a leaf's 32 points are measured by one lane each. The earlier form, 32 points
+// per warp walking the union of their searches in lockstep, kept 7 of 32 lanes
+// busy in a leaf and left single warps with thousands of serial steps (1M points,
+// 8-d blobs, the same tree: core distances 26.8 ms against 7.3 here, and 8 to 13 ms
+// in each early round for one straggling warp against 0.8 to 1.1). The instruction
+// count bounds it: about 20 leaves and 10 groups per point, and 12 blocks per SM
+// (40 registers) gain only a tenth over 8.
+constexpr int MST_WARPS = 4;   // warps per block
+template <int DIMP>
+constexpr int mst_blocks() { return DIMP <= 8 ? 12 : 8; }  // blocks per SM (registers)
+constexpr int MST_LEVELS = 6;  // of five binary levels: 2^28 leaves at most
+constexpr uint32_t INF_BITS = 0x7f800000u;
 
 template <int DIMP>
-struct MstLeafStage {
-  float4 pt[MST_LEAF][DIMP / 4];
-  uint32_t comp[MST_LEAF];
-  float core[MST_LEAF];
-  uint32_t orig[MST_LEAF];
+struct MstTree {
+  const float* xs;
+  const float* lo;
+  const float* hi;
+  int64_t n, P;
+  int depth;  // binary levels: P = 2^depth leaves
 };
 
-template <int DIMP>
-__device__ __forceinline__ void mst_stage_leaf(MstLeafStage<DIMP>& st,
-                                               const float* __restrict__ xs, int64_t b0, int cnt,
-                                               int lane) {
-  if (lane < cnt) {
-    const float4* src = reinterpret_cast<const float4*>(xs + (b0 + lane) * DIMP);
-#pragma unroll
-    for (int q = 0; q < DIMP / 4; ++q) st.pt[lane][q] = __ldg(src + q);
-  }
+// Position of a walk: the group of nodes in hand, each lane holding the bound of
+// its node (INF: done, pruned or none). The groups above wait in shared memory.
+struct MstWalk {
+  int64_t base;  // first node of the group
+  int level;     // depth of the group's nodes
+  int up;        // groups waiting above
+  float p;       // this lane's bound
+};
+
+__device__ __forceinline__ int mst_first_bits(int depth) {
+  return depth == 0 ? 0 : (depth - 1) % 5 + 1;
 }
 
-template <int DIMP>
-__device__ __forceinline__ void mst_staged(const MstLeafStage<DIMP>& st, int s2,
-                                           float (&y)[DIMP]) {
+// The next node whose bound does not exceed `limit`, nearest first, or -1 when
+// the group is done.
+__device__ __forceinline__ int64_t mst_next(MstWalk& w, float limit, int lane) {
+  const unsigned FULL = 0xffffffffu;
+  const uint32_t m = __reduce_min_sync(FULL, __float_as_uint(w.p));
+  if (m == INF_BITS || __uint_as_float(m) > limit) return -1;
+  const int sel = __ffs(__ballot_sync(FULL, __float_as_uint(w.p) == m)) - 1;
+  if (lane == sel) w.p = __uint_as_float(INF_BITS);
+  return w.base + sel;
+}
+
+// Back to the waiting group above; false at the top.
+__device__ __forceinline__ bool mst_ascend(MstWalk& w, const float (*stack)[32], int first_bits,
+                                           int lane) {
+  if (w.up == 0) return false;
+  --w.up;
+  w.p = stack[w.up][lane];
+  w.base = w.up == 0 ? (int64_t)1 << first_bits : (w.base >> 5) & ~(int64_t)31;
+  w.level -= 5;
+  return true;
+}
+
+__device__ __forceinline__ void mst_descend(MstWalk& w, float (*stack)[32], int64_t node, int lane) {
+  stack[w.up][lane] = w.p;
+  ++w.up;
+  w.base = node << 5;
+  w.level += 5;
+}
+
+// Ascending bitonic sort of (d, j) across the warp.
+__device__ __forceinline__ void mst_sort32(float& d, uint32_t& j, int lane) {
 #pragma unroll
-  for (int q = 0; q < DIMP / 4; ++q) {
-    const float4 t = st.pt[s2][q];
-    y[4 * q] = t.x;
-    y[4 * q + 1] = t.y;
-    y[4 * q + 2] = t.z;
-    y[4 * q + 3] = t.w;
-  }
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride >= 1; stride >>= 1) {
+      const float od = __shfl_xor_sync(0xffffffffu, d, stride);
+      const uint32_t oj = __shfl_xor_sync(0xffffffffu, j, stride);
+      const bool low = ((lane & size) == 0) == ((lane & stride) == 0);
+      const bool take = low ? (od < d || (od == d && oj < j)) : (od > d || (od == d && oj > j));
+      if (take) {
+        d = od;
+        j = oj;
+      }
+    }
 }
 
 // Core distances: per sorted point, the k-th smallest squared distance to
-// another point (the k smallest kept sorted in registers); a node is skipped
-// when its box bound exceeds the current k-th distance (kd_tree.rs:499).
-template <int DIMP, int KMAX>
-__global__ void __launch_bounds__(32 * MST_WARPS) k_mst_core(
-    const float* __restrict__ xs, int64_t n, int64_t P, int64_t L, const float* __restrict__ lo,
-    const float* __restrict__ hi, int k, float* __restrict__ core, uint32_t* __restrict__ knn_j,
-    float* __restrict__ knn_d, int32_t* __restrict__ status) {
-  __shared__ MstLeafStage<DIMP> stage_s[MST_WARPS];
+// another point; a node is skipped when its box bound exceeds the current k-th
+// distance (kd_tree.rs:499). The k smallest are kept sorted across the lanes
+// (entry t in lane t, with WIDE entries 32.. in a second register), started
+// from the point's own leaf.
+template <int DIMP, bool WIDE>
+__global__ void __launch_bounds__(32 * MST_WARPS, mst_blocks<DIMP>()) k_mst_core(
+    MstTree<DIMP> tree, int k, unsigned long long* __restrict__ work, float* __restrict__ core,
+    uint32_t* __restrict__ knn_j, float* __restrict__ knn_d, uint8_t* __restrict__ tie_out) {
+  __shared__ float stack_s[MST_WARPS][MST_LEVELS][32];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t q0 = ((int64_t)blockIdx.x * MST_WARPS + wid) * 32;
-  if (q0 >= n) return;
-  MstLeafStage<DIMP>& st = stage_s[wid];
-  const int64_t pos = q0 + lane;
-  const bool act = pos < n;
-  float q[DIMP];
-  mst_load<DIMP>(xs, act ? pos : q0, q);
-  const float INF = __int_as_float(0x7f800000);
-  float kd[KMAX];
-  uint32_t kj[KMAX];
-#pragma unroll
-  for (int t = 0; t < KMAX; ++t) {
-    kd[t] = INF;
-    kj[t] = NO_POINT;
-  }
-  float kth = act ? INF : -1.0f;  // an idle lane needs no node
-  const unsigned actm = __ballot_sync(FULL, act);
-  uint32_t stk = 0;
-  int sp = 0;
-  int64_t v = 1;
-  float lbv = 0.0f;
+  float (*stack)[32] = stack_s[wid];
+  const float INF = __uint_as_float(INF_BITS);
+  const int g0 = mst_first_bits(tree.depth);
   for (;;) {
-    if (__any_sync(FULL, lbv <= kth)) {
-      if (v >= P) {
-        const int64_t l = v - P;
-        if (l < L) {
-          const int64_t b0 = l * MST_LEAF;
-          const int cnt = (int)min((int64_t)MST_LEAF, n - b0);
-          __syncwarp();
-          mst_stage_leaf<DIMP>(st, xs, b0, cnt, lane);
-          __syncwarp();
-          if (lbv <= kth) {
-            for (int s2 = 0; s2 < cnt; ++s2) {
-              if (b0 + s2 == pos) continue;
-              float y[DIMP];
-              mst_staged<DIMP>(st, s2, y);
-              const float d = mst_sqd<DIMP>(q, y);
-              if (d < kth) {
-                const uint32_t j = (uint32_t)(b0 + s2);
-#pragma unroll
-                for (int t = KMAX - 1; t > 0; --t) {
-                  if (kd[t - 1] > d) {
-                    kd[t] = kd[t - 1];
-                    kj[t] = kj[t - 1];
-                  } else if (kd[t] > d) {
-                    kd[t] = d;
-                    kj[t] = j;
-                  }
-                }
-                if (kd[0] > d) {
-                  kd[0] = d;
-                  kj[0] = j;
-                }
-                float kt = kd[0];
-#pragma unroll
-                for (int t = 1; t < KMAX; ++t)
-                  if (t == k - 1) kt = kd[t];
-                kth = kt;
-              }
-            }
-          }
-        }
-      } else {
-        const float l0 = mst_box_lb<DIMP>(lo, hi, 2 * v, q);
-        const float l1 = mst_box_lb<DIMP>(lo, hi, 2 * v + 1, q);
-        const bool n0 = __any_sync(FULL, l0 <= kth), n1 = __any_sync(FULL, l1 <= kth);
-        if (n0 || n1) {
-          const bool left = 2 * __popc(__ballot_sync(FULL, l0 <= l1) & actm) >= __popc(actm);
-          const bool na = left ? n0 : n1, nb = left ? n1 : n0;
-          const int64_t a = left ? 2 * v : 2 * v + 1;
-          if (na && nb) {
-            if (sp >= 32) {
-              if (lane == 0) set_status(status, ST_INTERNAL);
-              return;
-            }
-            if (lane == sp) stk = (uint32_t)(a ^ 1);
-            ++sp;
-          }
-          const int64_t c = na ? a : (a ^ 1);
-          lbv = (c == 2 * v) ? l0 : l1;
-          v = c;
-          continue;
-        }
+    int64_t pos = 0;
+    if (lane == 0) pos = (int64_t)atomicAdd(work, 1ull);
+    pos = __shfl_sync(FULL, pos, 0);
+    if (pos >= tree.n) return;
+    float q[DIMP];
+    mst_load<DIMP>(tree.xs, pos, q);
+    float kd0 = INF, kd1 = INF;
+    uint32_t kj0 = NO_POINT, kj1 = NO_POINT;
+    const int64_t own = pos / MST_LEAF;
+    {
+      const int64_t j = own * MST_LEAF + lane;
+      if (j < tree.n && j != pos) {
+        float y[DIMP];
+        mst_load<DIMP>(tree.xs, j, y);
+        kd0 = mst_sqd<DIMP>(q, y);
+        if (kd0 < INF) kj0 = (uint32_t)j;
       }
+      mst_sort32(kd0, kj0, lane);
     }
-    if (sp == 0) break;
-    --sp;
-    v = __shfl_sync(FULL, stk, sp);
-    lbv = mst_box_lb<DIMP>(lo, hi, v, q);
-  }
-  if (act) {
-    core[pos] = kth;
-#pragma unroll
-    for (int t = 0; t < KMAX; ++t)
-      if (t < k) {
-        knn_j[pos * k + t] = kj[t];
-        knn_d[pos * k + t] = kd[t];
+    const bool high = WIDE && k > 32;  // the k-th entry is in the second register
+    float kth = __shfl_sync(FULL, high ? kd1 : kd0, (k - 1) & 31);
+    // a point outside the first k is exactly kth away
+    bool tie = !high && __any_sync(FULL, lane >= k && kd0 == kth);
+    MstWalk w{(int64_t)1 << g0, g0, 0, INF};
+    if (tree.depth > 0 && lane < (1 << g0)) w.p = mst_box_lb<DIMP>(tree.lo, tree.hi, w.base + lane, q);
+    for (;;) {
+      if (w.level == tree.depth && w.base + lane == tree.P + own) w.p = INF;  // its own leaf is in
+      const int64_t node = mst_next(w, kth, lane);
+      if (node < 0) {
+        if (!mst_ascend(w, stack, g0, lane)) break;
+        continue;
       }
+      if (w.level < tree.depth) {
+        mst_descend(w, stack, node, lane);
+        w.p = mst_box_lb<DIMP>(tree.lo, tree.hi, w.base + lane, q);
+        continue;
+      }
+      const int64_t j = (node - tree.P) * MST_LEAF + lane;
+      float d = INF;
+      if (j < tree.n) {
+        float y[DIMP];
+        mst_load<DIMP>(tree.xs, j, y);
+        d = mst_sqd<DIMP>(q, y);
+      }
+      for (uint32_t in; (in = __ballot_sync(FULL, d < kth)) != 0u;) {
+        const int src = __ffs(in) - 1;
+        const float dv = __shfl_sync(FULL, d, src);
+        const uint32_t jv = (uint32_t)(j - lane + src);
+        if (lane == src) d = INF;
+        const int at = __popc(__ballot_sync(FULL, kd0 <= dv));  // after equal entries
+        const float ud = __shfl_up_sync(FULL, kd0, 1);
+        const uint32_t uj = __shfl_up_sync(FULL, kj0, 1);
+        if (WIDE) {
+          const int at1 = 32 + __popc(__ballot_sync(FULL, kd1 <= dv)), slot = at < 32 ? at : at1;
+          const float ld = __shfl_sync(FULL, kd0, 31);
+          const uint32_t lj = __shfl_sync(FULL, kj0, 31);
+          const float vd = __shfl_up_sync(FULL, kd1, 1);
+          const uint32_t vj = __shfl_up_sync(FULL, kj1, 1);
+          if (lane + 32 == slot) {
+            kd1 = dv;
+            kj1 = jv;
+          } else if (lane + 32 > slot) {
+            kd1 = lane == 0 ? ld : vd;
+            kj1 = lane == 0 ? lj : vj;
+          }
+        }
+        if (lane == at) {
+          kd0 = dv;
+          kj0 = jv;
+        } else if (lane > at) {
+          kd0 = ud;
+          kj0 = uj;
+        }
+        const float was = kth;
+        kth = __shfl_sync(FULL, high ? kd1 : kd0, (k - 1) & 31);
+        tie = was == kth;  // the entry pushed out was at the distance that stays
+      }
+      tie = tie || __any_sync(FULL, d == kth && j < tree.n);
+    }
+    if (lane < k) {
+      knn_j[pos * k + lane] = kj0;
+      knn_d[pos * k + lane] = kd0;
+    }
+    if (WIDE && lane + 32 < k) {
+      knn_j[pos * k + lane + 32] = kj1;
+      knn_d[pos * k + lane + 32] = kd1;
+    }
+    if (lane == 0) {
+      core[pos] = kth;
+      tie_out[pos] = tie ? 1 : 0;
+    }
   }
 }
 
-// Upper bounds before a round's queries: per component, the smallest mutual
-// reachability value over the kNN edges (from the core-distance pass) that
-// leave it. Each is the value of a real edge leaving the component, so it is
-// never below the component's pick and starting the queries just above it
-// changes no pick.
-__global__ void k_mst_knn_bound(int64_t n, int k, const uint32_t* __restrict__ knn_j,
-                                const float* __restrict__ knn_d,
-                                const uint32_t* __restrict__ comp, const float* __restrict__ core,
-                                uint32_t* __restrict__ cbest) {
+// What a point knows of its nearest point of another component carries over
+// between rounds, because components only grow: near_j is that point (or
+// NO_POINT) and near_v its value, or, without a point, a value below which there
+// is none. A point whose near_j is still foreign needs no search, and neither
+// does one whose near_v is not below its component's bound.
+//
+// First round, from the kNN lists: every value is at least the point's own core
+// distance, and the points at exactly that value are those within it whose own
+// core distance is no larger, that is entries of its list (unless a point outside
+// the list ties with the last one). The smallest index among them is the answer.
+__global__ void k_mst_near_init(int64_t n, int k, const uint32_t* __restrict__ knn_j,
+                                const uint8_t* __restrict__ tie, const float* __restrict__ core,
+                                const uint32_t* __restrict__ orig, uint32_t* __restrict__ near_j,
+                                float* __restrict__ near_v) {
   const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= n) return;
-  const uint32_t qc = comp[pos];
+  const float cq = core[pos];
+  uint32_t best = NO_POINT, bo = NO_POINT;
+  if (k > 0 && cq < __uint_as_float(FMAX_BITS) && !tie[pos]) {
+    for (int t = 0; t < k; ++t) {
+      const uint32_t j = knn_j[pos * k + t];
+      if (j >= n || core[j] > cq) continue;  // unfilled, or a larger value
+      const uint32_t oj = orig[j];
+      if (oj < bo) {
+        bo = oj;
+        best = j;
+      }
+    }
+  }
+  near_j[pos] = best;
+  near_v[pos] = cq;
+}
+
+// Upper bounds before a round's queries: per component, the smallest value of its
+// points' nearest foreign points where those are known, of the kNN edges
+// (from the core-distance pass) that leave it, and of the neighbours in tree order
+// that do (a component of a whole cluster often has no other). Each is the value of a real edge
+// leaving the component, so it is never below the component's pick and starting
+// the queries just above it changes no pick.
+template <int DIMP>
+__global__ void k_mst_bound(const float* __restrict__ xs, int64_t n, int k,
+                            const uint32_t* __restrict__ knn_j,
+                            const float* __restrict__ knn_d, const uint32_t* __restrict__ comp,
+                            const float* __restrict__ core, uint32_t* __restrict__ near_j,
+                            const float* __restrict__ near_v, uint32_t* __restrict__ cbest) {
+  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pos >= n) return;
+  const uint32_t qc = comp[pos], nj = near_j[pos];
+  if (pos + 1 < n && comp[pos + 1] != qc) {
+    const uint32_t oc = comp[pos + 1];
+    float a[DIMP], b[DIMP];
+    mst_load<DIMP>(xs, pos, a);
+    mst_load<DIMP>(xs, pos + 1, b);
+    const float mr = fmaxf(fmaxf(mst_sqd<DIMP>(a, b), core[pos]), core[pos + 1]);
+    const uint32_t v = __float_as_uint(mr);
+    if (v < __ldcg(cbest + qc)) atomicMin(cbest + qc, v);
+    if (v < __ldcg(cbest + oc)) atomicMin(cbest + oc, v);
+  }
+  if (nj != NO_POINT) {
+    if (comp[nj] != qc) {
+      const uint32_t v = __float_as_uint(near_v[pos]);
+      if (v < __ldcg(cbest + qc)) atomicMin(cbest + qc, v);
+      return;  // its nearest: no kNN edge of it leaves with less
+    }
+    near_j[pos] = NO_POINT;
+  }
   const float cq = core[pos];
   float best = __uint_as_float(FMAX_BITS);
-  bool any = false;
   for (int t = 0; t < k; ++t) {
     const uint32_t j = knn_j[pos * k + t];
     if (j >= n || comp[j] == qc) continue;  // an unfilled entry (no finite distance)
-    const float mr = fmaxf(fmaxf(knn_d[pos * k + t], cq), core[j]);
-    if (mr < best) {
-      best = mr;
-      any = true;
+    best = fminf(best, fmaxf(fmaxf(knn_d[pos * k + t], cq), core[j]));
+  }
+  const uint32_t v = __float_as_uint(best);
+  if (v < __ldcg(cbest + qc)) atomicMin(cbest + qc, v);
+}
+
+// Known nearest points enter their component's pick; need[pos] = 1 for the
+// points that have to search.
+__global__ void k_mst_select(int64_t n, const uint32_t* __restrict__ comp,
+                             const float* __restrict__ core, const uint32_t* __restrict__ orig,
+                             const uint32_t* __restrict__ near_j, const float* __restrict__ near_v,
+                             const uint32_t* __restrict__ cbest,
+                             unsigned long long* __restrict__ ckey, int32_t* __restrict__ need) {
+  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pos >= n) return;
+  const uint32_t qc = comp[pos], cb = cbest[qc];
+  const float v = near_v[pos];
+  bool search = false;
+  if (near_j[pos] != NO_POINT) {
+    const uint32_t vb = __float_as_uint(v);
+    if (vb <= cb) atomicMin(ckey + qc, ((unsigned long long)vb << 32) | orig[pos]);
+  } else {
+    const float bd = __uint_as_float(cb < FMAX_BITS ? cb + 1u : FMAX_BITS);
+    search = v < bd && !(core[pos] > bd);
+  }
+  need[pos] = search ? 1 : 0;
+}
+
+__global__ void k_mst_search_list(int64_t n, const int32_t* __restrict__ need,
+                                  const int64_t* __restrict__ off, uint32_t* __restrict__ list) {
+  const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pos < n && need[pos]) list[off[pos]] = (uint32_t)pos;
+}
+
+// What a round's queries see of a node: a component `maj` that many of its points
+// belong to, the box of its other points, and the smallest core distance of all
+// (core_all) and of the other points (core_rest). A query of that component is
+// bounded by the other points' box and core (infinite for a node wholly of one
+// component), any other query by the full box and core_all. Otherwise a few stray
+// points next to a cluster keep the cluster's own points in every leaf that holds
+// one of them, although their large core distances rule them out (1M points: the
+// last three rounds 51.7 ms with pure-node marks only, 29.7 with this).
+template <int DIMP>
+struct MstParts {
+  uint32_t* maj;
+  int32_t* cnt;
+  float* lo;
+  float* hi;
+  float* core_all;
+  float* core_rest;
+};
+
+// Leaves: a warp per leaf; the most frequent component (the smallest id among
+// equals). No point belongs to NO_POINT, the majority of an empty leaf.
+template <int DIMP>
+__global__ void k_mst_leaf_parts(MstTree<DIMP> tree, const uint32_t* __restrict__ comp,
+                                 const float* __restrict__ core, MstParts<DIMP> parts) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t l = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (l >= tree.P) return;
+  const int64_t j = l * MST_LEAF + lane;
+  const bool on = j < tree.n;
+  const uint32_t c = on ? comp[j] : NO_POINT;
+  const uint32_t peers = __match_any_sync(FULL, c);  // every lane takes part
+  const int same = on ? __popc(peers) : 0;
+  const int most = __reduce_max_sync(FULL, same);
+  const uint32_t m = __reduce_min_sync(FULL, on && same == most ? c : NO_POINT);
+  const bool other = on && c != m;
+  float y[DIMP];
+  if (other) mst_load<DIMP>(tree.xs, j, y);
+  const bool any = __any_sync(FULL, other);
+  float* vl = parts.lo + (tree.P + l) * DIMP;
+  float* vh = parts.hi + (tree.P + l) * DIMP;
+  const uint32_t cb = on ? __float_as_uint(core[j]) : INF_BITS;  // not negative: bits order them
+  const uint32_t c_all = __reduce_min_sync(FULL, cb);
+  const uint32_t c_rest = __reduce_min_sync(FULL, other ? cb : INF_BITS);
+#pragma unroll
+  for (int d = 0; d < DIMP; ++d) {
+    float a = __uint_as_float(INF_BITS), b = -a;
+    if (any) {
+      const uint32_t o = other ? ord_of(y[d]) : 0u;
+      const uint32_t mn = __reduce_min_sync(FULL, other ? o : 0xffffffffu);
+      const uint32_t mx = __reduce_max_sync(FULL, o);
+      a = of_ord(mn);
+      b = of_ord(mx);
+    }
+    if (lane == 0) {
+      vl[d] = a;
+      vh[d] = b;
     }
   }
-  if (any) atomicMin(cbest + qc, __float_as_uint(best));
-}
-
-// Node components: a leaf's common component, NC_MIXED or NC_EMPTY.
-__global__ void k_mst_leaf_comp(const uint32_t* __restrict__ comp, int64_t n, int64_t P, int64_t L,
-                                uint32_t* __restrict__ nd) {
-  const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= P) return;
-  if (l >= L) {
-    nd[P + l] = NC_EMPTY;
-    return;
+  if (lane == 0) {
+    parts.maj[tree.P + l] = m;
+    parts.cnt[tree.P + l] = most;
+    parts.core_all[tree.P + l] = __uint_as_float(c_all);
+    parts.core_rest[tree.P + l] = __uint_as_float(c_rest);
   }
-  const int64_t b = l * MST_LEAF, e = min(n, b + MST_LEAF);
-  const uint32_t c = comp[b];
-  bool same = true;
-  for (int64_t j = b + 1; j < e; ++j) same &= comp[j] == c;
-  nd[P + l] = same ? c : NC_MIXED;
 }
 
-__global__ void k_mst_level_comp(uint32_t* __restrict__ nd, int64_t first, int64_t count) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const int64_t v = first + k;
-  const uint32_t a = nd[2 * v], b = nd[2 * v + 1];
-  nd[v] = a == NC_EMPTY ? b : (b == NC_EMPTY ? a : (a == b ? a : NC_MIXED));
+// Inner nodes, up to eight levels per launch (as k_mst_boxes_up): the majority
+// of the child whose majority is larger, and the union of what the children hold
+// besides it.
+template <int DIMP>
+__global__ void __launch_bounds__(UP_NODES / 2) k_mst_parts_up(MstTree<DIMP> tree,
+                                                             MstParts<DIMP> parts, int64_t first) {
+  constexpr int Q = DIMP / 4;
+  float4* lo4 = reinterpret_cast<float4*>(parts.lo);
+  float4* hi4 = reinterpret_cast<float4*>(parts.hi);
+  const float4* fl4 = reinterpret_cast<const float4*>(tree.lo);
+  const float4* fh4 = reinterpret_cast<const float4*>(tree.hi);
+  int64_t base = (first + (int64_t)blockIdx.x * UP_NODES) >> 1;
+  for (int c = (int)min((int64_t)UP_NODES, first) >> 1; c >= 1; c >>= 1, base >>= 1) {
+    if ((int)threadIdx.x < c) {
+      const int64_t v = base + threadIdx.x, l = 2 * v, r = 2 * v + 1;
+      const uint32_t ml = parts.maj[l], mr = parts.maj[r];
+      const int32_t cl = parts.cnt[l], cr = parts.cnt[r];
+      const uint32_t m = cl >= cr ? ml : mr;
+      parts.maj[v] = m;
+      parts.cnt[v] = ml == mr ? cl + cr : max(cl, cr);
+      parts.core_all[v] = fminf(parts.core_all[l], parts.core_all[r]);
+      parts.core_rest[v] = fminf(ml == m ? parts.core_rest[l] : parts.core_all[l],
+                                 mr == m ? parts.core_rest[r] : parts.core_all[r]);
+      const float4* la = (ml == m ? lo4 : fl4) + l * Q;
+      const float4* ha = (ml == m ? hi4 : fh4) + l * Q;
+      const float4* lb = (mr == m ? lo4 : fl4) + r * Q;
+      const float4* hb = (mr == m ? hi4 : fh4) + r * Q;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const float4 a = la[q], b = lb[q], e = ha[q], f = hb[q];
+        lo4[v * Q + q] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), fminf(a.w, b.w));
+        hi4[v * Q + q] = make_float4(fmaxf(e.x, f.x), fmaxf(e.y, f.y), fmaxf(e.z, f.z), fmaxf(e.w, f.w));
+      }
+    }
+    __syncthreads();
+  }
 }
 
 __global__ void k_mst_round_reset(const uint32_t* __restrict__ A, int64_t m,
@@ -454,126 +765,99 @@ __global__ void k_mst_round_reset(const uint32_t* __restrict__ A, int64_t m,
 }
 
 // Nearest point of another component under squared mutual reachability
-// (kd_tree.rs:318-378): a lane keeps a node when its box bound and its own
-// core distance do not exceed the lane's best value and the node is not
-// wholly of the lane's component. After each pop a lane lowers its bound to
-// just above its component's best value so far this round; a pick it holds
+// (kd_tree.rs:318-378), for the listed points: a node is kept when the bound of
+// its foreign points and the point's own core distance do not exceed the best
+// value so far. After each leaf the bound is
+// lowered to just above the component's best value so far this round; a pick
 // above that bound is dropped (it cannot be the component's pick).
 template <int DIMP>
-__global__ void __launch_bounds__(32 * MST_WARPS) k_mst_noc(
-    const float* __restrict__ xs, int64_t n, int64_t P, int64_t L, const float* __restrict__ lo,
-    const float* __restrict__ hi, const uint32_t* __restrict__ nd,
-    const uint32_t* __restrict__ comp, const float* __restrict__ core,
-    const uint32_t* __restrict__ orig, uint32_t* __restrict__ cbest,
-    unsigned long long* __restrict__ ckey, uint32_t* __restrict__ bj_out,
-    int32_t* __restrict__ status) {
-  __shared__ MstLeafStage<DIMP> stage_s[MST_WARPS];
+__global__ void __launch_bounds__(32 * MST_WARPS, mst_blocks<DIMP>()) k_mst_noc(
+    MstTree<DIMP> tree, MstParts<DIMP> parts, const uint32_t* __restrict__ comp,
+    const float* __restrict__ core, const uint32_t* __restrict__ orig,
+    const uint32_t* __restrict__ list, const int64_t* __restrict__ n_list,
+    unsigned long long* __restrict__ work, uint32_t* __restrict__ cbest,
+    unsigned long long* __restrict__ ckey, uint32_t* __restrict__ near_j,
+    float* __restrict__ near_v) {
+  __shared__ float stack_s[MST_WARPS][MST_LEVELS][32];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t q0 = ((int64_t)blockIdx.x * MST_WARPS + wid) * 32;
-  if (q0 >= n) return;
-  MstLeafStage<DIMP>& st = stage_s[wid];
-  const int64_t pos = q0 + lane;
-  const bool act = pos < n;
-  if (act) bj_out[pos] = NO_POINT;
-  const uint32_t root_c = nd[1];
-  const uint32_t qc = act ? comp[pos] : NC_MIXED;
-  const float cq = act ? core[pos] : 0.0f;
-  float bd = __uint_as_float(FMAX_BITS);
-  bool live = act && root_c != qc;  // root_c == qc: a single component
-  if (live) {
-    const uint32_t bb = __ldcg(cbest + qc);
-    if (bb < FMAX_BITS) bd = __uint_as_float(bb + 1u);
-    live = !(cq > bd);
-  }
-  if (!__any_sync(FULL, live)) return;
-  const unsigned actm = __ballot_sync(FULL, act);
-  float q[DIMP];
-  mst_load<DIMP>(xs, act ? pos : q0, q);
-  uint32_t bj = NO_POINT, bo = 0;
-  uint32_t stk = 0;
-  int sp = 0;
-  int64_t v = 1;
-  float lbv = 0.0f;
+  float (*stack)[32] = stack_s[wid];
+  const float INF = __uint_as_float(INF_BITS);
+  const int g0 = mst_first_bits(tree.depth);
+  const int64_t items = *n_list;
   for (;;) {
-    const bool need = live && !(lbv > bd) && nd[v] != qc;
-    if (__any_sync(FULL, need)) {
-      if (v >= P) {
-        const int64_t l = v - P;
-        if (l < L) {
-          const int64_t b0 = l * MST_LEAF;
-          const int cnt = (int)min((int64_t)MST_LEAF, n - b0);
-          __syncwarp();
-          mst_stage_leaf<DIMP>(st, xs, b0, cnt, lane);
-          if (lane < cnt) {
-            st.comp[lane] = comp[b0 + lane];
-            st.core[lane] = core[b0 + lane];
-            st.orig[lane] = orig[b0 + lane];
-          }
-          __syncwarp();
-          if (need) {
-            for (int s2 = 0; s2 < cnt; ++s2) {
-              if (st.comp[s2] == qc) continue;
-              const float cj = st.core[s2];
-              if (cj > bd) continue;
-              float y[DIMP];
-              mst_staged<DIMP>(st, s2, y);
-              const float mr = fmaxf(fmaxf(mst_sqd<DIMP>(q, y), cq), cj);
-              const uint32_t oj = st.orig[s2];
-              if (mr < bd || (mr == bd && bj != NO_POINT && oj < bo)) {
-                bd = mr;
-                bj = (uint32_t)(b0 + s2);
-                bo = oj;
-              }
-            }
-          }
-        }
-      } else {
-        const float l0 = mst_box_lb<DIMP>(lo, hi, 2 * v, q);
-        const float l1 = mst_box_lb<DIMP>(lo, hi, 2 * v + 1, q);
-        const bool ok = live && !(cq > bd);
-        const bool n0 = __any_sync(FULL, ok && !(l0 > bd) && nd[2 * v] != qc);
-        const bool n1 = __any_sync(FULL, ok && !(l1 > bd) && nd[2 * v + 1] != qc);
-        if (n0 || n1) {
-          const bool left = 2 * __popc(__ballot_sync(FULL, l0 <= l1) & actm) >= __popc(actm);
-          const bool na = left ? n0 : n1, nb = left ? n1 : n0;
-          const int64_t a = left ? 2 * v : 2 * v + 1;
-          if (na && nb) {
-            if (sp >= 32) {
-              if (lane == 0) set_status(status, ST_INTERNAL);
-              return;
-            }
-            if (lane == sp) stk = (uint32_t)(a ^ 1);
-            ++sp;
-          }
-          const int64_t c = na ? a : (a ^ 1);
-          lbv = (c == 2 * v) ? l0 : l1;
-          v = c;
-          continue;
+    int64_t item = 0;
+    if (lane == 0) item = (int64_t)atomicAdd(work, 1ull);
+    item = __shfl_sync(FULL, item, 0);
+    if (item >= items) return;
+    const int64_t pos = list[item];
+    const uint32_t qc = comp[pos];
+    const float cq = core[pos];
+    float q[DIMP];
+    mst_load<DIMP>(tree.xs, pos, q);
+    float bd = __uint_as_float(FMAX_BITS);
+    uint32_t bj = NO_POINT, bo = 0;
+    auto refresh = [&]() {  // the component's best so far, found by other warps
+      // one lane reads it (it changes meanwhile) and tells the others: the warp's
+      // path through the tree has to be one
+      const uint32_t cb = __shfl_sync(FULL, lane == 0 ? __ldcg(cbest + qc) : 0u, 0);
+      const float nb = __uint_as_float(cb < FMAX_BITS ? cb + 1u : FMAX_BITS);
+      if (nb < bd) {
+        bd = nb;
+        bj = NO_POINT;
+      }
+    };
+    refresh();
+    auto bound = [&](int64_t v) {
+      const bool own = parts.maj[v] == qc;
+      const float c = own ? parts.core_rest[v] : parts.core_all[v];
+      return fmaxf(mst_box_lb<DIMP>(own ? parts.lo : tree.lo, own ? parts.hi : tree.hi, v, q), c);
+    };
+    MstWalk w{(int64_t)1 << g0, g0, 0, INF};
+    if (lane < (1 << g0)) w.p = bound(w.base + lane);
+    while (!(cq > bd)) {
+      const int64_t node = mst_next(w, bd, lane);
+      if (node < 0) {
+        if (!mst_ascend(w, stack, g0, lane)) break;
+        continue;
+      }
+      if (w.level < tree.depth) {
+        mst_descend(w, stack, node, lane);
+        w.p = bound(w.base + lane);
+        continue;
+      }
+      const int64_t j = (node - tree.P) * MST_LEAF + lane;
+      float mr = INF;
+      if (j < tree.n && comp[j] != qc) {
+        const float cj = core[j];
+        if (!(cj > bd)) {
+          float y[DIMP];
+          mst_load<DIMP>(tree.xs, j, y);
+          mr = fmaxf(fmaxf(mst_sqd<DIMP>(q, y), cq), cj);
         }
       }
-    }
-    if (sp == 0) break;
-    --sp;
-    v = __shfl_sync(FULL, stk, sp);
-    lbv = mst_box_lb<DIMP>(lo, hi, v, q);
-    if (live) {  // the component's best so far, found by other lanes and warps
-      const uint32_t cb = __ldcg(cbest + qc);
-      if (cb < FMAX_BITS) {
-        const float nb = __uint_as_float(cb + 1u);
-        if (nb < bd) {
-          bd = nb;
-          bj = NO_POINT;
+      const uint32_t mb = __float_as_uint(mr), best = __reduce_min_sync(FULL, mb);
+      if (best < __float_as_uint(bd) || (best == __float_as_uint(bd) && bj != NO_POINT)) {
+        const uint32_t oj = mb == best ? orig[j] : NO_POINT;
+        const uint32_t o = __reduce_min_sync(FULL, oj);
+        if (best < __float_as_uint(bd) || o < bo) {
+          const int src = __ffs(__ballot_sync(FULL, mb == best && oj == o)) - 1;
+          if (lane == 0 && best < __float_as_uint(bd)) atomicMin(cbest + qc, best);
+          bd = __uint_as_float(best);
+          bo = o;
+          bj = (uint32_t)(j - lane + src);
         }
       }
-      live = !(cq > bd);
+      refresh();
     }
-  }
-  if (bj != NO_POINT) {
-    bj_out[pos] = bj;
-    const uint32_t db = __float_as_uint(bd);
-    atomicMin(cbest + qc, db);
-    atomicMin(ckey + qc, ((unsigned long long)db << 32) | orig[pos]);
+    if (lane == 0) {
+      near_j[pos] = bj;
+      near_v[pos] = fmaxf(near_v[pos], bd);  // the value found, or nothing below the last bound
+      if (bj != NO_POINT) {
+        const uint32_t db = __float_as_uint(bd);
+        atomicMin(ckey + qc, ((unsigned long long)db << 32) | orig[pos]);
+      }
+    }
   }
 }
 
@@ -714,46 +998,51 @@ int log2_ceil(int64_t m) {
 }
 
 template <int DIMP>
-void launch_core(int kmax_bucket, const float* xs, int64_t n, int64_t P, int64_t L,
-                 const float* lo, const float* hi, int k, float* core, uint32_t* kj, float* kd,
-                 int32_t* st, cudaStream_t s) {
-  const unsigned g = grid_of((n + 31) / 32, MST_WARPS);
-  switch (kmax_bucket) {
-    case 8: k_mst_core<DIMP, 8><<<g, 32 * MST_WARPS, 0, s>>>(xs, n, P, L, lo, hi, k, core, kj, kd, st); break;
-    case 16: k_mst_core<DIMP, 16><<<g, 32 * MST_WARPS, 0, s>>>(xs, n, P, L, lo, hi, k, core, kj, kd, st); break;
-    case 32: k_mst_core<DIMP, 32><<<g, 32 * MST_WARPS, 0, s>>>(xs, n, P, L, lo, hi, k, core, kj, kd, st); break;
-    default: k_mst_core<DIMP, 64><<<g, 32 * MST_WARPS, 0, s>>>(xs, n, P, L, lo, hi, k, core, kj, kd, st); break;
-  }
-  EVOC_CHECK_LAUNCH();
-}
-
-template <int DIMP>
 int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, int64_t* d_u,
                 int64_t* d_v, float* d_w) {
   cudaStream_t s = ctx->stream;
   int32_t* st = ctx->status.get();
   StageTrace tr(s);
-  // bounding box and Morton order
-  DevBuf<uint32_t> bmin(dim, s), bmax(dim, s);
-  EVOC_CUDA(cudaMemsetAsync(bmin.get(), 0xff, bmin.bytes(), s));
-  EVOC_CUDA(cudaMemsetAsync(bmax.get(), 0, bmax.bytes(), s));
   {
-    const unsigned gx = (unsigned)std::min<int64_t>(grid_of(n), 4 * ctx->num_sms);
-    k_mst_bbox<<<dim3(gx, dim), 256, 0, s>>>(d_data, n, dim, bmin.get(), bmax.get(), st);
+    const unsigned g = (unsigned)std::min<int64_t>(grid_of(n * dim), 4 * ctx->num_sms);
+    k_mst_finite<<<g, 256, 0, s>>>(d_data, n * dim, st);
     EVOC_CHECK_LAUNCH();
   }
   check_status(ctx, "build_mst");  // non-finite coordinates are rejected before any search
-  const int bits = std::min(16, 64 / dim), total_bits = bits * dim;
+  // tree order of the points
+  const int64_t L = (n + MST_LEAF - 1) / MST_LEAF;
+  int64_t P = 1;
+  while (P < L) P <<= 1;
   DevBuf<uint32_t> key(n, s);
   DevBuf<uint2> val(n, s);
-  k_mst_morton<<<grid_of(n), 256, 0, s>>>(d_data, n, dim, bits, bmin.get(), bmax.get(), key.get(),
-                                          val.get());
+  k_mst_iota_pairs<<<grid_of(n), 256, 0, s>>>(val.get(), n);
   EVOC_CHECK_LAUNCH();
-  radix_sort_pairs(ctx, key, val, n, std::min(32, total_bits));
-  if (total_bits > 32) {
-    k_mst_hi_keys<<<grid_of(n), 256, 0, s>>>(val.get(), n, key.get());
-    EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(ctx, key, val, n, total_bits - 32);
+  {
+    int64_t size = P * MST_LEAF;
+    const int64_t max_nodes = (n + 2 * KD_BLOCK - 1) / (2 * KD_BLOCK);
+    DevBuf<uint32_t> box(2 * max_nodes * dim, s);
+    for (; size > KD_BLOCK; size >>= 1) {
+      const int64_t nodes = (n + size - 1) / size;
+      uint32_t *bmin = box.get(), *bmax = box.get() + nodes * dim;
+      EVOC_CUDA(cudaMemsetAsync(bmin, 0xff, nodes * dim * sizeof(uint32_t), s));
+      EVOC_CUDA(cudaMemsetAsync(bmax, 0, nodes * dim * sizeof(uint32_t), s));
+      k_kd_box<<<grid_of((n + KD_RUN - 1) / KD_RUN, 128), 128, 0, s>>>(d_data, n, dim, size,
+                                                                     val.get(), bmin, bmax);
+      EVOC_CHECK_LAUNCH();
+      const int nb = bits_for((uint64_t)(nodes - 1)), bits = std::min(24, 32 - nb);
+      k_kd_key<<<grid_of(n), 256, 0, s>>>(d_data, n, dim, size, bits, val.get(), bmin, bmax,
+                                          key.get());
+      EVOC_CHECK_LAUNCH();
+      radix_sort_pairs(ctx, key, val, n, nb + bits);
+    }
+    if (size >= 2 * MST_LEAF) {
+      EVOC_CUDA(cudaFuncSetAttribute((const void*)k_kd_block,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(KdSmem)));
+      k_kd_block<<<(unsigned)((n + size - 1) / size), KD_THREADS, sizeof(KdSmem), s>>>(
+          d_data, n, dim, (int)size, val.get());
+      EVOC_CHECK_LAUNCH();
+    }
   }
   DevBuf<float> xs(n * DIMP, s);
   DevBuf<uint32_t> orig(n, s), pos_of(n, s);
@@ -762,32 +1051,42 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
   EVOC_CHECK_LAUNCH();
   key.release();
   val.release();
-  tr.mark("morton order");
-  // implicit tree
-  const int64_t L = (n + MST_LEAF - 1) / MST_LEAF;
-  int64_t P = 1;
-  while (P < L) P <<= 1;
+  tr.mark("tree order");
   DevBuf<float> lo(2 * P * DIMP, s), hi(2 * P * DIMP, s);
   k_mst_leaf_boxes<DIMP><<<grid_of(P), 256, 0, s>>>(xs.get(), n, P, L, lo.get(), hi.get());
   EVOC_CHECK_LAUNCH();
-  for (int64_t first = P >> 1; first >= 1; first >>= 1) {
-    k_mst_level_boxes<DIMP><<<grid_of(first), 256, 0, s>>>(lo.get(), hi.get(), first, first);
+  for (int64_t first = P; first > 1; first = std::max<int64_t>(first / UP_NODES, 1)) {
+    k_mst_boxes_up<DIMP><<<grid_of(first, UP_NODES), UP_NODES / 2, 0, s>>>(lo.get(), hi.get(),
+                                                                         first);
     EVOC_CHECK_LAUNCH();
   }
   tr.mark("tree boxes");
   // core distances
+  const MstTree<DIMP> tree{xs.get(), lo.get(), hi.get(), n, P, log2_ceil(P)};
+  auto search_grid = [&](int64_t items) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)mst_blocks<DIMP>() * ctx->num_sms,
+                                                           (items + MST_WARPS - 1) / MST_WARPS));
+  };
+  DevBuf<unsigned long long> work(1, s);  // the searches' next point
+  EVOC_CUDA(cudaMemsetAsync(work.get(), 0, work.bytes(), s));
   DevBuf<float> core(n, s), knn_d(n * (int64_t)k, s);
   DevBuf<uint32_t> knn_j(n * (int64_t)k, s);
+  DevBuf<uint8_t> tie(n, s);
   if (k == 0) {
     EVOC_CUDA(cudaMemsetAsync(core.get(), 0, core.bytes(), s));
   } else {
-    const int kb = k <= 8 ? 8 : k <= 16 ? 16 : k <= 32 ? 32 : 64;
-    launch_core<DIMP>(kb, xs.get(), n, P, L, lo.get(), hi.get(), k, core.get(), knn_j.get(),
-                      knn_d.get(), st, s);
+    auto* kern = k <= 32 ? k_mst_core<DIMP, false> : k_mst_core<DIMP, true>;
+    kern<<<search_grid(n), 32 * MST_WARPS, 0, s>>>(tree, k, work.get(), core.get(), knn_j.get(),
+                                                   knn_d.get(), tie.get());
+    EVOC_CHECK_LAUNCH();
   }
   tr.mark("core distances");
   // Boruvka rounds
-  DevBuf<uint32_t> comp(n, s), nd(2 * P, s), cbest(n, s), bj(n, s), succ(n, s);
+  DevBuf<uint32_t> comp(n, s), maj(2 * P, s), cbest(n, s), near_j(n, s), list(n, s), succ(n, s);
+  DevBuf<float> near_v(n, s), plo(2 * P * DIMP, s), phi(2 * P * DIMP, s), pcore(4 * P, s);
+  DevBuf<int32_t> mcnt(2 * P, s);
+  const MstParts<DIMP> parts{maj.get(), mcnt.get(),  plo.get(),
+                             phi.get(), pcore.get(), pcore.get() + 2 * P};
   DevBuf<unsigned long long> ckey(n, s);
   DevBuf<uint32_t> jA(n, s), jB(n, s), mA(n, s), mB(n, s), oncyc(n, s), nid(n, s), lab(n, s);
   DevBuf<uint32_t> A(n, s), A2(n, s), eu(n, s), ev(n, s), ew(n, s);
@@ -796,28 +1095,36 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
   EVOC_CUDA(cudaMemcpyAsync(comp.get(), orig.get(), comp.bytes(), cudaMemcpyDeviceToDevice, s));
   k_mst_iota<<<grid_of(n), 256, 0, s>>>(A.get(), n);
   EVOC_CHECK_LAUNCH();
+  k_mst_near_init<<<grid_of(n), 256, 0, s>>>(n, k, knn_j.get(), tie.get(), core.get(), orig.get(),
+                                             near_j.get(), near_v.get());
+  EVOC_CHECK_LAUNCH();
   int64_t m = n, len = 0;
   int64_t h_tot[2];
   while (m > 1 && len < n - 1) {
     const unsigned gm = grid_of(m), gn = grid_of(n);
-    k_mst_leaf_comp<<<grid_of(P), 256, 0, s>>>(comp.get(), n, P, L, nd.get());
+    k_mst_leaf_parts<DIMP><<<grid_of(P * 32), 256, 0, s>>>(tree, comp.get(), core.get(), parts);
     EVOC_CHECK_LAUNCH();
-    for (int64_t first = P >> 1; first >= 1; first >>= 1) {
-      k_mst_level_comp<<<grid_of(first), 256, 0, s>>>(nd.get(), first, first);
+    for (int64_t first = P; first > 1; first = std::max<int64_t>(first / UP_NODES, 1)) {
+      k_mst_parts_up<DIMP><<<grid_of(first, UP_NODES), UP_NODES / 2, 0, s>>>(tree, parts, first);
       EVOC_CHECK_LAUNCH();
     }
     k_mst_round_reset<<<gm, 256, 0, s>>>(A.get(), m, cbest.get(), ckey.get());
     EVOC_CHECK_LAUNCH();
-    if (k > 0) {
-      k_mst_knn_bound<<<gn, 256, 0, s>>>(n, k, knn_j.get(), knn_d.get(), comp.get(), core.get(),
-                                         cbest.get());
-      EVOC_CHECK_LAUNCH();
-    }
-    k_mst_noc<DIMP><<<grid_of((n + 31) / 32, MST_WARPS), 32 * MST_WARPS, 0, s>>>(xs.get(), n, P, L, lo.get(), hi.get(),
-                                                     nd.get(), comp.get(), core.get(), orig.get(),
-                                                     cbest.get(), ckey.get(), bj.get(), st);
+    k_mst_bound<DIMP><<<gn, 256, 0, s>>>(xs.get(), n, k, knn_j.get(), knn_d.get(), comp.get(), core.get(),
+                                   near_j.get(), near_v.get(), cbest.get());
     EVOC_CHECK_LAUNCH();
-    k_mst_picks<<<gm, 256, 0, s>>>(A.get(), m, ckey.get(), pos_of.get(), bj.get(), orig.get(),
+    k_mst_select<<<gn, 256, 0, s>>>(n, comp.get(), core.get(), orig.get(), near_j.get(),
+                                    near_v.get(), cbest.get(), ckey.get(), has.get());
+    EVOC_CHECK_LAUNCH();
+    exclusive_scan_i32_to_i64(ctx, has.get(), off.get(), n);
+    k_mst_search_list<<<gn, 256, 0, s>>>(n, has.get(), off.get(), list.get());
+    EVOC_CHECK_LAUNCH();
+    EVOC_CUDA(cudaMemsetAsync(work.get(), 0, work.bytes(), s));
+    k_mst_noc<DIMP><<<search_grid(n), 32 * MST_WARPS, 0, s>>>(
+        tree, parts, comp.get(), core.get(), orig.get(), list.get(), off.get() + n, work.get(),
+        cbest.get(), ckey.get(), near_j.get(), near_v.get());
+    EVOC_CHECK_LAUNCH();
+    k_mst_picks<<<gm, 256, 0, s>>>(A.get(), m, ckey.get(), pos_of.get(), near_j.get(), orig.get(),
                                    comp.get(), succ.get(), eu.get(), ev.get(), ew.get(), has.get());
     EVOC_CHECK_LAUNCH();
     // cycles of the pick graph: 2^K >= m doubling steps
