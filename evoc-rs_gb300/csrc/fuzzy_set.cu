@@ -10,20 +10,18 @@
 // Pipeline (all on the context stream):
 //   k_knn_rowlen     warp per row: row length (first EVOC_KNN_PAD) and index
 //                    validation.
-//   k_smooth_knn     lane per row (a pool of rows per warp, a finished lane
-//                    takes the next): rho and the sigma bisection with the
-//                    rows' distances staged in shared memory. The sum over the
-//                    row is serial in row order, as in the reference
-//                    (fuzzy_graph.rs:72-76), so sigma is bit-identical to a
-//                    serial CPU evaluation.
-//   k_knn_weights    elementwise membership weights (fuzzy_graph.rs:138-145).
-//   k_forward_rows   thread per row: drop self loops, sort by column keeping
+//   k_smooth_knn     lane per row: rho, the sigma bisection (steps whose outcome
+//                    is certain are not evaluated) and the membership weights
+//                    (fuzzy_graph.rs:138-145). An evaluated sum is serial in
+//                    row order, as in the reference (fuzzy_graph.rs:72-76), so
+//                    sigma is bit-identical to a serial CPU evaluation.
+//   k_forward_*      drop self loops, sort by column keeping
 //                    the last of equal columns (HashMap::insert overwrites,
 //                    fuzzy_graph.rs:189), count in-degrees.
 //   radix sort       stable sort of the forward entries by column: each
 //                    column bucket lists its source rows in ascending order,
 //                    which is the backward map of fuzzy_graph.rs:190.
-//   k_union          thread per row: merge the sorted forward and backward
+//   k_union          warp per row: merge the sorted forward and backward
 //                    lists, w = w_ij + w_ji - w_ij * w_ji, keep w > 0
 //                    (fuzzy_graph.rs:196-204); once to count, once to write.
 #include "evoc_device.cuh"
@@ -64,38 +62,50 @@ __global__ void k_knn_rowlen(const uint32_t* __restrict__ idx, int64_t n,
 }
 
 // ---------------------------------------------------------------------------
-// smooth_knn_dist (fuzzy_graph.rs:33-98): rho and the sigma bisection, one
-// row per lane at a time. The sum over the row stays serial in row order, so
-// sigma is bit-identical to a serial CPU evaluation. Rows need different
-// numbers of bisection steps (a handful up to n_iter), so instead of one row
-// per lane for the whole launch, each warp owns a pool of rows staged in
-// shared memory (odd row stride: lanes on different rows hit different banks)
-// and a lane that finishes its row takes the pool's next one at the end of
-// the step; the warp runs about the mean step count of its rows rather than
-// their maximum. The membership weights are a separate elementwise pass.
+// smooth_knn_dist (fuzzy_graph.rs:33-98): rho, the sigma bisection and the
+// membership weights, one row per lane, a warp's rows staged in shared memory (odd
+// row stride: lanes on different rows hit different banks).
+//
+// The bisection's outcome is defined by the f32 sum val(mid) of the row's
+// exponentials, added serially in row order, and by the side of the target it
+// falls on. Most of its steps (27 on average) lie so far from the target that the
+// side is certain, so their sums are never formed. In real arithmetic S(x) = sum
+// exp(-a_j x), x = 1 / mid, is decreasing and convex: Newton's iteration from
+// x = 0 approaches the solution from below, with hardware ex2 (4 instructions per
+// term, against about 45 of an exactly rounded term). Two points on either side of
+// it are then certified: where the approximate sum is further than W from the
+// target, with W = 1e-5 (the bisection's own tolerance) + a bound M on all
+// rounding, val is on that side and not converged, and by monotony so it is for
+// every mid beyond that point. Steps between the two points (about three) are
+// evaluated exactly as written in the reference, so sigma and the step count are
+// bit-identical to a serial evaluation of every step. Rows for which nothing can
+// be certified (no solution, extreme distances) evaluate every step.
+//
+// M, for len terms of at most 1 each: the exact terms are off by at most 1.5e-7
+// (quotient, own exp at 1.2 ulp), the approximate ones by 2.4e-7 (ex2.approx
+// 2^-22.5, argument 3 roundings), either sum by len * sum * 2^-24, the target's
+// rounding by 5e-7. 2M rows of 30: 3.3 ms when every step was
+// evaluated, 0.90 now; it is bound by instruction issue.
 // ---------------------------------------------------------------------------
-constexpr int SK_WARPS = 4;
-
 struct RowState {
-  int32_t row;   // pool slot, or >= pool size when the lane is done
   int32_t len;
   int32_t it;
   float rho, lo, hi, mid;
 };
 
-__device__ __forceinline__ void sk_start_row(RowState& st, const float* __restrict__ d,
-                                             int32_t len, float lc, int32_t* __restrict__ status,
-                                             bool& ok) {
+// Checks a row, takes its rho and replaces its distances by max(0, d - rho).
+__device__ __forceinline__ bool sk_start_row(RowState& st, float* __restrict__ d, int32_t len,
+                                             float lc, int32_t* __restrict__ status) {
   st.len = len;
   st.it = 0;
   st.lo = 0.0f;
   st.hi = 3.40282347e+38f;
   st.mid = 1.0f;
-  ok = true;
+  st.rho = 0.0f;
+  bool ok = true;
   for (int32_t j = 0; j < len; ++j)
     if (d[j] != d[j]) ok = false;
   if (!ok) set_status(status, ST_BAD_VALUE);
-  float rho = 0.0f;
   if (lc > 0.0f) {  // fuzzy_graph.rs:49-62
     if (len <= 0) {
       set_status(status, ST_EMPTY_ROW);
@@ -107,130 +117,257 @@ __device__ __forceinline__ void sk_start_row(RowState& st, const float* __restri
       if (id > len - 1) id = len - 1;
       const float frac = fsub(lm1, fl);
       if (frac > 0.0f && id + 1 < len)
-        rho = fadd(fmul(d[id], fsub(1.0f, frac)), fmul(d[id + 1], frac));
+        st.rho = fadd(fmul(d[id], fsub(1.0f, frac)), fmul(d[id + 1], frac));
       else
-        rho = d[id];
+        st.rho = d[id];
     }
   }
-  st.rho = rho;
+  for (int32_t j = 0; j < len; ++j) d[j] = max0(fsub(d[j], st.rho));
+  return ok;
 }
 
-__global__ void __launch_bounds__(32 * SK_WARPS) k_smooth_knn(
-    const float* __restrict__ dist, const int32_t* __restrict__ row_len, int64_t n, int32_t k,
-    int32_t kp, int32_t pool, double target, float lc, int32_t n_iter,
-    float* __restrict__ sigma_out, float* __restrict__ rho_out, int32_t* __restrict__ status,
-    unsigned long long* __restrict__ steps) {
+__device__ __forceinline__ float sk_ex2(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Certified sides of the target: above for mid >= *up, below for mid <= *down
+// (infinity and 0 where nothing is certified).
+__device__ __forceinline__ void sk_certify(const float* __restrict__ a, int32_t len, double target,
+                                           bool on, float* up, float* down) {
+  const float INF = __int_as_float(0x7f800000);
+  constexpr float LOG2E = 1.44269504f;
+  const float t = (float)target, flen = (float)len;
+  const float w = 1.05e-5f + 5e-7f + flen * (4e-7f + 1.2e-7f * (fabsf(t) + 1.0f));
+  float sum = 0.0f;
+  int32_t zeros = 0;
+  for (int32_t j = 0; j < len; ++j) {
+    sum += a[j];
+    zeros += a[j] == 0.0f;
+  }
+  *up = INF;
+  *down = 0.0f;
+  if (on && (float)zeros - t > w) {  // the zeros alone exceed the target at every mid
+    *up = 0.0f;
+    on = false;
+  }
+  if (on && t - flen > w) {  // every term at 1 does not reach it
+    *down = INF;
+    on = false;
+  }
+  float x = (flen - t) / sum, g = 0.0f;
+  on = on && x > 1e-30f && x < 1e30f;
+  bool solved = false;
+  for (int it = 0; it < 16; ++it) {
+    if (!__any_sync(0xffffffffu, on && !solved)) break;
+    if (on && !solved) {
+      const float c = -x * LOG2E;
+      float s = 0.0f, d = 0.0f;
+#pragma unroll 4
+      for (int32_t j = 0; j < len; ++j) {
+        const float e = sk_ex2(a[j] * c);
+        s += e;
+        d = fmaf(a[j], e, d);
+      }
+      g = x * d;
+      const float r = s - t;
+      if (fabsf(r) <= 0.25f * w)
+        solved = true;
+      else
+        x += r / d;
+      on = x > 1e-30f && x < 1e30f;  // also not NaN
+    }
+  }
+  const float del = 1.5f * w / g;
+  if (on && solved && del < 0.3f) {
+    const float xl = x * (1.0f - del), xh = x * (1.0f + del);
+    const float cl = -xl * LOG2E, ch = -xh * LOG2E;
+    float sl = 0.0f, sh = 0.0f;
+#pragma unroll 4
+    for (int32_t j = 0; j < len; ++j) {
+      sl += sk_ex2(a[j] * cl);
+      sh += sk_ex2(a[j] * ch);
+    }
+    if (sl - t > w) *up = 1.000001f / xl;
+    if (t - sh > w) *down = 0.999999f / xh;
+  }
+}
+
+__global__ void k_smooth_knn(const float* __restrict__ dist, const int32_t* __restrict__ row_len,
+                             int64_t n, int32_t k, int32_t kp, double target, float lc,
+                             int32_t n_iter, float* __restrict__ sigma_out,
+                             float* __restrict__ rho_out, float* __restrict__ w_out,
+                             int32_t* __restrict__ status, unsigned long long* __restrict__ steps) {
   extern __shared__ float sm[];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  float* sd = sm + (size_t)wid * pool * kp;
-  const int64_t row0 = ((int64_t)blockIdx.x * SK_WARPS + wid) * pool;
+  float* sd = sm + (size_t)wid * 32 * kp;
+  const int64_t row0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + wid) * 32;
   if (row0 >= n) return;  // whole warp
-  const int rows = (int)min((int64_t)pool, n - row0);
+  const int rows = (int)min((int64_t)32, n - row0);
+  const uint32_t elems = (uint32_t)rows * (uint32_t)k;
   {
     const float* src = dist + row0 * (int64_t)k;
-    const int64_t elems = (int64_t)rows * k;
-    for (int64_t e = lane; e < elems; e += 32) {
-      const int64_t r = e / k;
+    for (uint32_t e = lane; e < elems; e += 32) {
+      const uint32_t r = e / (uint32_t)k;
       sd[r * kp + (e - r * k)] = src[e];
     }
   }
   __syncwarp();
-  const uint32_t lt = (1u << lane) - 1u;
-  RowState st;
-  bool ok = false;
-  st.row = lane;
-  int next = 32;  // the pool's next unstarted row (warp-uniform)
-  uint32_t nsteps = 0;  // row sums evaluated by this lane
-  if (st.row < rows) {
-    sk_start_row(st, sd + st.row * kp, row_len ? row_len[row0 + st.row] : k, lc, status, ok);
+  float* a = sd + lane * kp;
+  const int64_t row = row0 + lane;
+  RowState st{};
+  bool live = lane < rows, ok = false;
+  if (live) ok = sk_start_row(st, a, row_len ? row_len[row] : k, lc, status);
+  if (live && !ok) {
+    st.mid = 0.0f;
+    st.rho = 0.0f;
+    live = false;
   }
-  for (;;) {
-    const bool active = st.row < rows;
-    if (__ballot_sync(FULL, active) == 0) break;
-    bool done = false;
-    if (active) {
-      if (!ok) {
-        st.mid = 0.0f;
-        st.rho = 0.0f;
-        done = true;
-      } else if (st.it >= n_iter) {
-        done = true;
-      } else {  // one bisection step, fuzzy_graph.rs:71-93
-        const float* d = sd + st.row * kp;
-        ++nsteps;
-        float val = 0.0f;
-        for (int32_t j = 0; j < st.len; ++j) {
-          const float adjusted = max0(fsub(d[j], st.rho));
-          val = fadd(val, evoc_expf(-fdiv(adjusted, st.mid)));
-        }
-        const double vd = (double)val;
-        if (fabs(vd - target) < 1e-5) {
-          done = true;
+  float up, down;
+  sk_certify(a, live ? st.len : 0, target, live, &up, &down);
+  uint32_t nsteps = 0;  // bisection steps of this lane's row
+  while (__any_sync(FULL, live)) {
+    // steps whose side is certain, then one exact evaluation (fuzzy_graph.rs:71-93)
+    bool above = false;
+    while (live) {
+      if (st.it >= n_iter) {
+        live = false;
+        break;
+      }
+      const bool in_range = st.mid > 1e-30f && st.mid < 1e30f;
+      above = in_range && st.mid >= up;
+      if (!above && !(in_range && st.mid <= down)) break;
+      ++nsteps;
+      if (above) {
+        st.hi = st.mid;
+        st.mid = fdiv(fadd(st.lo, st.hi), 2.0f);
+      } else {
+        st.lo = st.mid;
+        st.mid = st.hi == 3.40282347e+38f ? fmul(st.mid, 2.0f) : fdiv(fadd(st.lo, st.hi), 2.0f);
+      }
+      ++st.it;
+    }
+    __syncwarp();
+    if (live) {
+      ++nsteps;
+      float val = 0.0f;
+#pragma unroll 2
+      for (int32_t j = 0; j < st.len; ++j) val = fadd(val, evoc_expf(-fdiv(a[j], st.mid)));
+      const double vd = (double)val;
+      if (fabs(vd - target) < 1e-5) {
+        live = false;
+      } else {
+        if (vd > target) {
+          st.hi = st.mid;
+          st.mid = fdiv(fadd(st.lo, st.hi), 2.0f);
         } else {
-          if (vd > target) {
-            st.hi = st.mid;
-            st.mid = fdiv(fadd(st.lo, st.hi), 2.0f);
-          } else {
-            st.lo = st.mid;
-            if (st.hi == 3.40282347e+38f)
-              st.mid = fmul(st.mid, 2.0f);
-            else
-              st.mid = fdiv(fadd(st.lo, st.hi), 2.0f);
-          }
-          ++st.it;
+          st.lo = st.mid;
+          st.mid = st.hi == 3.40282347e+38f ? fmul(st.mid, 2.0f) : fdiv(fadd(st.lo, st.hi), 2.0f);
         }
-      }
-      if (done) {
-        sigma_out[row0 + st.row] = st.mid;
-        rho_out[row0 + st.row] = st.rho;
+        ++st.it;
       }
     }
-    // lanes whose row is done take the pool's next rows, in lane order
-    const uint32_t need = __ballot_sync(FULL, done);
-    if (done) {
-      st.row = next + __popc(need & lt);
-      if (st.row < rows)
-        sk_start_row(st, sd + st.row * kp, row_len ? row_len[row0 + st.row] : k, lc, status, ok);
-    }
-    next += __popc(need);
+  }
+  if (lane < rows) {
+    sigma_out[row] = st.mid;
+    rho_out[row] = st.rho;
   }
   const unsigned tot = __reduce_add_sync(FULL, nsteps);
   if (lane == 0 && tot) atomicAdd(steps, (unsigned long long)tot);
-}
-
-// knn_to_coo's membership weights (fuzzy_graph.rs:138-145), elementwise:
-// w = exp(-max(0, d - rho) / sigma), or 0 / 1 when sigma <= 0.
-__global__ void k_knn_weights(const float* __restrict__ dist, const int32_t* __restrict__ row_len,
-                              int64_t n, int32_t k, const float* __restrict__ sigma,
-                              const float* __restrict__ rho, float* __restrict__ w) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n * (int64_t)k) return;
-  const int64_t i = e / k;
-  const int32_t j = (int32_t)(e - i * k);
-  const int32_t len = row_len ? row_len[i] : k;
-  float out = 0.0f;
-  if (j < len) {
-    const float mid = sigma[i];
-    const float adjusted = max0(fsub(dist[e], rho[i]));
-    if (mid > 0.0f)
-      out = evoc_expf(-fdiv(adjusted, mid));
-    else
-      out = (adjusted > 0.0f) ? 0.0f : 1.0f;
+  if (!w_out) return;
+  // knn_to_coo's membership weights (fuzzy_graph.rs:138-145): w = exp(-max(0, d -
+  // rho) / sigma), or 0 / 1 when sigma <= 0 (and 0 past the row's end; a rejected
+  // row's are never read)
+  __syncwarp();
+  for (uint32_t e0 = 0; e0 < elems; e0 += 32) {
+    const uint32_t e = e0 + lane;
+    const int r = (int)min(e / (uint32_t)k, 31u);
+    const int32_t j = (int32_t)(e - (uint32_t)r * k);
+    const float mid = __shfl_sync(FULL, st.mid, r);
+    const int32_t len = __shfl_sync(FULL, st.len, r);
+    if (e < elems) {
+      float out = 0.0f;
+      if (j < len) {
+        const float adjusted = sd[r * kp + j];
+        out = mid > 0.0f ? evoc_expf(-fdiv(adjusted, mid)) : (adjusted > 0.0f ? 0.0f : 1.0f);
+      }
+      w_out[row0 * (int64_t)k + e] = out;
+    }
   }
-  w[e] = out;
 }
 
 // ---------------------------------------------------------------------------
-// Forward lists: drop self loops, stable insertion sort by column, keep the
-// last entry of each column, count in-degrees. Rows stay padded to k.
+// Forward lists: drop self loops, sort by column (stable), keep the last entry
+// of each column, count in-degrees. Rows stay padded to k. The lists leave twice:
+// as (fcol, fw) for the union, and as (column, (row, weight)) pairs, PAD past a
+// row's end, which the stable sort by column turns into the backward lists.
+// Rows of up to 32: G lanes per row sort (column, position) in registers, 2M rows
+// of 30 in 0.63 ms (the insertion sort 0.98, and 0.4 for the pairs). Longer rows: a
+// thread per row, insertion sort in shared memory.
 // ---------------------------------------------------------------------------
+template <int G>
+__global__ void __launch_bounds__(256) k_forward_short(
+    const uint32_t* __restrict__ idx, const float* __restrict__ w,
+    const int32_t* __restrict__ row_len, int64_t n, int32_t k, uint32_t* __restrict__ fcol,
+    float* __restrict__ fw, uint32_t* __restrict__ keys, uint2* __restrict__ vals,
+    int32_t* __restrict__ fcnt, int32_t* __restrict__ indeg) {
+  const unsigned FULL = 0xffffffffu;
+  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const int lane = threadIdx.x & 31, sub = threadIdx.x & (G - 1);
+  const bool valid = row < n;
+  const int32_t len = valid ? row_len[row] : 0;
+  const int64_t at = row * (int64_t)k + sub;
+  uint32_t c = PAD, pos = sub;
+  float wv = 0.0f;
+  if (sub < len) {
+    c = idx[at];
+    wv = w[at];
+    if ((int64_t)c == row) c = PAD;  // self loop (fuzzy_graph.rs:135)
+  }
+#pragma unroll
+  for (int size = 2; size <= G; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride >= 1; stride >>= 1) {
+      const uint32_t oc = __shfl_xor_sync(FULL, c, stride), op = __shfl_xor_sync(FULL, pos, stride);
+      const bool low = ((sub & size) == 0) == ((sub & stride) == 0);
+      const bool less = oc < c || (oc == c && op < pos);
+      if (low == less) {
+        c = oc;
+        pos = op;
+      }
+    }
+  wv = __shfl_sync(FULL, wv, (int)pos, G);
+  const uint32_t next = __shfl_down_sync(FULL, c, 1, G);
+  const bool keep = c != PAD && (sub == G - 1 || next != c);  // the last of equal columns
+  uint32_t kept = __ballot_sync(FULL, keep);
+  if (G < 32) kept = (kept >> (lane & ~(G - 1))) & ((1u << (G & 31)) - 1u);
+  const int cnt = __popc(kept);
+  if (!valid) return;
+  if (keep) {
+    const int64_t o = row * (int64_t)k + __popc(kept & ((1u << sub) - 1u));
+    fcol[o] = c;
+    fw[o] = wv;
+    keys[o] = c;
+    vals[o] = make_uint2((uint32_t)row, __float_as_uint(wv));
+    atomicAdd(&indeg[c], 1);
+  }
+  if (sub >= cnt && sub < k) {
+    keys[at] = PAD;
+    vals[at] = make_uint2(0u, 0u);
+  }
+  if (sub == 0) fcnt[row] = cnt;
+}
+
 __global__ void k_forward_rows(const uint32_t* __restrict__ idx,
                                const float* __restrict__ w,
                                const int32_t* __restrict__ row_len, int64_t n,
                                int32_t k, int32_t kp,
                                uint32_t* __restrict__ fcol,
                                float* __restrict__ fw,
+                               uint32_t* __restrict__ keys,
+                               uint2* __restrict__ vals,
                                int32_t* __restrict__ fcnt,
                                int32_t* __restrict__ indeg) {
   extern __shared__ uint32_t smu[];
@@ -284,26 +421,11 @@ __global__ void k_forward_rows(const uint32_t* __restrict__ idx,
   __syncthreads();
   for (int64_t e = threadIdx.x; e < elems; e += R) {
     const int64_t r = e / k, j = e - r * k;
-    fcol[row0 * (int64_t)k + e] = sc[r * kp + j];
-    fw[row0 * (int64_t)k + e] = sw[r * kp + j];
-  }
-}
-
-// Compact the padded forward lists into (column key, (row, weight)) pairs in
-// row-major order: the input of the stable transpose.
-__global__ void k_forward_compact(const uint32_t* __restrict__ fcol,
-                                  const float* __restrict__ fw,
-                                  const int64_t* __restrict__ fptr, int64_t n,
-                                  int32_t k, uint32_t* __restrict__ keys,
-                                  uint2* __restrict__ vals) {
-  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const int64_t o = fptr[row];
-  const int32_t cnt = (int32_t)(fptr[row + 1] - o);
-  for (int32_t j = lane; j < cnt; j += 32) {
-    keys[o + j] = fcol[row * (int64_t)k + j];
-    vals[o + j] = make_uint2((uint32_t)row, __float_as_uint(fw[row * (int64_t)k + j]));
+    const int64_t o = row0 * (int64_t)k + e;
+    fcol[o] = sc[r * kp + j];
+    fw[o] = sw[r * kp + j];
+    keys[o] = sc[r * kp + j];
+    vals[o] = make_uint2((uint32_t)(row0 + r), __float_as_uint(sw[r * kp + j]));
   }
 }
 
@@ -464,27 +586,23 @@ void smooth_knn_device(evoc_ctx* ctx, const float* d_dist,
                        float* d_weights_out, const uint32_t* /*unused*/) {
   if (n == 0) return;
   const int32_t kp = k | 1;
-  // rows per warp: 64 where they fit in 48 KB per block, else one per lane
-  int pool = 64;
-  while (pool > 32 && (size_t)SK_WARPS * pool * kp * sizeof(float) > 48 * 1024) pool /= 2;
-  const size_t smem = (size_t)SK_WARPS * pool * kp * sizeof(float);
-  if (smem > 200 * 1024)
+  // four warps per block, one where that leaves SMs idle or the rows are long
+  int warps = 4;
+  while (warps > 1 && (n < (int64_t)64 * warps * ctx->num_sms ||
+                       (size_t)warps * 32 * kp * sizeof(float) > 200 * 1024))
+    warps /= 2;
+  const size_t smem = (size_t)warps * 32 * kp * sizeof(float);
+  if ((size_t)4 * 32 * kp * sizeof(float) > 200 * 1024)
     throw Error(EVOC_ERR_UNSUPPORTED, "k too large (k <= 399 supported)");
   set_smem_limit((const void*)k_smooth_knn, smem);
   const double target = std::log2((double)k_target);
-  const int64_t per_block = (int64_t)SK_WARPS * pool;
+  const int64_t per_block = (int64_t)warps * 32;
   const int64_t blocks = (n + per_block - 1) / per_block;
   EVOC_CUDA(cudaMemsetAsync(ctx->sk_steps.get(), 0, sizeof(unsigned long long), ctx->stream));
-  k_smooth_knn<<<(unsigned)blocks, 32 * SK_WARPS, smem, ctx->stream>>>(
-      d_dist, d_row_len, n, k, kp, pool, target, local_connectivity, n_iter, d_sigma, d_rho,
-      ctx->status.get(), ctx->sk_steps.get());
+  k_smooth_knn<<<(unsigned)blocks, 32 * warps, smem, ctx->stream>>>(
+      d_dist, d_row_len, n, k, kp, target, local_connectivity, n_iter, d_sigma, d_rho,
+      d_weights_out, ctx->status.get(), ctx->sk_steps.get());
   EVOC_CHECK_LAUNCH();
-  if (d_weights_out) {
-    const int64_t elems = n * (int64_t)k;
-    k_knn_weights<<<(unsigned)((elems + 255) / 256), 256, 0, ctx->stream>>>(
-        d_dist, d_row_len, n, k, d_sigma, d_rho, d_weights_out);
-    EVOC_CHECK_LAUNCH();
-  }
 }
 
 void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
@@ -506,7 +624,6 @@ void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
         d_idx, n, k, row_len.get(), ctx->status.get());
     EVOC_CHECK_LAUNCH();
   }
-  check_status(ctx, "fuzzy set");
   trace.mark("row lengths");
 
   // k = effective_n_neighbors.to_usize().unwrap_or(knn_dists[0].len())
@@ -562,52 +679,43 @@ void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
     return;
   }
 
-  // forward lists
-  const int32_t kp = k | 1;
-  int R = rows_per_block(kp);
-  const size_t smem = (size_t)R * kp * 8;
-  if (smem > 200 * 1024)
-    throw Error(EVOC_ERR_UNSUPPORTED, "k too large (k <= 1599 supported)");
-  set_smem_limit((const void*)k_forward_rows, smem);
-  DevBuf<uint32_t> fcol(n * (int64_t)k, s);
-  DevBuf<float> fw(n * (int64_t)k, s);
+  // forward lists, and their pairs for the transpose
+  const int64_t nk = n * (int64_t)k;
+  DevBuf<uint32_t> fcol(nk, s), keys(nk, s);
+  DevBuf<float> fw(nk, s);
+  DevBuf<uint2> vals(nk, s);
   DevBuf<int32_t> fcnt(n, s), indeg(n, s);
   EVOC_CUDA(cudaMemsetAsync(indeg.get(), 0, n * sizeof(int32_t), s));
-  k_forward_rows<<<(unsigned)((n + R - 1) / R), R, smem, s>>>(
-      d_idx, wts.get(), row_len.get(), n, k, kp, fcol.get(), fw.get(),
-      fcnt.get(), indeg.get());
+  if (k <= 32) {
+    auto* kern = k <= 16 ? k_forward_short<16> : k_forward_short<32>;
+    const int64_t threads = n * (k <= 16 ? 16 : 32);
+    kern<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+        d_idx, wts.get(), row_len.get(), n, k, fcol.get(), fw.get(), keys.get(), vals.get(),
+        fcnt.get(), indeg.get());
+  } else {
+    const int32_t kp = k | 1;
+    int R = rows_per_block(kp);
+    const size_t smem = (size_t)R * kp * 8;
+    if (smem > 200 * 1024)
+      throw Error(EVOC_ERR_UNSUPPORTED, "k too large (k <= 1599 supported)");
+    set_smem_limit((const void*)k_forward_rows, smem);
+    k_forward_rows<<<(unsigned)((n + R - 1) / R), R, smem, s>>>(
+        d_idx, wts.get(), row_len.get(), n, k, kp, fcol.get(), fw.get(), keys.get(), vals.get(),
+        fcnt.get(), indeg.get());
+  }
   EVOC_CHECK_LAUNCH();
   wts.release();
   trace.mark("forward rows");
 
-  DevBuf<int64_t> fptr(n + 1, s), bptr(n + 1, s);
-  exclusive_scan_i32_to_i64(ctx, fcnt.get(), fptr.get(), n);
+  // stable transpose: the pairs by column (PAD, above every column, last)
+  DevBuf<int64_t> bptr(n + 1, s);
   exclusive_scan_i32_to_i64(ctx, indeg.get(), bptr.get(), n);
-  int64_t nf = 0;
-  EVOC_CUDA(cudaMemcpyAsync(&nf, fptr.get() + n, sizeof(int64_t),
-                            cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaStreamSynchronize(s));
-
-  // stable transpose: sort forward entries by column
-  DevBuf<uint32_t> keys(nf, s);
-  DevBuf<uint2> vals(nf, s);
-  if (nf > 0) {
-    const int64_t threads = n * 32;
-    k_forward_compact<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
-        fcol.get(), fw.get(), fptr.get(), n, k, keys.get(), vals.get());
-    EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(ctx, keys, vals, nf, bits_for((uint64_t)(n - 1)));
-  }
+  radix_sort_pairs(ctx, keys, vals, nk, bits_for((uint64_t)n));
   keys.release();
-  fptr.release();
   trace.mark("transpose");
 
   DevBuf<int32_t> ucnt(n, s);
-  int64_t nb_total = 0;
-  EVOC_CUDA(cudaMemcpyAsync(&nb_total, bptr.get() + n, sizeof(int64_t),
-                            cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaStreamSynchronize(s));
-  DevBuf<uint2> utmp(n * (int64_t)k + nb_total, s);
+  DevBuf<uint2> utmp(2 * nk, s);  // at most k entries each way per row
   k_union<<<(unsigned)((n * 32 + 255) / 256), 256, 0, s>>>(
       fcol.get(), fw.get(), fcnt.get(), bptr.get(), vals.get(), n, k, ucnt.get(), utmp.get());
   EVOC_CHECK_LAUNCH();
