@@ -3,33 +3,23 @@
 // Replaces evoc_embedding, src/graph/embedding.rs:48-298 (evoc-rs 0.2.7).
 //
 // Set-up (once per plan, embedding.rs:78-175):
-//   k_row_counts   warp per row: upper (i < j) and lower entries per row.
-//   k_edge_fill    warp per row: undirected edge list in adjacency order
-//                  (eidx = rank among upper entries, embedding.rs:79-90) and
-//                  the per-problem maximum weight (embedding.rs:99).
-//   k_edge_ps      thread per edge: epochs_per_sample (embedding.rs:101-111).
-//   radix sort     (general graphs only) edges by larger endpoint, stable, to
-//                  list each node's "is_smaller = false" incidences in edge
-//                  order (embedding.rs:130-135).
-//   k_inc_fill     warp per node: the per-node incidence list of
-//                  embedding.rs:121-135 (lower part in edge order, then the
-//                  node's own upper entries).
-//   k_schedule     thread per incidence entry: runs the epochs-per-sample
-//                  recurrence of embedding.rs:274-286 for every epoch and
-//                  stores, per epoch, one bit "fires" and P bits "negative
-//                  count" (embedding.rs:225-228) for each entry. Both copies of
-//                  an edge evaluate the same f32 recurrence, so they agree.
+//   k_row_counts   warp per row: upper (i < j) and lower entries per row, and the
+//                  per-problem maximum weight (embedding.rs:99).
+//   A canonical graph's rows are its nodes' incidence lists (embedding.rs:121-135:
+//   the lower part in edge order, then the node's own upper entries). Of a general
+//   graph they are built: edge list (k_edge_fill, eidx = rank among upper entries,
+//   embedding.rs:79-90), epochs_per_sample (k_edge_ps), a stable radix sort of
+//   the edges by larger endpoint, and k_inc_fill.
+//   k_tile_masks   the epochs-per-sample recurrence of embedding.rs:274-286 for
+//                  every entry, as bit words per epoch: who fires, and the
+//                  negative counts (embedding.rs:225-228). Both copies of an
+//                  edge evaluate the same f32 recurrence, so they agree.
+//   k_tile_fill    the gradient slots of every epoch and tile from them.
+//   (k_sched_count and k_sched_fill beyond the masks' range; k_schedule_* and bit
+//   planes for k_epoch when the slots would not fit.)
 // Epoch loop (embedding.rs:178-292), one launch per epoch, captured in a CUDA
-// graph:
-//   k_epoch        G lanes per node (pull-based): the node's fire words are
-//                  read G at a time and its fired entries compacted (prefix
-//                  sum + __fns), so each lane takes a fired entry, gathers the
-//                  partner row (float4) and the Philox negatives, and adds into
-//                  partial sum (fired rank mod 32) in shared memory; the 32
-//                  partials are combined by a pairwise tree (strides 16..1);
-//                  the lane that owns a dimension applies Adam
-//                  (embedding.rs:256-272) and writes the next embedding buffer
-//                  (ping-pong). No float atomics; results do not depend on G.
+// graph, or one cooperative launch for all: k_epoch_slot (k_epoch on bit planes).
+// No float atomics; results do not depend on the launch shape.
 #include "evoc_device.cuh"
 #include "evoc_internal.h"
 
@@ -86,10 +76,13 @@ struct evoc_plan {
   float one_m_b1 = 0, one_m_b2 = 0;
   std::vector<evoc_epoch_stats_t> stats;
   // per-epoch gradient slots (the fast path): for epoch t and tile T, slots
-  // [tile_off[t * ntiles + T], tile_off[t * ntiles + T + 1]); a slot is
-  // (source row, tile-local node | 32 for a negative sample)
+  // [tile_off[T * n_epochs + t], tile_off[T * n_epochs + t + 1]); a slot is
+  // (source row, tile-local node | 32 for a negative sample). A tile's epochs are
+  // adjacent, so that the fill pass, which writes them all at once, stays within
+  // one page of the address translation
   bool use_slots = false;
   int64_t ntiles = 0;
+  int32_t tile_nodes = 32;            // nodes per tile
   int64_t n_slots = 0;
   evoc::DevBuf<int64_t> tile_off;
   evoc::DevBuf<uint32_t> tile_order;  // tiles by descending slot count (launch order)
@@ -123,25 +116,39 @@ __device__ __forceinline__ uint32_t prob_of(const uint32_t* pon, uint32_t v) {
 // ---------------------------------------------------------------------------
 // Set-up kernels
 // ---------------------------------------------------------------------------
+// Upper and lower entries per row; with weights (canonical graphs) also each
+// problem's largest weight.
 __global__ void k_row_counts(const int64_t* __restrict__ indptr,
-                             const uint32_t* __restrict__ indices, int64_t n,
+                             const uint32_t* __restrict__ indices,
+                             const float* __restrict__ weights, int64_t n,
+                             const uint32_t* __restrict__ prob_of_node,
                              int32_t* __restrict__ ucnt,
-                             int32_t* __restrict__ lcnt_own) {
+                             int32_t* __restrict__ lcnt_own,
+                             int32_t* __restrict__ max_w_bits) {
   const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= n) return;
   const int64_t a = indptr[r], b = indptr[r + 1];
-  int32_t u = 0, l = 0;
+  int32_t u = 0, l = 0, mx = 0;
   for (int64_t p = a + lane; p < b; p += 32) {
     const uint32_t c = indices[p];
     u += (int64_t)c > r;
     l += (int64_t)c < r;
+    if (weights) {
+      const float w = weights[p];
+      if (w == w) mx = max(mx, __float_as_int(w));  // f32::max ignores NaN
+    }
   }
   u = __reduce_add_sync(0xffffffffu, (unsigned)u);
   l = __reduce_add_sync(0xffffffffu, (unsigned)l);
+  mx = __reduce_max_sync(0xffffffffu, mx);
   if (lane == 0) {
     ucnt[r] = u;
     lcnt_own[r] = l;
+    if (mx > 0) {
+      int32_t* dst = &max_w_bits[prob_of(prob_of_node, (uint32_t)r)];
+      if (mx > *(volatile int32_t*)dst) atomicMax(dst, mx);
+    }
   }
 }
 
@@ -216,12 +223,9 @@ __global__ void k_inc_fill(const int64_t* __restrict__ indptr,
                            const int64_t* __restrict__ inc_ptr,
                            const uint32_t* __restrict__ prob_of_node,
                            const int32_t* __restrict__ max_w_bits,
-                           const int64_t* __restrict__ ebase,
                            uint32_t* __restrict__ inc_other,
                            float* __restrict__ inc_ps,
-                           uint8_t* __restrict__ inc_up,
-                           int64_t* __restrict__ eidx_base,
-                           uint32_t* __restrict__ inc_eidx) {
+                           uint8_t* __restrict__ inc_up) {
   const int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (v >= n) return;
@@ -244,7 +248,6 @@ __global__ void k_inc_fill(const int64_t* __restrict__ indptr,
         inc_other[q] = c;
         inc_ps[q] = ps_from_w(weights[p], mw);
         inc_up[q] = 0;
-        inc_eidx[q] = 0xffffffffu;  // lower entries draw no negatives
       }
       o += __popc(bal);
     }
@@ -255,7 +258,6 @@ __global__ void k_inc_fill(const int64_t* __restrict__ indptr,
       inc_other[p0 + j] = pe.y;
       inc_ps[p0 + j] = e_ps[pe.x];
       inc_up[p0 + j] = 0;
-      inc_eidx[p0 + j] = 0xffffffffu;  // lower entries draw no negatives
     }
   }
   int64_t o = p0 + nl;
@@ -268,11 +270,19 @@ __global__ void k_inc_fill(const int64_t* __restrict__ indptr,
       inc_other[q] = indices[p];
       inc_ps[q] = ps_from_w(weights[p], mw);
       inc_up[q] = 1;
-      inc_eidx[q] = (uint32_t)(uptr[v] + (q - (p0 + nl)));
     }
     o += __popc(bal);
   }
-  if (lane == 0) eidx_base[v] = (uptr[v] - ebase[pr]) - (p0 + nl);
+}
+
+// Edge id of upper entry p of node v, within its problem: p + eidx_base[v].
+__global__ void k_eidx_base(const int64_t* __restrict__ inc_ptr, const int64_t* __restrict__ uptr,
+                            const int32_t* __restrict__ lcnt, int64_t n,
+                            const uint32_t* __restrict__ prob_of_node,
+                            const int64_t* __restrict__ ebase, int64_t* __restrict__ eidx_base) {
+  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < n)
+    eidx_base[v] = (uptr[v] - ebase[prob_of(prob_of_node, (uint32_t)v)]) - (inc_ptr[v] + lcnt[v]);
 }
 
 // Epochs-per-sample recurrence of one incidence entry (embedding.rs:274-286)
@@ -464,29 +474,108 @@ struct EpochArgs {
   float* grad_out;
   const uint32_t* prob_of_node;
   const ProbInfo* prob;
-  const int64_t* tile_off;     // slot offsets of this epoch (slots path)
+  const int64_t* tile_off;     // this epoch's first slot offset; a tile's is n_epochs apart
   const uint32_t* tile_order;  // slots path: tiles in launch order, heaviest first
   const uint32_t* slots;
   unsigned long long* work_ctr;  // slots path: next tile of this epoch (zeroed per launch)
   uint32_t n_total;
   uint32_t epoch;
+  int32_t n_epochs;
+  int32_t tn;      // slots path: nodes per tile
+  int64_t ntiles;  // slots path
   uint64_t seed;
   float noise, gamma, lr_ad, epsc, one_m_b1, one_m_b2;
 };
 
+// Eight floats in one 256-bit access (sm_100 and later). A warp's rows lie in 32
+// different places, and the load unit takes one of them per cycle and instruction:
+// a 32-byte row in two 128-bit loads costs twice the cycles of one 256-bit load.
+__device__ __forceinline__ void ldg8(const float* p, float* r) {  // read-only data
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]),
+        "=f"(r[7])
+      : "l"(p));
+}
+__device__ __forceinline__ void ldcg8(const float* p, float* r) {  // through L2
+  asm volatile("ld.global.cg.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]),
+                 "=f"(r[6]), "=f"(r[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void ldcs8(const float* p, float* r) {  // streamed
+  asm volatile("ld.global.cs.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]),
+                 "=f"(r[6]), "=f"(r[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void stcs8(float* p, const float* r) {
+  asm volatile("st.global.cs.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(r[0]),
+               "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "l"(p)
+               : "memory");
+}
+
+// A row of DIMP floats (DIMP a multiple of 8: 32-byte aligned, else 16).
 // COH: the row may have been written earlier in the same launch (the
 // persistent all-epochs kernel), so it is read through L2 (ld.global.cg)
 // rather than the non-coherent read-only path.
 template <int DIMP, bool COH = false>
 __device__ __forceinline__ void load_row(const float* __restrict__ p, float (&r)[DIMP]) {
-  const float4* p4 = reinterpret_cast<const float4*>(p);
+  if constexpr (DIMP % 8 == 0) {
 #pragma unroll
-  for (int i = 0; i < DIMP / 4; ++i) {
-    const float4 x = COH ? __ldcg(p4 + i) : __ldg(p4 + i);
-    r[4 * i + 0] = x.x;
-    r[4 * i + 1] = x.y;
-    r[4 * i + 2] = x.z;
-    r[4 * i + 3] = x.w;
+    for (int i = 0; i < DIMP; i += 8) {
+      if constexpr (COH)
+        ldcg8(p + i, r + i);
+      else
+        ldg8(p + i, r + i);
+    }
+  } else {
+    const float4* p4 = reinterpret_cast<const float4*>(p);
+#pragma unroll
+    for (int i = 0; i < DIMP / 4; ++i) {
+      const float4 x = COH ? __ldcg(p4 + i) : __ldg(p4 + i);
+      r[4 * i + 0] = x.x;
+      r[4 * i + 1] = x.y;
+      r[4 * i + 2] = x.z;
+      r[4 * i + 3] = x.w;
+    }
+  }
+}
+
+// An Adam moment row, streamed (through L2 with COH), and a row's streamed store.
+template <int DIMP, bool COH>
+__device__ __forceinline__ void load_moment(const float* p, float (&r)[DIMP]) {
+  if constexpr (DIMP % 8 == 0) {
+#pragma unroll
+    for (int i = 0; i < DIMP; i += 8) {
+      if constexpr (COH)
+        ldcg8(p + i, r + i);
+      else
+        ldcs8(p + i, r + i);
+    }
+  } else {
+    const float4* p4 = reinterpret_cast<const float4*>(p);
+#pragma unroll
+    for (int i = 0; i < DIMP / 4; ++i) {
+      const float4 x = COH ? __ldcg(p4 + i) : __ldcs(p4 + i);
+      r[4 * i + 0] = x.x;
+      r[4 * i + 1] = x.y;
+      r[4 * i + 2] = x.z;
+      r[4 * i + 3] = x.w;
+    }
+  }
+}
+template <int DIMP>
+__device__ __forceinline__ void store_row(float* p, const float (&r)[DIMP]) {
+  if constexpr (DIMP % 8 == 0) {
+#pragma unroll
+    for (int i = 0; i < DIMP; i += 8) stcs8(p + i, r + i);
+  } else {
+    float4* p4 = reinterpret_cast<float4*>(p);
+#pragma unroll
+    for (int i = 0; i < DIMP / 4; ++i)
+      __stcs(p4 + i, make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]));
   }
 }
 
@@ -763,60 +852,12 @@ __global__ void __launch_bounds__(128) k_epoch(EpochArgs a) {
 // Fast path: per-epoch gradient slots.
 //
 // The epochs-per-sample schedule and the negative draws do not depend on the
-// embedding, so the set-up lists, for every epoch and every 32-node tile, the
+// embedding, so the set-up lists, for every epoch and every tile of 4 to 32 nodes, the
 // terms of the reference's gradient sums in their order: one slot (source
 // row, tile-local node | 32 for a negative) per fired incidence entry and per
 // negative sample it draws. The epoch kernel streams its tile's slots instead
 // of scanning fire bits.
 // ---------------------------------------------------------------------------
-// Per-edge schedule (n_epochs <= 64): thread per undirected edge runs the
-// recurrence once (embedding.rs:274-286) and stores the epochs in which the
-// edge fires as a bit mask, and its negative count per epoch as two bit
-// planes (bit 0 and bit 1 of the count; counts above 3 are caught through
-// max_neg, and the per-entry path is used then). Both incidence copies of the
-// edge take their fire pattern from here.
-__global__ void k_edge_sched(const float* __restrict__ e_ps, int64_t U, int32_t ne,
-                             float neg_factor, unsigned long long* __restrict__ fire_mask,
-                             unsigned long long* __restrict__ neg_lo,
-                             unsigned long long* __restrict__ neg_hi,
-                             unsigned long long* __restrict__ max_neg) {
-  const unsigned FULL = 0xffffffffu;
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = e < U;
-  const float ps = valid ? e_ps[e] : 3.0e38f;
-  const float pn = fmul(ps, neg_factor);
-  float ns = ps, nn = pn, mx = 0.0f;
-  uint32_t fm[2] = {0u, 0u}, n0[2] = {0u, 0u}, n1[2] = {0u, 0u};  // epochs 0-31, 32-63
-  // the same recurrence as Sched::stepf, with the count kept in float and its
-  // two low bits taken by comparisons (count 3 stands for 3 or more)
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int32_t t_end = min(ne, 32 * (h + 1));
-    float tf = (float)(32 * h);
-    uint32_t bit = 1u;
-    for (int32_t t = 32 * h; t < t_end; ++t, tf = fadd(tf, 1.0f), bit <<= 1) {
-      if (!(ns > tf)) fm[h] |= bit;  // fires (also for a NaN schedule, which never updates)
-      if (ns <= tf) {
-        ns = fadd(ns, ps);
-        const float x = floorf(fdiv(fsub(tf, nn), pn));
-        const float c = (x > 0.0f && x < 18446744073709551616.0f) ? x : 0.0f;
-        nn = fadd(nn, fmul(c, pn));
-        if (c == 1.0f || c >= 3.0f) n0[h] |= bit;
-        if (c >= 2.0f) n1[h] |= bit;
-        mx = fmaxf(mx, c);
-      }
-    }
-  }
-  if (valid) {
-    fire_mask[e] = ((unsigned long long)fm[1] << 32) | fm[0];
-    neg_lo[e] = ((unsigned long long)n0[1] << 32) | n0[0];
-    neg_hi[e] = ((unsigned long long)n1[1] << 32) | n1[0];
-  }
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
-  if ((threadIdx.x & 31) == 0 && mx > 0.0f)
-    atomicMax(max_neg, mx >= 1.8446744e19f ? ~0ull : (unsigned long long)mx);
-}
-
 // 32 x 32 bit transpose across a warp: lane l passes row word x (bit c =
 // element (l, c)); lane c receives column c (bit l = element (l, c)), which
 // is __ballot_sync of bit c. Five butterfly stages swap off-diagonal blocks.
@@ -834,153 +875,241 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
   return x;
 }
 
-// Fire and negative-count bit planes in incidence order (n_epochs <= 64).
-// F[t * W + w] bit l = entry 32 w + l fires in epoch t; N0 / N1 hold bits 0 /
-// 1 of its negative count (upper entries only). Block of 8 warps per 32 words:
-// each warp takes the masks of 4 words and transposes them (lane t receives
-// epoch t and t + 32); the words are staged in shared memory and every plane
-// row leaves as one 128-byte line. Upper entries read their edge's masks
-// (consecutive edges); a lower entry's fire mask is the same recurrence run
-// on its own epochs-per-sample, which equals its upper twin's (both copies of
-// an edge carry the same value).
-constexpr int PLANE_BLOCK_WORDS = 32;
-__global__ void __launch_bounds__(256) k_inc_planes(
-    const uint32_t* __restrict__ inc_eidx, const uint8_t* __restrict__ inc_up,
-    const float* __restrict__ inc_ps, int64_t n_inc,
-    int64_t W, int32_t ne, const unsigned long long* __restrict__ edge_fire,
-    const unsigned long long* __restrict__ edge_neg_lo,
-    const unsigned long long* __restrict__ edge_neg_hi, uint32_t* __restrict__ fplane,
-    uint32_t* __restrict__ nplane0, uint32_t* __restrict__ nplane1) {
-  __shared__ uint32_t sbuf[3][64][PLANE_BLOCK_WORDS + 1];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t w0 = (int64_t)blockIdx.x * PLANE_BLOCK_WORDS;
-  constexpr int J = PLANE_BLOCK_WORDS / 8;
-  uint32_t e[J];
-  bool up[J], ok[J];
-  float ps[J];
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    const int64_t p = ((w0 + wid * J + j) << 5) + lane;
-    ok[j] = p < n_inc;
-    up[j] = ok[j] && inc_up[p];
-    e[j] = up[j] ? inc_eidx[p] : 0u;
-    ps[j] = (ok[j] && !up[j]) ? inc_ps[p] : 3.0e38f;
-  }
-  unsigned long long fm[J], g0[J], g1[J];
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    fm[j] = up[j] ? edge_fire[e[j]] : 0ull;
-    g0[j] = up[j] ? edge_neg_lo[e[j]] : 0ull;
-    g1[j] = up[j] ? edge_neg_hi[e[j]] : 0ull;
-  }
-#pragma unroll
-  for (int j = 0; j < J; ++j) {  // lower entries: fires only (embedding.rs:274-279)
-    if (ok[j] && !up[j]) {
-      float ns = ps[j];
-      uint32_t m[2] = {0u, 0u};
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int32_t t_end = min(ne, 32 * (h + 1));
-        for (int32_t t = 32 * h; t < t_end; ++t) {
-          const float tf = (float)t;
-          m[h] |= (!(ns > tf) ? 1u : 0u) << (t - 32 * h);
-          if (ns <= tf) ns = fadd(ns, ps[j]);
-        }
-      }
-      fm[j] = ((unsigned long long)m[1] << 32) | m[0];
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    const int col = wid * J + j;
-    sbuf[0][lane][col] = warp_transpose32((uint32_t)fm[j], lane);
-    sbuf[0][lane + 32][col] = warp_transpose32((uint32_t)(fm[j] >> 32), lane);
-    sbuf[1][lane][col] = warp_transpose32((uint32_t)g0[j], lane);
-    sbuf[1][lane + 32][col] = warp_transpose32((uint32_t)(g0[j] >> 32), lane);
-    sbuf[2][lane][col] = warp_transpose32((uint32_t)g1[j], lane);
-    sbuf[2][lane + 32][col] = warp_transpose32((uint32_t)(g1[j] >> 32), lane);
-  }
-  __syncthreads();
-  const int64_t w = w0 + lane;
-  if (w >= W) return;
-  for (int r = wid; r < 3 * ne; r += 8) {
-    const int kind = r / ne, t = r - kind * ne;
-    uint32_t* dst = kind == 0 ? fplane : kind == 1 ? nplane0 : nplane1;
-    dst[(int64_t)t * W + w] = sbuf[kind][t][lane];
-  }
+// The schedule of planes (MASK_EPOCHS epochs, counts of MASK_NEGS) covers the
+// default 50 epochs and one negative per edge and any moderate multiple of them;
+// beyond, an entry's recurrence runs in the count pass and again in the fill pass.
+constexpr int MASK_EPOCHS = 128;
+constexpr uint64_t MASK_NEGS = 15;
+
+// The incidence lists the schedule reads: node v's entries [ptr[v], ptr[v + 1]),
+// the lower part (other < v) first, each part in edge order. val is the edge
+// weight (raw: epochs-per-sample is formed from it and the problem's largest
+// weight) or the epochs-per-sample itself. A canonical graph's CSR is such a list.
+struct IncView {
+  const int64_t* ptr;
+  const uint32_t* other;
+  const float* val;
+  bool raw;
+  const int32_t* max_w_bits;
+  const uint32_t* prob_of_node;
+  int64_t n, ntiles;
+  int32_t tn;  // nodes per tile
+  int32_t ne;
+  float neg_factor;
+};
+
+__global__ void k_tile_words(const int64_t* __restrict__ ptr, int64_t n, int64_t ntiles,
+                             int32_t tn, int32_t* __restrict__ words) {
+  const int64_t tile = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (tile >= ntiles) return;
+  const int64_t len = ptr[min((tile + 1) * tn, n)] - ptr[tile * tn];
+  words[tile] = (int32_t)((len + 31) >> 5);
 }
 
-// Words [wb, we) of a tile's entries [P0, P1) with the bits outside masked.
-__device__ __forceinline__ uint32_t tile_word(const uint32_t* __restrict__ plane, int64_t w,
-                                              int64_t wb, int64_t we, uint32_t lo_mask,
-                                              uint32_t hi_mask) {
-  if (w >= we) return 0u;
-  uint32_t x = plane[w];
-  if (w == wb) x &= lo_mask;
-  if (w == we - 1) x &= hi_mask;
-  return x;
-}
+// Schedule of a tile's entries (embedding.rs:274-286): which epochs each fires in
+// and, for upper entries, its negative count there (embedding.rs:225-228), as bit
+// words in tile order. A word covers 32 entries, a chunk of a tile at most
+// MASK_CHUNK entries (nw words); plane 0 holds who fires, plane 1 + b bit b of the
+// count. Word w of plane b and epoch t of the chunk that starts at word w0 of all is
+// planes[w0 * (1 + NB) * ne + (b * ne + t) * nw + w]: the fill pass reads an epoch's
+// words of a chunk in one line. Per epoch and tile the slots (fired entries and
+// their negatives) are counted on the way.
+//
+// An entry's recurrence only changes when it fires (8 of 50 epochs on average,
+// but 49 for the strongest edges), so a lane steps from fire to fire, and the
+// entries in hand are first grouped by kind and by about how often they fire, so
+// that the lanes of a warp run out of epochs together. Stepping all entries
+// through all epochs took 2.95 ms for the edges of the 2M graph alone, and their
+// planes, twin recurrences, lists and counts 7 ms more (3.7 ms here, bound by
+// instruction issue). The masks are turned from entry-major to epoch-major by a
+// 32 x 32 bit transpose. NW 32-epoch words, NB count bits; counts above
+// 2^NB - 1 are caught through max_neg by the host.
+constexpr int MASK_THREADS = 128;
+constexpr int MASK_CHUNK = 1024;  // entries in hand
+constexpr int MASK_BINS = 32;     // of firing frequency, for lower and for upper entries
+template <int NW, int NB>
+struct MaskSmem {
+  uint32_t mask[1 + NB][NW][MASK_CHUNK];
+  float ps[MASK_CHUNK];        // negative for upper entries
+  uint16_t list[MASK_CHUNK];   // entries by bin, the most frequent upper ones first
+  int64_t pb[TILE + 1];
+  float mw[TILE];
+  int32_t fires[32 * NW], negs[32 * NW];
+  int32_t bin[2 * MASK_BINS];
+};
 
-// Count pass from the planes: warp per tile; slots per epoch = fired entries
-// + their negatives (N0 + 2 N1), written to counts[t * ntiles + tile]. The
-// loads of 8 epochs are issued together (the pass is latency-bound), and the
-// per-epoch totals of fired entries and negatives (fired[t], negs[t]) are
-// summed in shared memory by the block's 8 warps before one global atomic each.
-constexpr int COUNT_EU = 8;
-__global__ void __launch_bounds__(256) k_plane_count(
-    const int64_t* __restrict__ inc_ptr, int64_t n, int64_t ntiles, int64_t W, int32_t ne,
-    const uint32_t* __restrict__ fplane, const uint32_t* __restrict__ nplane0,
-    const uint32_t* __restrict__ nplane1, int32_t* __restrict__ counts,
-    unsigned long long* __restrict__ fired, unsigned long long* __restrict__ negs) {
-  __shared__ unsigned long long sfired[64], snegs[64];
+template <int NW, int NB>
+__global__ void __launch_bounds__(MASK_THREADS) k_tile_masks(
+    IncView a, const int64_t* __restrict__ wbase, uint32_t* __restrict__ planes,
+    int32_t* __restrict__ counts, int32_t* __restrict__ fires,
+    unsigned long long* __restrict__ max_neg) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  MaskSmem<NW, NB>& sm = *reinterpret_cast<MaskSmem<NW, NB>*>(smem_raw);
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < 64; i += blockDim.x) sfired[i] = snegs[i] = 0ull;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t tile = blockIdx.x, v0 = tile * a.tn;
+  const int nt = (int)min((int64_t)a.tn, a.n - v0);
+  const float fne = (float)a.ne;
+  if (threadIdx.x <= TILE) sm.pb[threadIdx.x] = a.ptr[v0 + min((int)threadIdx.x, nt)];
+  if (threadIdx.x < TILE && (int)threadIdx.x < nt && a.raw)
+    sm.mw[threadIdx.x] =
+        __int_as_float(a.max_w_bits[prob_of(a.prob_of_node, (uint32_t)(v0 + threadIdx.x))]);
+  for (int t = threadIdx.x; t < 32 * NW; t += MASK_THREADS) sm.fires[t] = sm.negs[t] = 0;
   __syncthreads();
-  const int64_t tile = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (tile < ntiles) {
-    const int64_t v0 = tile * TILE;
-    const int nt = (int)min((int64_t)TILE, n - v0);
-    const int64_t P0 = inc_ptr[v0], P1 = inc_ptr[v0 + nt];
-    const int64_t wb = P0 >> 5, we = P1 > P0 ? ((P1 - 1) >> 5) + 1 : wb;
-    const uint32_t lo_mask = ~0u << (P0 & 31);
-    const uint32_t hi_mask = ~0u >> (31 - (int)((P1 - 1) & 31));
-    for (int32_t t0 = 0; t0 < ne; t0 += COUNT_EU) {
-      int cf[COUNT_EU], cn[COUNT_EU];
+  const int64_t P0 = sm.pb[0], P1 = sm.pb[nt];
+  float mx = 0.0f;
+  for (int64_t c0 = P0; c0 < P1; c0 += MASK_CHUNK) {
+    const int m = (int)min((int64_t)MASK_CHUNK, P1 - c0), m32 = (m + 31) & ~31;
+    if (threadIdx.x < 2 * MASK_BINS) sm.bin[threadIdx.x] = 0;
+    __syncthreads();
+    int where[MASK_CHUNK / MASK_THREADS];  // bin | rank in it << 8
 #pragma unroll
-      for (int u = 0; u < COUNT_EU; ++u) cf[u] = cn[u] = 0;
-      for (int64_t w = wb + lane; w < we; w += 32) {
-        uint32_t x[COUNT_EU], y0[COUNT_EU], y1[COUNT_EU];
+    for (int r = 0; r < MASK_CHUNK / MASK_THREADS; ++r) {
+      const int e = r * MASK_THREADS + threadIdx.x;
+      where[r] = -1;
+      if (e < m) {
+        const int64_t p = c0 + e;
+        int node = 0;
 #pragma unroll
-        for (int u = 0; u < COUNT_EU; ++u) {
-          const int64_t po = (int64_t)min(t0 + u, ne - 1) * W;
-          x[u] = tile_word(fplane + po, w, wb, we, lo_mask, hi_mask);
-          y0[u] = tile_word(nplane0 + po, w, wb, we, lo_mask, hi_mask);
-          y1[u] = tile_word(nplane1 + po, w, wb, we, lo_mask, hi_mask);
-        }
+        for (int step = 16; step >= 1; step >>= 1)
+          if (node + step < nt && sm.pb[node + step] <= p) node += step;
+        const float x = a.val[p], ps = a.raw ? ps_from_w(x, sm.mw[node]) : x;
+        const bool up = (int64_t)a.other[p] > v0 + node;
+        sm.ps[e] = up ? -ps : ps;
+        // about (MASK_BINS - 1) / ps, the share of epochs it fires in; bins in falling order
+        const int often = min(MASK_BINS - 1, (int)__fdividef((float)(MASK_BINS - 1), ps));
+        const int b = (up ? 0 : MASK_BINS) + MASK_BINS - 1 - often;
+        where[r] = b | (atomicAdd(&sm.bin[b], 1) << 8);
+      } else if (e < m32) {  // past the end: no epoch
 #pragma unroll
-        for (int u = 0; u < COUNT_EU; ++u) {
-          cf[u] += __popc(x[u]);
-          cn[u] += __popc(y0[u]) + 2 * __popc(y1[u]);
+        for (int b = 0; b < 1 + NB; ++b)
+#pragma unroll
+          for (int w = 0; w < NW; ++w) sm.mask[b][w][e] = 0u;
+      }
+    }
+    __syncthreads();
+    if (wid == 0) {  // exclusive prefix of the 64 bins, two per lane
+      const int b0 = sm.bin[2 * lane], b1 = sm.bin[2 * lane + 1];
+      int incl = b0 + b1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+      }
+      sm.bin[2 * lane] = incl - b0 - b1;
+      sm.bin[2 * lane + 1] = incl - b1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < MASK_CHUNK / MASK_THREADS; ++r)
+      if (where[r] >= 0)
+        sm.list[sm.bin[where[r] & 255] + (where[r] >> 8)] = (uint16_t)(r * MASK_THREADS + threadIdx.x);
+    __syncthreads();
+    for (int g = wid; 32 * g < m; g += MASK_THREADS / 32) {
+      const bool on = 32 * g + lane < m;
+      const int e = on ? sm.list[32 * g + lane] : 0;
+      const float x = on ? sm.ps[e] : 3.0e38f;
+      const bool up = __float_as_int(x) < 0;
+      const float ps = fabsf(x), pn = fmul(ps, a.neg_factor);
+      float ns = ps, nn = pn;
+      uint32_t cur[1 + NB][NW];
+#pragma unroll
+      for (int b = 0; b < 1 + NB; ++b)
+#pragma unroll
+        for (int w = 0; w < NW; ++w) cur[b][w] = 0u;
+      // epochs that fire: the smallest t >= 0 with !(ns > t), then the smallest above the
+      // last one (a NaN schedule fires in every epoch and never updates)
+      for (float tf = fmaxf(ceilf(ns), 0.0f); tf < fne; tf = fmaxf(ceilf(ns), tf + 1.0f)) {
+        const int t = (int)tf;
+        const uint32_t bit = 1u << (t & 31);
+#pragma unroll
+        for (int w = 0; w < NW; ++w) cur[0][w] |= (t >> 5) == w ? bit : 0u;
+        if (ns <= tf) {
+          ns = fadd(ns, ps);
+          if (up) {
+            const float q = floorf(fdiv(fsub(tf, nn), pn));
+            const float c = (q > 0.0f && q < 18446744073709551616.0f) ? q : 0.0f;
+            nn = fadd(nn, fmul(c, pn));
+            mx = fmaxf(mx, c);
+            const uint32_t ci = (uint32_t)fminf(c, 255.0f);
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+              const uint32_t wb = (t >> 5) == w ? bit : 0u;
+#pragma unroll
+              for (int b = 0; b < NB; ++b) cur[1 + b][w] |= (ci >> b) & 1u ? wb : 0u;
+            }
+          }
         }
       }
+      if (on) {
 #pragma unroll
-      for (int u = 0; u < COUNT_EU; ++u) {
-        const int32_t t = t0 + u;
-        const int f = __reduce_add_sync(FULL, cf[u]), g = __reduce_add_sync(FULL, cn[u]);
-        if (lane == 0 && t < ne) {
-          counts[(int64_t)t * ntiles + tile] = f + g;
-          if (f) atomicAdd_block(&sfired[t], (unsigned long long)f);
-          if (g) atomicAdd_block(&snegs[t], (unsigned long long)g);
+        for (int b = 0; b < 1 + NB; ++b)
+#pragma unroll
+          for (int w = 0; w < NW; ++w) sm.mask[b][w][e] = cur[b][w];
+      }
+    }
+    __syncthreads();
+    // entry-major words to epoch-major ones, in place (word w's epoch l at 32 w + (l ^ w):
+    // the rows that leave below then come from 32 banks), and their counts
+    int32_t cf[NW], cn[NW];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) cf[w] = cn[w] = 0;
+    const int nw = m32 >> 5;
+    for (int word = wid; word < nw; word += MASK_THREADS / 32) {
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+#pragma unroll
+        for (int b = 0; b < 1 + NB; ++b) {
+          uint32_t x = sm.mask[b][w][32 * word + lane];
+          if (b < 2 || __any_sync(FULL, x != 0u)) x = warp_transpose32(x, lane);  // counts above 1 are rare
+          __syncwarp();  // the word is read
+          sm.mask[b][w][32 * word + (lane ^ word)] = x;
+          if (b == 0)
+            cf[w] += __popc(x);
+          else
+            cn[w] += __popc(x) << (b - 1);
         }
       }
     }
+    __syncthreads();
+    uint32_t* dst = planes + (wbase[tile] + ((c0 - P0) >> 5)) * (1 + NB) * a.ne;
+#pragma unroll
+    for (int b = 0; b < 1 + NB; ++b)
+      for (int t = wid; t < a.ne; t += MASK_THREADS / 32)
+        if (lane < nw)
+          dst[(b * a.ne + t) * nw + lane] = sm.mask[b][t >> 5][32 * lane + ((t & 31) ^ lane)];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if (cf[w]) atomicAdd(&sm.fires[32 * w + lane], cf[w]);
+      if (cn[w]) atomicAdd(&sm.negs[32 * w + lane], cn[w]);
+    }
+    __syncthreads();  // before the next chunk's masks
   }
-  __syncthreads();
-  for (int t = threadIdx.x; t < ne; t += blockDim.x) {
-    if (sfired[t]) atomicAdd(&fired[t], sfired[t]);
-    if (snegs[t]) atomicAdd(&negs[t], snegs[t]);
+  for (int t = threadIdx.x; t < a.ne; t += MASK_THREADS) {
+    counts[tile * a.ne + t] = sm.fires[t] + sm.negs[t];
+    fires[tile * a.ne + t] = sm.fires[t];
   }
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
+  if (lane == 0 && mx > 0.0f) {
+    const unsigned long long x = mx >= 1.8446744e19f ? ~0ull : (unsigned long long)mx;
+    if (x > *(volatile unsigned long long*)max_neg) atomicMax(max_neg, x);
+  }
+}
+
+// Per-epoch totals fired[t] and negs[t]: thread per epoch, blocks over the tiles.
+__global__ void k_epoch_totals(const int32_t* __restrict__ counts,
+                               const int32_t* __restrict__ fires, int64_t ntiles, int32_t ne,
+                               unsigned long long* __restrict__ fired,
+                               unsigned long long* __restrict__ negs) {
+  const int32_t t = threadIdx.x;
+  if (t >= ne) return;
+  unsigned long long f = 0, c = 0;
+  for (int64_t i = blockIdx.x; i < ntiles; i += gridDim.x) {
+    f += (unsigned)fires[i * ne + t];
+    c += (unsigned)counts[i * ne + t];
+  }
+  if (f) atomicAdd(&fired[t], f);
+  if (c > f) atomicAdd(&negs[t], c - f);
 }
 
 // Position of the r-th (from 0) set bit of m; some lane index for r >= popc(m).
@@ -997,35 +1126,6 @@ __device__ __forceinline__ int nth_set_bit(uint32_t m, int r) {
   }
   return pos;
 }
-
-// Fill pass from the planes, block per (tile, FILL_EPB epochs). The block
-// stages the tile's partner ids and each entry's tile-local node in shared
-// memory (FILL_SEG entries at a time, coalesced); warp w then writes the
-// slots of epoch FILL_EPB * g + w. Per 32-word window of fire bits, lane l
-// takes word l: its slot count (fired entries + their negatives) and its
-// negative-draw count are prefix-summed over the lanes, and the lane walks its
-// word's fired entries in order, storing each attraction slot at its place and
-// queueing its negatives (slot position, edge, draw index) in shared memory.
-// The queue is then drawn (Philox) 32 at a time by the whole warp. A window
-// with more draws than the queue holds draws them inline instead (the same
-// draws at the same places). Every (epoch, tile) segment holds the terms in
-// the order of the reference's serial sum: entries in incidence order, each
-// attraction followed by its negatives.
-constexpr int FILL_EPB = 8;
-constexpr int FILL_SEG = 4096;
-constexpr int FILL_Q = 128;  // queued draws per warp and window
-struct FillJob {
-  int64_t q;        // slot index
-  uint32_t eidx;    // edge id
-  uint32_t jn;      // draw index j | tile-local node << 8
-};
-struct PlaneFillSmem {
-  uint32_t part[FILL_SEG];           // partner of each staged entry
-  uint8_t node[FILL_SEG];            // tile-local node of each staged entry
-  int64_t pb[TILE + 1];              // incidence offsets of the tile's nodes
-  int64_t eb[TILE];                  // edge-id bases of the tile's nodes
-  FillJob job[FILL_EPB][FILL_Q];     // per-warp draw queues
-};
 
 // A gradient slot is one word: (source row << 6) | (1 << 5 for a negative
 // sample) | tile-local node. Plans with 2^26 or more nodes take the scan path.
@@ -1050,97 +1150,135 @@ __device__ __forceinline__ uint32_t negative_slot(uint64_t seed, uint32_t j, int
   return make_slot(nb + negative_draw(sd, j, (uint32_t)t, eidx, np), node | 32u);
 }
 
-__global__ void __launch_bounds__(32 * FILL_EPB) k_plane_fill(
-    const int64_t* __restrict__ inc_ptr, const uint32_t* __restrict__ inc_other,
-    const int64_t* __restrict__ eidx_base, int64_t n, int64_t ntiles, int64_t W, int32_t ne,
-    const uint32_t* __restrict__ fplane, const uint32_t* __restrict__ nplane0,
-    const uint32_t* __restrict__ nplane1, const int64_t* __restrict__ tile_off,
-    const uint32_t* __restrict__ prob_of_node, const ProbInfo* __restrict__ prob,
-    uint64_t seed, uint32_t* __restrict__ slots) {
-  __shared__ PlaneFillSmem sm;
+// Fill pass, block per tile (heaviest first), the epochs dealt to its warps. Per
+// chunk the entries' slot words are staged in shared memory once for all epochs.
+// Per epoch lane l lists the fired entries of word l (its place by a prefix sum);
+// then every lane takes one listed entry, writes its attraction slot (32 entries
+// lie in a few neighbouring sectors) and queues its negatives (slot position, edge,
+// draw index), which are drawn (Philox) by full warps, 32 at a time. Every (epoch,
+// tile) segment holds the terms in the order of the reference's serial sum: entries
+// in incidence order, each attraction followed by its negatives. Two other forms
+// at 2M points (1.29 G slots): lane per fire word writing as it walks, 8 epochs to a
+// block, 7.3 ms; lane per epoch with shuffled slot words, 9.2 ms (each of its
+// stores went to 32 sectors, one per cycle and SM); this one 4.9 ms, bound by
+// instruction issue, the draws being a third of it.
+constexpr int FILL_WARPS = 8;
+struct FillJob {
+  int64_t q;       // slot index
+  uint32_t eidx;   // edge id
+  uint32_t jnt;    // draw index | tile-local node << 8 | epoch << 16
+};
+struct FillSmem {
+  uint32_t slot[MASK_CHUNK];               // slot word of each entry of the chunk
+  uint16_t list[FILL_WARPS][MASK_CHUNK];   // fired entries of a warp's epoch
+  FillJob job[FILL_WARPS][64];
+  int64_t pb[TILE + 1];
+  int64_t eb[TILE];
+  int64_t cur[MASK_EPOCHS];                // next slot of each epoch
+};
+
+template <int NB>
+__global__ void __launch_bounds__(32 * FILL_WARPS, 6) k_tile_fill(
+    IncView a, const int64_t* __restrict__ wbase, const uint32_t* __restrict__ planes,
+    const uint32_t* __restrict__ tile_order, const int64_t* __restrict__ tile_off,
+    const int64_t* __restrict__ eidx_base, const ProbInfo* __restrict__ prob, uint64_t seed,
+    uint32_t* __restrict__ slots) {
+  __shared__ FillSmem sm;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int ngroups = (ne + FILL_EPB - 1) / FILL_EPB;
-  const int64_t tile = blockIdx.x / ngroups;
-  const int32_t t = (int32_t)(blockIdx.x % ngroups) * FILL_EPB + wid;
-  const int64_t v0 = tile * TILE;
-  const int nt = (int)min((int64_t)TILE, n - v0);
-  if (threadIdx.x <= TILE) sm.pb[threadIdx.x] = inc_ptr[v0 + min((int)threadIdx.x, nt)];
-  if (threadIdx.x < TILE) sm.eb[threadIdx.x] = (int)threadIdx.x < nt ? eidx_base[v0 + threadIdx.x] : 0;
+  const uint32_t lt = (1u << lane) - 1u;
+  const int64_t tile = tile_order[blockIdx.x], v0 = tile * a.tn;
+  const int nt = (int)min((int64_t)a.tn, a.n - v0);
+  if (threadIdx.x <= TILE) sm.pb[threadIdx.x] = a.ptr[v0 + min((int)threadIdx.x, nt)];
+  if (threadIdx.x < TILE)
+    sm.eb[threadIdx.x] = (int)threadIdx.x < nt ? eidx_base[v0 + threadIdx.x] : 0;
+  for (int t = threadIdx.x; t < a.ne; t += 32 * FILL_WARPS) sm.cur[t] = tile_off[tile * a.ne + t];
   __syncthreads();
   const int64_t P0 = sm.pb[0], P1 = sm.pb[nt];
-  if (P1 <= P0) return;  // the whole block: no entries
-  const bool active = t < ne;
-  int64_t cur = active ? tile_off[(int64_t)t * ntiles + tile] : 0;
-  const int64_t po = (int64_t)t * W;
   FillJob* job = sm.job[wid];
-  for (int64_t sb = P0; sb < P1; sb += FILL_SEG) {
-    const int64_t se = min(sb + (int64_t)FILL_SEG, P1);
-    __syncthreads();  // the previous segment's readers are done
-    for (int64_t p = sb + threadIdx.x; p < se; p += blockDim.x) {
-      sm.part[p - sb] = inc_other[p];
-      int l = 0;  // last node l < nt with pb[l] <= p (empty rows are skipped)
+  uint16_t* list = sm.list[wid];
+  int queued = 0;
+  auto draw = [&](int cnt) {  // the first cnt jobs; the rest move down
+    __syncwarp();
+    if (lane < cnt) {
+      const FillJob jb = job[lane];
+      slots[jb.q] = negative_slot(seed, jb.jnt & 0xffu, (int32_t)(jb.jnt >> 16), jb.eidx,
+                                  (jb.jnt >> 8) & 31u, v0, (uint32_t)a.n, a.prob_of_node, prob);
+    }
+    __syncwarp();
+    queued -= cnt;
+    if (lane < queued) job[lane] = job[cnt + lane];
+    __syncwarp();
+  };
+  for (int64_t c0 = P0; c0 < P1; c0 += MASK_CHUNK) {
+    const int m = (int)min((int64_t)MASK_CHUNK, P1 - c0), nw = (m + 31) >> 5;
+    __syncthreads();  // the previous chunk's readers are done
+    for (int e = threadIdx.x; e < m; e += 32 * FILL_WARPS) {
+      const int64_t p = c0 + e;
+      int node = 0;
 #pragma unroll
       for (int step = 16; step >= 1; step >>= 1)
-        if (l + step < nt && sm.pb[l + step] <= p) l += step;
-      sm.node[p - sb] = (uint8_t)l;
+        if (node + step < nt && sm.pb[node + step] <= p) node += step;
+      sm.slot[e] = make_slot(a.other[p], (uint32_t)node);
     }
     __syncthreads();
-    if (!active) continue;
-    const int64_t wb = sb >> 5, we = ((se - 1) >> 5) + 1;
-    const uint32_t lo_mask = ~0u << (sb & 31);
-    const uint32_t hi_mask = ~0u >> (31 - (int)((se - 1) & 31));
-    for (int64_t ws = wb; ws < we; ws += 32) {
-      const int64_t w = ws + lane;
-      uint32_t f = tile_word(fplane + po, w, wb, we, lo_mask, hi_mask);
-      // negative bits are set only on fired entries: masking by f keeps the segment's
-      const uint32_t g0 = f ? nplane0[po + w] & f : 0u, g1 = f ? nplane1[po + w] & f : 0u;
-      const int nneg = __popc(g0) + 2 * __popc(g1);
-      int sincl = __popc(f) + nneg, jincl = nneg;  // inclusive prefix sums over lanes
+    const uint32_t* src = planes + (wbase[tile] + ((c0 - P0) >> 5)) * (1 + NB) * a.ne;
+    for (int t = wid; t < a.ne; t += FILL_WARPS) {
+      uint32_t f = lane < nw ? src[t * nw + lane] : 0u, g[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) g[b] = lane < nw ? src[((1 + b) * a.ne + t) * nw + lane] : 0u;
+      const int fired = __popc(f);
+      int incl = fired;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(FULL, sincl, o), z = __shfl_up_sync(FULL, jincl, o);
-        if (lane >= o) {
-          sincl += y;
-          jincl += z;
-        }
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
       }
-      const int stot = __shfl_sync(FULL, sincl, 31), jtot = __shfl_sync(FULL, jincl, 31);
-      if (stot == 0) continue;
-      const bool queued = jtot <= FILL_Q;
-      int64_t q = cur + sincl - (__popc(f) + nneg);
-      int jq = jincl - nneg;
-      __syncwarp();  // the previous window's drain has read its jobs
-      while (f) {
-        const int b = __ffs(f) - 1;
-        f &= f - 1;
-        const int64_t p = (w << 5) + b;
-        const int li = (int)(p - sb);
-        const uint32_t node = sm.node[li];
-        slots[q++] = make_slot(sm.part[li], node);
-        const uint32_t nn = ((g0 >> b) & 1u) | (((g1 >> b) & 1u) << 1);
-        if (nn) {
-          const uint32_t eidx = (uint32_t)(p + sm.eb[node]);
-          for (uint32_t j = 0; j < nn; ++j, ++q) {
-            if (queued)
-              job[jq++] = FillJob{q, eidx, j | (node << 8)};
-            else
-              slots[q] = negative_slot(seed, j, t, eidx, node, v0, (uint32_t)n, prob_of_node, prob);
+      const int tot = __shfl_sync(FULL, incl, 31);
+      if (tot == 0) continue;
+      __syncwarp();  // the previous epoch's list is read
+      for (uint16_t* dst = list + incl - fired; f; f &= f - 1)
+        *dst++ = (uint16_t)(32 * lane + __ffs(f) - 1);
+      __syncwarp();
+      int64_t cur = sm.cur[t];
+      for (int r0 = 0; r0 < tot; r0 += 32) {
+        const bool on = r0 + lane < tot;
+        const int e = on ? list[r0 + lane] : 0;
+        const uint32_t sw = sm.slot[e];
+        uint32_t nn = 0, most = 0;
+        int before = 0, all = 0;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const uint32_t w = __shfl_sync(FULL, g[b], e >> 5);
+          const bool set = on && ((w >> (e & 31)) & 1u);
+          const uint32_t bal = __ballot_sync(FULL, set);
+          if (bal) {
+            nn |= (uint32_t)set << b;
+            before += __popc(bal & lt) << b;
+            all += __popc(bal) << b;
+            most = 2u << b;  // counts are below this
           }
         }
-      }
-      cur += stot;
-      if (queued && jtot > 0) {
-        __syncwarp();  // the jobs are in shared memory
-        for (int i = lane; i < jtot; i += 32) {
-          const FillJob jb = job[i];
-          const uint32_t node = jb.jn >> 8;
-          slots[jb.q] = negative_slot(seed, jb.jn & 0xffu, t, jb.eidx, node, v0, (uint32_t)n,
-                                      prob_of_node, prob);
+        const int64_t pos = cur + lane + before;
+        if (on) slots[pos] = sw;
+        for (uint32_t j = 0; j + 1 < most; ++j) {
+          const uint32_t push = __ballot_sync(FULL, nn > j);
+          if (push == 0u) break;
+          if (nn > j) {
+            const uint32_t node = sw & 31u;
+            job[queued + __popc(push & lt)] =
+                FillJob{pos + 1 + j, (uint32_t)(c0 + e + sm.eb[node]), j | (node << 8) | ((uint32_t)t << 16)};
+          }
+          queued += __popc(push);
+          if (queued >= 32) draw(32);
         }
+        cur += min(32, tot - r0) + all;
       }
+      __syncwarp();
+      if (lane == 0) sm.cur[t] = cur;
     }
   }
+  if (queued) draw(queued);
 }
 
 // Count pass (general path): warp per tile; each lane runs the
@@ -1152,7 +1290,7 @@ __global__ void __launch_bounds__(32 * FILL_EPB) k_plane_fill(
 __global__ void k_sched_count(const int64_t* __restrict__ inc_ptr,
                               const float* __restrict__ inc_ps,
                               const uint8_t* __restrict__ inc_up, int64_t n,
-                              int64_t ntiles, int32_t ne, float neg_factor,
+                              int64_t ntiles, int32_t tn, int32_t ne, float neg_factor,
                               int32_t* __restrict__ counts,
                               unsigned long long* __restrict__ max_neg,
                               unsigned long long* __restrict__ fired,
@@ -1165,8 +1303,8 @@ __global__ void k_sched_count(const int64_t* __restrict__ inc_ptr,
   if (tile >= ntiles) return;
   for (int32_t t = lane; t < ne; t += 32) cnt[t] = 0;
   __syncwarp();
-  const int64_t v0 = tile * TILE;
-  const int nt = (int)min((int64_t)TILE, n - v0);
+  const int64_t v0 = tile * tn;
+  const int nt = (int)min((int64_t)tn, n - v0);
   const int64_t P0 = inc_ptr[v0], P1 = inc_ptr[v0 + nt];
   float mx = 0.0f;
   for (int64_t base = P0 & ~(int64_t)31; base < P1; base += 32) {
@@ -1190,7 +1328,7 @@ __global__ void k_sched_count(const int64_t* __restrict__ inc_ptr,
     }
   }
   __syncwarp();
-  for (int32_t t = lane; t < ne; t += 32) counts[(int64_t)t * ntiles + tile] = cnt[t];
+  for (int32_t t = lane; t < ne; t += 32) counts[tile * ne + t] = cnt[t];
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
   if (lane == 0 && mx > 0.0f)
     atomicMax(max_neg, mx >= 1.8446744e19f ? ~0ull : (unsigned long long)mx);
@@ -1205,7 +1343,7 @@ __global__ void k_sched_fill(const int64_t* __restrict__ inc_ptr,
                              const float* __restrict__ inc_ps,
                              const uint8_t* __restrict__ inc_up,
                              const int64_t* __restrict__ eidx_base, int64_t n,
-                             int64_t ntiles, int32_t ne, float neg_factor,
+                             int64_t ntiles, int32_t tn, int32_t ne, float neg_factor,
                              const int64_t* __restrict__ tile_off,
                              const uint32_t* __restrict__ prob_of_node,
                              const ProbInfo* __restrict__ prob, uint64_t seed,
@@ -1216,14 +1354,14 @@ __global__ void k_sched_fill(const int64_t* __restrict__ inc_ptr,
   int64_t* cur = cursors + (size_t)wib * ne;
   const int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
   if (tile >= ntiles) return;
-  const int64_t v0 = tile * TILE;
-  const int nt = (int)min((int64_t)TILE, n - v0);
+  const int64_t v0 = tile * tn;
+  const int nt = (int)min((int64_t)tn, n - v0);
   const int64_t pbl = inc_ptr[v0 + min(lane, nt)];  // lanes >= nt hold the end
   const int64_t ebl = (lane < nt) ? eidx_base[v0 + lane] : 0;
   const int64_t P0 = __shfl_sync(FULL, pbl, 0);
   const int64_t P1 = inc_ptr[v0 + nt];  // nt may be 32: no lane holds the end
   if (lane == 0)
-    for (int32_t t = 0; t < ne; ++t) cur[t] = tile_off[(int64_t)t * ntiles + tile];
+    for (int32_t t = 0; t < ne; ++t) cur[t] = tile_off[tile * ne + t];
   const uint32_t n_total = (uint32_t)n;
   for (int64_t base = P0 & ~(int64_t)31; base < P1; base += 32) {
     const int64_t p = base + lane;
@@ -1283,8 +1421,8 @@ __global__ void k_slot_stats(const int64_t* __restrict__ tile_off,
   const int lane = threadIdx.x & 31;
   if (tile >= ntiles) return;
   for (int32_t t = 0; t < ne; ++t) {
-    const int64_t r0 = tile_off[(int64_t)t * ntiles + tile];
-    const int64_t r1 = tile_off[(int64_t)t * ntiles + tile + 1];
+    const int64_t r0 = tile_off[tile * ne + t];
+    const int64_t r1 = tile_off[tile * ne + t + 1];
     uint32_t mask = 0;
     for (int64_t r = r0 + lane; r < r1; r += 32) {
       const uint32_t y = slots[r];
@@ -1295,7 +1433,7 @@ __global__ void k_slot_stats(const int64_t* __restrict__ tile_off,
   }
 }
 
-// One epoch, slots path: persistent warps; each takes the next 32-node tile
+// One epoch, slots path: persistent warps; each takes the next tile (4 to 32 nodes)
 // in tile_order (heaviest first) from the epoch's work counter. The tile's
 // slots of the epoch come in windows of SLOT_WIN. Phase 1: each lane computes
 // slot contributions (attraction, embedding.rs:213-221, or repulsion,
@@ -1313,7 +1451,7 @@ constexpr int slot_parts() { return DIMP >= 8 ? 2 : 1; }
 template <int DIMP, int WIN>
 struct alignas(16) SlotSmem {
   float rows[TILE][DIMP];      // e_cur rows of the tile's nodes
-  float c[WIN][DIMP];          // contributions of the window's slots
+  float4 c[DIMP / 4][WIN + 1];  // contributions of the window's slots, a plane per four dims
   float S[TILE][DIMP];         // running gradients
   int32_t start[TILE];         // first window slot of each node's run (or none)
   int32_t end[TILE];           // one past its last
@@ -1390,10 +1528,9 @@ __device__ __forceinline__ void slot_group(const EpochArgs& a, SlotSmem<DIMP, WI
 #pragma unroll
       for (int d = 0; d < DIMP; ++d) ev[d] = sm.rows[node][d];
       slot_contrib<DIMP>(c, (sl[u] & 32u) != 0, ev, row[u], two_noise, gamma4);
-      float4* cd = reinterpret_cast<float4*>(&sm.c[i][0]);
 #pragma unroll
       for (int q = 0; q < DIMP / 4; ++q)
-        cd[q] = make_float4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+        sm.c[q][i] = make_float4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
     }
   }
 }
@@ -1402,16 +1539,16 @@ template <int DIMP, int WIN, int SU, bool COH>
 __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN>& sm, int64_t tile,
                                           int lane) {
   const unsigned FULL = 0xffffffffu;
-  const int64_t v0 = tile * TILE;
-  const int nt = (int)min((int64_t)TILE, (int64_t)a.n_total - v0);
-  const int64_t s0 = a.tile_off[tile], s1 = a.tile_off[tile + 1];
+  const int64_t v0 = tile * a.tn;
+  const int nt = (int)min((int64_t)a.tn, (int64_t)a.n_total - v0);
+  const int64_t s0 = a.tile_off[tile * a.n_epochs], s1 = a.tile_off[tile * a.n_epochs + 1];
   __syncwarp();  // the previous tile's readers of the shared rows and sums are done
   {
     const float4* src = reinterpret_cast<const float4*>(a.e_cur + (size_t)v0 * DIMP);
     float4* dst = reinterpret_cast<float4*>(&sm.rows[0][0]);
     for (int i = lane; i < nt * (DIMP / 4); i += 32) dst[i] = COH ? __ldcg(src + i) : __ldg(src + i);
     float4* sz = reinterpret_cast<float4*>(&sm.S[0][0]);
-    for (int i = lane; i < TILE * (DIMP / 4); i += 32) sz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = lane; i < nt * (DIMP / 4); i += 32) sz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const float two_noise = fmul(2.0f, a.noise);
   const float gamma4 = fmul(a.gamma, 4.0f);
@@ -1454,10 +1591,9 @@ __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN
 #pragma unroll
       for (int q = 0; q < PD / 4; ++q) acc[q] = srow[q];
       for (int s2 = s2b; s2 < s2e; ++s2) {
-        const float4* cd = reinterpret_cast<const float4*>(&sm.c[s2][d0]);
 #pragma unroll
         for (int q = 0; q < PD / 4; ++q) {
-          const float4 x = cd[q];
+          const float4 x = sm.c[d0 / 4 + q][s2];
           const float2 lo = fadd2(make_float2(acc[q].x, acc[q].y), make_float2(x.x, x.y));
           const float2 hi = fadd2(make_float2(acc[q].z, acc[q].w), make_float2(x.z, x.w));
           acc[q] = make_float4(lo.x, lo.y, hi.x, hi.y);
@@ -1480,17 +1616,9 @@ __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN
       g[d] = act ? sm.S[lane][d] : 0.0f;
     }
     if (act) {
-      const float4* m4 = reinterpret_cast<const float4*>(a.m + q);
-      const float4* v4 = reinterpret_cast<const float4*>(a.v + q);
       float mm[DIMP], vv[DIMP];
-#pragma unroll
-      for (int i = 0; i < DIMP / 4; ++i) {
-        const float4 x = COH ? __ldcg(m4 + i) : __ldcs(m4 + i);
-        const float4 y = COH ? __ldcg(v4 + i) : __ldcs(v4 + i);
-        mm[4 * i] = x.x; mm[4 * i + 1] = x.y; mm[4 * i + 2] = x.z; mm[4 * i + 3] = x.w;
-        vv[4 * i] = y.x; vv[4 * i + 1] = y.y; vv[4 * i + 2] = y.z; vv[4 * i + 3] = y.w;
-      }
-#pragma unroll
+      load_moment<DIMP, COH>(a.m + q, mm);
+      load_moment<DIMP, COH>(a.v + q, vv);
 #pragma unroll
       for (int d = 0; d < DIMP; ++d) {  // scalar: a packed multiply feeding a packed
         // add did not reproduce the unfused result
@@ -1498,18 +1626,10 @@ __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN
         vv[d] = fadd(vv[d], fmul(a.one_m_b2, fsub(fmul(g[d], g[d]), vv[d])));
         e[d] = fadd(e[d], fdiv(fmul(a.lr_ad, mm[d]), fadd(fsqrt(vv[d]), a.epsc)));
       }
-      float4* mo = reinterpret_cast<float4*>(a.m + q);
-      float4* vo = reinterpret_cast<float4*>(a.v + q);
-#pragma unroll
-      for (int i = 0; i < DIMP / 4; ++i) {
-        __stcs(mo + i, make_float4(mm[4 * i], mm[4 * i + 1], mm[4 * i + 2], mm[4 * i + 3]));
-        __stcs(vo + i, make_float4(vv[4 * i], vv[4 * i + 1], vv[4 * i + 2], vv[4 * i + 3]));
-      }
+      store_row<DIMP>(a.m + q, mm);
+      store_row<DIMP>(a.v + q, vv);
     }
-    float4* eo = reinterpret_cast<float4*>(a.e_next + q);
-#pragma unroll
-    for (int i = 0; i < DIMP / 4; ++i)  // evict-first: keep e_cur's rows in L2 for the gathers
-      __stcs(eo + i, make_float4(e[4 * i], e[4 * i + 1], e[4 * i + 2], e[4 * i + 3]));
+    store_row<DIMP>(a.e_next + q, e);  // evict-first: keep e_cur's rows in L2 for the gathers
     if (a.grad_out) {
       float4* go = reinterpret_cast<float4*>(a.grad_out + q);
 #pragma unroll
@@ -1528,7 +1648,7 @@ __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4) k_epoch_slot(EpochArgs
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   SlotSmem<DIMP, WIN>& sm = reinterpret_cast<SlotSmem<DIMP, WIN>*>(smem_raw)[threadIdx.x >> 5];
-  const int64_t ntiles = ((int64_t)a.n_total + TILE - 1) / TILE;
+  const int64_t ntiles = a.ntiles;
   for (;;) {
     unsigned long long w = 0;
     if (lane == 0) w = atomicAdd(a.work_ctr, 1ull);
@@ -1606,13 +1726,13 @@ __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   SlotSmem<DIMP, WIN>& sm = reinterpret_cast<SlotSmem<DIMP, WIN>*>(smem_raw)[threadIdx.x >> 5];
-  const int64_t ntiles = ((int64_t)base.n_total + TILE - 1) / TILE;
+  const int64_t ntiles = base.ntiles;
   for (int32_t t = x.t0; t < x.t1; ++t) {
     EpochArgs a = base;
     const int k = t - x.t0;
     a.e_cur = (k & 1) ? x.e1 : x.e0;
     a.e_next = (k & 1) ? x.e0 : x.e1;
-    a.tile_off = x.tile_off + (size_t)t * ntiles;
+    a.tile_off = x.tile_off + t;
     a.work_ctr = x.work_ctr + t;
     const float4 ep = x.ep[t];
     a.gamma = ep.x;
@@ -1721,6 +1841,9 @@ void launch_epoch(evoc_plan* pl, int32_t t, const float* e_cur, float* e_next,
   a.prob = pl->n_problems > 1 ? pl->prob.get() : nullptr;
   a.n_total = (uint32_t)pl->n;
   a.epoch = (uint32_t)t;
+  a.n_epochs = pl->params.n_epochs;
+  a.tn = pl->tile_nodes;
+  a.ntiles = pl->ntiles;
   a.seed = pl->seeds.empty() ? 0 : pl->seeds[0];
   a.noise = pl->params.noise_level;
   a.gamma = pl->gamma[t];
@@ -1733,10 +1856,10 @@ void launch_epoch(evoc_plan* pl, int32_t t, const float* e_cur, float* e_next,
   a.slots = nullptr;
   a.work_ctr = nullptr;
   const int wpb = pl->lanes;
-  const int64_t tiles = (pl->n + TILE - 1) / TILE;
+  const int64_t tiles = (pl->n + TILE - 1) / TILE;  // scan path
   const unsigned grid = (unsigned)((tiles + wpb - 1) / wpb);
   if (pl->use_slots) {
-    a.tile_off = pl->tile_off.get() + (size_t)t * pl->ntiles;
+    a.tile_off = pl->tile_off.get() + t;
     a.tile_order = pl->tile_order.get();
     a.slots = pl->slots.get();
     a.work_ctr = pl->work_ctr.get() + t;  // zeroed before the epoch loop
@@ -1759,6 +1882,9 @@ void launch_all_epochs(evoc_plan* pl, int32_t t0, int32_t t1, cudaStream_t s) {
   a.prob_of_node = pl->n_problems > 1 ? pl->prob_of_node.get() : nullptr;
   a.prob = pl->n_problems > 1 ? pl->prob.get() : nullptr;
   a.n_total = (uint32_t)pl->n;
+  a.n_epochs = pl->params.n_epochs;
+  a.tn = pl->tile_nodes;
+  a.ntiles = pl->ntiles;
   a.seed = pl->seeds.empty() ? 0 : pl->seeds[0];
   a.noise = pl->params.noise_level;
   a.one_m_b1 = pl->one_m_b1;
@@ -1805,7 +1931,7 @@ __global__ void k_tile_weight(const int32_t* __restrict__ counts, int64_t ntiles
   const int64_t tile = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tile >= ntiles) return;
   uint64_t tot = 0;
-  for (int32_t t = 0; t < ne; ++t) tot += (uint32_t)counts[(int64_t)t * ntiles + tile];
+  for (int32_t t = 0; t < ne; ++t) tot += (uint32_t)counts[tile * ne + t];
   keys[tile] = ~(uint32_t)min(tot, (uint64_t)0xffffffffu);
   vals[tile] = make_uint2((uint32_t)tile, 0u);
 }
@@ -1816,20 +1942,51 @@ __global__ void k_tile_order(const uint2* __restrict__ vals, int64_t ntiles,
   if (i < ntiles) order[i] = vals[i].x;
 }
 
-// Slots path of the schedule set-up: per-edge schedule and incidence planes
-// (n_epochs <= 64 and at most 3 negatives per edge and epoch) or the
-// per-entry recurrence (otherwise), then count pass, offset scan, tile order
-// and fill pass. Returns false (nothing built) when EVOC_EPOCH_PATH=scan,
-// when the epoch count exceeds the shared-memory cursors, or when the slots
-// would take more than half of the free device memory (unless
-// EVOC_EPOCH_PATH=slots).
-static bool build_slots(evoc_plan* pl, const float* inc_ps, const uint8_t* inc_up,
-                        const uint32_t* inc_eidx, const float* e_ps, int64_t U,
-                        float neg_factor) {
-  cudaStream_t s = pl->ctx->stream;
-  const int32_t ne = pl->params.n_epochs;
+namespace {
+// Nodes per tile: the largest of 32, 16, 8 and 4 that leaves the resident warps
+// (28 per SM) about three tiles for every four of them, since a warp works through
+// a tile in one latency-bound go and an epoch ends with its last tile. 50 epochs, dim
+// 8, tiles of 4 / 8 / 16 / 32 nodes: 2k points 0.33 / 0.38 / 0.47 / 0.61 ms, 20k
+// 0.57 / 0.55 / 0.57 / 0.70, 100k 1.59 / 1.09 / 1.03 / 1.11, 300k 4.2 / 2.7 / 2.10 /
+// 2.03, 2M 31.9 / 19.9 / 14.5 / 12.6.
+int32_t tile_nodes_for(int64_t n, int sms) {
+  int32_t tn = TILE;
+  while (tn > 4 && 4 * n < (int64_t)tn * 3 * 28 * sms) tn /= 2;
+  return tn;
+}
+
+// Masks, counts, offsets, order and fill of the slots for one (NW, NB).
+template <int NW, int NB>
+void launch_masks(const IncView& iv, const int64_t* wbase, uint32_t* planes, int32_t* counts,
+                  int32_t* fires, unsigned long long* max_neg, cudaStream_t s) {
+  const size_t smem = sizeof(MaskSmem<NW, NB>);
+  EVOC_CUDA(cudaFuncSetAttribute((const void*)k_tile_masks<NW, NB>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_tile_masks<NW, NB><<<(unsigned)iv.ntiles, MASK_THREADS, smem, s>>>(iv, wbase, planes, counts,
+                                                                      fires, max_neg);
+  EVOC_CHECK_LAUNCH();
+}
+}  // namespace
+
+// Incidence entries of the per-entry and scan paths: built on request.
+struct IncEntries {
+  DevBuf<float> ps;
+  DevBuf<uint8_t> up;
+};
+
+// Slots path of the schedule set-up: the schedule in bit planes per tile
+// (n_epochs <= MASK_EPOCHS and at most MASK_NEGS negatives per edge and epoch) or
+// the per-entry recurrence (otherwise), then offset scan, tile order and fill
+// pass. Returns false (nothing built) when EVOC_EPOCH_PATH=scan, when the epoch
+// count exceeds the shared-memory cursors, or when the slots would take more than
+// half of the free device memory (unless EVOC_EPOCH_PATH=slots).
+template <class Entries>
+static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_base,
+                        Entries entries) {
+  evoc_ctx* ctx = pl->ctx;
+  cudaStream_t s = ctx->stream;
+  const int32_t ne = iv.ne;
   const int64_t n = pl->n;
-  pl->ntiles = (n + TILE - 1) / TILE;
   const char* env = std::getenv("EVOC_EPOCH_PATH");
   const bool force_scan = env && std::strcmp(env, "scan") == 0;
   const bool force_slots = env && std::strcmp(env, "slots") == 0;
@@ -1841,62 +1998,71 @@ static bool build_slots(evoc_plan* pl, const float* inc_ps, const uint8_t* inc_u
   const int64_t cells = (int64_t)ne * pl->ntiles;
   StageTrace trace(s);
   DevBuf<int32_t> counts(cells, s);
-  DevBuf<unsigned long long> mx(1, s), tot(2 * ne, s);  // tot: fired[ne], negs[ne]
-  EVOC_CUDA(cudaMemsetAsync(mx.get(), 0, sizeof(unsigned long long), s));
+  DevBuf<unsigned long long> tot(2 * ne + 1, s);  // fired[ne], negs[ne], largest count
   EVOC_CUDA(cudaMemsetAsync(tot.get(), 0, tot.bytes(), s));
-  unsigned long long maxneg = 0;
-  // n_epochs <= 64: the recurrence runs once per edge into bit masks, turned
-  // into incidence-order bit planes that the count and fill passes read.
-  bool use_planes = ne <= 64;
-  DevBuf<uint32_t> fpl, npl0, npl1;
-  int64_t planes_w = 0;
-  if (use_planes) {
-    DevBuf<unsigned long long> efire(U, s), eneg_lo(U, s), eneg_hi(U, s);
-    trace.mark("alloc masks");
-    k_edge_sched<<<blocks_for(U), 256, 0, s>>>(e_ps, U, ne, neg_factor, efire.get(),
-                                               eneg_lo.get(), eneg_hi.get(), mx.get());
-    EVOC_CHECK_LAUNCH();
-    EVOC_CUDA(cudaMemcpyAsync(&maxneg, mx.get(), sizeof(maxneg), cudaMemcpyDeviceToHost, s));
+  unsigned long long* mx = tot.get() + 2 * ne;
+  std::vector<unsigned long long> htot(2 * ne + 1);
+  DevBuf<int64_t> off(cells + 1, s);
+  int64_t total = 0;
+  auto read_totals = [&]() {
+    exclusive_scan_i32_to_i64(ctx, counts.get(), off.get(), cells);
+    EVOC_CUDA(cudaMemcpyAsync(&total, off.get() + cells, sizeof(int64_t), cudaMemcpyDeviceToHost,
+                              s));
+    EVOC_CUDA(cudaMemcpyAsync(htot.data(), tot.get(), tot.bytes(), cudaMemcpyDeviceToHost, s));
     EVOC_CUDA(cudaStreamSynchronize(s));
-    trace.mark("edge schedule");
-    use_planes = maxneg <= 3;  // the planes hold negative counts 0..3
-    if (use_planes) {
-      planes_w = (pl->n_inc + 31) / 32;
-      const int64_t pw = planes_w * ne;
-      fpl.alloc(pw, s);
-      npl0.alloc(pw, s);
-      npl1.alloc(pw, s);
-      k_inc_planes<<<(unsigned)((planes_w + PLANE_BLOCK_WORDS - 1) / PLANE_BLOCK_WORDS), 256,
-                     0, s>>>(inc_eidx, inc_up, inc_ps, pl->n_inc, planes_w, ne, efire.get(),
-                             eneg_lo.get(), eneg_hi.get(), fpl.get(), npl0.get(), npl1.get());
+  };
+  bool use_planes = ne <= MASK_EPOCHS;
+  // at a rate r an edge draws about r / 1.5 negatives when it fires, one more at times
+  const bool wide_neg = pl->params.negative_sample_rate > 2.5f, wide_ep = ne > 64;
+  bool mask_neg4 = wide_neg;
+  DevBuf<uint32_t> planes;
+  DevBuf<int64_t> wbase;
+  if (use_planes) {
+    DevBuf<int32_t> words(pl->ntiles, s), fires(cells, s);
+    k_tile_words<<<blocks_for(pl->ntiles), 256, 0, s>>>(iv.ptr, n, pl->ntiles, iv.tn, words.get());
+    EVOC_CHECK_LAUNCH();
+    wbase.alloc(pl->ntiles + 1, s);
+    exclusive_scan_i32_to_i64(ctx, words.get(), wbase.get(), pl->ntiles);
+    // at most one partial word per tile
+    const int64_t max_words = pl->n_inc / 32 + pl->ntiles;
+    bool neg4 = wide_neg;
+    for (;;) {
+      planes.alloc(max_words * (neg4 ? 5 : 3) * ne, s);
+      (wide_ep ? (neg4 ? launch_masks<4, 4> : launch_masks<4, 2>)
+               : (neg4 ? launch_masks<2, 4> : launch_masks<2, 2>))(
+          iv, wbase.get(), planes.get(), counts.get(), fires.get(), mx, s);
+      k_epoch_totals<<<(unsigned)std::min<int64_t>(pl->ntiles, 4 * (int64_t)ctx->num_sms),
+                       MASK_EPOCHS, 0, s>>>(counts.get(), fires.get(), pl->ntiles, ne, tot.get(),
+                                            tot.get() + ne);
       EVOC_CHECK_LAUNCH();
-      trace.mark("incidence planes");
-      k_plane_count<<<blocks_for(pl->ntiles * 32), 256, 0, s>>>(
-          pl->inc_ptr.get(), n, pl->ntiles, planes_w, ne, fpl.get(), npl0.get(), npl1.get(),
-          counts.get(), tot.get(), tot.get() + ne);
-      EVOC_CHECK_LAUNCH();
+      trace.mark("schedule masks");
+      read_totals();
+      use_planes = htot[2 * ne] <= (neg4 ? MASK_NEGS : 3ull);
+      if (use_planes || neg4 || htot[2 * ne] > MASK_NEGS) break;
+      neg4 = true;  // counts of 4 to 15: once more with four bits
+      EVOC_CUDA(cudaMemsetAsync(tot.get(), 0, tot.bytes(), s));
     }
+    if (!use_planes) {
+      planes.release();
+      EVOC_CUDA(cudaMemsetAsync(tot.get(), 0, tot.bytes(), s));
+    }
+    mask_neg4 = neg4;
   }
+  IncEntries* ent = nullptr;
   if (!use_planes) {
+    ent = entries();
     const size_t csmem = (size_t)wpb * ne * sizeof(int32_t);
     if (csmem > 48 * 1024)
       EVOC_CUDA(cudaFuncSetAttribute((const void*)k_sched_count,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
-    k_sched_count<<<grid, 32 * wpb, csmem, s>>>(pl->inc_ptr.get(), inc_ps, inc_up, n,
-                                                pl->ntiles, ne, neg_factor, counts.get(),
-                                                mx.get(), tot.get(), tot.get() + ne);
+    k_sched_count<<<grid, 32 * wpb, csmem, s>>>(pl->inc_ptr.get(), ent->ps.get(), ent->up.get(), n,
+                                                pl->ntiles, iv.tn, ne, iv.neg_factor, counts.get(), mx,
+                                                tot.get(), tot.get() + ne);
     EVOC_CHECK_LAUNCH();
+    trace.mark("count pass");
+    read_totals();
   }
-  trace.mark("count pass");
-  DevBuf<int64_t> off(cells + 1, s);
-  exclusive_scan_i32_to_i64(pl->ctx, counts.get(), off.get(), cells);
-  int64_t total = 0;
-  std::vector<unsigned long long> htot(2 * ne);
-  EVOC_CUDA(cudaMemcpyAsync(&total, off.get() + cells, sizeof(int64_t),
-                            cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaMemcpyAsync(&maxneg, mx.get(), sizeof(maxneg), cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaMemcpyAsync(htot.data(), tot.get(), tot.bytes(), cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaStreamSynchronize(s));
+  const unsigned long long maxneg = htot[2 * ne];
   if (maxneg > (unsigned long long)NEG_LIMIT)
     throw Error(EVOC_ERR_UNSUPPORTED,
                 "more than 2^20 negative samples per edge and epoch "
@@ -1904,7 +2070,7 @@ static bool build_slots(evoc_plan* pl, const float* inc_ps, const uint8_t* inc_u
   size_t free_b = 0, total_b = 0;
   EVOC_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const double need = (double)sizeof(uint32_t) * (double)total;
-  const double avail = (double)free_b + (double)pl->ctx->slot_cache.bytes();  // the cache is reusable
+  const double avail = (double)free_b + (double)ctx->slot_cache.bytes();  // the cache is reusable
   if (!force_slots && need > 0.5 * avail) return false;
   pl->max_neg = maxneg;
   trace.mark("offset scan + sync");
@@ -1914,36 +2080,35 @@ static bool build_slots(evoc_plan* pl, const float* inc_ps, const uint8_t* inc_u
     k_tile_weight<<<blocks_for(pl->ntiles), 256, 0, s>>>(counts.get(), pl->ntiles, ne,
                                                           keys.get(), vals.get());
     EVOC_CHECK_LAUNCH();
-    radix_sort_pairs(pl->ctx, keys, vals, pl->ntiles, 32);
+    radix_sort_pairs(ctx, keys, vals, pl->ntiles, 32);
     pl->tile_order.alloc(pl->ntiles, s);
     k_tile_order<<<blocks_for(pl->ntiles), 256, 0, s>>>(vals.get(), pl->ntiles,
                                                          pl->tile_order.get());
     EVOC_CHECK_LAUNCH();
   }
   trace.mark("tile order");
-  if (total > 0 && pl->ctx->slot_cache.count >= (size_t)total) {
-    pl->slots = std::move(pl->ctx->slot_cache);
+  if (total > 0 && ctx->slot_cache.count >= (size_t)total) {
+    pl->slots = std::move(ctx->slot_cache);
   } else {
-    pl->ctx->slot_cache.release();
+    ctx->slot_cache.release();
     pl->slots.alloc(total, s);
   }
   trace.mark("alloc slots");
-  const uint32_t* pon = pl->n_problems > 1 ? pl->prob_of_node.get() : nullptr;
   const ProbInfo* pinfo = pl->n_problems > 1 ? pl->prob.get() : nullptr;
   const uint64_t seed0 = pl->seeds.empty() ? 0 : pl->seeds[0];
   if (use_planes) {
-    const int64_t ngroups = (ne + FILL_EPB - 1) / FILL_EPB;
-    k_plane_fill<<<(unsigned)(ngroups * pl->ntiles), 32 * FILL_EPB, 0, s>>>(
-        pl->inc_ptr.get(), pl->inc_other.get(), pl->eidx_base.get(), n, pl->ntiles, planes_w,
-        ne, fpl.get(), npl0.get(), npl1.get(), off.get(), pon, pinfo, seed0, pl->slots.get());
+    (mask_neg4 ? k_tile_fill<4> : k_tile_fill<2>)<<<(unsigned)pl->ntiles, 32 * FILL_WARPS, 0, s>>>(
+        iv, wbase.get(), planes.get(), pl->tile_order.get(), off.get(), eidx_base, pinfo, seed0,
+        pl->slots.get());
   } else {
     const size_t fsmem = (size_t)wpb * ne * sizeof(int64_t);
     if (fsmem > 48 * 1024)
       EVOC_CUDA(cudaFuncSetAttribute((const void*)k_sched_fill,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
     k_sched_fill<<<grid, 32 * wpb, fsmem, s>>>(
-        pl->inc_ptr.get(), pl->inc_other.get(), inc_ps, inc_up, pl->eidx_base.get(), n,
-        pl->ntiles, ne, neg_factor, off.get(), pon, pinfo, seed0, pl->slots.get());
+        pl->inc_ptr.get(), pl->inc_other.get(), ent->ps.get(), ent->up.get(), eidx_base, n,
+        pl->ntiles, iv.tn, ne, iv.neg_factor, off.get(), iv.prob_of_node, pinfo, seed0,
+        pl->slots.get());
   }
   EVOC_CHECK_LAUNCH();
   trace.mark("fill pass");
@@ -2351,10 +2516,11 @@ evoc_plan* plan_create(evoc_ctx* ctx, const std::vector<ProblemDesc>& probs,
 
   StageTrace trace(s);
   trace.mark("graph concat");
-  // upper / lower counts and the edge list
-  DevBuf<int32_t> ucnt(n, s), lcnt(n, s);
-  k_row_counts<<<blocks_for(n * 32), 256, 0, s>>>(indptr, indices, n, ucnt.get(),
-                                                  lcnt.get());
+  // upper / lower counts; canonical graphs: the largest weights too
+  DevBuf<int32_t> ucnt(n, s), lcnt(n, s), max_w(pl->n_problems, s);
+  EVOC_CUDA(cudaMemsetAsync(max_w.get(), 0, pl->n_problems * sizeof(int32_t), s));
+  k_row_counts<<<blocks_for(n * 32), 256, 0, s>>>(indptr, indices, canonical ? weights : nullptr,
+                                                  n, pon, ucnt.get(), lcnt.get(), max_w.get());
   EVOC_CHECK_LAUNCH();
   DevBuf<int64_t> uptr(n + 1, s);
   exclusive_scan_i32_to_i64(pl->ctx, ucnt.get(), uptr.get(), n);
@@ -2373,76 +2539,84 @@ evoc_plan* plan_create(evoc_ctx* ctx, const std::vector<ProblemDesc>& probs,
   if (U >= (int64_t)0xFFFFFFFFu)
     throw Error(EVOC_ERR_UNSUPPORTED, "more than 2^32-2 edges");
   pl->has_edges = true;
-
+  pl->n_inc = 2 * U;
+  pl->W = (pl->n_inc + 31) / 32;
+  pl->tile_nodes = tile_nodes_for(n, ctx->num_sms);
+  pl->ntiles = (n + pl->tile_nodes - 1) / pl->tile_nodes;
   trace.mark("row counts + scan");
-  DevBuf<float> e_w(U, s), e_ps(U, s);
-  DevBuf<uint32_t> e_dst(U, s), e_src(U, s);
-  DevBuf<int32_t> max_w(pl->n_problems, s);
-  EVOC_CUDA(cudaMemsetAsync(max_w.get(), 0, pl->n_problems * sizeof(int32_t), s));
-  if (!canonical) EVOC_CUDA(cudaMemsetAsync(lcnt.get(), 0, n * sizeof(int32_t), s));
-  k_edge_fill<<<blocks_for(n * 32), 256, 0, s>>>(
-      indptr, indices, weights, n, uptr.get(), pon, e_w.get(), e_dst.get(),
-      e_src.get(), max_w.get(), canonical ? nullptr : lcnt.get());
-  EVOC_CHECK_LAUNCH();
-  k_edge_ps<<<blocks_for(U), 256, 0, s>>>(e_w.get(), e_src.get(), U, pon,
-                                          max_w.get(), e_ps.get());
-  EVOC_CHECK_LAUNCH();
-  e_w.release();
 
+  // incidence lists. A canonical graph's rows are them; a general graph's lower
+  // parts are its edges sorted by their larger endpoint.
+  DevBuf<float> e_ps;
   DevBuf<int64_t> lptr;
   DevBuf<uint2> lower;
-  if (!canonical) {
-    DevBuf<uint32_t> keys(U, s);
+  if (canonical) {
+    if (nnz != pl->n_inc)
+      throw Error(EVOC_ERR_INTERNAL, "incidence count mismatch (graph not symmetric?)");
+  } else {
+    DevBuf<float> e_w(U, s);
+    DevBuf<uint32_t> e_dst(U, s), e_src(U, s);
+    e_ps.alloc(U, s);
+    EVOC_CUDA(cudaMemsetAsync(lcnt.get(), 0, n * sizeof(int32_t), s));
+    k_edge_fill<<<blocks_for(n * 32), 256, 0, s>>>(indptr, indices, weights, n, uptr.get(), pon,
+                                                   e_w.get(), e_dst.get(), e_src.get(),
+                                                   max_w.get(), lcnt.get());
+    EVOC_CHECK_LAUNCH();
+    k_edge_ps<<<blocks_for(U), 256, 0, s>>>(e_w.get(), e_src.get(), U, pon, max_w.get(),
+                                            e_ps.get());
+    EVOC_CHECK_LAUNCH();
     lower.alloc(U, s);
-    EVOC_CUDA(cudaMemcpyAsync(keys.get(), e_dst.get(), U * sizeof(uint32_t),
-                              cudaMemcpyDeviceToDevice, s));
     fill_eidx_src(lower.get(), e_src.get(), U, s);
-    radix_sort_pairs(pl->ctx, keys, lower, U, bits_for((uint64_t)(n - 1)));
+    radix_sort_pairs(pl->ctx, e_dst, lower, U, bits_for((uint64_t)(n - 1)));
     lptr.alloc(n + 1, s);
     exclusive_scan_i32_to_i64(pl->ctx, lcnt.get(), lptr.get(), n);
+    DevBuf<int32_t> deg(n, s);
+    add_counts(ucnt.get(), lcnt.get(), deg.get(), n, s);
+    pl->inc_ptr.alloc(n + 1, s);
+    exclusive_scan_i32_to_i64(pl->ctx, deg.get(), pl->inc_ptr.get(), n);
   }
-  e_dst.release();
-  e_src.release();
-
-  trace.mark("edges + transpose");
-  // incidence lists
-  DevBuf<int32_t> deg(n, s);
-  add_counts(ucnt.get(), lcnt.get(), deg.get(), n, s);
-  pl->inc_ptr.alloc(n + 1, s);
-  exclusive_scan_i32_to_i64(pl->ctx, deg.get(), pl->inc_ptr.get(), n);
-  deg.release();
-  int64_t n_inc = 0;
-  EVOC_CUDA(cudaMemcpyAsync(&n_inc, pl->inc_ptr.get() + n, sizeof(int64_t),
-                            cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaStreamSynchronize(s));
-  if (n_inc != 2 * U)
-    throw Error(EVOC_ERR_INTERNAL, "incidence count mismatch (graph not symmetric?)");
-  pl->n_inc = n_inc;
+  // entries as lists of their own: general graphs, and the paths that need them
+  IncEntries ent;
+  auto entries = [&]() {
+    if (ent.ps.count == 0) {
+      if (canonical) {
+        pl->inc_ptr.alloc(n + 1, s);
+        EVOC_CUDA(cudaMemcpyAsync(pl->inc_ptr.get(), indptr, (n + 1) * sizeof(int64_t),
+                                  cudaMemcpyDeviceToDevice, s));
+      }
+      pl->inc_other.alloc(pl->n_inc, s);
+      ent.ps.alloc(pl->n_inc, s);
+      ent.up.alloc(pl->n_inc, s);
+      k_inc_fill<<<blocks_for(n * 32), 256, 0, s>>>(
+          indptr, indices, weights, n, uptr.get(), lcnt.get(), lptr.get(), lower.get(),
+          e_ps.get(), pl->inc_ptr.get(), pon, max_w.get(), pl->inc_other.get(), ent.ps.get(),
+          ent.up.get());
+      EVOC_CHECK_LAUNCH();
+    }
+    return &ent;
+  };
+  if (!canonical) entries();
   DevBuf<int64_t> ebase(pl->n_problems, s);
   k_prob_ebase<<<blocks_for(pl->n_problems), 256, 0, s>>>(
       uptr.get(), pl->n_problems > 1 ? pl->prob.get() : nullptr,
       pl->n_problems, ebase.get());
   EVOC_CHECK_LAUNCH();
-  pl->inc_other.alloc(n_inc, s);
   pl->eidx_base.alloc(n, s);
-  DevBuf<float> inc_ps(n_inc, s);
-  DevBuf<uint8_t> inc_up(n_inc, s);
-  DevBuf<uint32_t> inc_eidx(n_inc, s);
-  k_inc_fill<<<blocks_for(n * 32), 256, 0, s>>>(
-      indptr, indices, weights, n, uptr.get(), lcnt.get(), lptr.get(),
-      lower.get(), e_ps.get(), pl->inc_ptr.get(), pon, max_w.get(), ebase.get(),
-      pl->inc_other.get(), inc_ps.get(), inc_up.get(), pl->eidx_base.get(),
-      inc_eidx.get());
+  k_eidx_base<<<blocks_for(n), 256, 0, s>>>(canonical ? indptr : pl->inc_ptr.get(), uptr.get(),
+                                            lcnt.get(), n, pon, ebase.get(),
+                                            pl->eidx_base.get());
   EVOC_CHECK_LAUNCH();
-  lower.release();
-  lptr.release();
-
   trace.mark("incidence lists");
   // schedule: per-epoch gradient slots (fast path) or bit planes (fallback)
   const float neg_factor = 1.5f / params.negative_sample_rate;  // embedding.rs:116
-  pl->W = (n_inc + 31) / 32;
-  if (ne > 0 && !build_slots(pl.get(), inc_ps.get(), inc_up.get(), inc_eidx.get(),
-                               e_ps.get(), U, neg_factor)) {
+  const IncView iv{canonical ? indptr : pl->inc_ptr.get(),
+                   canonical ? indices : pl->inc_other.get(),
+                   canonical ? weights : ent.ps.get(),
+                   canonical, max_w.get(), pon, n, pl->ntiles, pl->tile_nodes, ne, neg_factor};
+  if (ne > 0 && !build_slots(pl.get(), iv, pl->eidx_base.get(), entries)) {
+    const float* inc_ps = entries()->ps.get();
+    const uint8_t* inc_up = ent.up.get();
+    const int64_t n_inc = pl->n_inc;
     DevBuf<unsigned long long> mx(1, s), st(2 * ne, s);
     EVOC_CUDA(cudaMemsetAsync(mx.get(), 0, sizeof(unsigned long long), s));
     EVOC_CUDA(cudaMemsetAsync(st.get(), 0, st.bytes(), s));
@@ -2453,7 +2627,7 @@ evoc_plan* plan_create(evoc_ctx* ctx, const std::vector<ProblemDesc>& probs,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
     k_schedule_scan<<<blocks_for(n_inc), 256, smem, s>>>(
-        inc_ps.get(), inc_up.get(), n_inc, ne, neg_factor, mx.get(),
+        inc_ps, inc_up, n_inc, ne, neg_factor, mx.get(),
         want_stats ? st.get() : nullptr, want_stats ? st.get() + ne : nullptr);
     EVOC_CHECK_LAUNCH();
     unsigned long long maxneg = 0;
@@ -2475,7 +2649,7 @@ evoc_plan* plan_create(evoc_ctx* ctx, const std::vector<ProblemDesc>& probs,
     }
     pl->planes.alloc((size_t)ne * (1 + pl->P) * pl->W, s);
     k_schedule_write<<<blocks_for(pl->W * 32), 256, 0, s>>>(
-        inc_ps.get(), inc_up.get(), n_inc, ne, neg_factor, pl->P, pl->W,
+        inc_ps, inc_up, n_inc, ne, neg_factor, pl->P, pl->W,
         pl->planes.get());
     EVOC_CHECK_LAUNCH();
   }
