@@ -166,6 +166,7 @@ int evoc_ctx_create(int device, evoc_ctx_t** out) {
   }
   (void)cudaGetLastError();
   EVOC_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+  evoc::dev_pool_open(c->stream, prop.totalGlobalMem / 8);
   c->status.alloc(1, c->stream);
   EVOC_CUDA(cudaMemsetAsync(c->status.get(), 0, sizeof(int32_t), c->stream));
   c->sk_steps.alloc(1, c->stream);
@@ -181,7 +182,7 @@ void evoc_ctx_destroy(evoc_ctx_t* ctx) {
   cudaStream_t s = ctx->stream;
   ctx->status.release();
   ctx->sk_steps.release();
-  ctx->slot_cache.release();
+  evoc::dev_pool_close(s);
   if (s) {
     cudaStreamSynchronize(s);
     cudaStreamDestroy(s);

@@ -2070,7 +2070,7 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
   size_t free_b = 0, total_b = 0;
   EVOC_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const double need = (double)sizeof(uint32_t) * (double)total;
-  const double avail = (double)free_b + (double)ctx->slot_cache.bytes();  // the cache is reusable
+  const double avail = (double)free_b + (double)dev_pool_bytes(s);  // what the pool holds is reusable
   if (!force_slots && need > 0.5 * avail) return false;
   pl->max_neg = maxneg;
   trace.mark("offset scan + sync");
@@ -2087,12 +2087,7 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
     EVOC_CHECK_LAUNCH();
   }
   trace.mark("tile order");
-  if (total > 0 && ctx->slot_cache.count >= (size_t)total) {
-    pl->slots = std::move(ctx->slot_cache);
-  } else {
-    ctx->slot_cache.release();
-    pl->slots.alloc(total, s);
-  }
+  pl->slots.alloc(total, s);
   trace.mark("alloc slots");
   const ProbInfo* pinfo = pl->n_problems > 1 ? pl->prob.get() : nullptr;
   const uint64_t seed0 = pl->seeds.empty() ? 0 : pl->seeds[0];
@@ -2892,8 +2887,6 @@ void plan_upload_init_and_run(evoc_plan* pl, const float* const* h_inits,
 
 void plan_free(evoc_plan* pl) {
   if (!pl) return;
-  if (pl->ctx && pl->slots.count > pl->ctx->slot_cache.count)
-    pl->ctx->slot_cache = std::move(pl->slots);
   if (pl->graph_exec) cudaGraphExecDestroy(pl->graph_exec);
   if (pl->graph) cudaGraphDestroy(pl->graph);
   delete pl;

@@ -48,12 +48,19 @@ enum StatusBit : int32_t {
 };
 
 // ---------------------------------------------------------------------------
-// Stream-ordered device buffer.
+// Stream-ordered device buffer, from the stream's pool (pool.cu).
 // ---------------------------------------------------------------------------
+void dev_pool_open(cudaStream_t s, size_t limit);
+void dev_pool_close(cudaStream_t s);
+size_t dev_pool_bytes(cudaStream_t s);  // free bytes held
+cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s, size_t* held);
+void dev_free(void* ptr, size_t held, cudaStream_t s);
+
 template <typename T>
 struct DevBuf {
   T* ptr = nullptr;
   size_t count = 0;
+  size_t held = 0;  // bytes taken for it
   cudaStream_t stream = nullptr;
   DevBuf() = default;
   DevBuf(size_t n, cudaStream_t s) { alloc(n, s); }
@@ -63,7 +70,7 @@ struct DevBuf {
   DevBuf& operator=(DevBuf&& o) noexcept {
     if (this != &o) {
       release();
-      ptr = o.ptr; count = o.count; stream = o.stream;
+      ptr = o.ptr; count = o.count; held = o.held; stream = o.stream;
       o.ptr = nullptr; o.count = 0;
     }
     return *this;
@@ -74,7 +81,7 @@ struct DevBuf {
     stream = s;
     count = n;
     if (n == 0) return;
-    cudaError_t e = cudaMallocAsync((void**)&ptr, n * sizeof(T), s);
+    cudaError_t e = dev_alloc((void**)&ptr, n * sizeof(T), s, &held);
     if (e != cudaSuccess) {
       ptr = nullptr;
       count = 0;
@@ -85,7 +92,7 @@ struct DevBuf {
     }
   }
   void release() {
-    if (ptr) cudaFreeAsync(ptr, stream);
+    if (ptr) dev_free(ptr, held, stream);
     ptr = nullptr;
     count = 0;
   }
@@ -141,10 +148,6 @@ struct evoc_ctx {
   cudaStream_t stream = nullptr;
   std::string last_error;
   evoc::DevBuf<int32_t> status;  // device status word
-  // The largest gradient-slot buffer of a freed plan, handed to the next plan
-  // that fits in it (stream order makes the reuse safe): repeated one-shot
-  // embeddings skip a multi-gigabyte allocation each.
-  evoc::DevBuf<uint32_t> slot_cache;
   // Row-sum evaluations (bisection steps over all rows) of the most recent
   // smooth_knn pass on this context: the work figure of its ALU bound.
   evoc::DevBuf<unsigned long long> sk_steps;
