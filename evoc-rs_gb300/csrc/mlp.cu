@@ -20,6 +20,8 @@
 // with every weight matrix row-major, output by input (a Linear layer's
 // layout).
 #include "evoc_internal.h"
+
+#include <cuda_pipeline.h>
 #include "evoc_device.cuh"
 
 #include <cuda.h>
@@ -1180,24 +1182,33 @@ __global__ void k_head_combine(const float* __restrict__ ypart, int tiles, int64
 constexpr int MLP_MAX_OUT = 16;
 constexpr int HEAD_THREADS = 256;
 
-template <bool TRAIN>
+template <bool TRAIN, int OMAX>  // out <= OMAX
 __global__ void __launch_bounds__(HEAD_THREADS)
     k_head(const bf16* __restrict__ a2, const float* __restrict__ h2, int hid, int out,
            int64_t rows, const bf16* __restrict__ w3, const float* __restrict__ b3,
            float* __restrict__ y, const float* __restrict__ target, float grad_scale,
            float* __restrict__ dy, bf16* __restrict__ dh2, float* __restrict__ loss_part) {
-  extern __shared__ float w3s[];  // [out][hid]
+  // W3 as [out][8][hid / 8]: a lane's chunk of 8 columns is one float in each of 8
+  // rows, so a warp's reads of an element fall in 32 banks (as [out][hid] they fell
+  // in 4, which took most of the kernel's 73 us at 8192 rows; 23 us now)
+  extern __shared__ float w3s[];
   __shared__ float wsum[HEAD_THREADS / 32];
-  for (int i = threadIdx.x; i < out * hid; i += blockDim.x) w3s[i] = __bfloat162float(w3[i]);
+  const int nchunks = hid >> 3;
+  for (int i = threadIdx.x; i < out * nchunks; i += blockDim.x) {
+    const uint4 raw = reinterpret_cast<const uint4*>(w3)[i];
+    const bf16* wv = reinterpret_cast<const bf16*>(&raw);
+    const int o = i / nchunks, c = i - o * nchunks;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w3s[o * hid + e * nchunks + c] = __bfloat162float(wv[e]);
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nchunks = hid >> 3;
   float lsum = 0.0f;
   for (int64_t row = (int64_t)blockIdx.x * (HEAD_THREADS / 32) + warp; row < rows;
        row += (int64_t)gridDim.x * (HEAD_THREADS / 32)) {
-    float acc[MLP_MAX_OUT];
+    float acc[OMAX];
 #pragma unroll
-    for (int o = 0; o < MLP_MAX_OUT; ++o) acc[o] = 0.0f;
+    for (int o = 0; o < OMAX; ++o) acc[o] = 0.0f;
     for (int c = lane; c < nchunks; c += 32) {
       const uint4 raw = *reinterpret_cast<const uint4*>(a2 + row * hid + c * 8);
       const bf16* av = reinterpret_cast<const bf16*>(&raw);
@@ -1205,12 +1216,12 @@ __global__ void __launch_bounds__(HEAD_THREADS)
       for (int e = 0; e < 8; ++e) {
         const float x = __bfloat162float(av[e]);
 #pragma unroll
-        for (int o = 0; o < MLP_MAX_OUT; ++o)
-          if (o < out) acc[o] += x * w3s[o * hid + c * 8 + e];
+        for (int o = 0; o < OMAX; ++o)
+          if (o < out) acc[o] += x * w3s[o * hid + e * nchunks + c];
       }
     }
 #pragma unroll
-    for (int o = 0; o < MLP_MAX_OUT; ++o) {
+    for (int o = 0; o < OMAX; ++o) {
       if (o >= out) break;
 #pragma unroll
       for (int sh = 16; sh > 0; sh >>= 1) acc[o] += __shfl_xor_sync(0xffffffffu, acc[o], sh);
@@ -1218,14 +1229,14 @@ __global__ void __launch_bounds__(HEAD_THREADS)
     }
     if (!TRAIN) {
 #pragma unroll
-      for (int o = 0; o < MLP_MAX_OUT; ++o)
+      for (int o = 0; o < OMAX; ++o)
         if (o < out && lane == o) y[row * out + o] = acc[o];
       continue;
     }
-    float gy[MLP_MAX_OUT];
+    float gy[OMAX];
     float rsum = 0.0f;
 #pragma unroll
-    for (int o = 0; o < MLP_MAX_OUT; ++o) {
+    for (int o = 0; o < OMAX; ++o) {
       gy[o] = 0.0f;
       if (o < out) {
         const float d = acc[o] - target[row * out + o];
@@ -1244,8 +1255,8 @@ __global__ void __launch_bounds__(HEAD_THREADS)
       for (int e = 0; e < 8; ++e) {
         float da = 0.0f;
 #pragma unroll
-        for (int o = 0; o < MLP_MAX_OUT; ++o)
-          if (o < out) da += gy[o] * w3s[o * hid + c * 8 + e];
+        for (int o = 0; o < OMAX; ++o)
+          if (o < out) da += gy[o] * w3s[o * hid + e * nchunks + c];
         res[e] = __float2bfloat16_rn(da * gelu_grad(pv[e]));
       }
       *reinterpret_cast<uint4*>(dh2 + row * hid + c * 8) = *reinterpret_cast<const uint4*>(res);
@@ -1262,66 +1273,170 @@ __global__ void __launch_bounds__(HEAD_THREADS)
   }
 }
 
-// Column sums over row splits (thread per column c < hid):
-//   pw[z][o][c] = sum_{b in split z} dy[b][o] * a2[b][c]   (o < out; skipped if out == 0)
-//   pb[z][c]    = sum_{b in split z} dh[b][c]
+// Column sums over row splits (thread per column c < hid), in row order:
+//   pw[z][o][c] = sum_{b in split z} dy[b][o] * a2[b][c]   (o < out)
+//   pb2[z][c], pb1[z][c] = sum_{b in split z} dh2[b][c], dh1[b][c]
 //   pb3[z][o]   = sum_{b in split z} dy[b][o]               (threads c < out of block 0)
-__global__ void k_colreduce(const float* __restrict__ dy, int out, const bf16* __restrict__ a2,
-                            const bf16* __restrict__ dh, int hid, int64_t rows,
-                            int64_t rows_per_split, float* __restrict__ pw,
-                            float* __restrict__ pb, float* __restrict__ pb3) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// The chain of additions is short (about 100 rows); what counts is that the loads do
+// not wait for it: 64 rows of the three matrices and of dy are brought into shared
+// memory at a time, 16 bytes per load, all in flight together. At 8192 x 512: 127 us
+// in two launches with a dependent 2-byte load per row, 13 us now.
+constexpr int COL_THREADS = 128;
+constexpr int COL_ROWS = 64;  // rows staged at a time
+template <int OMAX>
+struct ColSmem {
+  bf16 m[3][COL_ROWS][COL_THREADS];  // a2, dh2, dh1
+  float dy[COL_ROWS][OMAX];
+};
+template <int OMAX>
+__global__ void __launch_bounds__(COL_THREADS) k_colreduce(
+    const float* __restrict__ dy, int out, const bf16* __restrict__ a2,
+    const bf16* __restrict__ dh2, const bf16* __restrict__ dh1, int hid, int64_t rows,
+    int64_t rows_per_split, float* __restrict__ pw, float* __restrict__ pb2,
+    float* __restrict__ pb1, float* __restrict__ pb3) {
+  extern __shared__ __align__(16) unsigned char col_raw[];
+  ColSmem<OMAX>& sm = *reinterpret_cast<ColSmem<OMAX>*>(col_raw);
+  const int c0 = blockIdx.x * COL_THREADS, c = c0 + threadIdx.x;
   const int z = blockIdx.y;
   const int64_t b0 = (int64_t)z * rows_per_split;
   const int64_t b1 = min(rows, b0 + rows_per_split);
-  if (c >= hid) return;
-  float acc[MLP_MAX_OUT];
+  const bool on = c < hid, do3 = blockIdx.x == 0 && (int)threadIdx.x < out;
+  const int pc = threadIdx.x & 15, pr = threadIdx.x >> 4;  // 8 columns, first row
+  const bool pon = c0 + 8 * pc < hid;
+  float acc[OMAX];
 #pragma unroll
-  for (int o = 0; o < MLP_MAX_OUT; ++o) acc[o] = 0.0f;
-  float accb = 0.0f, acc3 = 0.0f;
-  const bool do3 = pb3 && blockIdx.x == 0 && c < out;
-  for (int64_t b = b0; b < b1; ++b) {
-    accb += __bfloat162float(dh[b * hid + c]);
-    if (out > 0) {
-      const float x = __bfloat162float(a2[b * hid + c]);
+  for (int o = 0; o < OMAX; ++o) acc[o] = 0.0f;
+  float s2 = 0.0f, s1 = 0.0f, s3 = 0.0f;
+  for (int64_t r0 = b0; r0 < b1; r0 += COL_ROWS) {
+    const int m = (int)min((int64_t)COL_ROWS, b1 - r0);
+    __syncthreads();  // the previous rows are read
+    if (pon) {
 #pragma unroll
-      for (int o = 0; o < MLP_MAX_OUT; ++o)
-        if (o < out) acc[o] += dy[b * out + o] * x;
+      for (int q = 0; q < 3; ++q) {
+        const bf16* src = q == 0 ? a2 : q == 1 ? dh2 : dh1;
+#pragma unroll
+        for (int r = 0; r < COL_ROWS; r += 8)
+          if (r + pr < m)
+            __pipeline_memcpy_async(&sm.m[q][r + pr][8 * pc],
+                                    src + (r0 + r + pr) * hid + c0 + 8 * pc, 16);
+      }
     }
-    if (do3) acc3 += dy[b * out + c];
-  }
-  pb[(int64_t)z * hid + c] = accb;
+    for (int r = threadIdx.x; r < m; r += COL_THREADS)
 #pragma unroll
-  for (int o = 0; o < MLP_MAX_OUT; ++o)
-    if (o < out) pw[((int64_t)z * out + o) * hid + c] = acc[o];
-  if (do3) pb3[(int64_t)z * out + c] = acc3;
+      for (int o = 0; o < OMAX; ++o)
+        if (o < out) sm.dy[r][o] = dy[(r0 + r) * out + o];
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+    __syncthreads();
+    if (do3)
+      for (int r = 0; r < m; ++r) s3 += sm.dy[r][threadIdx.x];
+    if (on) {
+#pragma unroll 4
+      for (int r = 0; r < m; ++r) {
+        s2 += __bfloat162float(sm.m[1][r][threadIdx.x]);
+        s1 += __bfloat162float(sm.m[2][r][threadIdx.x]);
+        const float x = __bfloat162float(sm.m[0][r][threadIdx.x]);
+#pragma unroll
+        for (int o = 0; o < OMAX; ++o)
+          if (o < out) acc[o] += sm.dy[r][o] * x;
+      }
+    }
+  }
+  if (on) {
+    pb2[(int64_t)z * hid + c] = s2;
+    pb1[(int64_t)z * hid + c] = s1;
+#pragma unroll
+    for (int o = 0; o < OMAX; ++o)
+      if (o < out) pw[((int64_t)z * out + o) * hid + c] = acc[o];
+  }
+  if (do3) pb3[(int64_t)z * out + threadIdx.x] = s3;
 }
 
-// grad[i] = sum_{z < splits} part[z * count + i], in split order.
-__global__ void k_sum_splits(const float* __restrict__ part, int splits, int64_t count,
-                             float* __restrict__ grad) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  float s = 0.0f;
-  for (int z = 0; z < splits; ++z) s += part[(int64_t)z * count + i];
-  grad[i] = s;
-}
-
+// One parameter tensor's gradient partials: part[z * count + i], z < splits, for
+// the packed parameters [begin, begin + count).
+struct GradSegment {
+  const float* part;
+  int64_t begin, count;
+  int splits;
+};
+struct GradSegments {
+  GradSegment seg[6];
+};
 // Adam with bias correction (Kingma & Ba, 2015): bc1 = 1 / (1 - beta1^t),
 // bc2 = 1 / (1 - beta2^t).
-__global__ void k_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                       const float* __restrict__ g, bf16* __restrict__ pb, int64_t count,
-                       float lr, float beta1, float beta2, float eps, float bc1, float bc2) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const float gi = g[i];
-  const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
-  const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float pi = p[i] - lr * (mi * bc1) / (sqrtf(vi * bc2) + eps);
-  p[i] = pi;
-  pb[i] = __float2bfloat16_rn(pi);
+struct AdamArgs {
+  float *p, *m, *v;
+  bf16 *pb, *w2t;  // BF16 parameters, transposed W2
+  int64_t o_w2;
+  int hid;
+  float lr, beta1, beta2, eps, bc1, bc2;
+};
+
+// Thread per parameter: grad[i] = sum over its partials in split order and, with
+// ADAM, the step from it. The last block instead adds up the batch's loss, in
+// order (a single thread adds, all load).
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_finish_step(GradSegments gs, int64_t n_params,
+                                                     float* __restrict__ grad, AdamArgs a,
+                                                     const float* __restrict__ loss_part,
+                                                     int nparts, float loss_scale,
+                                                     float* __restrict__ loss) {
+  if (blockIdx.x == gridDim.x - 1) {
+    __shared__ float lp[1024];
+    float s = 0.0f;
+    for (int b = 0; b < nparts; b += 1024) {
+      const int m = min(1024, nparts - b);
+      __syncthreads();
+      for (int i = threadIdx.x; i < m; i += 256) lp[i] = loss_part[b + i];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+#pragma unroll 8
+        for (int i = 0; i < m; ++i) s += lp[i];
+      }
+    }
+    if (threadIdx.x == 0) *loss = s * loss_scale;
+    return;
+  }
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n_params) return;
+  int q = 0;
+#pragma unroll
+  for (int k = 1; k < 6; ++k)
+    if (i >= gs.seg[k].begin) q = k;
+  const float* part = nullptr;
+  int64_t count = 0;
+  int splits = 0;
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+    if (k == q) {
+      part = gs.seg[k].part + (i - gs.seg[k].begin);
+      count = gs.seg[k].count;
+      splits = gs.seg[k].splits;
+    }
+  float gi = 0.0f;
+  int z = 0;
+  for (; z + 8 <= splits; z += 8) {
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = part[(int64_t)(z + u) * count];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) gi += x[u];
+  }
+  for (; z < splits; ++z) gi += part[(int64_t)z * count];
+  grad[i] = gi;
+  if (!ADAM) return;
+  const float mi = a.beta1 * a.m[i] + (1.0f - a.beta1) * gi;
+  const float vi = a.beta2 * a.v[i] + (1.0f - a.beta2) * gi * gi;
+  a.m[i] = mi;
+  a.v[i] = vi;
+  const float pi = a.p[i] - a.lr * (mi * a.bc1) / (sqrtf(vi * a.bc2) + a.eps);
+  a.p[i] = pi;
+  const bf16 pb = __float2bfloat16_rn(pi);
+  a.pb[i] = pb;
+  if (q == 2) {  // W2: its transpose too
+    const int64_t w = i - a.o_w2, r = w / a.hid, c = w - r * a.hid;
+    a.w2t[c * a.hid + r] = pb;
+  }
 }
 
 __global__ void k_to_bf16(const float* __restrict__ x, int64_t count, bf16* __restrict__ y) {
@@ -1329,22 +1444,38 @@ __global__ void k_to_bf16(const float* __restrict__ x, int64_t count, bf16* __re
   if (i < count) y[i] = __float2bfloat16_rn(x[i]);
 }
 
-// dst[c][r] = src[r][c] for a rows x cols BF16 matrix (row strides lds, ldd),
-// through 64 x 64 shared-memory tiles; coalesced on both sides.
-__global__ void __launch_bounds__(256) k_transpose_bf16(const bf16* __restrict__ src, int64_t lds,
-                                                        int rows, int cols, bf16* __restrict__ dst,
-                                                        int64_t ldd) {
-  __shared__ bf16 tile[64][66];
+// dst[c][r] = src[r][c] for up to four rows x cols BF16 matrices (row strides cols
+// and ldd, multiples of 8; blockIdx.z: which), through 64 x 64 shared-memory tiles,
+// 16 bytes per access on both sides (2-byte accesses in a launch each took 70 us for
+// a step's four copies, 28 us now). Columns r >= rows of dst, up to ldd, get zeros.
+struct Transposes {
+  const bf16* src[4];
+  bf16* dst[4];
+  int cols[4];
+};
+__global__ void __launch_bounds__(256) k_transpose_bf16(Transposes t, int rows, int64_t ldd) {
+  __shared__ __align__(16) bf16 tile[64][72];
+  const bf16* __restrict__ src = t.src[blockIdx.z];
+  bf16* __restrict__ dst = t.dst[blockIdx.z];
+  const int cols = t.cols[blockIdx.z];
   const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;  // 64 x 4
-  for (int i = ty; i < 64; i += 4) {
-    const int r = r0 + i, c = c0 + tx;
-    tile[i][tx] = (r < rows && c < cols) ? src[(int64_t)r * lds + c] : __float2bfloat16_rn(0.0f);
+  if (c0 >= cols) return;
+  for (int i = threadIdx.x; i < 64 * 8; i += 256) {
+    const int r = i >> 3, c = (i & 7) * 8;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (r0 + r < rows && c0 + c < cols)
+      v = *reinterpret_cast<const uint4*>(src + (int64_t)(r0 + r) * cols + c0 + c);
+    *reinterpret_cast<uint4*>(&tile[r][c]) = v;
   }
   __syncthreads();
-  for (int i = ty; i < 64; i += 4) {
-    const int c = c0 + i, r = r0 + tx;
-    if (c < cols && r < rows) dst[(int64_t)c * ldd + r] = tile[tx][i];
+  for (int i = threadIdx.x; i < 64 * 8; i += 256) {
+    const int c = i & 63, r = (i >> 6) * 8;
+    if (c0 + c >= cols || r0 + r >= ldd) continue;
+    __align__(16) bf16 v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = tile[r + e][c];
+    *reinterpret_cast<uint4*>(dst + (int64_t)(c0 + c) * ldd + r0 + r) =
+        *reinterpret_cast<const uint4*>(v);
   }
 }
 
@@ -1358,14 +1489,31 @@ __global__ void k_sample_rows(uint32_t* __restrict__ rows, int64_t count, uint32
   rows[i] = __umulhi(o.x, n);
 }
 
-// dst[i][w] = src[rows[i]][w] for rows of `words` 32-bit words.
-__global__ void k_gather_rows(const uint32_t* __restrict__ src, int64_t words,
+// A training batch, warp per row: the row drawn (as k_sample_rows), its point (16
+// bytes per lane: instances are 16-byte aligned) and its layout copied.
+__global__ void k_draw_batch(const bf16* __restrict__ x, int in, const float* __restrict__ layout,
+                             int out, int64_t batch, uint32_t n, uint64_t seed, uint32_t draw,
+                             bf16* __restrict__ xd, float* __restrict__ td) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i >= batch) return;
+  const uint4 o = philox4x32_10(make_uint4((uint32_t)i, draw, 0x4D4C5052u, 0x53414D50u),
+                                make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
+  const int64_t row = __umulhi(o.x, n);
+  const uint4* src = reinterpret_cast<const uint4*>(x + row * in);
+  uint4* dst = reinterpret_cast<uint4*>(xd + i * in);
+  for (int w = lane; w < in / 8; w += 32) dst[w] = src[w];
+  if (lane < out) td[i * out + lane] = layout[row * out + lane];
+}
+
+// dst[i] = src[rows[i]] for rows of `words` 16-byte words, warp per row.
+__global__ void k_gather_rows(const uint4* __restrict__ src, int words,
                               const uint32_t* __restrict__ rows, int64_t count,
-                              uint32_t* __restrict__ dst) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count * words) return;
-  const int64_t i = t / words, w = t - i * words;
-  dst[t] = src[(int64_t)rows[i] * words + w];
+                              uint4* __restrict__ dst) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= count) return;
+  const uint4* s = src + (int64_t)rows[i] * words;
+  for (int w = threadIdx.x & 31; w < words; w += 32) dst[i * words + w] = s[w];
 }
 
 // out[r][j] = sum_i (x[r][i] - xmean[i]) * R[i][j] + ymean[j], d <= 16.
@@ -1386,12 +1534,80 @@ __global__ void k_affine_rows(const float* __restrict__ x, int64_t rows, int d,
   }
 }
 
-__global__ void k_loss_total(const float* __restrict__ part, int nparts, float scale,
-                             float* __restrict__ dst) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  float s = 0.0f;
-  for (int i = 0; i < nparts; ++i) s += part[i];
-  *dst = s * scale;
+// Alignment sums of one instance's sample (rows s[r] of the layout, row r of the
+// prediction), in double and in a fixed order. First the column sums per block,
+// then, with the means formed from them by every block alike, the cross-covariance
+// sum (t - tmean) (p - pmean)^T per block. The host adds the blocks up: on it the
+// row loops took 1.2 of 1.7 ms per instance of 60,000 rows and their copies 0.3.
+constexpr int ALIGN_THREADS = 256;
+constexpr int ALIGN_ROWS = 32;  // rows staged at a time
+__global__ void __launch_bounds__(ALIGN_THREADS) k_align_sums(
+    const float* __restrict__ layout, const uint32_t* __restrict__ sample,
+    const float* __restrict__ pred, int64_t rows, int d, double* __restrict__ sums) {
+  __shared__ double part[ALIGN_THREADS / 32][2 * MLP_MAX_OUT];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double st[MLP_MAX_OUT], sp[MLP_MAX_OUT];
+#pragma unroll
+  for (int j = 0; j < MLP_MAX_OUT; ++j) st[j] = sp[j] = 0.0;
+  for (int64_t r = (int64_t)blockIdx.x * ALIGN_THREADS + threadIdx.x; r < rows;
+       r += (int64_t)gridDim.x * ALIGN_THREADS) {
+    const int64_t t = (int64_t)sample[r] * d;
+#pragma unroll
+    for (int j = 0; j < MLP_MAX_OUT; ++j)
+      if (j < d) {
+        st[j] += layout[t + j];
+        sp[j] += pred[r * d + j];
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < MLP_MAX_OUT; ++j) {
+    if (j >= d) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      st[j] += __shfl_xor_sync(0xffffffffu, st[j], o);
+      sp[j] += __shfl_xor_sync(0xffffffffu, sp[j], o);
+    }
+    if (lane == 0) {
+      part[wid][j] = st[j];
+      part[wid][MLP_MAX_OUT + j] = sp[j];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * MLP_MAX_OUT && (int)(threadIdx.x % MLP_MAX_OUT) < d) {
+    double x = 0.0;
+    for (int w = 0; w < ALIGN_THREADS / 32; ++w) x += part[w][threadIdx.x];
+    sums[blockIdx.x * 2 * MLP_MAX_OUT + threadIdx.x] = x;
+  }
+}
+
+__global__ void __launch_bounds__(ALIGN_THREADS) k_align_cov(
+    const float* __restrict__ layout, const uint32_t* __restrict__ sample,
+    const float* __restrict__ pred, int64_t rows, int d, const double* __restrict__ sums,
+    int nsums, double* __restrict__ means, double* __restrict__ cov) {
+  __shared__ double mean[2 * MLP_MAX_OUT];
+  __shared__ double t_s[ALIGN_ROWS][MLP_MAX_OUT], p_s[ALIGN_ROWS][MLP_MAX_OUT];
+  if (threadIdx.x < 2 * MLP_MAX_OUT && (int)(threadIdx.x % MLP_MAX_OUT) < d) {
+    double x = 0.0;
+    for (int b = 0; b < nsums; ++b) x += sums[b * 2 * MLP_MAX_OUT + threadIdx.x];
+    mean[threadIdx.x] = x / (double)rows;
+    if (blockIdx.x == 0) means[threadIdx.x] = mean[threadIdx.x];
+  }
+  const int a = threadIdx.x / d, b = threadIdx.x - a * d;  // d * d <= 256 pairs
+  double m = 0.0;
+  for (int64_t r0 = (int64_t)blockIdx.x * ALIGN_ROWS; r0 < rows;
+       r0 += (int64_t)gridDim.x * ALIGN_ROWS) {
+    const int n = (int)min((int64_t)ALIGN_ROWS, rows - r0);
+    __syncthreads();  // the means, and the previous rows' readers
+    for (int i = threadIdx.x; i < n * d; i += ALIGN_THREADS) {
+      const int r = i / d, j = i - r * d;
+      t_s[r][j] = (double)layout[(int64_t)sample[r0 + r] * d + j] - mean[j];
+      p_s[r][j] = (double)pred[(r0 + r) * d + j] - mean[MLP_MAX_OUT + j];
+    }
+    __syncthreads();
+    if (a < d)
+      for (int r = 0; r < n; ++r) m += t_s[r][a] * p_s[r][b];
+  }
+  if (a < d) cov[(int64_t)blockIdx.x * d * d + threadIdx.x] = m;
 }
 
 // ---------------------------------------------------------------------------
@@ -1553,10 +1769,11 @@ void launch_forward_head(const GemmArgs& ga, const HeadArgs& ha, evoc_ctx* ctx) 
 
 int tc_col_tiles(int n) { return (n + TC_BN - 1) / TC_BN; }
 
-void transpose_bf16(const bf16* src, int64_t lds, int rows, int cols, bf16* dst, int64_t ldd,
-                    cudaStream_t s) {
-  dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64));
-  k_transpose_bf16<<<grid, 256, 0, s>>>(src, lds, rows, cols, dst, ldd);
+void transpose_bf16(const Transposes& t, int count, int rows, int64_t ldd, cudaStream_t s) {
+  int cols = 0;
+  for (int i = 0; i < count; ++i) cols = std::max(cols, t.cols[i]);
+  dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64), (unsigned)count);
+  k_transpose_bf16<<<grid, 256, 0, s>>>(t, rows, ldd);
   EVOC_CHECK_LAUNCH();
 }
 
@@ -1580,7 +1797,6 @@ struct MlpScratch {
   DevBuf<bf16> x, a1, a2, dh1, dh2;
   DevBuf<bf16> xt, a1t, dh1t, dh2t;  // [features][batch] copies for the weight gradients
   DevBuf<float> h1, h2, target, dy, part, loss_part, loss, ypart;
-  DevBuf<uint32_t> rows;
   int64_t cap = 0;
   int head_grid = 0;
 };
@@ -1594,28 +1810,41 @@ size_t head_smem(const evoc_mlp* net) { return (size_t)net->out * net->hid * siz
 
 void set_head_smem(const evoc_mlp* net) {
   const int bytes = (int)head_smem(net);
-  EVOC_CUDA(cudaFuncSetAttribute(k_head<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  EVOC_CUDA(cudaFuncSetAttribute(k_head<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  for (const void* f : {(const void*)k_head<true, 8>, (const void*)k_head<true, MLP_MAX_OUT>,
+                        (const void*)k_head<false, 8>, (const void*)k_head<false, MLP_MAX_OUT>})
+    EVOC_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
-// Split-K partial buffer size of one training pass: the largest of the three
-// weight-gradient reductions.
-int64_t partial_floats(const evoc_mlp* net, int64_t rows, int* s1, int* kc1, int* s2, int* kc2,
-                       int* s3, int64_t* rps3) {
+// Splits of a training pass's gradient reductions, and where their partials lie:
+// dW1 [s1][hid][in], dW2 [s2][hid][hid], dW3 [s3][out][hid], db2, db1 [s3][hid],
+// db3 [s3][out].
+struct GradSplits {
+  int s1, kc1, s2, kc2, s3;
+  int64_t rps3;
+  int64_t w1, w2, w3, b2, b1, b3, total;  // offsets in floats
+};
+GradSplits grad_splits(const evoc_mlp* net, int64_t rows) {
   const int sms = net->ctx->num_sms;
-  choose_splits(net->hid, net->in, (int)rows, sms, s1, kc1);
-  choose_splits(net->hid, net->hid, (int)rows, sms, s2, kc2);
+  GradSplits g{};
+  if (use_tcgen05()) {
+    choose_splits_tc(net->hid, net->in, (int)rows, sms, &g.s1, &g.kc1);
+    choose_splits_tc(net->hid, net->hid, (int)rows, sms, &g.s2, &g.kc2);
+  } else {
+    choose_splits(net->hid, net->in, (int)rows, sms, &g.s1, &g.kc1);
+    choose_splits(net->hid, net->hid, (int)rows, sms, &g.s2, &g.kc2);
+  }
   const int colblocks = (net->hid + 127) / 128;
-  int want3 = std::max(1, (2 * sms + colblocks - 1) / colblocks);
-  *rps3 = std::max<int64_t>(1, (rows + want3 - 1) / want3);
-  *s3 = (int)((rows + *rps3 - 1) / *rps3);
-  int t1, tk1, t2, tk2;  // the tcgen05 weight-gradient splits
-  choose_splits_tc(net->hid, net->in, (int)rows, sms, &t1, &tk1);
-  choose_splits_tc(net->hid, net->hid, (int)rows, sms, &t2, &tk2);
-  const int64_t p1 = (int64_t)std::max(*s1, t1) * net->hid * net->in;
-  const int64_t p2 = (int64_t)std::max(*s2, t2) * net->hid * net->hid;
-  const int64_t p3 = (int64_t)*s3 * ((int64_t)net->out * net->hid + 2 * net->hid + net->out);
-  return std::max(p1, std::max(p2, p3));
+  const int want3 = std::max(1, (2 * sms + colblocks - 1) / colblocks);
+  g.rps3 = std::max<int64_t>(1, (rows + want3 - 1) / want3);
+  g.s3 = (int)((rows + g.rps3 - 1) / g.rps3);
+  g.w1 = 0;
+  g.w2 = g.w1 + (int64_t)g.s1 * net->hid * net->in;
+  g.w3 = g.w2 + (int64_t)g.s2 * net->hid * net->hid;
+  g.b2 = g.w3 + (int64_t)g.s3 * net->out * net->hid;
+  g.b1 = g.b2 + (int64_t)g.s3 * net->hid;
+  g.b3 = g.b1 + (int64_t)g.s3 * net->hid;
+  g.total = g.b3 + (int64_t)g.s3 * net->out;
+  return g;
 }
 
 void alloc_scratch(const evoc_mlp* net, MlpScratch& sc, int64_t rows, bool train) {
@@ -1629,16 +1858,13 @@ void alloc_scratch(const evoc_mlp* net, MlpScratch& sc, int64_t rows, bool train
     sc.ypart.alloc((size_t)tc_col_tiles(net->hid) * rows * net->out, s);
     return;
   }
-  int s1, kc1, s2, kc2, s3;
-  int64_t rps3;
-  const int64_t pf = partial_floats(net, rows, &s1, &kc1, &s2, &kc2, &s3, &rps3);
   sc.h1.alloc((size_t)rows * net->hid, s);
   sc.h2.alloc((size_t)rows * net->hid, s);
   sc.dh1.alloc((size_t)rows * net->hid, s);
   sc.dh2.alloc((size_t)rows * net->hid, s);
   sc.target.alloc((size_t)rows * net->out, s);
   sc.dy.alloc((size_t)rows * net->out, s);
-  sc.part.alloc((size_t)pf, s);
+  sc.part.alloc((size_t)grad_splits(net, rows).total, s);
   sc.loss_part.alloc((size_t)sc.head_grid, s);
   if (use_tcgen05()) {
     const int64_t ldt = transposed_ld(rows);
@@ -1647,7 +1873,6 @@ void alloc_scratch(const evoc_mlp* net, MlpScratch& sc, int64_t rows, bool train
     sc.dh1t.alloc((size_t)net->hid * ldt, s);
     sc.dh2t.alloc((size_t)net->hid * ldt, s);
   }
-  sc.rows.alloc((size_t)rows, s);
 }
 
 // Forward over `rows` rows of BF16 input x (device); inference writes y.
@@ -1681,7 +1906,7 @@ void forward(const evoc_mlp* net, const bf16* x, int64_t rows, MlpScratch& sc, b
   }
   launch_forward_gemm(g2, net->ctx);
   if (!train) {
-    k_head<false><<<head_grid_for(net, rows), HEAD_THREADS, head_smem(net), s>>>(
+    (net->out <= 8 ? k_head<false, 8> : k_head<false, MLP_MAX_OUT>)<<<head_grid_for(net, rows), HEAD_THREADS, head_smem(net), s>>>(
         sc.a2.get(), nullptr, net->hid, net->out, rows, wb + net->o_w3, mp + net->o_b3, y,
         nullptr, 0.0f, nullptr, nullptr, nullptr);
     EVOC_CHECK_LAUNCH();
@@ -1689,132 +1914,105 @@ void forward(const evoc_mlp* net, const bf16* x, int64_t rows, MlpScratch& sc, b
 }
 
 // Forward + backward over the batch in sc.x / sc.target (rows rows); leaves
-// the packed gradient in net->grad and the mean-squared error in *loss_dst.
-void forward_backward(evoc_mlp* net, int64_t rows, MlpScratch& sc, float* loss_dst) {
+// the packed gradient in net->grad and the mean-squared error in *loss_dst, and
+// with `adam` takes its step.
+void forward_backward(evoc_mlp* net, int64_t rows, MlpScratch& sc, float* loss_dst,
+                      const AdamArgs* adam) {
   cudaStream_t s = net->ctx->stream;
   const bf16* wb = net->wb.get();
   const float* mp = net->master.get();
   forward(net, sc.x.get(), rows, sc, true, nullptr);
   const int hg = head_grid_for(net, rows);
   const float scale = 1.0f / (float)((double)rows * net->out);
-  k_head<true><<<hg, HEAD_THREADS, head_smem(net), s>>>(
+  (net->out <= 8 ? k_head<true, 8> : k_head<true, MLP_MAX_OUT>)<<<hg, HEAD_THREADS, head_smem(net), s>>>(
       sc.a2.get(), sc.h2.get(), net->hid, net->out, rows, wb + net->o_w3, mp + net->o_b3,
       nullptr, sc.target.get(), 2.0f * scale, sc.dy.get(), sc.dh2.get(), sc.loss_part.get());
   EVOC_CHECK_LAUNCH();
-  k_loss_total<<<1, 32, 0, s>>>(sc.loss_part.get(), hg, scale, loss_dst);
-  EVOC_CHECK_LAUNCH();
-  int s1, kc1, s2, kc2, s3;
-  int64_t rps3;
-  partial_floats(net, rows, &s1, &kc1, &s2, &kc2, &s3, &rps3);
-  float* grad = net->grad.get();
-  const int64_t cw1 = (int64_t)net->hid * net->in, cw2 = (int64_t)net->hid * net->hid;
+  const GradSplits gsp = grad_splits(net, rows);
+  float* part = sc.part.get();
+  GemmArgs gd{};  // dH1 = (dH2 W2) * gelu'(H1)
+  gd.a = sc.dh2.get(); gd.lda = net->hid;
+  gd.M = (int)rows; gd.N = net->hid; gd.K = net->hid;
+  gd.pre = sc.h1.get();
+  gd.outb = sc.dh1.get();
+  GemmArgs gw2{}, gw1{};  // dW2 = dH2^T A1, dW1 = dH1^T X
+  gw2.M = net->hid; gw2.N = net->hid; gw2.K = (int)rows; gw2.kchunk = gsp.kc2;
+  gw2.outf = part + gsp.w2;
+  gw1.M = net->hid; gw1.N = net->in; gw1.K = (int)rows; gw1.kchunk = gsp.kc1;
+  gw1.outf = part + gsp.w1;
   if (use_tcgen05()) {
-    // dH1 = (dH2 W2) * gelu'(H1) with W2^T as the K-major B operand.
     const HeadArgs none{};
-    GemmArgs gd{};
-    gd.a = sc.dh2.get(); gd.lda = net->hid;
-    gd.b = net->w2t.get(); gd.ldb = net->hid;
-    gd.M = (int)rows; gd.N = net->hid; gd.K = net->hid;
+    gd.b = net->w2t.get(); gd.ldb = net->hid;  // W2^T as the K-major B operand
     gd.kchunk = (net->hid + TC_BK - 1) / TC_BK * TC_BK;
-    gd.pre = sc.h1.get();
-    gd.outb = sc.dh1.get();
     launch_tc<2, TC_GRAD>(gd, none, net->ctx);
     // Weight gradients over the batch: K-major copies [features][batch].
     const int64_t ldt = transposed_ld(rows);
-    transpose_bf16(sc.dh2.get(), net->hid, (int)rows, net->hid, sc.dh2t.get(), ldt, s);
-    transpose_bf16(sc.a1.get(), net->hid, (int)rows, net->hid, sc.a1t.get(), ldt, s);
-    transpose_bf16(sc.dh1.get(), net->hid, (int)rows, net->hid, sc.dh1t.get(), ldt, s);
-    transpose_bf16(sc.x.get(), net->in, (int)rows, net->in, sc.xt.get(), ldt, s);
-    int t2, tk2, t1, tk1;
-    choose_splits_tc(net->hid, net->hid, (int)rows, net->ctx->num_sms, &t2, &tk2);
-    choose_splits_tc(net->hid, net->in, (int)rows, net->ctx->num_sms, &t1, &tk1);
-    GemmArgs gw2{};  // dW2 = dH2^T A1
+    const Transposes tr{{sc.dh2.get(), sc.a1.get(), sc.dh1.get(), sc.x.get()},
+                        {sc.dh2t.get(), sc.a1t.get(), sc.dh1t.get(), sc.xt.get()},
+                        {net->hid, net->hid, net->hid, net->in}};
+    transpose_bf16(tr, 4, (int)rows, ldt, s);
     gw2.a = sc.dh2t.get(); gw2.lda = ldt;
     gw2.b = sc.a1t.get(); gw2.ldb = ldt;
-    gw2.M = net->hid; gw2.N = net->hid; gw2.K = (int)rows; gw2.kchunk = tk2;
-    gw2.outf = sc.part.get();
-    launch_tc<2, TC_F32>(gw2, none, net->ctx, t2);
-    k_sum_splits<<<blocks_for(cw2, 256), 256, 0, s>>>(sc.part.get(), t2, cw2, grad + net->o_w2);
-    EVOC_CHECK_LAUNCH();
-    GemmArgs gw1{};  // dW1 = dH1^T X
+    launch_tc<2, TC_F32>(gw2, none, net->ctx, gsp.s2);
     gw1.a = sc.dh1t.get(); gw1.lda = ldt;
     gw1.b = sc.xt.get(); gw1.ldb = ldt;
-    gw1.M = net->hid; gw1.N = net->in; gw1.K = (int)rows; gw1.kchunk = tk1;
-    gw1.outf = sc.part.get();
-    launch_tc<2, TC_F32>(gw1, none, net->ctx, t1);
-    k_sum_splits<<<blocks_for(cw1, 256), 256, 0, s>>>(sc.part.get(), t1, cw1, grad + net->o_w1);
-    EVOC_CHECK_LAUNCH();
+    launch_tc<2, TC_F32>(gw1, none, net->ctx, gsp.s1);
   } else {
-    // dH1 = (dH2 W2) * gelu'(H1): W2 is [out][in] = [K][N], read MN-major.
-    GemmArgs gd{};
-    gd.a = sc.dh2.get(); gd.lda = net->hid;
-    gd.b = wb + net->o_w2; gd.ldb = net->hid;
-    gd.M = (int)rows; gd.N = net->hid; gd.K = net->hid;
+    gd.b = wb + net->o_w2; gd.ldb = net->hid;  // W2 is [out][in] = [K][N], read MN-major
     gd.kchunk = ((net->hid + GBK - 1) / GBK) * GBK;
-    gd.pre = sc.h1.get();
-    gd.outb = sc.dh1.get();
     launch_gemm<true, false, EPI_GELU_GRAD>(gd, 1, s);
-    // dW2 = dH2^T A1 (both [batch][hidden]: MN-major with the batch as K).
-    GemmArgs gw2{};
+    // [batch][features] operands: MN-major with the batch as K
     gw2.a = sc.dh2.get(); gw2.lda = net->hid;
     gw2.b = sc.a1.get(); gw2.ldb = net->hid;
-    gw2.M = net->hid; gw2.N = net->hid; gw2.K = (int)rows; gw2.kchunk = kc2;
-    gw2.outf = sc.part.get();
-    launch_gemm<false, false, EPI_PARTIAL>(gw2, s2, s);
-    k_sum_splits<<<blocks_for(cw2, 256), 256, 0, s>>>(sc.part.get(), s2, cw2, grad + net->o_w2);
-    EVOC_CHECK_LAUNCH();
-    // dW1 = dH1^T X.
-    GemmArgs gw1{};
+    launch_gemm<false, false, EPI_PARTIAL>(gw2, gsp.s2, s);
     gw1.a = sc.dh1.get(); gw1.lda = net->hid;
     gw1.b = sc.x.get(); gw1.ldb = net->in;
-    gw1.M = net->hid; gw1.N = net->in; gw1.K = (int)rows; gw1.kchunk = kc1;
-    gw1.outf = sc.part.get();
-    launch_gemm<false, false, EPI_PARTIAL>(gw1, s1, s);
-    k_sum_splits<<<blocks_for(cw1, 256), 256, 0, s>>>(sc.part.get(), s1, cw1, grad + net->o_w1);
-    EVOC_CHECK_LAUNCH();
+    launch_gemm<false, false, EPI_PARTIAL>(gw1, gsp.s1, s);
   }
-  // dW3, db2, db3 in one column pass; then db1.
-  float* pw3 = sc.part.get();
-  float* pb2 = pw3 + (int64_t)s3 * net->out * net->hid;
-  float* pb3 = pb2 + (int64_t)s3 * net->hid;
-  float* pb1 = pb3 + (int64_t)s3 * net->out;
-  dim3 cg((unsigned)((net->hid + 127) / 128), (unsigned)s3);
-  k_colreduce<<<cg, 128, 0, s>>>(sc.dy.get(), net->out, sc.a2.get(), sc.dh2.get(), net->hid,
-                                 rows, rps3, pw3, pb2, pb3);
+  dim3 cg((unsigned)((net->hid + COL_THREADS - 1) / COL_THREADS), (unsigned)gsp.s3);
+  auto* col = net->out <= 8 ? k_colreduce<8> : k_colreduce<16>;
+  const size_t csmem = net->out <= 8 ? sizeof(ColSmem<8>) : sizeof(ColSmem<16>);
+  EVOC_CUDA(cudaFuncSetAttribute((const void*)col, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)csmem));
+  col<<<cg, COL_THREADS, csmem, s>>>(
+      sc.dy.get(), net->out, sc.a2.get(), sc.dh2.get(), sc.dh1.get(), net->hid, rows, gsp.rps3,
+      part + gsp.w3, part + gsp.b2, part + gsp.b1, part + gsp.b3);
   EVOC_CHECK_LAUNCH();
-  k_colreduce<<<cg, 128, 0, s>>>(nullptr, 0, nullptr, sc.dh1.get(), net->hid, rows, rps3,
-                                 nullptr, pb1, nullptr);
-  EVOC_CHECK_LAUNCH();
-  const int64_t cw3 = (int64_t)net->out * net->hid;
-  k_sum_splits<<<blocks_for(cw3, 256), 256, 0, s>>>(pw3, s3, cw3, grad + net->o_w3);
-  k_sum_splits<<<blocks_for(net->hid, 256), 256, 0, s>>>(pb2, s3, net->hid, grad + net->o_b2);
-  k_sum_splits<<<1, 32, 0, s>>>(pb3, s3, net->out, grad + net->o_b3);
-  k_sum_splits<<<blocks_for(net->hid, 256), 256, 0, s>>>(pb1, s3, net->hid, grad + net->o_b1);
+  const int64_t hid = net->hid;
+  const GradSegments gs{{{part + gsp.w1, net->o_w1, hid * net->in, gsp.s1},
+                         {part + gsp.b1, net->o_b1, hid, gsp.s3},
+                         {part + gsp.w2, net->o_w2, hid * hid, gsp.s2},
+                         {part + gsp.b2, net->o_b2, hid, gsp.s3},
+                         {part + gsp.w3, net->o_w3, net->out * hid, gsp.s3},
+                         {part + gsp.b3, net->o_b3, net->out, gsp.s3}}};
+  const unsigned fgrid = blocks_for(net->n_params, 256) + 1;
+  if (adam)
+    k_finish_step<true><<<fgrid, 256, 0, s>>>(gs, net->n_params, net->grad.get(), *adam,
+                                              sc.loss_part.get(), hg, scale, loss_dst);
+  else
+    k_finish_step<false><<<fgrid, 256, 0, s>>>(gs, net->n_params, net->grad.get(), AdamArgs{},
+                                               sc.loss_part.get(), hg, scale, loss_dst);
   EVOC_CHECK_LAUNCH();
 }
 
-void refresh_w2t(evoc_mlp* net) {
-  transpose_bf16(net->wb.get() + net->o_w2, net->hid, net->hid, net->hid, net->w2t.get(),
-                 net->hid, net->ctx->stream);
-}
-
-void adam_step(evoc_mlp* net, float lr, float beta1, float beta2, float eps) {
+// The next Adam step's arguments.
+AdamArgs adam_args(evoc_mlp* net, float lr, float beta1, float beta2, float eps) {
   net->adam_steps += 1;
   const double t = (double)net->adam_steps;
   const float bc1 = (float)(1.0 / (1.0 - std::pow((double)beta1, t)));
   const float bc2 = (float)(1.0 / (1.0 - std::pow((double)beta2, t)));
-  k_adam<<<blocks_for(net->n_params, 256), 256, 0, net->ctx->stream>>>(
-      net->master.get(), net->adam_m.get(), net->adam_v.get(), net->grad.get(), net->wb.get(),
-      net->n_params, lr, beta1, beta2, eps, bc1, bc2);
-  EVOC_CHECK_LAUNCH();
-  refresh_w2t(net);
+  return AdamArgs{net->master.get(), net->adam_m.get(), net->adam_v.get(), net->wb.get(),
+                  net->w2t.get(),    net->o_w2,         net->hid,          lr,
+                  beta1,             beta2,             eps,               bc1,
+                  bc2};
 }
 
 void refresh_bf16(evoc_mlp* net) {
   k_to_bf16<<<blocks_for(net->n_params, 256), 256, 0, net->ctx->stream>>>(
       net->master.get(), net->n_params, net->wb.get());
   EVOC_CHECK_LAUNCH();
-  refresh_w2t(net);
+  const Transposes t{{net->wb.get() + net->o_w2}, {net->w2t.get()}, {net->hid}};
+  transpose_bf16(t, 1, net->hid, net->hid, net->ctx->stream);
 }
 
 // splitmix64: the host-side generator of the initial weights.
@@ -2064,7 +2262,7 @@ void mlp_gradients_host(evoc_mlp* net, const float* x, const float* target, int6
   EVOC_CUDA(cudaMemcpyAsync(sc.target.get(), target, (size_t)n * net->out * sizeof(float),
                             cudaMemcpyHostToDevice, s));
   to_bf16_device(net->ctx, xf.get(), n * net->in, reinterpret_cast<uint16_t*>(sc.x.get()));
-  forward_backward(net, n, sc, ld.get());
+  forward_backward(net, n, sc, ld.get(), nullptr);
   EVOC_CUDA(cudaMemcpyAsync(grad, net->grad.get(), net->grad.bytes(), cudaMemcpyDeviceToHost, s));
   EVOC_CUDA(cudaMemcpyAsync(loss, ld.get(), sizeof(float), cudaMemcpyDeviceToHost, s));
   check_status(net->ctx, "evoc_mlp_gradients");
@@ -2110,81 +2308,77 @@ void mlp_fit_device(evoc_mlp* net, int32_t m, const uint16_t* const* xs,
   MlpScratch sp;  // prediction on an alignment sample
   alloc_scratch(net, sp, std::min<int64_t>(max_sample, PREDICT_CHUNK), false);
   DevBuf<bf16> xs_s((size_t)max_sample * net->in, s);
-  DevBuf<float> pred((size_t)max_sample * d, s), tsamp((size_t)max_sample * d, s);
-  DevBuf<float> aff((size_t)d * d + 2 * d, s);
+  DevBuf<float> pred((size_t)max_sample * d, s);
   DevBuf<float> losses((size_t)std::max(1, p->steps), s);
-  std::vector<float> hp((size_t)max_sample * d), ht((size_t)max_sample * d);
-  std::vector<float> haff((size_t)d * d + 2 * d);
+  // per instance: block sums of the columns, means, block cross-covariances
+  const int ab = (int)std::min<int64_t>(net->ctx->num_sms, blocks_for(max_sample, ALIGN_ROWS));
+  const size_t per_inst = (size_t)ab * 2 * MLP_MAX_OUT + 2 * MLP_MAX_OUT + (size_t)ab * d * d;
+  const size_t host_off = (size_t)ab * 2 * MLP_MAX_OUT, host_len = per_inst - host_off;
+  const size_t naff = (size_t)d * d + 2 * d;
+  DevBuf<double> sums(per_inst * m, s);
+  DevBuf<float> aff(naff * m, s);
+  std::vector<double> hsum(host_len * m);
+  std::vector<float> haff(naff * m);
 
-  auto realign = [&](int32_t i) {
-    const int64_t k = ns_sample[i];
-    k_gather_rows<<<blocks_for(k * net->in / 2, 256), 256, 0, s>>>(
-        reinterpret_cast<const uint32_t*>(xs[i]), net->in / 2, sample[i].get(), k,
-        reinterpret_cast<uint32_t*>(xs_s.get()));
-    EVOC_CHECK_LAUNCH();
-    k_gather_rows<<<blocks_for(k * d, 256), 256, 0, s>>>(
-        reinterpret_cast<const uint32_t*>(layouts[i]), d, sample[i].get(), k,
-        reinterpret_cast<uint32_t*>(tsamp.get()));
-    EVOC_CHECK_LAUNCH();
-    const int64_t chunk = std::min<int64_t>(k, PREDICT_CHUNK);
-    for (int64_t r0 = 0; r0 < k; r0 += chunk) {
-      const int64_t rows = std::min(chunk, k - r0);
-      forward(net, xs_s.get() + r0 * net->in, rows, sp, false, pred.get() + r0 * d);
+  // Every instance's prediction sums, one wait, the rotations on the host, then
+  // the aligned layouts.
+  auto realign = [&]() {
+    for (int32_t i = 0; i < m; ++i) {
+      const int64_t k = ns_sample[i];
+      k_gather_rows<<<blocks_for(k * 32, 256), 256, 0, s>>>(
+          reinterpret_cast<const uint4*>(xs[i]), net->in / 8, sample[i].get(), k,
+          reinterpret_cast<uint4*>(xs_s.get()));
+      EVOC_CHECK_LAUNCH();
+      const int64_t chunk = std::min<int64_t>(k, PREDICT_CHUNK);
+      for (int64_t r0 = 0; r0 < k; r0 += chunk) {
+        const int64_t rows = std::min(chunk, k - r0);
+        forward(net, xs_s.get() + r0 * net->in, rows, sp, false, pred.get() + r0 * d);
+      }
+      double* si = sums.get() + per_inst * i;
+      k_align_sums<<<ab, ALIGN_THREADS, 0, s>>>(layouts[i], sample[i].get(), pred.get(), k, d, si);
+      EVOC_CHECK_LAUNCH();
+      k_align_cov<<<ab, ALIGN_THREADS, 0, s>>>(layouts[i], sample[i].get(), pred.get(), k, d, si,
+                                               ab, si + host_off, si + host_off + 2 * MLP_MAX_OUT);
+      EVOC_CHECK_LAUNCH();
+      EVOC_CUDA(cudaMemcpyAsync(hsum.data() + host_len * i, si + host_off,
+                                host_len * sizeof(double), cudaMemcpyDeviceToHost, s));
     }
-    EVOC_CUDA(cudaMemcpyAsync(hp.data(), pred.get(), (size_t)k * d * sizeof(float),
-                              cudaMemcpyDeviceToHost, s));
-    EVOC_CUDA(cudaMemcpyAsync(ht.data(), tsamp.get(), (size_t)k * d * sizeof(float),
-                              cudaMemcpyDeviceToHost, s));
-    EVOC_CUDA(cudaStreamSynchronize(s));
-    std::vector<double> tm(d, 0.0), pm(d, 0.0), mm((size_t)d * d, 0.0), rr((size_t)d * d);
-    for (int64_t r = 0; r < k; ++r)
+    check_status(net->ctx, "evoc_mlp_fit_device (alignment)");  // synchronises
+    for (int32_t i = 0; i < m; ++i) {
+      const double* means = hsum.data() + host_len * i;
+      const double* cov = means + 2 * MLP_MAX_OUT;
+      std::vector<double> mm((size_t)d * d, 0.0), rr((size_t)d * d);
+      for (int b = 0; b < ab; ++b)
+        for (int q = 0; q < d * d; ++q) mm[q] += cov[(size_t)b * d * d + q];
+      procrustes(mm.data(), d, rr.data());
+      float* ha = haff.data() + naff * i;
+      for (int j = 0; j < d * d; ++j) ha[j] = (float)rr[j];
       for (int j = 0; j < d; ++j) {
-        tm[j] += ht[(size_t)r * d + j];
-        pm[j] += hp[(size_t)r * d + j];
+        ha[(size_t)d * d + j] = (float)means[j];
+        ha[(size_t)d * d + d + j] = (float)means[MLP_MAX_OUT + j];
       }
-    for (int j = 0; j < d; ++j) {
-      tm[j] /= (double)k;
-      pm[j] /= (double)k;
     }
-    for (int64_t r = 0; r < k; ++r)
-      for (int a = 0; a < d; ++a) {
-        const double ta = ht[(size_t)r * d + a] - tm[a];
-        for (int b = 0; b < d; ++b) mm[(size_t)a * d + b] += ta * (hp[(size_t)r * d + b] - pm[b]);
-      }
-    procrustes(mm.data(), d, rr.data());
-    for (int j = 0; j < d * d; ++j) haff[j] = (float)rr[j];
-    for (int j = 0; j < d; ++j) {
-      haff[(size_t)d * d + j] = (float)tm[j];
-      haff[(size_t)d * d + d + j] = (float)pm[j];
-    }
-    check_status(net->ctx, "evoc_mlp_fit_device (alignment)");
     EVOC_CUDA(cudaMemcpyAsync(aff.get(), haff.data(), haff.size() * sizeof(float),
                               cudaMemcpyHostToDevice, s));
-    k_affine_rows<<<blocks_for(ns[i], 256), 256, 0, s>>>(layouts[i], ns[i], d, aff.get(),
-                                                         aligned[i].get());
-    EVOC_CHECK_LAUNCH();
-    EVOC_CUDA(cudaStreamSynchronize(s));  // haff is reused by the next call
+    for (int32_t i = 0; i < m; ++i) {
+      k_affine_rows<<<blocks_for(ns[i], 256), 256, 0, s>>>(layouts[i], ns[i], d,
+                                                           aff.get() + naff * i,
+                                                           aligned[i].get());
+      EVOC_CHECK_LAUNCH();
+    }
   };
 
   for (int32_t step = 0; step < p->steps; ++step) {
-    if (step % p->align_every == 0)
-      for (int32_t i = 0; i < m; ++i) realign(i);
+    if (step % p->align_every == 0) realign();
     const int32_t i = step % m;
-    k_sample_rows<<<blocks_for(batch, 256), 256, 0, s>>>(sc.rows.get(), batch, (uint32_t)ns[i],
-                                                         p->seed, (uint32_t)step);
+    k_draw_batch<<<blocks_for(batch * 32, 256), 256, 0, s>>>(
+        reinterpret_cast<const bf16*>(xs[i]), net->in, aligned[i].get(), d, batch,
+        (uint32_t)ns[i], p->seed, (uint32_t)step, sc.x.get(), sc.target.get());
     EVOC_CHECK_LAUNCH();
-    k_gather_rows<<<blocks_for(batch * net->in / 2, 256), 256, 0, s>>>(
-        reinterpret_cast<const uint32_t*>(xs[i]), net->in / 2, sc.rows.get(), batch,
-        reinterpret_cast<uint32_t*>(sc.x.get()));
-    EVOC_CHECK_LAUNCH();
-    k_gather_rows<<<blocks_for(batch * d, 256), 256, 0, s>>>(
-        reinterpret_cast<const uint32_t*>(aligned[i].get()), d, sc.rows.get(), batch,
-        reinterpret_cast<uint32_t*>(sc.target.get()));
-    EVOC_CHECK_LAUNCH();
-    forward_backward(net, batch, sc, losses.get() + step);
     const double frac = p->steps > 1 ? (double)step / (double)(p->steps - 1) : 0.0;
     const float lr = (float)((double)p->lr + ((double)p->lr_end - (double)p->lr) * frac);
-    adam_step(net, lr, p->beta1, p->beta2, p->eps);
+    const AdamArgs adam = adam_args(net, lr, p->beta1, p->beta2, p->eps);
+    forward_backward(net, batch, sc, losses.get() + step, &adam);
   }
   if (loss_history && p->steps > 0)
     EVOC_CUDA(cudaMemcpyAsync(loss_history, losses.get(), (size_t)p->steps * sizeof(float),
