@@ -503,13 +503,6 @@ __device__ __forceinline__ void ldcg8(const float* p, float* r) {  // through L2
                : "l"(p)
                : "memory");
 }
-__device__ __forceinline__ void ldcs8(const float* p, float* r) {  // streamed
-  asm volatile("ld.global.cs.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]),
-                 "=f"(r[6]), "=f"(r[7])
-               : "l"(p)
-               : "memory");
-}
 __device__ __forceinline__ void stcs8(float* p, const float* r) {
   asm volatile("st.global.cs.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(r[0]),
                "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "l"(p)
@@ -543,29 +536,7 @@ __device__ __forceinline__ void load_row(const float* __restrict__ p, float (&r)
   }
 }
 
-// An Adam moment row, streamed (through L2 with COH), and a row's streamed store.
-template <int DIMP, bool COH>
-__device__ __forceinline__ void load_moment(const float* p, float (&r)[DIMP]) {
-  if constexpr (DIMP % 8 == 0) {
-#pragma unroll
-    for (int i = 0; i < DIMP; i += 8) {
-      if constexpr (COH)
-        ldcg8(p + i, r + i);
-      else
-        ldcs8(p + i, r + i);
-    }
-  } else {
-    const float4* p4 = reinterpret_cast<const float4*>(p);
-#pragma unroll
-    for (int i = 0; i < DIMP / 4; ++i) {
-      const float4 x = COH ? __ldcg(p4 + i) : __ldcs(p4 + i);
-      r[4 * i + 0] = x.x;
-      r[4 * i + 1] = x.y;
-      r[4 * i + 2] = x.z;
-      r[4 * i + 3] = x.w;
-    }
-  }
-}
+// A row's streamed store.
 template <int DIMP>
 __device__ __forceinline__ void store_row(float* p, const float (&r)[DIMP]) {
   if constexpr (DIMP % 8 == 0) {
@@ -1433,18 +1404,29 @@ __global__ void k_slot_stats(const int64_t* __restrict__ tile_off,
   }
 }
 
-// One epoch, slots path: persistent warps; each takes the next tile (4 to 32 nodes)
-// in tile_order (heaviest first) from the epoch's work counter. The tile's
-// slots of the epoch come in windows of SLOT_WIN. Phase 1: each lane computes
-// slot contributions (attraction, embedding.rs:213-221, or repulsion,
-// embedding.rs:237-245, from the slot's source row and the node's own row)
-// into shared memory, SLOT_U slots at a time with all loads and gathers
-// issued first; the first slot of each node run records its position.
+// One epoch, slots path: persistent warps. Tiles (4 to 32 nodes) are taken in
+// tile_order (heaviest first): a warp's first by its own number, the others from
+// the epoch's work counter. The tile's slots of the epoch come in windows of WIN.
+// Phase 1: each lane computes slot contributions (attraction,
+// embedding.rs:213-221, or repulsion, embedding.rs:237-245, from the slot's
+// source row and the node's own row) into shared memory, SU slots at a time with
+// all gathers issued first; the first slot of each node run records its position.
 // Phase 2: the slots are node-major in the order of the reference's serial
 // sum (embedding.rs:194-253); each node present in the window is summed by
 // SLOT_PARTS lanes, each adding its DIMP / SLOT_PARTS dims of the node's run,
 // in slot order, onto the node's running gradient in shared memory.
 // Then Adam (embedding.rs:256-272), lane per node.
+//
+// Bound by latency: a slot (from DRAM) names the row to gather (from L2, at about
+// half its bandwidth), and seven blocks per SM are all the registers allow. So the
+// next group's slots are on their way while a group is gathered, and rows go
+// past L1, where no two gathers of a tile meet often enough to pay for the lines
+// that they evict. 50 epochs of 2 M nodes 12.4 ms -> 11.6 past L1
+// -> 10.9 with the slots ahead; 1.6 k nodes, 50 epochs 0.33 -> 0.31 ms with the
+// first tile taken without the counter -> 0.30. Without gain: the counter read
+// before Adam; moments prefetched to L2; the sums' shared loads one step ahead. A
+// loss: the counter read at the tile's start, 3.2 -> 3.6 ms at 500 k nodes (a warp
+// then holds two tiles, the heaviest first order ends unevenly).
 template <int DIMP>
 constexpr int slot_parts() { return DIMP >= 8 ? 2 : 1; }
 
@@ -1493,23 +1475,17 @@ __device__ __forceinline__ void slot_contrib(float (&c)[DIMP], bool neg,
   }
 }
 
-// Phase 1 for U slots per lane: window slots ib + 32 u + lane, u < U.
-template <int DIMP, int WIN, int U, bool COH>
+// Phase 1 for U slots per lane: window slots ib + 32 u + lane, u < U, in sl (past the
+// window's end: its last slot again, which is gathered but adds nothing).
+template <int DIMP, int WIN, int U>
 __device__ __forceinline__ void slot_group(const EpochArgs& a, SlotSmem<DIMP, WIN>& sm,
-                                           const uint32_t* __restrict__ wslots, int ib, int wn,
-                                           int lane, int& carry,
-                                           float two_noise, float gamma4) {
+                                           const uint32_t (&sl)[U], int ib, int wn, int lane,
+                                           int& carry, float two_noise, float gamma4) {
   const unsigned FULL = 0xffffffffu;
-  uint32_t sl[U];
   float row[U][DIMP];
 #pragma unroll
-  for (int u = 0; u < U; ++u) {  // past the end: the window's last slot again
-    const int i = ib + 32 * u + lane;
-    sl[u] = __ldcs(wslots + (i < wn ? i : wn - 1));
-  }
-#pragma unroll
   for (int u = 0; u < U; ++u)
-    load_row<DIMP, COH>(a.e_cur + (size_t)(sl[u] >> SLOT_ROW_SHIFT) * DIMP, row[u]);
+    load_row<DIMP, true>(a.e_cur + (size_t)(sl[u] >> SLOT_ROW_SHIFT) * DIMP, row[u]);
 #pragma unroll
   for (int u = 0; u < U; ++u) {  // run starts (a repeated last slot starts nothing)
     const int i = ib + 32 * u + lane;
@@ -1535,7 +1511,7 @@ __device__ __forceinline__ void slot_group(const EpochArgs& a, SlotSmem<DIMP, WI
   }
 }
 
-template <int DIMP, int WIN, int SU, bool COH>
+template <int DIMP, int WIN, int SU>
 __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN>& sm, int64_t tile,
                                           int lane) {
   const unsigned FULL = 0xffffffffu;
@@ -1546,26 +1522,36 @@ __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN
   {
     const float4* src = reinterpret_cast<const float4*>(a.e_cur + (size_t)v0 * DIMP);
     float4* dst = reinterpret_cast<float4*>(&sm.rows[0][0]);
-    for (int i = lane; i < nt * (DIMP / 4); i += 32) dst[i] = COH ? __ldcg(src + i) : __ldg(src + i);
+    for (int i = lane; i < nt * (DIMP / 4); i += 32) dst[i] = __ldcg(src + i);
     float4* sz = reinterpret_cast<float4*>(&sm.S[0][0]);
     for (int i = lane; i < nt * (DIMP / 4); i += 32) sz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const float two_noise = fmul(2.0f, a.noise);
   const float gamma4 = fmul(a.gamma, 4.0f);
   uint32_t act_mask = 0;
+  uint32_t nx[SU];  // the next group's slots, fetched while the group before it is gathered
+  if (s0 < s1) {
+#pragma unroll
+    for (int u = 0; u < SU; ++u) nx[u] = __ldcs(a.slots + min(s0 + 32 * u + lane, s1 - 1));
+  }
+  static_assert(WIN % (32 * SU) == 0, "a group does not cross a window");
   for (int64_t w0 = s0; w0 < s1; w0 += WIN) {
     const int wn = (int)min((int64_t)WIN, s1 - w0);
-    const uint32_t* wslots = a.slots + w0;
     sm.start[lane] = WIN;  // none
     __syncwarp();
     int carry = -1;  // node of the previous slot of the window
-    int ib = 0;
-    for (; ib + 32 * SU <= wn; ib += 32 * SU)
-      slot_group<DIMP, WIN, SU, COH>(a, sm, wslots, ib, wn, lane, carry, two_noise,
-                                     gamma4);
-    for (; ib < wn; ib += 32)
-      slot_group<DIMP, WIN, 1, COH>(a, sm, wslots, ib, wn, lane, carry, two_noise,
-                                    gamma4);
+    for (int ib = 0; ib < wn; ib += 32 * SU) {
+      uint32_t sl[SU];
+#pragma unroll
+      for (int u = 0; u < SU; ++u) sl[u] = nx[u];
+      const int64_t next = w0 + ib + 32 * SU;
+      if (next < s1) {
+#pragma unroll
+        for (int u = 0; u < SU; ++u)
+          nx[u] = __ldcs(a.slots + min(next + 32 * u + lane, s1 - 1));
+      }
+      slot_group<DIMP, WIN, SU>(a, sm, sl, ib, wn, lane, carry, two_noise, gamma4);
+    }
     __syncwarp();
     // run of node l: [start[l], first start of a later node or wn)
     const int st = sm.start[lane];
@@ -1617,8 +1603,8 @@ __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN
     }
     if (act) {
       float mm[DIMP], vv[DIMP];
-      load_moment<DIMP, COH>(a.m + q, mm);
-      load_moment<DIMP, COH>(a.v + q, vv);
+      load_row<DIMP, true>(a.m + q, mm);
+      load_row<DIMP, true>(a.v + q, vv);
 #pragma unroll
       for (int d = 0; d < DIMP; ++d) {  // scalar: a packed multiply feeding a packed
         // add did not reproduce the unfused result
@@ -1649,21 +1635,20 @@ __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4) k_epoch_slot(EpochArgs
   const int lane = threadIdx.x & 31;
   SlotSmem<DIMP, WIN>& sm = reinterpret_cast<SlotSmem<DIMP, WIN>*>(smem_raw)[threadIdx.x >> 5];
   const int64_t ntiles = a.ntiles;
-  for (;;) {
-    unsigned long long w = 0;
-    if (lane == 0) w = atomicAdd(a.work_ctr, 1ull);
+  const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  unsigned long long w = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  while ((int64_t)w < ntiles) {
+    slot_tile<DIMP, WIN, SU>(a, sm, (int64_t)a.tile_order[w], lane);
+    if (lane == 0) w = warps + atomicAdd(a.work_ctr, 1ull);
     w = __shfl_sync(0xffffffffu, w, 0);
-    if ((int64_t)w >= ntiles) break;
-    slot_tile<DIMP, WIN, SU, false>(a, sm, (int64_t)a.tile_order[w], lane);
   }
 }
 
 // ---------------------------------------------------------------------------
 // All epochs in one persistent launch (cooperative: every block resident).
-// Each epoch runs exactly as k_epoch_slot (tiles from the epoch's work
-// counter, heaviest first), reading rows and moments through L2 because they
-// were written earlier in the same launch; a grid-wide barrier separates the
-// epochs. The barrier waits at most GRID_WAIT_NS; on expiry it records
+// Each epoch runs exactly as k_epoch_slot, whose rows and moments are read
+// through L2 and may so have been written earlier in the same launch; a
+// grid-wide barrier separates the epochs. The barrier waits at most GRID_WAIT_NS; on expiry it records
 // ST_WAIT_TIMEOUT, raises an abort word that every block checks, and the
 // launch returns.
 // ---------------------------------------------------------------------------
@@ -1727,6 +1712,9 @@ __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4)
   const int lane = threadIdx.x & 31;
   SlotSmem<DIMP, WIN>& sm = reinterpret_cast<SlotSmem<DIMP, WIN>*>(smem_raw)[threadIdx.x >> 5];
   const int64_t ntiles = base.ntiles;
+  const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+  const unsigned long long first =
+      (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (int32_t t = x.t0; t < x.t1; ++t) {
     EpochArgs a = base;
     const int k = t - x.t0;
@@ -1739,12 +1727,11 @@ __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4)
     a.lr_ad = ep.y;
     a.epsc = ep.z;
     a.epoch = (uint32_t)t;
-    for (;;) {
-      unsigned long long w = 0;
-      if (lane == 0) w = atomicAdd(a.work_ctr, 1ull);
+    unsigned long long w = first;
+    while ((int64_t)w < ntiles) {
+      slot_tile<DIMP, WIN, SU>(a, sm, (int64_t)a.tile_order[w], lane);
+      if (lane == 0) w = warps + atomicAdd(a.work_ctr, 1ull);
       w = __shfl_sync(0xffffffffu, w, 0);
-      if ((int64_t)w >= ntiles) break;
-      slot_tile<DIMP, WIN, SU, true>(a, sm, (int64_t)a.tile_order[w], lane);
     }
     if (t + 1 < x.t1 && !grid_barrier(x.bar, x.nblocks, x.status)) return;
   }
