@@ -29,7 +29,6 @@
 #include "evoc_internal.h"
 #include "row_groups.cuh"
 
-#include <cuda_pipeline.h>
 
 #include <algorithm>
 #include <cmath>
@@ -592,77 +591,254 @@ __global__ void k_expand_rows(const int64_t* __restrict__ eptr, const uint2* __r
   }
 }
 
-// Column centring (serial column sums over all rows), then scaling.
-// One block: warps 1.. bring the rows into shared memory in chunks (a ring of
-// three filled by cp.async, rows padded to DIMP) while lane j < dim of warp 0
-// adds column j's values serially in row order. The chain of additions (4 cycles
-// each) is the bound, so the adding warp loads nothing from global memory, its
-// addresses are constant offsets and 16 values are read ahead of their additions.
-constexpr int COLMEAN_THREADS = 512;
-constexpr int COLMEAN_FLOATS = 4096;  // per chunk: 4096 / DIMP rows, a multiple of 16
-template <int DIMP>
-__global__ void __launch_bounds__(COLMEAN_THREADS) k_col_mean(const float* __restrict__ res,
-                                                             int64_t n, int32_t dim, float inv_n,
-                                                             float* __restrict__ mean) {
-  __shared__ __align__(16) float buf[3][COLMEAN_FLOATS];
-  constexpr int ROWS = COLMEAN_FLOATS / DIMP, U = 16, LOADERS = COLMEAN_THREADS - 32;
-  const int j = threadIdx.x;
-  const int64_t nch = (n + ROWS - 1) / ROWS;
-  const bool wide = dim == DIMP && (reinterpret_cast<uintptr_t>(res) & 15u) == 0;
-  auto load = [&](int64_t c) {
-    if (c < nch) {
-      float* dst = buf[c % 3];
-      const int64_t r0 = c * ROWS;
-      const int rows = (int)min((int64_t)ROWS, n - r0);
-      const float* src = res + r0 * dim;
-      if (wide) {
-        for (int q = j - 32; q < rows * (DIMP / 4); q += LOADERS)
-          __pipeline_memcpy_async(dst + 4 * q, src + 4 * q, 16);
-      } else {
-        for (int q = j - 32; q < rows * dim; q += LOADERS) {
-          const int r = q / dim;
-          __pipeline_memcpy_async(dst + r * DIMP + (q - r * dim), src + q, 4);
+// Column centring: serial column sums over all rows, then scaling.
+//
+// The sum s + x0 + x1 + ... rounds after each addition, so added one by one it is a
+// chain of n additions (5.8 cycles each fed from shared memory: 6.0 ms for 2 M rows).
+// But while the sum stays inside one binade its values are integers m of one unit
+// u, 2^23 < m < 2^24, and an addition is m += rint(x / u), where only a tie looks
+// at the sum: it goes to the even neighbour, so its step depends on m's parity. A
+// run of additions is then a pair of integers, its total step from an even and from
+// an odd m, and two runs compose: (a b)_p = a_p + b_((p + a_p) & 1). One block per
+// column takes CM_CHUNK values at a time: a thread composes CM_K of them, a block
+// scan gives each thread the m that its run begins with, and the thread checks that
+// its run keeps inside the binade. From the first run that does not (or whose
+// values are not finite, or above a quarter of the sum), warp 0 adds one by one;
+// twice as many each time that a chunk ends early, so that sums which never settle
+// cost little more than the chain. The result is the chain's, bit for bit.
+// 2 M rows of 8 columns, by the chain 6.0 ms whatever they hold: 0.42 ms with a mean
+// of three deviations, 0.74 ms of 0.01, 2.9 ms for pure noise (a sum that crosses
+// binades all the time), 5.9 ms for x, -x, x, -x (never in chunks).
+constexpr int CM_THREADS = 512;
+constexpr int CM_K = 16;
+constexpr int CM_CHUNK = CM_THREADS * CM_K;
+constexpr int CM_RUN = 256;        // additions of one serial unit
+constexpr int CM_MAX_UNITS = 64;
+constexpr float CM_ROUND = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
+constexpr int CM_WORTH = 512;      // values in steps that pay for a chunk's work
+// The first values are always added one by one: a young sum soon leaves its binade
+// (8192 values of noise 24 us so, 45 us in chunks).
+constexpr int64_t CM_HEAD = CM_CHUNK;
+// Above this many rows the columns are first copied out (k_columns): value i of a
+// column then lies in plane (i / 4) % 4, at float 4 (i / 16) + i % 4, so that the 16
+// values of each thread are four coalesced loads of a warp rather than 16 scattered.
+constexpr int64_t CM_DIRECT = CM_HEAD;
+__device__ __forceinline__ int64_t cm_index(int64_t i, int64_t groups) {
+  return ((i >> 2) & 3) * 4 * groups + 4 * (i >> 4) + (i & 3);
+}
+
+struct SumStep {
+  int even, odd;  // total step from an even and from an odd sum
+};
+// (Sums wrap where a run is already known to leave the binade.)
+__device__ __forceinline__ int wrap_add(int a, int b) { return (int)((unsigned)a + (unsigned)b); }
+__device__ __forceinline__ SumStep then(SumStep a, SumStep b) {
+  return {wrap_add(a.even, (a.even & 1) ? b.odd : b.even),
+          wrap_add(a.odd, (a.odd & 1) ? b.even : b.odd)};
+}
+// Lane l: the composition of lanes 0..l.
+__device__ __forceinline__ SumStep warp_steps(SumStep x, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    SumStep y;
+    y.even = __shfl_up_sync(0xffffffffu, x.even, o);
+    y.odd = __shfl_up_sync(0xffffffffu, x.odd, o);
+    if (lane >= o) x = then(y, x);
+  }
+  return x;
+}
+
+// COLS: column j is x[16 j ld ..], ld groups of CM_K values in cm_index order with
+// zeros from n up; else value i of column j is x[i * ld + j].
+template <bool COLS>
+__global__ void __launch_bounds__(CM_THREADS) k_col_mean(const float* __restrict__ x, int64_t n,
+                                                        int64_t ld, float inv_n,
+                                                        float* __restrict__ mean) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int WARPS = CM_THREADS / 32;
+  __shared__ SumStep agg[WARPS];
+  __shared__ int first_sh, m_sh;
+  __shared__ float s_sh;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  __shared__ __align__(16) float run[CM_RUN];
+  const float* col = COLS ? x + blockIdx.x * CM_K * ld : x + blockIdx.x;
+  auto at = [&](int64_t i) {
+    return i < n ? col[COLS ? cm_index(i, ld) : i * ld] : 0.0f;
+  };
+  auto load = [&](int64_t p, float (&v)[CM_K]) {  // values p .. p + CM_K - 1
+    if constexpr (COLS) {
+      const float4* c4 = reinterpret_cast<const float4*>(col) + p / CM_K;
+#pragma unroll
+      for (int q = 0; q < CM_K / 4; ++q) {
+        const float4 t = p < n ? __ldg(c4 + q * ld) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[4 * q] = t.x, v[4 * q + 1] = t.y, v[4 * q + 2] = t.z, v[4 * q + 3] = t.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < CM_K; ++k) v[k] = at(p + k);
+    }
+  };
+  float s = 0.0f;  // the sum of the values below pos, in every thread
+  int64_t pos = 0;  // a multiple of CM_K
+  int units = 1;
+  float v[CM_K];
+  int64_t held = -1;  // the chunk that v belongs to
+  while (pos < n) {
+    const int bits = __float_as_int(s), ex = (bits >> 23) & 255;
+    int first = 0;
+    if (ex >= 27 && ex <= 227) {  // a normal sum, and so are its unit and the inverse
+      const bool neg = bits < 0;
+      const float inv = __int_as_float((277 - ex) << 23 | (bits & 0x80000000));  // +-1 / u
+      const int m = (bits & 0x7fffff) | 0x800000;
+      if (held != pos) {
+        load(pos + tid * CM_K, v);
+        held = pos;
+      }
+      SumStep d = {0, 0};
+      int lo = 0, hi = 0;
+      bool near = true, tie = false;
+#pragma unroll
+      for (int k = 0; k < CM_K; ++k) {
+        const float t = fmul(v[k], inv);  // exact, or far below half a unit
+        near = near && fabsf(t) < 4194304.0f;  // no for NaN
+        const float y = fadd(t, CM_ROUND);
+        tie = tie || fabsf(fsub(t, fsub(y, CM_ROUND))) == 0.5f;
+        d.even = wrap_add(d.even, __float_as_int(y) - __float_as_int(CM_ROUND));
+        lo = min(lo, d.even);
+        hi = max(hi, d.even);
+      }
+      if (!near) d.even = lo = hi = 0;
+      d.odd = d.even;
+      if (near && tie) {
+        d = {0, 0};
+        lo = hi = 0;
+#pragma unroll
+        for (int k = 0; k < CM_K; ++k) {
+          const float t = fmul(v[k], inv), y = fadd(t, CM_ROUND);
+          const float rem = fsub(t, fsub(y, CM_ROUND));
+          const int i = __float_as_int(y) - __float_as_int(CM_ROUND);
+          const int w = fabsf(rem) == 0.5f ? (rem > 0.0f ? 1 : -1) : 0;  // from an odd sum
+          d.even += i + ((d.even & 1) ? w : 0);
+          d.odd += i + ((d.odd & 1) ? 0 : w);
+          lo = min(lo, d.even);
+          hi = max(hi, d.even);
         }
       }
+      const int64_t ahead = pos + CM_CHUNK;
+      if (ahead < n) {
+        load(ahead + tid * CM_K, v);
+        held = ahead;
+      }
+      const SumStep inc = warp_steps(d, lane);
+      SumStep before;
+      before.even = __shfl_up_sync(FULL, inc.even, 1);
+      before.odd = __shfl_up_sync(FULL, inc.odd, 1);
+      if (lane == 0) before = {0, 0};
+      if (lane == 31) agg[wid] = inc;
+      if (tid == 0) first_sh = CM_THREADS;
+      __syncthreads();
+      const SumStep all = warp_steps(lane < WARPS ? agg[lane] : SumStep{0, 0}, lane);
+      SumStep base;
+      base.even = __shfl_sync(FULL, all.even, max(wid - 1, 0));
+      base.odd = __shfl_sync(FULL, all.odd, max(wid - 1, 0));
+      if (wid > 0) before = then(base, before);
+      const int mt = wrap_add(m, (m & 1) ? before.odd : before.even);
+      // a run's values from an odd sum are within 2 of lo and hi
+      const bool leaves =
+          !near || wrap_add(mt, lo - 2) <= (1 << 23) || wrap_add(mt, hi + 2) >= (1 << 24);
+      const unsigned out = __ballot_sync(FULL, leaves);
+      if (lane == 0 && out) atomicMin(&first_sh, wid * 32 + __ffs(out) - 1);
+      __syncthreads();
+      first = first_sh;
+      if (first < CM_THREADS) {
+        if (tid == first) m_sh = mt;
+      } else if (tid == CM_THREADS - 1) {
+        m_sh = mt + ((mt & 1) ? d.odd : d.even);
+      }
+      __syncthreads();
+      // m_sh * u with the sign of s: exact, m_sh stays below 2^24
+      const float mag = fmul((float)m_sh, __int_as_float((ex - 23) << 23));
+      s = neg ? -mag : mag;
+      pos = min(n, pos + (int64_t)first * CM_K);
     }
-    __pipeline_commit();
-  };
-  float s = 0.0f;
-  if (j >= 32) {
-    load(0);
-    load(1);
-    __pipeline_wait_prior(1);
+    if (first < CM_THREADS && pos < n) {
+      if (first * CM_K >= CM_WORTH) units = 1;
+      const int64_t end = min(n, pos == 0 ? CM_HEAD : pos + (int64_t)CM_RUN * units);
+      if (wid == 0) {
+        float a = s, c[CM_RUN / 32];
+#pragma unroll
+        for (int q = 0; q < CM_RUN / 32; ++q) c[q] = at(pos + 32 * q + lane);
+        for (int64_t p = pos; p < end; p += CM_RUN) {
+          float nx[CM_RUN / 32];
+#pragma unroll
+          for (int q = 0; q < CM_RUN / 32; ++q) nx[q] = at(p + CM_RUN + 32 * q + lane);
+#pragma unroll
+          for (int q = 0; q < CM_RUN / 32; ++q) run[32 * q + lane] = c[q];
+          __syncwarp();
+#pragma unroll 16
+          for (int q = 0; q < CM_RUN / 4; ++q) {  // past the end: + 0, the sum is never -0
+            const float4 t = reinterpret_cast<const float4*>(run)[q];
+            a = fadd(fadd(fadd(fadd(a, t.x), t.y), t.z), t.w);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < CM_RUN / 32; ++q) c[q] = nx[q];
+        }
+        if (lane == 0) s_sh = a;
+      }
+      __syncthreads();
+      s = s_sh;
+      __syncthreads();
+      pos = end;
+      units = end == CM_HEAD ? 1 : min(2 * units, CM_MAX_UNITS);
+    } else {
+      units = 1;
+    }
+  }
+  if (tid == 0) mean[blockIdx.x] = fmul(s, inv_n);
+}
+
+// Rows (n x dim, dim <= 16) to columns of ld groups of CM_K floats in cm_index order,
+// zeros from n up.
+__global__ void __launch_bounds__(256) k_columns(const float* __restrict__ x, int64_t n,
+                                                int32_t dim, int64_t ld,
+                                                float* __restrict__ cols) {
+  __shared__ float tile[16][256 + 1];
+  const int64_t r0 = (int64_t)blockIdx.x * 256;
+  const int tid = threadIdx.x;
+  const int rows = (int)min((int64_t)256, n - r0);
+  for (int q = tid; q < rows * dim; q += 256) {
+    const int r = q / dim;
+    tile[q - r * dim][r] = __ldg(x + r0 * dim + q);
   }
   __syncthreads();
-  for (int64_t c = 0; c < nch; ++c) {
-    if (j >= 32) {
-      load(c + 2);
-      __pipeline_wait_prior(1);  // chunk c + 1 has landed
-    } else if (j < dim) {
-      const float* col = buf[c % 3] + j;
-      const int rows = (int)min((int64_t)ROWS, n - c * ROWS);
-      int r = 0;
-      if (rows >= U) {
-        float t[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) t[u] = col[u * DIMP];
-        for (r = U; r + U <= rows; r += U) {
-          float nx[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) nx[u] = col[(r + u) * DIMP];
-#pragma unroll
-          for (int u = 0; u < U; ++u) s = fadd(s, t[u]);
-#pragma unroll
-          for (int u = 0; u < U; ++u) t[u] = nx[u];
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) s = fadd(s, t[u]);  // rows r - U .. r - 1
-      }
-      for (; r < rows; ++r) s = fadd(s, col[r * DIMP]);
-    }
-    __syncthreads();
+  if (r0 + tid < ld * CM_K) {
+    cols += cm_index(r0 + tid, ld);
+    for (int j = 0; j < dim; ++j) cols[j * ld * CM_K] = tid < rows ? tile[j][tid] : 0.0f;
   }
-  if (j < dim) mean[j] = fmul(s, inv_n);
+}
+
+// mean[j] = inv_n * (the serial sum of column j of x).
+void column_means(const float* x, int64_t n, int32_t dim, float inv_n, float* mean,
+                  cudaStream_t s) {
+  DevBuf<float> cols;
+  const int64_t ld = (n + CM_K - 1) / CM_K;
+  bool by_cols = n > CM_DIRECT;
+  if (by_cols) {
+    try {
+      cols.alloc(ld * CM_K * dim, s);
+    } catch (const Error&) {  // no room for the copy: the strided form needs none
+      by_cols = false;
+    }
+  }
+  if (by_cols) {
+    k_columns<<<grid_of(ld * CM_K), 256, 0, s>>>(x, n, dim, ld, cols.get());
+    EVOC_CHECK_LAUNCH();
+    k_col_mean<true><<<dim, CM_THREADS, 0, s>>>(cols.get(), n, ld, inv_n, mean);
+  } else {
+    k_col_mean<false><<<dim, CM_THREADS, 0, s>>>(x, n, dim, inv_n, mean);
+  }
+  EVOC_CHECK_LAUNCH();
 }
 
 __global__ void k_center_scale(float* __restrict__ res, int64_t n, int32_t dim,
@@ -1082,9 +1258,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
     mark("expansion: rows");
     DevBuf<float> mean(dim, s);
     const float inv_n = (float)(1.0 / (double)n);
-    auto* col_mean = dim <= 4 ? k_col_mean<4> : dim <= 8 ? k_col_mean<8> : k_col_mean<16>;
-    col_mean<<<1, COLMEAN_THREADS, 0, s>>>(d_out, n, dim, inv_n, mean.get());
-    EVOC_CHECK_LAUNCH();
+    column_means(d_out, n, dim, inv_n, mean.get(), s);
     k_center_scale<<<grid_of(n * dim), 256, 0, s>>>(d_out, n, dim, mean.get(),
                                                     (float)lp.scaling);
     EVOC_CHECK_LAUNCH();
