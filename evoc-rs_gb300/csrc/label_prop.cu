@@ -43,9 +43,18 @@ __device__ __forceinline__ uint32_t lp_outlier_draw(uint64_t seed, uint64_t i, u
   return __umulhi(o.x, range);
 }
 
-__global__ void k_lp_fill(int32_t* __restrict__ labels, int64_t n) {
+// Unlabelled nodes, and the length of the longest row (starts below 0).
+__global__ void __launch_bounds__(256) k_lp_fill(int32_t* __restrict__ labels,
+                                                 const int64_t* __restrict__ indptr, int64_t n,
+                                                 int32_t* __restrict__ longest) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) labels[i] = -1;
+  int32_t len = 0;
+  if (i < n) {
+    labels[i] = -1;
+    len = (int32_t)min(indptr[i + 1] - indptr[i], (int64_t)0x7fffffff);
+  }
+  len = __reduce_max_sync(0xffffffffu, len);
+  if ((threadIdx.x & 31) == 0 && len > *(volatile int32_t*)longest) atomicMax(longest, len);
 }
 
 // Draw i labels node lp_seed_draw(i); the largest i drawn for a node is the
@@ -160,7 +169,7 @@ __global__ void k_lp_mark_seeds(const int64_t* __restrict__ indptr,
   lp_mark_row(indices, indptr[v], indptr[v + 1], threadIdx.x & 31, 32, 0, mark);
 }
 
-// One conservative iteration for labels below RG_LABELS, a warp per 32 nodes:
+// One conservative iteration for labels below RG_LABELS, a warp per npw nodes:
 // labelled nodes pass their label on, and each unlabelled node's row is read by
 // the whole warp (coalesced, 32 label gathers in flight), its labelled entries
 // are compacted and grouped on the SM (row_groups.cuh). The winner is the
@@ -177,16 +186,20 @@ __global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_lp_iter_rows(
     const float* __restrict__ w, int64_t n, const int32_t* __restrict__ in,
     int32_t* __restrict__ out, const int32_t* __restrict__ prev_changed,
     int32_t* __restrict__ changed, uint32_t* __restrict__ longs, int32_t* __restrict__ n_long,
-    int32_t round, const uint8_t* __restrict__ mark, uint8_t* __restrict__ next_mark) {
+    int32_t round, const uint8_t* __restrict__ mark, uint8_t* __restrict__ next_mark, int npw) {
   __shared__ RgWarp<RG_CAP> sm_all[RG_WARPS];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // launched while the round before ends (see the launch); the next may come likewise
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (prev_changed && *prev_changed == 0) return;
-  const int64_t v0 = ((int64_t)blockIdx.x * RG_WARPS + wid) * 32;
+  const int64_t v0 = ((int64_t)blockIdx.x * RG_WARPS + wid) * npw;
   if (v0 >= n) return;
   RgWarp<RG_CAP>& sm = sm_all[wid];
   const int64_t v = v0 + lane;
-  int32_t mine = v < n ? in[v] : 0;
+  const bool node = lane < npw && v < n;
+  int32_t mine = node ? in[v] : 0;
   const bool look = mine < 0 && (!mark || mark[v] == (uint8_t)round);
   const int64_t pb = look ? indptr[v] : 0, pe = look ? indptr[v + 1] : 0;
   const uint32_t lt = (1u << lane) - 1u;
@@ -253,7 +266,7 @@ __global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_lp_iter_rows(
       if (mark) lp_mark_row(indices, b, e, lane, 32, (uint8_t)(round + 1), next_mark);
     }
   }
-  if (v < n) out[v] = mine;
+  if (node) out[v] = mine;
   if (won) *changed = 1;
 }
 
@@ -402,16 +415,19 @@ __global__ void __launch_bounds__(32 * LP_WALK_WARPS) k_lp_walk(
   if (lane == 0) res[u] = (int32_t)lp_outlier_draw(seed, i, (uint32_t)max_label + 1u);
 }
 
-// Pointer jumping over the walk results; pointers only go to earlier
-// outliers, so the chains end.
-__global__ void k_lp_jump(int32_t* __restrict__ res, int64_t count, int32_t* __restrict__ changed) {
+// Pointer jumping over the walk results, up to LP_HOPS pointers a pass; pointers
+// only go to earlier outliers, so the chains end. *changed: one is left.
+constexpr int LP_HOPS = 64;
+__global__ void k_lp_jump(int32_t* res, int64_t count, int32_t* __restrict__ changed) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= count) return;
-  const int32_t r = res[u];
+  int32_t r = res[u];
   if (r >= 0) return;
-  const int32_t rk = res[-2 - (int64_t)r];
-  res[u] = rk;
-  *changed = 1;
+  // others' results are read as they are written: each is on the chain's way on
+  for (int h = 0; h < LP_HOPS && r < 0; ++h)
+    r = *(volatile const int32_t*)(res + (-2 - (int64_t)r));
+  *(volatile int32_t*)(res + u) = r;
+  if (r < 0) *changed = 1;
 }
 
 __global__ void k_lp_assign(const uint32_t* __restrict__ list, const int32_t* __restrict__ res,
@@ -486,11 +502,15 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
     throw Error(EVOC_ERR_INVALID_ARGUMENT, "approx_n_parts outside [0, 2^31)");
   if (n_iter < 0) throw Error(EVOC_ERR_INVALID_ARGUMENT, "n_iter < 0");
   DevBuf<int32_t> la(n, s), lb(n, s), flag(std::max(n_iter, 1), s);
-  k_lp_fill<<<grid_for(n), 256, 0, s>>>(la.get(), n);
+  DevBuf<int32_t> mx(2, s);  // largest label, longest row
+  EVOC_CUDA(cudaMemsetAsync(mx.get(), 0xff, mx.bytes(), s));  // -1
+  k_lp_fill<<<grid_for(n), 256, 0, s>>>(la.get(), g->indptr.get(), n, mx.get() + 1);
   if (approx_n_parts > 0)
     k_lp_seed<<<grid_for(approx_n_parts), 256, 0, s>>>(la.get(), n, approx_n_parts, seed);
   EVOC_CHECK_LAUNCH();
   if (approx_n_parts <= RG_LABELS) {
+    int32_t longest = 0;  // read while the seeds' kernels run
+    EVOC_CUDA(cudaMemcpyAsync(&longest, mx.get() + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     // n_iter rounds without the host: a round sees from the one before whether
     // anything is left to do
     DevBuf<uint32_t> longs(n, s);
@@ -513,17 +533,34 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
         EVOC_CHECK_LAUNCH();
       }
     }
-    const unsigned grid = (unsigned)((n + 32 * RG_WARPS - 1) / (32 * RG_WARPS));
+    // A warp takes its nodes' rows one after the other, 1 us and more each: as many
+    // as leave RG_NODE_WARPS warps per SM, down to one.
+    int npw = 32;
+    while (npw > 1 && n < (int64_t)npw * ctx->num_sms * RG_NODE_WARPS) npw /= 2;
+    const unsigned grid = (unsigned)((n + npw * RG_WARPS - 1) / (npw * RG_WARPS));
     const unsigned lgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms, nnz / RG_CAP));
+    EVOC_CUDA(cudaStreamSynchronize(s));
     for (int32_t it = 0; it < n_iter; ++it) {
       uint8_t* mark = use_marks ? marks.get() + (it & 1) * n : nullptr;
       uint8_t* next = use_marks ? marks.get() + (1 - (it & 1)) * n : nullptr;
-      k_lp_iter_rows<<<grid, 32 * RG_WARPS, 0, s>>>(
-          g->indptr.get(), g->indices.get(), g->weights.get(), n, la.get(), lb.get(),
-          it > 0 ? flag.get() + it - 1 : nullptr, flag.get() + it, longs.get(),
-          n_long.get() + it, it, mark, next);
-      EVOC_CHECK_LAUNCH();
-      if (nnz > RG_CAP) {
+      // A round may be brought onto the SMs while the one before still runs and waits
+      // there for its end (and for all that came before: the first has no such leave).
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(grid);
+      cfg.blockDim = dim3(32 * RG_WARPS);
+      cfg.stream = s;
+      cfg.attrs = &attr;
+      cfg.numAttrs = it > 0 ? 1 : 0;
+      EVOC_CUDA(cudaLaunchKernelEx(
+          &cfg, k_lp_iter_rows, (const int64_t*)g->indptr.get(),
+          (const uint32_t*)g->indices.get(), (const float*)g->weights.get(), n,
+          (const int32_t*)la.get(), lb.get(),
+          (const int32_t*)(it > 0 ? flag.get() + it - 1 : nullptr), flag.get() + it, longs.get(),
+          n_long.get() + it, it, (const uint8_t*)mark, next, npw));
+      if (longest > RG_CAP) {  // else no row can be left over
         k_lp_iter_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLongVotes), s>>>(
             g->indptr.get(), g->indices.get(), g->weights.get(), la.get(), lb.get(),
             flag.get() + it, longs.get(), n_long.get() + it, it, next);
@@ -535,15 +572,13 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
     lp_rounds_any_label(ctx, g, n_iter, la, lb, flag.get());
   }
   // mop-up of the nodes still unlabelled, in node order
-  DevBuf<int32_t> mx(1, s), unl(n, s);
+  DevBuf<int32_t> unl(n, s);
   DevBuf<int64_t> pos(n + 1, s);
-  EVOC_CUDA(cudaMemsetAsync(mx.get(), 0xff, sizeof(int32_t), s));  // -1
   k_lp_max<<<grid_for(n), 256, 0, s>>>(la.get(), n, mx.get(), unl.get());
   EVOC_CHECK_LAUNCH();
   exclusive_scan_i32_to_i64(ctx, unl.get(), pos.get(), n);
   int64_t count = 0;
   EVOC_CUDA(cudaMemcpyAsync(&count, pos.get() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  EVOC_CUDA(cudaStreamSynchronize(s));
   int32_t max_label = -1;
   EVOC_CUDA(cudaMemcpyAsync(&max_label, mx.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   EVOC_CUDA(cudaStreamSynchronize(s));
@@ -555,7 +590,7 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
         g->indptr.get(), g->indices.get(), la.get(), pos.get(), list.get(), count, max_label,
         seed + 2000, res.get());
     EVOC_CHECK_LAUNCH();
-    for (int pass = 0; pass < 64; ++pass) {  // chains halve per pass
+    for (int pass = 0; pass < 64; ++pass) {  // chains shrink at least by half per pass
       EVOC_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int32_t), s));
       k_lp_jump<<<grid_for(count), 256, 0, s>>>(res.get(), count, flag.get());
       EVOC_CHECK_LAUNCH();

@@ -25,6 +25,7 @@ constexpr uint32_t RG_POS = (1u << RG_POS_BITS) - 1u;
 constexpr int RG_LABELS = 16384;   // labels are below this (the long rows' dense table)
 constexpr int RG_WARPS = 8;        // warps per block of the short-row kernels
 constexpr int RG_BLOCKS = 6;       // and their blocks per SM (the rows' load chains need warps)
+constexpr int RG_NODE_WARPS = 12;  // warps per SM below which a warp takes fewer rows
 constexpr int RG_MID_WARPS = 4;    // and of the middle-row kernels
 
 template <int CAP>
