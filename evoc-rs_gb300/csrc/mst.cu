@@ -27,7 +27,8 @@
 //      kd_tree.rs:275-378), with the same three pruning rules; among equal
 //      values the smallest point index. A point whose nearest foreign point is
 //      known from an earlier round or from the kNN lists is not searched for
-//      again (k_mst_near_init). A per-component bound starts each other
+//      again (k_mst_near_init); late rounds search for the points of a leaf together
+//      (k_mst_noc_group). A per-component bound starts each other
 //      query just above it and is lowered while the round runs: first the
 //      smallest known value leaving the component (k_mst_bound), then the best
 //      value found so far by its points.
@@ -623,25 +624,63 @@ __global__ void k_mst_bound(const float* __restrict__ xs, int64_t n, int k,
 }
 
 // Known nearest points enter their component's pick; need[pos] = 1 for the
-// points that have to search.
+// points that have to search. With `groups`, the searching points of one component
+// in `width` consecutive places are put up for a common search
+// (k_mst_noc_group) when they are at least half of them: (leaf, lanes) is appended.
 __global__ void k_mst_select(int64_t n, const uint32_t* __restrict__ comp,
                              const float* __restrict__ core, const uint32_t* __restrict__ orig,
                              const uint32_t* __restrict__ near_j, const float* __restrict__ near_v,
                              const uint32_t* __restrict__ cbest,
-                             unsigned long long* __restrict__ ckey, int32_t* __restrict__ need) {
+                             unsigned long long* __restrict__ ckey, int32_t* __restrict__ need,
+                             uint2* __restrict__ groups, unsigned long long* __restrict__ n_groups,
+                             int width) {
+  const unsigned FULL = 0xffffffffu;
   const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= n) return;
-  const uint32_t qc = comp[pos], cb = cbest[qc];
-  const float v = near_v[pos];
+  const bool on = pos < n;
+  uint32_t qc = NO_POINT;
   bool search = false;
-  if (near_j[pos] != NO_POINT) {
-    const uint32_t vb = __float_as_uint(v);
-    if (vb <= cb) atomicMin(ckey + qc, ((unsigned long long)vb << 32) | orig[pos]);
-  } else {
-    const float bd = __uint_as_float(cb < FMAX_BITS ? cb + 1u : FMAX_BITS);
-    search = v < bd && !(core[pos] > bd);
+  if (on) {
+    qc = comp[pos];
+    const uint32_t cb = cbest[qc];
+    const float v = near_v[pos];
+    if (near_j[pos] != NO_POINT) {
+      const uint32_t vb = __float_as_uint(v);
+      if (vb <= cb) atomicMin(ckey + qc, ((unsigned long long)vb << 32) | orig[pos]);
+    } else {
+      const float bd = __uint_as_float(cb < FMAX_BITS ? cb + 1u : FMAX_BITS);
+      search = v < bd && !(core[pos] > bd);
+    }
   }
-  need[pos] = search ? 1 : 0;
+  if (groups && __popc(__ballot_sync(FULL, search)) >= width / 2) {  // the same in the warp
+    const uint32_t peers = __match_any_sync(FULL, search ? qc : NO_POINT);
+    const int same = search ? __popc(peers) : 0;
+    const int most = __reduce_max_sync(FULL, same);
+    const uint32_t c = __reduce_min_sync(FULL, search && same == most ? qc : NO_POINT);
+    if (most >= width / 2) {
+      const uint32_t lanes = __ballot_sync(FULL, search && qc == c);
+      const int lane = threadIdx.x & 31;
+      for (int at = 0; at < 32; at += width) {
+        const uint32_t some = lanes & (0xffffffffu >> (32 - width) << at);
+        if (__popc(some) >= width / 2 && lane == 0)
+          groups[atomicAdd(n_groups, 1ull)] = make_uint2((uint32_t)(pos / MST_LEAF), some);
+      }
+    }
+  }
+  if (on) need[pos] = search ? 1 : 0;
+}
+
+// Takes the groups' points off the others' list, unless there are fewer groups than
+// warps to serve them: a group's search is the longer one, and then sets the
+// round's time (1M points, the round of 1,465 components: 1.21 ms with, 0.79 without).
+__global__ void k_mst_take_groups(const uint2* __restrict__ groups,
+                                  const unsigned long long* __restrict__ n_groups,
+                                  unsigned long long min_groups, int32_t* __restrict__ need) {
+  const unsigned long long ng = *n_groups;
+  const unsigned long long g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (ng < min_groups || g >= ng) return;
+  const uint2 group = groups[g];
+  for (uint32_t m = group.y; m; m &= m - 1)
+    need[(int64_t)group.x * MST_LEAF + __ffs(m) - 1] = 0;
 }
 
 __global__ void k_mst_search_list(int64_t n, const int32_t* __restrict__ need,
@@ -657,7 +696,7 @@ __global__ void k_mst_search_list(int64_t n, const int32_t* __restrict__ need,
 // component), any other query by the full box and core_all. Otherwise a few stray
 // points next to a cluster keep the cluster's own points in every leaf that holds
 // one of them, although their large core distances rule them out (1M points: the
-// last three rounds 51.7 ms with pure-node marks only, 29.7 with this).
+// last three rounds 51.7 ms with pure-node marks only, 29.7 with this, walked by points).
 template <int DIMP>
 struct MstParts {
   uint32_t* maj;
@@ -857,6 +896,175 @@ __global__ void __launch_bounds__(32 * MST_WARPS, mst_blocks<DIMP>()) k_mst_noc(
         const uint32_t db = __float_as_uint(bd);
         atomicMin(ckey + qc, ((unsigned long long)db << 32) | orig[pos]);
       }
+    }
+  }
+}
+
+// The same for the searching points of one component in one leaf, a warp per
+// group: late rounds have most points search again up to their component's bound
+// and find nothing (1M points: 60 node groups and 63 leaves per point in the round
+// of 24 components, 34 of 727,000 points have a find), and neighbours walk the same
+// nodes. The walk tests nodes against the box of the group's points, so a node is
+// met once for all of them; at a leaf each lane tests its own point against the
+// leaf's box, and the leaf's foreign points (one per lane) are measured against
+// each point that it may still matter to. Bound by instructions, about 35 for a
+// point and leaf and 100 for a node group, as the walk by points. The last four rounds
+// 26.7 -> 9.5 ms (the test of the points before a group of nodes is entered: 24.6 ->
+// 22.5 of the whole tree, in the middle rounds, whose groups' boxes are loose).
+constexpr int MST_GROUP_BLOCKS = 8;  // per SM (registers)
+template <int DIMP>
+__global__ void __launch_bounds__(32 * MST_WARPS, MST_GROUP_BLOCKS) k_mst_noc_group(
+    MstTree<DIMP> tree, MstParts<DIMP> parts, const uint32_t* __restrict__ comp,
+    const float* __restrict__ core, const uint32_t* __restrict__ orig,
+    const uint2* __restrict__ groups, const unsigned long long* __restrict__ n_groups,
+    unsigned long long min_groups, unsigned long long* __restrict__ work,
+    uint32_t* __restrict__ cbest,
+    unsigned long long* __restrict__ ckey, uint32_t* __restrict__ near_j,
+    float* __restrict__ near_v) {
+  constexpr int Q = DIMP / 4;
+  __shared__ float stack_s[MST_WARPS][MST_LEVELS][32];
+  __shared__ float4 q_s[MST_WARPS][32][Q];
+  __shared__ float4 box_s[MST_WARPS][2][Q];  // of the group's points
+  __shared__ float cq_s[MST_WARPS][32];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  float (*stack)[32] = stack_s[wid];
+  const float INF = __uint_as_float(INF_BITS);
+  const int g0 = mst_first_bits(tree.depth);
+  const unsigned long long items = *n_groups;
+  if (items < min_groups) return;  // their points are on the others' list
+  for (;;) {
+    unsigned long long item = 0;
+    if (lane == 0) item = atomicAdd(work, 1ull);
+    item = __shfl_sync(FULL, item, 0);
+    if (item >= items) return;
+    const uint2 group = groups[item];
+    const int64_t pos = (int64_t)group.x * MST_LEAF + lane;
+    const bool active = (group.y >> lane) & 1u;
+    const uint32_t qc = comp[(int64_t)group.x * MST_LEAF + __ffs(group.y) - 1];
+    float q[DIMP];
+    float cq = INF;
+#pragma unroll
+    for (int d = 0; d < DIMP; ++d) q[d] = 0.0f;
+    if (active) {
+      mst_load<DIMP>(tree.xs, pos, q);
+      cq = core[pos];
+    }
+    const float cmin = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(cq)));
+    float blo[DIMP], bhi[DIMP];
+#pragma unroll
+    for (int d = 0; d < DIMP; ++d) {
+      const uint32_t o = ord_of(q[d]);
+      blo[d] = of_ord(__reduce_min_sync(FULL, active ? o : 0xffffffffu));
+      bhi[d] = of_ord(__reduce_max_sync(FULL, active ? o : 0u));
+    }
+    __syncwarp();  // the group before is done with the shared copies
+    cq_s[wid][lane] = cq;
+#pragma unroll
+    for (int t = 0; t < Q; ++t) {
+      q_s[wid][lane][t] = make_float4(q[4 * t], q[4 * t + 1], q[4 * t + 2], q[4 * t + 3]);
+      if (lane == 0) {
+        box_s[wid][0][t] = make_float4(blo[4 * t], blo[4 * t + 1], blo[4 * t + 2], blo[4 * t + 3]);
+        box_s[wid][1][t] = make_float4(bhi[4 * t], bhi[4 * t + 1], bhi[4 * t + 2], bhi[4 * t + 3]);
+      }
+    }
+    __syncwarp();
+    float bd = __uint_as_float(FMAX_BITS), limit = bd;  // limit: of the component, at least bd
+    uint32_t bj = NO_POINT, bo = 0;
+    auto refresh = [&]() {
+      const uint32_t cb = __shfl_sync(FULL, lane == 0 ? __ldcg(cbest + qc) : 0u, 0);
+      limit = __uint_as_float(cb < FMAX_BITS ? cb + 1u : FMAX_BITS);
+      if (limit < bd) {
+        bd = limit;
+        bj = NO_POINT;
+      }
+    };
+    refresh();
+    auto bound = [&](int64_t v) {  // box to box, monotone as mst_box_lb
+      const bool own = parts.maj[v] == qc;
+      const float c = own ? parts.core_rest[v] : parts.core_all[v];
+      const float4* l4 = reinterpret_cast<const float4*>(own ? parts.lo : tree.lo) + v * Q;
+      const float4* h4 = reinterpret_cast<const float4*>(own ? parts.hi : tree.hi) + v * Q;
+      float r = 0.0f;
+#pragma unroll
+      for (int t = 0; t < Q; ++t) {
+        const float4 a = __ldg(l4 + t), b = __ldg(h4 + t);
+        const float4 ql = box_s[wid][0][t], qh = box_s[wid][1][t];
+        const float2 l0 = fsub2(make_float2(a.x, a.y), make_float2(qh.x, qh.y));
+        const float2 l1 = fsub2(make_float2(a.z, a.w), make_float2(qh.z, qh.w));
+        const float2 h0 = fsub2(make_float2(ql.x, ql.y), make_float2(b.x, b.y));
+        const float2 h1 = fsub2(make_float2(ql.z, ql.w), make_float2(b.z, b.w));
+        const float2 d0 = make_float2(fmaxf(fmaxf(l0.x, h0.x), 0.0f), fmaxf(fmaxf(l0.y, h0.y), 0.0f));
+        const float2 d1 = make_float2(fmaxf(fmaxf(l1.x, h1.x), 0.0f), fmaxf(fmaxf(l1.y, h1.y), 0.0f));
+        const float2 s0 = fmul2(d0, d0), s1 = fmul2(d1, d1);
+        r = fadd(fadd(fadd(fadd(r, s0.x), s0.y), s1.x), s1.y);
+      }
+      return fmaxf(r, c);
+    };
+    MstWalk w{(int64_t)1 << g0, g0, 0, INF};
+    if (lane < (1 << g0)) w.p = bound(w.base + lane);
+    while (!(cmin > limit)) {
+      const int64_t node = mst_next(w, limit, lane);
+      if (node < 0) {
+        if (!mst_ascend(w, stack, g0, lane)) break;
+        continue;
+      }
+      // the points that the node may still matter to
+      const bool own = parts.maj[node] == qc;
+      const float lb = fmaxf(mst_box_lb<DIMP>(own ? parts.lo : tree.lo, own ? parts.hi : tree.hi,
+                                              node, q),
+                             own ? parts.core_rest[node] : parts.core_all[node]);
+      uint32_t todo = __ballot_sync(FULL, active && !(cq > bd) && !(lb > bd));
+      if (todo == 0u) continue;
+      if (w.level < tree.depth) {
+        mst_descend(w, stack, node, lane);
+        w.p = bound(w.base + lane);
+        continue;
+      }
+      const int64_t j = (node - tree.P) * MST_LEAF + lane;
+      float cj = INF;
+      bool foreign = false;
+      if (j < tree.n && comp[j] != qc) {
+        cj = core[j];
+        foreign = !(cj > limit);
+      }
+      if (__ballot_sync(FULL, foreign) == 0u) continue;
+      float y[DIMP];
+#pragma unroll
+      for (int d = 0; d < DIMP; ++d) y[d] = 0.0f;
+      if (foreign) mst_load<DIMP>(tree.xs, j, y);
+      for (; todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        float p[DIMP];
+#pragma unroll
+        for (int t = 0; t < Q; ++t) {
+          const float4 x = q_s[wid][src][t];
+          p[4 * t] = x.x, p[4 * t + 1] = x.y, p[4 * t + 2] = x.z, p[4 * t + 3] = x.w;
+        }
+        const float mr = foreign ? fmaxf(fmaxf(mst_sqd<DIMP>(p, y), cq_s[wid][src]), cj) : INF;
+        if (__ballot_sync(FULL, mr <= limit) == 0u) continue;
+        const uint32_t mb = __float_as_uint(mr), best = __reduce_min_sync(FULL, mb);
+        const uint32_t sb = __float_as_uint(__shfl_sync(FULL, bd, src));
+        const uint32_t sj = __shfl_sync(FULL, bj, src);
+        if (best < sb || (best == sb && sj != NO_POINT)) {  // as in k_mst_noc
+          const uint32_t oj = mb == best ? orig[j] : NO_POINT;
+          const uint32_t o = __reduce_min_sync(FULL, oj);
+          const int at = __ffs(__ballot_sync(FULL, mb == best && oj == o)) - 1;
+          if (lane == src && (best < sb || o < bo)) {
+            if (best < sb) atomicMin(cbest + qc, best);
+            bd = __uint_as_float(best);
+            bo = o;
+            bj = (uint32_t)(j - lane + at);
+          }
+        }
+      }
+      refresh();
+    }
+    if (active) {
+      near_j[pos] = bj;
+      near_v[pos] = fmaxf(near_v[pos], bd);
+      if (bj != NO_POINT)
+        atomicMin(ckey + qc, ((unsigned long long)__float_as_uint(bd) << 32) | orig[pos]);
     }
   }
 }
@@ -1067,7 +1275,7 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)mst_blocks<DIMP>() * ctx->num_sms,
                                                            (items + MST_WARPS - 1) / MST_WARPS));
   };
-  DevBuf<unsigned long long> work(1, s);  // the searches' next point
+  DevBuf<unsigned long long> work(3, s);  // the searches' next point, groups and their next
   EVOC_CUDA(cudaMemsetAsync(work.get(), 0, work.bytes(), s));
   DevBuf<float> core(n, s), knn_d(n * (int64_t)k, s);
   DevBuf<uint32_t> knn_j(n * (int64_t)k, s);
@@ -1088,6 +1296,18 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
   const MstParts<DIMP> parts{maj.get(), mcnt.get(),  plo.get(),
                              phi.get(), pcore.get(), pcore.get() + 2 * P};
   DevBuf<unsigned long long> ckey(n, s);
+  // Groups pay where their searches fill the chip: none below one leaf per resident
+  // warp of that kernel (100 k points: 4.7 ms without, 5.0 to 5.5 with), half leaves up
+  // to four (200 k: 9.2 ms without, 7.9 by 16, 8.3 by 32 points; 16 dimensions,
+  // 300 k: 88, 49 and 55 ms), whole leaves above (1 M: 38.8, 23.3 and 22.5 ms).
+  const int64_t resident = (int64_t)MST_GROUP_BLOCKS * MST_WARPS * ctx->num_sms;
+  const bool by_group = L >= resident;
+  const int width = L >= 4 * resident ? 32 : 16;
+  const int64_t max_groups = by_group ? L * (MST_LEAF / width) : 0;
+  // 16 dimensions: searches are so long that few groups still beat them (48.7 and 58.0 ms)
+  const unsigned long long min_groups = DIMP > 8 ? 1 : (unsigned long long)resident;
+  DevBuf<uint2> groups(max_groups, s);
+  const unsigned group_grid = (unsigned)(MST_GROUP_BLOCKS * ctx->num_sms);
   DevBuf<uint32_t> jA(n, s), jB(n, s), mA(n, s), mB(n, s), oncyc(n, s), nid(n, s), lab(n, s);
   DevBuf<uint32_t> A(n, s), A2(n, s), eu(n, s), ev(n, s), ew(n, s);
   DevBuf<int32_t> has(n, s), keep(n, s), alive(n, s);
@@ -1113,13 +1333,25 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
     k_mst_bound<DIMP><<<gn, 256, 0, s>>>(xs.get(), n, k, knn_j.get(), knn_d.get(), comp.get(), core.get(),
                                    near_j.get(), near_v.get(), cbest.get());
     EVOC_CHECK_LAUNCH();
+    EVOC_CUDA(cudaMemsetAsync(work.get(), 0, work.bytes(), s));
     k_mst_select<<<gn, 256, 0, s>>>(n, comp.get(), core.get(), orig.get(), near_j.get(),
-                                    near_v.get(), cbest.get(), ckey.get(), has.get());
+                                    near_v.get(), cbest.get(), ckey.get(), has.get(),
+                                    by_group ? groups.get() : nullptr, work.get() + 1, width);
     EVOC_CHECK_LAUNCH();
+    if (by_group) {
+      k_mst_take_groups<<<grid_of(max_groups), 256, 0, s>>>(groups.get(), work.get() + 1,
+                                                            min_groups, has.get());
+      EVOC_CHECK_LAUNCH();
+    }
     exclusive_scan_i32_to_i64(ctx, has.get(), off.get(), n);
     k_mst_search_list<<<gn, 256, 0, s>>>(n, has.get(), off.get(), list.get());
     EVOC_CHECK_LAUNCH();
-    EVOC_CUDA(cudaMemsetAsync(work.get(), 0, work.bytes(), s));
+    if (by_group) {
+      k_mst_noc_group<DIMP><<<group_grid, 32 * MST_WARPS, 0, s>>>(
+          tree, parts, comp.get(), core.get(), orig.get(), groups.get(), work.get() + 1,
+          min_groups, work.get() + 2, cbest.get(), ckey.get(), near_j.get(), near_v.get());
+      EVOC_CHECK_LAUNCH();
+    }
     k_mst_noc<DIMP><<<search_grid(n), 32 * MST_WARPS, 0, s>>>(
         tree, parts, comp.get(), core.get(), orig.get(), list.get(), off.get() + n, work.get(),
         cbest.get(), ckey.get(), near_j.get(), near_v.get());
