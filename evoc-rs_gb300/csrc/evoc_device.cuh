@@ -46,6 +46,12 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
   return unpack2(r);
 }
 
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)), "l"(pack2(c)));
+  return unpack2(r);
+}
+
 // max(a, 0) with NaN -> 0, the result of Rust's f32::max(a, 0.0).
 __device__ __forceinline__ float max0(float a) { return (a > 0.0f) ? a : 0.0f; }
 
