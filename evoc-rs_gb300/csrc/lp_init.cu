@@ -261,6 +261,10 @@ __global__ void k_runs_to_csr(const uint2* __restrict__ vals, int64_t m, float l
 // lists column j's entries too, so both products of a level are sums over one
 // row, grouped by the part of the neighbour (row_groups.cuh), and no entry has
 // to be sorted across rows. Needs at most RG_LABELS parts.
+// The coarse graphs of a canonical one have sorted rows and entries both ways, with
+// weights that need not be equal: there (TWIN) an entry's other weight is searched
+// for in its column's row. Levels of 644 and 11,274 nodes spend 0.20 and 0.54 ms on both
+// products so, 0.43 and 1.09 with a transpose and sorts of all entries.
 // ---------------------------------------------------------------------------
 struct RowGraph {
   const int64_t* indptr;
@@ -270,36 +274,50 @@ struct RowGraph {
   const float* inv;
 };
 
-// Entry q's label and product: inv_P * w of the coarse graph, or (SYM) the
-// expansion's (w * w) * inv_Q (the symmetric part of an equal pair).
-template <bool SYM>
-__device__ __forceinline__ uint32_t row_entry(const RowGraph& g, int64_t q, float* v) {
-  const uint32_t l = g.part[g.indices[q]];
-  const float w = g.w[q];
-  *v = SYM ? fmul(fmul(w, w), g.inv[l]) : fmul(g.inv[l], w);
+// The weight of (j, i): a binary search of row j for column i, which is there.
+__device__ __forceinline__ float twin_weight(const RowGraph& g, uint32_t j, uint32_t i) {
+  int64_t a = g.indptr[j], b = g.indptr[j + 1] - 1;
+  while (a < b) {
+    const int64_t m = (a + b) >> 1;
+    if (g.indices[m] < i)
+      a = m + 1;
+    else
+      b = m;
+  }
+  return g.w[a];
+}
+
+// Entry q = (i, j)'s label and product: inv_P * w_ji of the coarse graph, or (SYM) the
+// expansion's (w_ij * w_ji) * inv_Q (the symmetric part).
+template <bool SYM, bool TWIN>
+__device__ __forceinline__ uint32_t row_entry(const RowGraph& g, uint32_t i, int64_t q, float* v) {
+  const uint32_t j = g.indices[q], l = g.part[j];
+  const float w = g.w[q], t = TWIN ? twin_weight(g, j, i) : w;
+  *v = SYM ? fmul(fmul(w, t), g.inv[l]) : fmul(g.inv[l], t);
   return l;
 }
 
-template <bool SYM, int CAP>
-__device__ __forceinline__ int row_groups(const RowGraph& g, RgWarp<CAP>& sm, int64_t b, int len,
-                                          int lane) {
+template <bool SYM, bool TWIN, int CAP>
+__device__ __forceinline__ int row_groups(const RowGraph& g, RgWarp<CAP>& sm, int64_t i, int64_t b,
+                                          int len, int lane) {
   for (int p = lane; p < len; p += 32) {
     float v;
-    const uint32_t l = row_entry<SYM>(g, b + p, &v);
+    const uint32_t l = row_entry<SYM, TWIN>(g, (uint32_t)i, b + p, &v);
     sm.key[p] = (l << RG_POS_BITS) | (uint32_t)p;
     sm.val[p] = v;
   }
   return rg_group(sm, len, lane);
 }
 
-template <bool SYM>
-__device__ __forceinline__ int long_row_groups(const RowGraph& g, RgLong& sm, int64_t b, int64_t e) {
+template <bool SYM, bool TWIN>
+__device__ __forceinline__ int long_row_groups(const RowGraph& g, RgLong& sm, uint32_t i) {
+  const int64_t b = g.indptr[i], e = g.indptr[i + 1];
   rg_long_clear(sm);
   for (int64_t c = b; c < e; c += RG_CHUNK) {
     for (int q = threadIdx.x; q < RG_CHUNK; q += RG_LONG_THREADS) {
       uint32_t key = 0xffffffffu;
       float v = 0.0f;
-      if (c + q < e) key = (row_entry<SYM>(g, c + q, &v) << 10) | (uint32_t)q;
+      if (c + q < e) key = (row_entry<SYM, TWIN>(g, i, c + q, &v) << 10) | (uint32_t)q;
       sm.key[q] = key;
       sm.val[q] = v;
     }
@@ -310,16 +328,17 @@ __device__ __forceinline__ int long_row_groups(const RowGraph& g, RgLong& sm, in
 
 // Coarse graph, first product: row j's (P, sum of inv_P w_ij over i in P), P
 // ascending, at the head of the row's CSR range in tmp; cnt[j] of them.
-template <int CAP>
+template <bool TWIN, int CAP>
 __device__ __forceinline__ void coarse_row(const RowGraph& g, RgWarp<CAP>& sm, int64_t j, int64_t b,
                                            int len, int lane, uint2* __restrict__ tmp,
                                            int32_t* __restrict__ cnt) {
-  const int runs = row_groups<false>(g, sm, b, len, lane);
+  const int runs = row_groups<false, TWIN>(g, sm, j, b, len, lane);
   for (int r = lane; r < runs; r += 32)
     tmp[b + r] = make_uint2(sm.key[sm.start[r]] >> RG_POS_BITS, __float_as_uint(sm.sum[r]));
   if (lane == 0) cnt[j] = runs;
 }
 
+template <bool TWIN>
 __global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_coarse_rows(RowGraph g, int64_t n,
                                                                uint2* __restrict__ tmp,
                                                                int32_t* __restrict__ cnt,
@@ -330,9 +349,10 @@ __global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_coarse_rows(RowGra
   if (j >= n) return;
   const int64_t b = g.indptr[j], len = g.indptr[j + 1] - b;
   if (rg_defer(lists, j, len, lane)) return;
-  coarse_row(g, sm_all[wid], j, b, (int)len, lane, tmp, cnt);
+  coarse_row<TWIN>(g, sm_all[wid], j, b, (int)len, lane, tmp, cnt);
 }
 
+template <bool TWIN>
 __global__ void __launch_bounds__(32 * RG_MID_WARPS) k_coarse_rows_mid(RowGraph g,
                                                                        uint2* __restrict__ tmp,
                                                                        int32_t* __restrict__ cnt,
@@ -342,10 +362,11 @@ __global__ void __launch_bounds__(32 * RG_MID_WARPS) k_coarse_rows_mid(RowGraph 
   RgWarp<RG_MID>& sm = reinterpret_cast<RgWarp<RG_MID>*>(rg_raw)[wid];
   for (int64_t j; (j = rg_next_mid(lists, lane)) >= 0;) {
     __syncwarp();  // the previous row's readers are done
-    coarse_row(g, sm, j, g.indptr[j], (int)(g.indptr[j + 1] - g.indptr[j]), lane, tmp, cnt);
+    coarse_row<TWIN>(g, sm, j, g.indptr[j], (int)(g.indptr[j + 1] - g.indptr[j]), lane, tmp, cnt);
   }
 }
 
+template <bool TWIN>
 __global__ void __launch_bounds__(RG_LONG_THREADS) k_coarse_rows_long(
     RowGraph g, uint2* __restrict__ tmp, int32_t* __restrict__ cnt, RgLists lists) {
   extern __shared__ __align__(16) unsigned char rg_raw[];
@@ -354,7 +375,7 @@ __global__ void __launch_bounds__(RG_LONG_THREADS) k_coarse_rows_long(
   for (int item = blockIdx.x; item < nl; item += gridDim.x) {
     const uint32_t j = lists.longs[item];
     const int64_t b = g.indptr[j];
-    const int runs = long_row_groups<false>(g, sm, b, g.indptr[j + 1]);
+    const int runs = long_row_groups<false, TWIN>(g, sm, j);
     for (int r = threadIdx.x; r < runs; r += RG_LONG_THREADS) {
       const uint32_t l = sm.list[r];
       tmp[b + r] = make_uint2(l, __float_as_uint(sm.acc[l]));
@@ -416,18 +437,19 @@ __device__ __forceinline__ void expand_row(int64_t i, int runs, int lane, int32_
   res[i * dim + lane] = fmul(fadd(acc, direct), 0.5f);
 }
 
-template <int CAP>
+template <bool TWIN, int CAP>
 __device__ __forceinline__ void expand_warp_row(const RowGraph& g, RgWarp<CAP>& sm, int64_t i,
                                                 int64_t b, int len, int lane, int32_t dim,
                                                 const float* __restrict__ layout,
                                                 const float* __restrict__ u,
                                                 float* __restrict__ res) {
-  const int runs = row_groups<true>(g, sm, b, len, lane);
+  const int runs = row_groups<true, TWIN>(g, sm, i, b, len, lane);
   expand_row(
       i, runs, lane, dim, layout, g.part, u, res,
       [&](int r) { return sm.key[sm.start[r]] >> RG_POS_BITS; }, [&](int r) { return sm.sum[r]; });
 }
 
+template <bool TWIN>
 __global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_expand_groups(
     RowGraph g, int64_t n, int32_t dim, const float* __restrict__ layout,
     const float* __restrict__ u, float* __restrict__ res, RgLists lists) {
@@ -437,9 +459,10 @@ __global__ void __launch_bounds__(32 * RG_WARPS, RG_BLOCKS) k_expand_groups(
   if (i >= n) return;
   const int64_t b = g.indptr[i], len = g.indptr[i + 1] - b;
   if (rg_defer(lists, i, len, lane)) return;
-  expand_warp_row(g, sm_all[wid], i, b, (int)len, lane, dim, layout, u, res);
+  expand_warp_row<TWIN>(g, sm_all[wid], i, b, (int)len, lane, dim, layout, u, res);
 }
 
+template <bool TWIN>
 __global__ void __launch_bounds__(32 * RG_MID_WARPS) k_expand_groups_mid(
     RowGraph g, int32_t dim, const float* __restrict__ layout, const float* __restrict__ u,
     float* __restrict__ res, RgLists lists) {
@@ -448,11 +471,12 @@ __global__ void __launch_bounds__(32 * RG_MID_WARPS) k_expand_groups_mid(
   RgWarp<RG_MID>& sm = reinterpret_cast<RgWarp<RG_MID>*>(rg_raw)[wid];
   for (int64_t i; (i = rg_next_mid(lists, lane)) >= 0;) {
     __syncwarp();  // the previous row's readers are done
-    expand_warp_row(g, sm, i, g.indptr[i], (int)(g.indptr[i + 1] - g.indptr[i]), lane, dim, layout,
+    expand_warp_row<TWIN>(g, sm, i, g.indptr[i], (int)(g.indptr[i + 1] - g.indptr[i]), lane, dim, layout,
                     u, res);
   }
 }
 
+template <bool TWIN>
 __global__ void __launch_bounds__(RG_LONG_THREADS) k_expand_groups_long(
     RowGraph g, int32_t dim, const float* __restrict__ layout, const float* __restrict__ u,
     float* __restrict__ res, RgLists lists) {
@@ -461,7 +485,7 @@ __global__ void __launch_bounds__(RG_LONG_THREADS) k_expand_groups_long(
   const int nl = lists.count[1];
   for (int item = blockIdx.x; item < nl; item += gridDim.x) {
     const uint32_t i = lists.longs[item];
-    const int runs = long_row_groups<true>(g, sm, g.indptr[i], g.indptr[i + 1]);
+    const int runs = long_row_groups<true, TWIN>(g, sm, i);
     if (threadIdx.x < 32)
       expand_row(
           (int64_t)i, runs, (int)threadIdx.x, dim, layout, g.part, u, res,
@@ -977,10 +1001,11 @@ struct LpParams {
 };
 
 // One level of label_prop_init_inner on graph g (device), data (device n x d
-// or null): writes the n x dim initial embedding into d_out (device).
+// or null): writes the n x dim initial embedding into d_out (device). twin: g has
+// sorted rows and every entry's (j, i) too.
 void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float* d_data,
                    int64_t d, int32_t n_emb_epochs, int64_t approx_parts, uint64_t seed,
-                   const LpParams& lp, float* d_out) {
+                   const LpParams& lp, float* d_out, bool twin = false) {
   cudaStream_t s = ctx->stream;
   const int64_t n = g->n;
   if (n < lp.base_thr) {  // label_prop.rs:440-445
@@ -1030,8 +1055,9 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
     EVOC_CHECK_LAUNCH();
     radix_sort_pairs(ctx, pk, nodes, n, pbits);
   }
-  // canonical graphs sum within their rows; others by sorting all entries
-  const bool by_rows = g->canonical && np <= RG_LABELS && g->nnz > 0;
+  // canonical graphs and those made from them sum within their rows; others by
+  // sorting all entries
+  const bool by_rows = (g->canonical || twin) && np <= RG_LABELS && g->nnz > 0;
   const RowGraph rg{g->indptr.get(), g->indices.get(), g->weights.get(), part.get(), inv.get()};
   DevBuf<uint32_t> row_lists;  // rows above RG_CAP: middle, long
   DevBuf<int32_t> row_counts;  // their counters: coarse graph, expansion
@@ -1042,16 +1068,22 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
       4 * (int64_t)ctx->num_sms, (g->nnz / RG_CAP + RG_MID_WARPS - 1) / RG_MID_WARPS);
   const unsigned lgrid = (unsigned)std::min<int64_t>(2 * (int64_t)ctx->num_sms, g->nnz / RG_MID);
   const size_t msmem = RG_MID_WARPS * sizeof(RgWarp<RG_MID>);
+  auto* coarse_short = twin ? k_coarse_rows<true> : k_coarse_rows<false>;
+  auto* coarse_mid = twin ? k_coarse_rows_mid<true> : k_coarse_rows_mid<false>;
+  auto* coarse_long = twin ? k_coarse_rows_long<true> : k_coarse_rows_long<false>;
+  auto* expand_short = twin ? k_expand_groups<true> : k_expand_groups<false>;
+  auto* expand_mid = twin ? k_expand_groups_mid<true> : k_expand_groups_mid<false>;
+  auto* expand_long = twin ? k_expand_groups_long<true> : k_expand_groups_long<false>;
   if (by_rows) {
     row_lists.alloc(2 * n, s);
     row_counts.alloc(6, s);
     EVOC_CUDA(cudaMemsetAsync(row_counts.get(), 0, row_counts.bytes(), s));
     lists = RgLists{row_lists.get(), row_lists.get() + n, row_counts.get()};
     lists2 = RgLists{row_lists.get(), row_lists.get() + n, row_counts.get() + 3};
-    for (const void* f : {(const void*)k_coarse_rows_long, (const void*)k_expand_groups_long})
+    for (const void* f : {(const void*)coarse_long, (const void*)expand_long})
       EVOC_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(RgLong)));
-    for (const void* f : {(const void*)k_coarse_rows_mid, (const void*)k_expand_groups_mid})
+    for (const void* f : {(const void*)coarse_mid, (const void*)expand_mid})
       EVOC_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem));
   }
   // 3. coarse graph clip(N^T G B)
@@ -1069,15 +1101,15 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
       // (P, a) per row j, gathered in (Q, j) order and sorted by P: (P, Q, j)
       DevBuf<uint2> tmp(m, s);
       DevBuf<int32_t> rcnt(n, s), pcnt(n, s);
-      k_coarse_rows<<<rgrid, 32 * RG_WARPS, 0, s>>>(rg, n, tmp.get(), rcnt.get(), lists);
+      coarse_short<<<rgrid, 32 * RG_WARPS, 0, s>>>(rg, n, tmp.get(), rcnt.get(), lists);
       EVOC_CHECK_LAUNCH();
       if (lgrid) {
-        k_coarse_rows_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLong), s>>>(rg, tmp.get(),
+        coarse_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLong), s>>>(rg, tmp.get(),
                                                                           rcnt.get(), lists);
         EVOC_CHECK_LAUNCH();
       }
       if (mgrid) {
-        k_coarse_rows_mid<<<mgrid, 32 * RG_MID_WARPS, msmem, s>>>(rg, tmp.get(), rcnt.get(),
+        coarse_mid<<<mgrid, 32 * RG_MID_WARPS, msmem, s>>>(rg, tmp.get(), rcnt.get(),
                                                                   lists);
         EVOC_CHECK_LAUNCH();
       }
@@ -1152,7 +1184,7 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
   const int32_t e = std::min(n_emb_epochs, 255);
   DevBuf<float> cinit(np * dim, s), layout(np * dim, s);
   lp_init_inner(ctx, &coarse, dim, d_data ? cdata.get() : nullptr, d, e, approx_parts / 4,
-                seed + 3000, lp, cinit.get());
+                seed + 3000, lp, cinit.get(), g->canonical || twin);
   mark("coarser levels");
   // 6. short embedding of the coarse graph (label_prop.rs:486-498)
   {
@@ -1175,16 +1207,16 @@ void lp_init_inner(evoc_ctx* ctx, const evoc_graph* g, int32_t dim, const float*
   // 7. expansion (label_prop.rs:500-534)
   {
     if (by_rows) {
-      k_expand_groups<<<rgrid, 32 * RG_WARPS, 0, s>>>(rg, n, dim, layout.get(), u.get(), d_out,
+      expand_short<<<rgrid, 32 * RG_WARPS, 0, s>>>(rg, n, dim, layout.get(), u.get(), d_out,
                                                       lists2);
       EVOC_CHECK_LAUNCH();
       if (lgrid) {
-        k_expand_groups_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLong), s>>>(
+        expand_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLong), s>>>(
             rg, dim, layout.get(), u.get(), d_out, lists2);
         EVOC_CHECK_LAUNCH();
       }
       if (mgrid) {
-        k_expand_groups_mid<<<mgrid, 32 * RG_MID_WARPS, msmem, s>>>(rg, dim, layout.get(),
+        expand_mid<<<mgrid, 32 * RG_MID_WARPS, msmem, s>>>(rg, dim, layout.get(),
                                                                     u.get(), d_out, lists2);
         EVOC_CHECK_LAUNCH();
       }
