@@ -17,7 +17,7 @@
 //   k_tile_fill    the gradient slots of every epoch and tile from them.
 //   (k_sched_count and k_sched_fill beyond the masks' range; k_schedule_* and bit
 //   planes for k_epoch when the slots would not fit.)
-// Epoch loop (embedding.rs:178-292), one launch per epoch, captured in a CUDA
+// Epoch loop (embedding.rs:178-292), one launch per epoch, from a second run on as a CUDA
 // graph, or one cooperative launch for all: k_epoch_slot (k_epoch on bit planes).
 // No float atomics; results do not depend on the launch shape.
 #include "evoc_device.cuh"

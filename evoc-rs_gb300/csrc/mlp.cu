@@ -883,11 +883,11 @@ __global__ void __launch_bounds__(TC_THREADS, (STAGES <= 2 ? 2 : 1))
 //   warps 4..11:     epilogue, warp w on TMEM lanes 32 (w % 4) and column half
 //                    (w - 4) / 4; with HEAD the BF16 activations go to a
 //                    dedicated 64 KB swizzled tile instead of global memory.
-// What bounds it is the mainloop: shared memory feeds the MMA 12 KB and takes 12 KB
-// from the TMA per 128 cycles of tensor time, 192 of its 128 bytes per cycle. Without
-// GELU and stores a prediction of 1 M points still takes 1.13 of its 1.26 ms;
-// sharing the weight tile over a cluster of two by multicast changes nothing, and
-// neither do four more warps that take the head's results off the epilogue warps.
+// A prediction of 1 M points takes 1.26 ms, twice the tensor time; without GELU and
+// stores still 1.13. It is neither the feeding of the MMA from shared memory (CTA
+// pairs, which halve it: 1.28 ms), nor the weight tile's way from L2 (multicast over
+// clusters of two: the same), nor the head's turn-around (its results read by four
+// more warps: 1.26), nor the timer in the waits (read after 16 tries only: 1.24).
 // The epilogue of tile i overlaps the mainloop of tile i + 1. Every wait is
 // bounded (2 s each); a timeout sets ST_WAIT_TIMEOUT and an abort flag that
 // every role checks before its next wait.

@@ -309,11 +309,11 @@ EVOC_API int evoc_gather_peak(evoc_ctx_t* ctx, int64_t bytes, double* gbs);
 
 /* Epoch-kernel configuration of a plan (no counterpart): variant 0..3 of the
  * gradient-slots kernel as (slot window, slots per lane per group) = (128, 2),
- * (64, 2), (256, 2), (128, 1), launched once per epoch (the epoch loop is
- * captured in a CUDA graph); variants 4..7 the same kernels with all epochs
+ * (64, 2), (256, 2), (128, 1), launched once per epoch (replayed as a
+ * CUDA graph from a plan's second run on); variants 4..7 the same kernels with all epochs
  * in one persistent cooperative launch, a grid-wide barrier between epochs
  * (a barrier wait that exceeds 2 s ends the launch with EVOC_ERR_INTERNAL);
- * warps (32-node tiles) per thread block 1, 2 or 4; persistent blocks per SM
+ * warps (node tiles) per thread block 1, 2 or 4; persistent blocks per SM
  * capped at blocks_per_sm (0: as many as fit). Every configuration gives
  * identical results; only speed differs. */
 EVOC_API int evoc_plan_set_config(evoc_plan_t* plan, int32_t variant,
@@ -334,7 +334,7 @@ EVOC_API int evoc_plan_autotune(evoc_plan_t* plan, int32_t* config, float* ms_pe
 
 /* Layout facts of a plan (any pointer may be NULL): undirected edges,
  * per-node incidence entries (2 per edge), negative-count bit planes per
- * epoch, warps (32-node tiles) per thread block of the epoch kernel, and the
+ * epoch, warps (node tiles) per thread block of the epoch kernel, and the
  * number of gradient slots over all epochs (one per fired incidence entry and
  * one per negative sample; 0 when the epoch kernel scans the bit planes
  * instead) (no counterpart). */
