@@ -1194,6 +1194,167 @@ __global__ void k_mst_compact(const uint32_t* __restrict__ A, int64_t m,
   if (k < m && alive[k]) A2[off[k]] = A[k];
 }
 
+// The whole merge (k_mst_picks to k_mst_compact but the relabelling) of at most
+// MERGE_ONE components in one block: by itself each of the 2 K + 10 steps is a launch
+// of 2 us for a microsecond's work. Components are held by their rank in A (ascending
+// ids, so ranks order them the same), everything but the picks and the outputs in
+// shared memory. tot: picks kept, components left. Rounds of 2,003, 63, 15 and 2
+// components take 344 us in all, 690 in launches of their own.
+constexpr int MERGE_ONE = 2048;
+constexpr int MERGE_THREADS = MERGE_ONE / 2;  // ranks 2 t and 2 t + 1 each
+struct MergeArgs {
+  const uint32_t* A;
+  const unsigned long long* ckey;
+  const uint32_t* pos_of;
+  const uint32_t* bj;
+  const uint32_t* orig;
+  const uint32_t* comp;
+  uint32_t* rank;  // scratch by component id
+  uint32_t* lab;   // out, by component id
+  uint32_t* A2;    // out: components left
+  int64_t* u;      // out: edges from base on
+  int64_t* v;
+  float* w;
+  int64_t base;
+  int64_t* tot;
+  int m, K;
+};
+__global__ void __launch_bounds__(MERGE_THREADS) k_mst_merge_one(MergeArgs a) {
+  __shared__ uint16_t succ[MERGE_ONE], ja[MERGE_ONE], jb[MERGE_ONE], ma[MERGE_ONE], mb[MERGE_ONE];
+  __shared__ uint8_t oncyc[MERGE_ONE];
+  __shared__ uint32_t nid[MERGE_ONE];
+  __shared__ int2 sums[32];
+  const unsigned FULL = 0xffffffffu;
+  const int t = threadIdx.x, lane = t & 31, k0 = 2 * t;
+  uint32_t id[2], eu[2], ev[2], ew[2];
+  bool has[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    id[q] = 0;
+    if (k0 + q < a.m) {
+      id[q] = a.A[k0 + q];
+      a.rank[id[q]] = (uint32_t)(k0 + q);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int k = k0 + q;
+    has[q] = false;
+    if (k >= a.m) continue;
+    const unsigned long long key = a.ckey[id[q]];
+    uint32_t s = (uint32_t)k;
+    if (key != ~0ull) {
+      eu[q] = (uint32_t)key;
+      const uint32_t pj = a.bj[a.pos_of[eu[q]]];
+      s = *(volatile const uint32_t*)(a.rank + a.comp[pj]);
+      ev[q] = a.orig[pj];
+      ew[q] = (uint32_t)(key >> 32);
+      has[q] = true;
+    }
+    succ[k] = ja[k] = (uint16_t)s;
+    ma[k] = (uint16_t)max((uint32_t)k, s);
+    oncyc[k] = 0;
+    nid[k] = 0xffffffffu;
+  }
+  __syncthreads();
+  uint16_t *jin = ja, *jout = jb, *min_ = ma, *mout = mb;
+  for (int step = 0; step < a.K; ++step) {  // as k_mst_dbl_step
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int k = k0 + q;
+      if (k >= a.m) continue;
+      const uint16_t j = jin[k];
+      jout[k] = jin[j];
+      mout[k] = max(min_[k], min_[j]);
+    }
+    __syncthreads();
+    uint16_t* x = jin;
+    jin = jout;
+    jout = x;
+    x = min_;
+    min_ = mout;
+    mout = x;
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    if (k0 + q < a.m) oncyc[jin[k0 + q]] = 1;
+  __syncthreads();
+  bool keep[2], alive[2];
+  uint16_t *pin = jout, *pout = mout;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int k = k0 + q;
+    keep[q] = alive[q] = false;
+    if (k >= a.m) continue;
+    const bool root = oncyc[k] != 0 && min_[k] == k;
+    pin[k] = root ? (uint16_t)k : succ[k];
+    keep[q] = has[q] && !root;
+  }
+  __syncthreads();
+  for (int step = 0; step <= a.K; ++step) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (k0 + q < a.m) pout[k0 + q] = pin[pin[k0 + q]];
+    __syncthreads();
+    uint16_t* x = pin;
+    pin = pout;
+    pout = x;
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    if (k0 + q < a.m) atomicMin(nid + pin[k0 + q], (uint32_t)(k0 + q));
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int k = k0 + q;
+    if (k >= a.m) continue;
+    const uint32_t l = nid[pin[k]];
+    a.lab[id[q]] = a.A[l];
+    alive[q] = l == (uint32_t)k;
+  }
+  // ranks among the kept and the living before this thread's
+  int2 c = make_int2((int)keep[0] + (int)keep[1], (int)alive[0] + (int)alive[1]), inc = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(FULL, inc.x, o), y = __shfl_up_sync(FULL, inc.y, o);
+    if (lane >= o) {
+      inc.x += x;
+      inc.y += y;
+    }
+  }
+  if (lane == 31) sums[t >> 5] = inc;
+  __syncthreads();
+  int2 all = sums[lane];
+  const int2 own = all;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(FULL, all.x, o), y = __shfl_up_sync(FULL, all.y, o);
+    if (lane >= o) {
+      all.x += x;
+      all.y += y;
+    }
+  }
+  const int before = t >> 5;
+  const int bx = __shfl_sync(FULL, all.x - own.x, before), by = __shfl_sync(FULL, all.y - own.y, before);
+  if (t == MERGE_THREADS - 1) {
+    a.tot[0] = bx + inc.x;
+    a.tot[1] = by + inc.y;
+  }
+  int64_t e = a.base + bx + inc.x - c.x;
+  int l = by + inc.y - c.y;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    if (keep[q]) {
+      a.u[e] = eu[q];
+      a.v[e] = ev[q];
+      a.w[e] = fsqrt(__uint_as_float(ew[q]));
+      ++e;
+    }
+    if (alive[q]) a.A2[l++] = id[q];
+  }
+}
+
 __global__ void k_mst_iota(uint32_t* __restrict__ a, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] = (uint32_t)i;
@@ -1311,7 +1472,7 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
   DevBuf<uint32_t> jA(n, s), jB(n, s), mA(n, s), mB(n, s), oncyc(n, s), nid(n, s), lab(n, s);
   DevBuf<uint32_t> A(n, s), A2(n, s), eu(n, s), ev(n, s), ew(n, s);
   DevBuf<int32_t> has(n, s), keep(n, s), alive(n, s);
-  DevBuf<int64_t> off(n + 1, s), off2(n + 1, s);
+  DevBuf<int64_t> off(n + 1, s), off2(n + 1, s), tot(2, s);
   EVOC_CUDA(cudaMemcpyAsync(comp.get(), orig.get(), comp.bytes(), cudaMemcpyDeviceToDevice, s));
   k_mst_iota<<<grid_of(n), 256, 0, s>>>(A.get(), n);
   EVOC_CHECK_LAUNCH();
@@ -1356,47 +1517,57 @@ int64_t mst_run(evoc_ctx* ctx, const float* d_data, int64_t n, int dim, int k, i
         tree, parts, comp.get(), core.get(), orig.get(), list.get(), off.get() + n, work.get(),
         cbest.get(), ckey.get(), near_j.get(), near_v.get());
     EVOC_CHECK_LAUNCH();
-    k_mst_picks<<<gm, 256, 0, s>>>(A.get(), m, ckey.get(), pos_of.get(), near_j.get(), orig.get(),
-                                   comp.get(), succ.get(), eu.get(), ev.get(), ew.get(), has.get());
-    EVOC_CHECK_LAUNCH();
-    // cycles of the pick graph: 2^K >= m doubling steps
-    const int K = std::max(1, log2_ceil(m));
-    k_mst_dbl_init<<<gm, 256, 0, s>>>(A.get(), m, succ.get(), jA.get(), mA.get(), oncyc.get());
-    EVOC_CHECK_LAUNCH();
-    uint32_t *jin = jA.get(), *jout = jB.get(), *min_ = mA.get(), *mout = mB.get();
-    for (int t = 0; t < K; ++t) {  // after t steps: jmp = succ^(2^(t+1)), mx over that path
-      k_mst_dbl_step<<<gm, 256, 0, s>>>(A.get(), m, jin, min_, jout, mout);
+    if (m <= MERGE_ONE) {
+      const MergeArgs ma{A.get(),    ckey.get(), pos_of.get(), near_j.get(), orig.get(),
+                         comp.get(), nid.get(),  lab.get(),    A2.get(),     d_u,
+                         d_v,        d_w,        len,          tot.get(),    (int)m,
+                         std::max(1, log2_ceil(m))};
+      k_mst_merge_one<<<1, MERGE_THREADS, 0, s>>>(ma);
       EVOC_CHECK_LAUNCH();
-      std::swap(jin, jout);
-      std::swap(min_, mout);
-    }
-    k_mst_mark<<<gm, 256, 0, s>>>(A.get(), m, jin, oncyc.get());
-    EVOC_CHECK_LAUNCH();
-    // the skipped picks, then the merged components by pointer jumping
-    uint32_t *pin = jout, *pout = mout;  // free ping-pong buffers
-    k_mst_skip<<<gm, 256, 0, s>>>(A.get(), m, succ.get(), min_, oncyc.get(), has.get(), pin,
-                                  nid.get(), keep.get());
-    EVOC_CHECK_LAUNCH();
-    for (int t = 0; t <= K; ++t) {
-      k_mst_jump<<<gm, 256, 0, s>>>(A.get(), m, pin, pout);
+      EVOC_CUDA(cudaMemcpyAsync(h_tot, tot.get(), sizeof(h_tot), cudaMemcpyDeviceToHost, s));
+    } else {
+      k_mst_picks<<<gm, 256, 0, s>>>(A.get(), m, ckey.get(), pos_of.get(), near_j.get(), orig.get(),
+                                     comp.get(), succ.get(), eu.get(), ev.get(), ew.get(), has.get());
       EVOC_CHECK_LAUNCH();
-      std::swap(pin, pout);
+      // cycles of the pick graph: 2^K >= m doubling steps
+      const int K = std::max(1, log2_ceil(m));
+      k_mst_dbl_init<<<gm, 256, 0, s>>>(A.get(), m, succ.get(), jA.get(), mA.get(), oncyc.get());
+      EVOC_CHECK_LAUNCH();
+      uint32_t *jin = jA.get(), *jout = jB.get(), *min_ = mA.get(), *mout = mB.get();
+      for (int t = 0; t < K; ++t) {  // after t steps: jmp = succ^(2^(t+1)), mx over that path
+        k_mst_dbl_step<<<gm, 256, 0, s>>>(A.get(), m, jin, min_, jout, mout);
+        EVOC_CHECK_LAUNCH();
+        std::swap(jin, jout);
+        std::swap(min_, mout);
+      }
+      k_mst_mark<<<gm, 256, 0, s>>>(A.get(), m, jin, oncyc.get());
+      EVOC_CHECK_LAUNCH();
+      // the skipped picks, then the merged components by pointer jumping
+      uint32_t *pin = jout, *pout = mout;  // free ping-pong buffers
+      k_mst_skip<<<gm, 256, 0, s>>>(A.get(), m, succ.get(), min_, oncyc.get(), has.get(), pin,
+                                    nid.get(), keep.get());
+      EVOC_CHECK_LAUNCH();
+      for (int t = 0; t <= K; ++t) {
+        k_mst_jump<<<gm, 256, 0, s>>>(A.get(), m, pin, pout);
+        EVOC_CHECK_LAUNCH();
+        std::swap(pin, pout);
+      }
+      k_mst_newid<<<gm, 256, 0, s>>>(A.get(), m, pin, nid.get());
+      EVOC_CHECK_LAUNCH();
+      k_mst_label<<<gm, 256, 0, s>>>(A.get(), m, pin, nid.get(), lab.get(), alive.get());
+      EVOC_CHECK_LAUNCH();
+      exclusive_scan_i32_to_i64(ctx, keep.get(), off.get(), m);
+      exclusive_scan_i32_to_i64(ctx, alive.get(), off2.get(), m);
+      k_mst_emit<<<gm, 256, 0, s>>>(m, keep.get(), off.get(), eu.get(), ev.get(), ew.get(), len,
+                                    d_u, d_v, d_w);
+      EVOC_CHECK_LAUNCH();
+      k_mst_compact<<<gm, 256, 0, s>>>(A.get(), m, alive.get(), off2.get(), A2.get());
+      EVOC_CHECK_LAUNCH();
+      EVOC_CUDA(cudaMemcpyAsync(&h_tot[0], off.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      EVOC_CUDA(cudaMemcpyAsync(&h_tot[1], off2.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     }
-    k_mst_newid<<<gm, 256, 0, s>>>(A.get(), m, pin, nid.get());
-    EVOC_CHECK_LAUNCH();
-    k_mst_label<<<gm, 256, 0, s>>>(A.get(), m, pin, nid.get(), lab.get(), alive.get());
-    EVOC_CHECK_LAUNCH();
-    exclusive_scan_i32_to_i64(ctx, keep.get(), off.get(), m);
-    exclusive_scan_i32_to_i64(ctx, alive.get(), off2.get(), m);
-    k_mst_emit<<<gm, 256, 0, s>>>(m, keep.get(), off.get(), eu.get(), ev.get(), ew.get(), len,
-                                  d_u, d_v, d_w);
-    EVOC_CHECK_LAUNCH();
     k_mst_relabel<<<gn, 256, 0, s>>>(comp.get(), n, lab.get());
     EVOC_CHECK_LAUNCH();
-    k_mst_compact<<<gm, 256, 0, s>>>(A.get(), m, alive.get(), off2.get(), A2.get());
-    EVOC_CHECK_LAUNCH();
-    EVOC_CUDA(cudaMemcpyAsync(&h_tot[0], off.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    EVOC_CUDA(cudaMemcpyAsync(&h_tot[1], off2.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     EVOC_CUDA(cudaStreamSynchronize(s));
     std::swap(A, A2);
     const int64_t kept = h_tot[0];
