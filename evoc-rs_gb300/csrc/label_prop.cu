@@ -282,6 +282,9 @@ __global__ void __launch_bounds__(RG_LONG_THREADS) k_lp_iter_long(
   __shared__ float wb[RG_LONG_THREADS / 32];
   __shared__ uint32_t wf[RG_LONG_THREADS / 32], wl[RG_LONG_THREADS / 32];
   const unsigned FULL = 0xffffffffu;
+  // launched while the short rows' kernel ends, and the next round while this one does
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int nl = *n_long;
   for (int item = blockIdx.x; item < nl; item += gridDim.x) {
     const uint32_t i = longs[item];
@@ -561,10 +564,15 @@ int64_t label_prop_partition(evoc_ctx* ctx, const evoc_graph* g, int64_t approx_
           (const int32_t*)(it > 0 ? flag.get() + it - 1 : nullptr), flag.get() + it, longs.get(),
           n_long.get() + it, it, (const uint8_t*)mark, next, npw));
       if (longest > RG_CAP) {  // else no row can be left over
-        k_lp_iter_long<<<lgrid, RG_LONG_THREADS, sizeof(RgLongVotes), s>>>(
-            g->indptr.get(), g->indices.get(), g->weights.get(), la.get(), lb.get(),
-            flag.get() + it, longs.get(), n_long.get() + it, it, next);
-        EVOC_CHECK_LAUNCH();
+        cfg.gridDim = dim3(lgrid);
+        cfg.blockDim = dim3(RG_LONG_THREADS);
+        cfg.dynamicSmemBytes = sizeof(RgLongVotes);
+        cfg.numAttrs = 1;
+        EVOC_CUDA(cudaLaunchKernelEx(
+            &cfg, k_lp_iter_long, (const int64_t*)g->indptr.get(),
+            (const uint32_t*)g->indices.get(), (const float*)g->weights.get(),
+            (const int32_t*)la.get(), lb.get(), flag.get() + it, (const uint32_t*)longs.get(),
+            (const int32_t*)(n_long.get() + it), it, next));
       }
       std::swap(la, lb);
     }
