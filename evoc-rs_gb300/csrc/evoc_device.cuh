@@ -52,6 +52,27 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   return unpack2(r);
 }
 
+// Loads of data that the launch before this one wrote, where this one was allowed to
+// start while that one still ran (programmatic launch, griddepcontrol.wait). Such data
+// is not read-only for as long as the grid lives, so it must not go through
+// const __restrict__ (ld.global.nc, which may also be moved above the wait): it is read
+// from L2, in program order after the wait.
+__device__ __forceinline__ int32_t load_l2(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t load_l2(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint8_t load_l2(const uint8_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.cg.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return (uint8_t)v;
+}
+
 // max(a, 0) with NaN -> 0, the result of Rust's f32::max(a, 0.0).
 __device__ __forceinline__ float max0(float a) { return (a > 0.0f) ? a : 0.0f; }
 
