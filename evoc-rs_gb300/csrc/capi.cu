@@ -166,7 +166,7 @@ int evoc_ctx_create(int device, evoc_ctx_t** out) {
   }
   (void)cudaGetLastError();
   EVOC_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  evoc::dev_pool_open(c->stream, prop.totalGlobalMem / 8);
+  evoc::dev_pool_open(c->stream, device, prop.totalGlobalMem / 8);
   c->status.alloc(1, c->stream);
   EVOC_CUDA(cudaMemsetAsync(c->status.get(), 0, sizeof(int32_t), c->stream));
   c->sk_steps.alloc(1, c->stream);

@@ -2771,6 +2771,7 @@ void plan_run_device(evoc_plan* pl, const float* d_init, float* d_out) {
       pl->ran = true;
     } else {
       if (!pl->graph_exec) {
+        const PoolCapture hold(s);
         EVOC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         try {
           launch_all();

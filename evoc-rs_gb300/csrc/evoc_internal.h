@@ -50,9 +50,18 @@ enum StatusBit : int32_t {
 // ---------------------------------------------------------------------------
 // Stream-ordered device buffer, from the stream's pool (pool.cu).
 // ---------------------------------------------------------------------------
-void dev_pool_open(cudaStream_t s, size_t limit);
+void dev_pool_open(cudaStream_t s, int device, size_t limit);
 void dev_pool_close(cudaStream_t s);
 size_t dev_pool_bytes(cudaStream_t s);  // free bytes held
+// Between the two calls the stream is being captured: no other context frees on it.
+void dev_pool_capture(cudaStream_t s, bool on);
+struct PoolCapture {
+  cudaStream_t s;
+  explicit PoolCapture(cudaStream_t st) : s(st) { dev_pool_capture(s, true); }
+  ~PoolCapture() { dev_pool_capture(s, false); }
+  PoolCapture(const PoolCapture&) = delete;
+  PoolCapture& operator=(const PoolCapture&) = delete;
+};
 cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s, size_t* held);
 void dev_free(void* ptr, size_t held, cudaStream_t s);
 

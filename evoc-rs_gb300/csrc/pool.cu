@@ -6,13 +6,20 @@
 // pass at 2,000 points). A call takes the same sizes as the one before, so freed
 // buffers are kept by size class and handed out again. A pool belongs to one
 // stream and only serves that stream, so a buffer's next use comes after its last
-// one in stream order, as with the driver's allocator. Free buffers are bounded by
-// an eighth of the device's memory (the least recently freed go first), are given
-// back when an allocation fails, and with the context.
+// one in stream order, as with the driver's allocator. A pool's free buffers are
+// bounded by an eighth of the device's memory (the least recently freed go first), are
+// given back when an allocation fails, and with the context. The bound is per context:
+// contexts on one device hold as many eighths between them as there are contexts, and
+// give them up to one another when an allocation fails.
+//
+// A pool is touched for another context only under the lock, only on the same device,
+// and only while its stream is not being captured: a free enqueued then would become a
+// part of the capture.
 #include "evoc_internal.h"
 
 #include <map>
 #include <mutex>
+#include <new>
 
 namespace evoc {
 namespace {
@@ -34,6 +41,8 @@ struct Pool {
   size_t bytes = 0;                                  // free bytes held
   size_t limit = 0;
   uint64_t stamp = 0;
+  int device = 0;
+  bool capturing = false;  // the context is capturing its stream (dev_pool_capture)
 
   // A block of the class, or of a little more for buffers that are worth it.
   void* take(size_t cls, size_t* held) {
@@ -49,6 +58,7 @@ struct Pool {
     }
     return nullptr;
   }
+  // Gives buffers back until `to` bytes are left; one that cannot be freed stays.
   void shrink(size_t to, cudaStream_t s) {
     while (bytes > to) {
       auto oldest = free_blocks.end();
@@ -58,7 +68,10 @@ struct Pool {
              it->second.front().stamp < oldest->second.front().stamp))
           oldest = it;
       if (oldest == free_blocks.end()) break;
-      cudaFreeAsync(oldest->second.front().ptr, s);
+      if (cudaFreeAsync(oldest->second.front().ptr, s) != cudaSuccess) {
+        (void)cudaGetLastError();
+        break;
+      }
       oldest->second.erase(oldest->second.begin());
       bytes -= oldest->first;
     }
@@ -70,9 +83,17 @@ std::map<cudaStream_t, Pool> g_pools;
 
 }  // namespace
 
-void dev_pool_open(cudaStream_t s, size_t limit) {
+void dev_pool_open(cudaStream_t s, int device, size_t limit) {
   std::lock_guard<std::mutex> lk(g_mu);
-  g_pools[s].limit = limit;
+  Pool& p = g_pools[s];
+  p.limit = limit;
+  p.device = device;
+}
+
+void dev_pool_capture(cudaStream_t s, bool on) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  auto it = g_pools.find(s);
+  if (it != g_pools.end()) it->second.capturing = on;
 }
 
 void dev_pool_close(cudaStream_t s) {
@@ -101,19 +122,32 @@ cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s, size_t* held) {
   cudaError_t e = cudaMallocAsync(ptr, cls, s);
   if (e == cudaSuccess) return e;
   (void)cudaGetLastError();
-  {  // give back what this stream holds, then what the others do
+  int device = -1;
+  {  // give back what this stream holds
     std::lock_guard<std::mutex> lk(g_mu);
     auto it = g_pools.find(s);
-    if (it != g_pools.end()) it->second.shrink(0, s);
+    if (it != g_pools.end()) {
+      it->second.shrink(0, s);
+      device = it->second.device;
+    }
   }
   e = cudaMallocAsync(ptr, cls, s);
   if (e == cudaSuccess) return e;
   (void)cudaGetLastError();
-  {
+  {  // then what the others on the device do, once their streams are done with it
     std::lock_guard<std::mutex> lk(g_mu);
-    for (auto& p : g_pools) p.second.shrink(0, p.first);
+    for (auto& p : g_pools) {
+      if (p.first == s || p.second.device != device || p.second.capturing || !p.second.bytes)
+        continue;
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;  // by the caller's own hand
+      if (cudaStreamIsCapturing(p.first, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        continue;
+      }
+      p.second.shrink(0, p.first);
+      cudaStreamSynchronize(p.first);
+    }
   }
-  cudaDeviceSynchronize();
   return cudaMallocAsync(ptr, cls, s);
 }
 
@@ -124,9 +158,12 @@ void dev_free(void* ptr, size_t held, cudaStream_t s) {
     if (it != g_pools.end() && held <= it->second.limit) {
       Pool& p = it->second;
       p.shrink(p.limit - held, s);
-      p.free_blocks[held].push_back(Block{ptr, ++p.stamp});
-      p.bytes += held;
-      return;
+      try {
+        p.free_blocks[held].push_back(Block{ptr, ++p.stamp});
+        p.bytes += held;
+        return;
+      } catch (const std::bad_alloc&) {  // no host memory for the entry: not kept
+      }
     }
   }
   cudaFreeAsync(ptr, s);
