@@ -2091,14 +2091,13 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
     throw Error(EVOC_ERR_UNSUPPORTED,
                 "more than 2^20 negative samples per edge and epoch "
                 "(negative_sample_rate too large)");
-  // Slots may take half of what is free, of which what the pool holds is a part; the
-  // driver (30 us a call) is asked for the rest only where that part does not settle it.
+  // Slots may take half of what an allocation could obtain, of which what this pool
+  // holds is a part; the driver (30 us a call) is asked for the rest only where that
+  // part does not settle it.
   const double need = (double)sizeof(uint32_t) * (double)total;
-  if (!force_slots && need > 0.5 * (double)dev_pool_bytes(s)) {
-    size_t free_b = 0, total_b = 0;
-    EVOC_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if (need > 0.5 * ((double)free_b + (double)dev_pool_bytes(s))) return false;
-  }
+  if (!force_slots && need > 0.5 * (double)dev_pool_bytes(s) &&
+      need > 0.5 * (double)dev_available(s))
+    return false;
   pl->max_neg = maxneg;
   trace.mark("offset scan + sync");
   {

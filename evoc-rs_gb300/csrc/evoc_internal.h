@@ -53,6 +53,7 @@ enum StatusBit : int32_t {
 void dev_pool_open(cudaStream_t s, int device, size_t limit);
 void dev_pool_close(cudaStream_t s);
 size_t dev_pool_bytes(cudaStream_t s);  // free bytes held
+size_t dev_available(cudaStream_t s);   // bytes that an allocation could obtain
 // Between the two calls the stream is being captured: no other context frees on it.
 void dev_pool_capture(cudaStream_t s, bool on);
 struct PoolCapture {

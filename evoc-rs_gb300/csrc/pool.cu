@@ -110,6 +110,32 @@ size_t dev_pool_bytes(cudaStream_t s) {
   return it == g_pools.end() ? 0 : it->second.bytes;
 }
 
+// Bytes that dev_alloc could obtain for the stream: the device's free memory, what the
+// driver's pool keeps of freed buffers (it returns none to the device), and what the
+// contexts' pools hold free. The same before a buffer's first use and after its free,
+// wherever the free has put it.
+size_t dev_available(cudaStream_t s) {
+  size_t free_b = 0, total_b = 0;
+  EVOC_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  int device = 0;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_pools.find(s);
+    if (it != g_pools.end()) device = it->second.device;
+    for (auto& p : g_pools)
+      if (p.second.device == device) free_b += p.second.bytes;
+  }
+  cudaMemPool_t pool;
+  uint64_t reserved = 0, used = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+      reserved > used)
+    free_b += reserved - used;
+  (void)cudaGetLastError();
+  return free_b;
+}
+
 // A buffer of at least `bytes`; *held is its size class, to be given to dev_free.
 cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s, size_t* held) {
   const size_t cls = class_of(bytes);

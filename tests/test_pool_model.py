@@ -112,6 +112,24 @@ void scenario() {
   DevBuf<char> b = take(0, 48);
   expect(b.get() != nullptr && st[1].frees == 32, "given up afterwards");
 }''',
+    # what can be had is the same before a buffer's first use and after its free, whether
+    # the free put it into this pool, another one or the driver's
+    "available": r'''
+void scenario() {
+  dev[0].capacity = 64 * MB;
+  open(0, 0, 8 * MB); open(1, 0, 8 * MB);
+  expect(dev_available(stream(0)) == 64 * MB, "all of it");
+  for (int round = 0; round < 3; ++round) {  // a plan built, freed and built again
+    expect(30 * MB <= dev_available(stream(0)) / 2, "half of it is enough for the slots");
+    { DevBuf<char> slots = take(0, 30); expect(dev_available(stream(0)) == 34 * MB, "in use"); }
+    expect(dev_available(stream(0)) == 64 * MB, "above the bound: back with the driver's pool");
+  }
+  fill(0, 8); fill(0, 4); fill(1, 8);
+  { DevBuf<char> b = take(0, 6); }  // evicts
+  expect(dev_available(stream(0)) == 64 * MB, "in this pool and the other's");
+  DevBuf<char> b = take(1, 20);
+  expect(dev_available(stream(0)) == 44 * MB, "less what is in use");
+}''',
     "devices": r'''
 void scenario() {
   dev[0].capacity = dev[1].capacity = 16 * MB;
@@ -120,6 +138,7 @@ void scenario() {
   bool refused = false;
   try { take(0, 20); } catch (const Error&) { refused = true; }
   expect(refused && st[1].frees == 0, "a pool on another device is of no use");
+  expect(dev_available(stream(0)) == 16 * MB, "nor is it counted");
 }''',
     # a buffer that cannot be freed is kept, not lost
     "failing_free": r'''
