@@ -1999,11 +1999,12 @@ struct IncEntries {
 };
 
 // Slots path of the schedule set-up: the schedule in bit planes per tile
-// (n_epochs <= MASK_EPOCHS and at most MASK_NEGS negatives per edge and epoch) or
-// the per-entry recurrence (otherwise), then offset scan, tile order and fill
-// pass. Returns false (nothing built) when EVOC_EPOCH_PATH=scan, when the epoch
-// count exceeds the shared-memory cursors, or when the slots would take more than
-// half of the free device memory (unless EVOC_EPOCH_PATH=slots).
+// (n_epochs <= MASK_EPOCHS and at most MASK_NEGS negatives per edge and epoch, where
+// there is room for the planes) or the per-entry recurrence (otherwise), then offset
+// scan, tile order and fill pass. Returns false (nothing built) when
+// EVOC_EPOCH_PATH=scan, when the epoch count exceeds the shared-memory cursors, or when
+// the slots would take more than half of the memory that can be had (unless
+// EVOC_EPOCH_PATH=slots).
 template <class Entries>
 static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_base,
                         Entries entries) {
@@ -2051,7 +2052,12 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
     const int64_t max_words = pl->n_inc / 32 + pl->ntiles;
     bool neg4 = wide_neg;
     for (;;) {
-      planes.alloc(max_words * (neg4 ? 5 : 3) * ne, s);
+      try {
+        planes.alloc(max_words * (neg4 ? 5 : 3) * ne, s);
+      } catch (const Error&) {  // no room: the recurrence per entry needs none of them
+        use_planes = false;
+        break;
+      }
       (wide_ep ? (neg4 ? launch_masks<4, 4> : launch_masks<4, 2>)
                : (neg4 ? launch_masks<2, 4> : launch_masks<2, 2>))(
           iv, wbase.get(), planes.get(), counts.get(), fires.get(), mx, s);
@@ -2073,6 +2079,13 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
     mask_neg4 = neg4;
   }
   IncEntries* ent = nullptr;
+  // The planes take up to 80 bytes an entry, the lists of the recurrence per entry 9:
+  // where the slots need that room, they are given up for the other fill.
+  auto drop_planes = [&]() {
+    planes.release();
+    ent = entries();
+    use_planes = false;
+  };
   if (!use_planes) {
     ent = entries();
     const size_t csmem = (size_t)wpb * ne * sizeof(int32_t);
@@ -2095,9 +2108,14 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
   // holds is a part; the driver (30 us a call) is asked for the rest only where that
   // part does not settle it.
   const double need = (double)sizeof(uint32_t) * (double)total;
-  if (!force_slots && need > 0.5 * (double)dev_pool_bytes(s) &&
-      need > 0.5 * (double)dev_available(s))
-    return false;
+  auto fits = [&]() {
+    return force_slots || need <= 0.5 * (double)dev_pool_bytes(s) ||
+           need <= 0.5 * (double)dev_available(s);
+  };
+  if (!fits()) {
+    if (use_planes) drop_planes();
+    if (!fits()) return false;
+  }
   pl->max_neg = maxneg;
   trace.mark("offset scan + sync");
   {
@@ -2113,7 +2131,13 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
     EVOC_CHECK_LAUNCH();
   }
   trace.mark("tile order");
-  pl->slots.alloc(total, s);
+  try {
+    pl->slots.alloc(total, s);
+  } catch (const Error&) {
+    if (!use_planes) throw;
+    drop_planes();
+    pl->slots.alloc(total, s);
+  }
   trace.mark("alloc slots");
   const ProbInfo* pinfo = pl->n_problems > 1 ? pl->prob.get() : nullptr;
   const uint64_t seed0 = pl->seeds.empty() ? 0 : pl->seeds[0];
