@@ -1476,17 +1476,30 @@ __device__ __forceinline__ void slot_contrib(float (&c)[DIMP], bool neg,
   }
 }
 
+// What changes from epoch to epoch, as the kernels see it. A launch per epoch has it in
+// its arguments.
+struct OneEpoch {
+  using Node = int64_t;
+  const EpochArgs& a;
+  __device__ __forceinline__ const float* e_cur() const { return a.e_cur; }
+  __device__ __forceinline__ float* e_next() const { return a.e_next; }
+  __device__ __forceinline__ const int64_t* tile_off() const { return a.tile_off; }
+  __device__ __forceinline__ float gamma() const { return a.gamma; }
+  __device__ __forceinline__ float lr_ad() const { return a.lr_ad; }
+  __device__ __forceinline__ float epsc() const { return a.epsc; }
+};
+
 // Phase 1 for U slots per lane: window slots ib + 32 u + lane, u < U, in sl (past the
 // window's end: its last slot again, which is gathered but adds nothing).
 template <int DIMP, int WIN, int U>
-__device__ __forceinline__ void slot_group(const EpochArgs& a, SlotSmem<DIMP, WIN>& sm,
+__device__ __forceinline__ void slot_group(const float* e_cur, SlotSmem<DIMP, WIN>& sm,
                                            const uint32_t (&sl)[U], int ib, int wn, int lane,
                                            int& carry, float two_noise, float gamma4) {
   const unsigned FULL = 0xffffffffu;
   float row[U][DIMP];
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    load_row<DIMP, true>(a.e_cur + (size_t)(sl[u] >> SLOT_ROW_SHIFT) * DIMP, row[u]);
+    load_row<DIMP, true>(e_cur + (size_t)(sl[u] >> SLOT_ROW_SHIFT) * DIMP, row[u]);
 #pragma unroll
   for (int u = 0; u < U; ++u) {  // run starts (a repeated last slot starts nothing)
     const int i = ib + 32 * u + lane;
@@ -1514,41 +1527,45 @@ __device__ __forceinline__ void slot_group(const EpochArgs& a, SlotSmem<DIMP, WI
 
 // The w-th tile in tile_order: its slots of the epoch and the first group of them.
 // Nothing here is written by an epoch.
-template <int SU>
+template <int SU, class Node>
 struct SlotHead {
-  int64_t v0, s0, s1;
+  Node v0;
+  int64_t s0, s1;
   uint32_t nx[SU];  // the next group's slots, fetched while the group before it is gathered
 };
-template <int SU>
-__device__ __forceinline__ SlotHead<SU> slot_head(const EpochArgs& a, unsigned long long w,
-                                                  int lane) {
-  SlotHead<SU> h;
+template <int SU, class Epoch>
+__device__ __forceinline__ SlotHead<SU, typename Epoch::Node> slot_head(const Epoch& ep, uint64_t w,
+                                                                       int lane) {
+  const EpochArgs& a = ep.a;
+  SlotHead<SU, typename Epoch::Node> h;
   const int64_t tile = (int64_t)a.tile_order[w];
-  h.v0 = tile * a.tn;
-  h.s0 = a.tile_off[tile * a.n_epochs];
-  h.s1 = a.tile_off[tile * a.n_epochs + 1];
+  h.v0 = (typename Epoch::Node)tile * a.tn;
+  h.s0 = ep.tile_off()[tile * a.n_epochs];
+  h.s1 = ep.tile_off()[tile * a.n_epochs + 1];
 #pragma unroll
   for (int u = 0; u < SU; ++u)
     h.nx[u] = h.s0 < h.s1 ? __ldcs(a.slots + min(h.s0 + 32 * u + lane, h.s1 - 1)) : 0u;
   return h;
 }
 
-template <int DIMP, int WIN, int SU>
-__device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN>& sm,
-                                          SlotHead<SU>& h, int lane) {
+template <int DIMP, int WIN, int SU, class Epoch>
+__device__ __forceinline__ void slot_tile(const Epoch& ep, SlotSmem<DIMP, WIN>& sm,
+                                          SlotHead<SU, typename Epoch::Node>& h, int lane) {
+  const EpochArgs& a = ep.a;
   const unsigned FULL = 0xffffffffu;
-  const int64_t v0 = h.v0, s0 = h.s0, s1 = h.s1;
-  const int nt = (int)min((int64_t)a.tn, (int64_t)a.n_total - v0);
+  const typename Epoch::Node v0 = h.v0;
+  const int64_t s0 = h.s0, s1 = h.s1;
+  const int nt = (int)min((typename Epoch::Node)a.tn, (typename Epoch::Node)a.n_total - v0);
   __syncwarp();  // the previous tile's readers of the shared rows and sums are done
   {
-    const float4* src = reinterpret_cast<const float4*>(a.e_cur + (size_t)v0 * DIMP);
+    const float4* src = reinterpret_cast<const float4*>(ep.e_cur() + (size_t)v0 * DIMP);
     float4* dst = reinterpret_cast<float4*>(&sm.rows[0][0]);
     for (int i = lane; i < nt * (DIMP / 4); i += 32) dst[i] = __ldcg(src + i);
     float4* sz = reinterpret_cast<float4*>(&sm.S[0][0]);
     for (int i = lane; i < nt * (DIMP / 4); i += 32) sz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const float two_noise = fmul(2.0f, a.noise);
-  const float gamma4 = fmul(a.gamma, 4.0f);
+  const float gamma4 = fmul(ep.gamma(), 4.0f);
   uint32_t act_mask = 0;
   static_assert(WIN % (32 * SU) == 0, "a group does not cross a window");
   for (int64_t w0 = s0; w0 < s1; w0 += WIN) {
@@ -1566,7 +1583,7 @@ __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN
         for (int u = 0; u < SU; ++u)
           h.nx[u] = __ldcs(a.slots + min(next + 32 * u + lane, s1 - 1));
       }
-      slot_group<DIMP, WIN, SU>(a, sm, sl, ib, wn, lane, carry, two_noise, gamma4);
+      slot_group<DIMP, WIN, SU>(ep.e_cur(), sm, sl, ib, wn, lane, carry, two_noise, gamma4);
     }
     __syncwarp();
     // run of node l: [start[l], first start of a later node or wn)
@@ -1621,17 +1638,18 @@ __device__ __forceinline__ void slot_tile(const EpochArgs& a, SlotSmem<DIMP, WIN
       float mm[DIMP], vv[DIMP];
       load_row<DIMP, true>(a.m + q, mm);
       load_row<DIMP, true>(a.v + q, vv);
+      const float lr_ad = ep.lr_ad(), epsc = ep.epsc();
 #pragma unroll
       for (int d = 0; d < DIMP; ++d) {  // scalar: a packed multiply feeding a packed
         // add did not reproduce the unfused result
         mm[d] = fadd(mm[d], fmul(a.one_m_b1, fsub(g[d], mm[d])));
         vv[d] = fadd(vv[d], fmul(a.one_m_b2, fsub(fmul(g[d], g[d]), vv[d])));
-        e[d] = fadd(e[d], fdiv(fmul(a.lr_ad, mm[d]), fadd(fsqrt(vv[d]), a.epsc)));
+        e[d] = fadd(e[d], fdiv(fmul(lr_ad, mm[d]), fadd(fsqrt(vv[d]), epsc)));
       }
       store_row<DIMP>(a.m + q, mm);
       store_row<DIMP>(a.v + q, vv);
     }
-    store_row<DIMP>(a.e_next + q, e);  // evict-first: keep e_cur's rows in L2 for the gathers
+    store_row<DIMP>(ep.e_next() + q, e);  // evict-first: keep e_cur's rows in L2 for the gathers
     if (a.grad_out) {
       float4* go = reinterpret_cast<float4*>(a.grad_out + q);
 #pragma unroll
@@ -1653,17 +1671,18 @@ __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4) k_epoch_slot(EpochArgs
   const int64_t ntiles = a.ntiles;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
   unsigned long long w = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  SlotHead<SU> h;
-  if ((int64_t)w < ntiles) h = slot_head<SU>(a, w, lane);
+  const OneEpoch ep{a};
+  SlotHead<SU, OneEpoch::Node> h;
+  if ((int64_t)w < ntiles) h = slot_head<SU>(ep, w, lane);
   // The epoch before this one may still run (launch_epoch): what it writes is touched
   // only from here on. The next one may then be brought onto the SMs.
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   while ((int64_t)w < ntiles) {
-    slot_tile<DIMP, WIN, SU>(a, sm, h, lane);
+    slot_tile<DIMP, WIN, SU>(ep, sm, h, lane);
     if (lane == 0) w = warps + atomicAdd(a.work_ctr, 1ull);
     w = __shfl_sync(0xffffffffu, w, 0);
-    if ((int64_t)w < ntiles) h = slot_head<SU>(a, w, lane);
+    if ((int64_t)w < ntiles) h = slot_head<SU>(ep, w, lane);
   }
 }
 
@@ -1677,7 +1696,7 @@ __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4) k_epoch_slot(EpochArgs
 // ---------------------------------------------------------------------------
 struct EpochAllArgs {
   const float4* ep;               // per epoch: gamma, lr * ad_scale, eps', 0
-  const int64_t* tile_off;        // all epochs: [t * ntiles + tile]
+  const int64_t* tile_off;        // all epochs: [tile * n_epochs + t]
   unsigned long long* work_ctr;   // per epoch, zeroed before the launch
   float* e0;                      // embedding at epoch t0 (ping-pong with e1)
   float* e1;
@@ -1728,33 +1747,36 @@ __device__ bool grid_barrier(unsigned* bar, unsigned nblocks, int32_t* status) {
   return ok_s != 0;
 }
 
+// Epoch t of all: formed from the arguments where it is used, not held. With a copy of
+// EpochArgs per epoch and 64-bit tile numbers <8, *, 2> spilled 48 bytes at its 72
+// registers (2M nodes, 4 warps: 13.8 ms, 13.0 without).
+struct EpochOfAll {
+  using Node = uint32_t;  // fewer than SLOT_MAX_ROWS
+  const EpochArgs& a;
+  const EpochAllArgs& x;
+  int32_t t;
+  __device__ __forceinline__ const float* e_cur() const { return ((t - x.t0) & 1) ? x.e1 : x.e0; }
+  __device__ __forceinline__ float* e_next() const { return ((t - x.t0) & 1) ? x.e0 : x.e1; }
+  __device__ __forceinline__ const int64_t* tile_off() const { return x.tile_off + t; }
+  __device__ __forceinline__ float gamma() const { return x.ep[t].x; }
+  __device__ __forceinline__ float lr_ad() const { return x.ep[t].y; }
+  __device__ __forceinline__ float epsc() const { return x.ep[t].z; }
+};
+
 template <int DIMP, int WIN, int SU>
 __global__ void __launch_bounds__(128, DIMP <= 8 ? 7 : 4)
     k_epoch_slot_all(EpochArgs base, EpochAllArgs x) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   SlotSmem<DIMP, WIN>& sm = reinterpret_cast<SlotSmem<DIMP, WIN>*>(smem_raw)[threadIdx.x >> 5];
-  const int64_t ntiles = base.ntiles;
-  const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-  const unsigned long long first =
-      (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t ntiles = (uint32_t)base.ntiles;
   for (int32_t t = x.t0; t < x.t1; ++t) {
-    EpochArgs a = base;
-    const int k = t - x.t0;
-    a.e_cur = (k & 1) ? x.e1 : x.e0;
-    a.e_next = (k & 1) ? x.e0 : x.e1;
-    a.tile_off = x.tile_off + t;
-    a.work_ctr = x.work_ctr + t;
-    const float4 ep = x.ep[t];
-    a.gamma = ep.x;
-    a.lr_ad = ep.y;
-    a.epsc = ep.z;
-    a.epoch = (uint32_t)t;
-    unsigned long long w = first;
-    while ((int64_t)w < ntiles) {
-      SlotHead<SU> h = slot_head<SU>(a, w, lane);
-      slot_tile<DIMP, WIN, SU>(a, sm, h, lane);
-      if (lane == 0) w = warps + atomicAdd(a.work_ctr, 1ull);
+    const EpochOfAll ep{base, x, t};
+    uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    while (w < ntiles) {
+      SlotHead<SU, EpochOfAll::Node> h = slot_head<SU>(ep, w, lane);
+      slot_tile<DIMP, WIN, SU>(ep, sm, h, lane);
+      if (lane == 0) w = gridDim.x * (blockDim.x >> 5) + (uint32_t)atomicAdd(x.work_ctr + t, 1ull);
       w = __shfl_sync(0xffffffffu, w, 0);
     }
     if (t + 1 < x.t1 && !grid_barrier(x.bar, x.nblocks, x.status)) return;
