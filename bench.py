@@ -224,13 +224,23 @@ def cpu_epochs_sample(ip, ix, w, dim, seed, stats, t0: int, n_ep: int, max_secon
     return fired / tsec, cores, tsec, emb, st
 
 
+def fuzzy_set_line(ms: float, n: int, k: int, nnz: int, steps: int, hbm_gbs: float) -> dict:
+    """The fuzzy simplicial set against its HBM bound: the kNN indices and
+    distances read (8 n k bytes), the CSR written (8 (n + 1) + 8 nnz) and sigma /
+    rho (8 n). The bisection steps are those of a serial evaluation; the kernel
+    decides most of them without their sums, so no rate of exps follows from them."""
+    hbm_bytes = 8 * n * k + 8 * (n + 1) + 8 * nnz + 8 * n
+    gbs = hbm_bytes / (ms / 1e3) / 1e9
+    return {"ms": round(ms, 3), "hbm_bytes": int(hbm_bytes), "achieved_gbs": round(gbs, 1),
+            "hbm_peak": hbm_gbs, "hbm_frac": round(gbs / hbm_gbs, 4),
+            "hbm_roofline_ms": round(hbm_bytes / (hbm_gbs * 1e9) * 1e3, 3),
+            "smooth_knn_steps": int(steps),
+            "mean_bisection_steps_per_row": round(steps / n, 2)}
+
+
 def fuzzy_set_roofline(ctx, idx32, dist, n: int, k: int, nnz: int, pk: dict, reps: int = 5):
     """Device time of the fuzzy simplicial set from the device kNN graph
-    (CUDA events on the library stream, mean of reps after one warm-up) with
-    its two bounds. HBM: the kNN indices and distances read (8 n k bytes), the
-    CSR written (8 (n + 1) + 8 nnz) and sigma / rho (8 n). ALU: exp
-    evaluations, k per bisection step of every row (the step count is
-    measured by the kernel) plus one per kNN entry for the weights."""
+    (CUDA events on the library stream, mean of reps after one warm-up)."""
     import torch
     stream = torch.cuda.ExternalStream(ctx.stream)
     g = ctx.fuzzy_set_device(idx32.data_ptr(), dist.data_ptr(), n, k, float(k), True)
@@ -244,16 +254,7 @@ def fuzzy_set_roofline(ctx, idx32, dist, n: int, k: int, nnz: int, pk: dict, rep
         g.free()
     e1.record(stream)
     torch.cuda.synchronize()
-    ms = e0.elapsed_time(e1) / reps
-    hbm_bytes = 8 * n * k + 8 * (n + 1) + 8 * nnz + 8 * n
-    exps = steps * k + n * k
-    gbs = hbm_bytes / (ms / 1e3) / 1e9
-    return {"ms": round(ms, 3), "hbm_bytes": int(hbm_bytes), "achieved_gbs": round(gbs, 1),
-            "hbm_peak": pk["hbm_gbs"], "hbm_frac": round(gbs / pk["hbm_gbs"], 4),
-            "hbm_roofline_ms": round(hbm_bytes / (pk["hbm_gbs"] * 1e9) * 1e3, 3),
-            "smooth_knn_steps": int(steps), "exp_evaluations": int(exps),
-            "exp_per_s": round(exps / (ms / 1e3), 1),
-            "mean_bisection_steps_per_row": round(steps / n, 2)}
+    return fuzzy_set_line(e0.elapsed_time(e1) / reps, n, k, nnz, steps, pk["hbm_gbs"])
 
 
 def _same_bits(a: np.ndarray, b: np.ndarray) -> bool:

@@ -158,8 +158,8 @@ struct evoc_ctx {
   cudaStream_t stream = nullptr;
   std::string last_error;
   evoc::DevBuf<int32_t> status;  // device status word
-  // Row-sum evaluations (bisection steps over all rows) of the most recent
-  // smooth_knn pass on this context: the work figure of its ALU bound.
+  // Bisection steps over all rows of the most recent smooth_knn pass on this
+  // context, whether a step's sum was evaluated or its side was certain.
   evoc::DevBuf<unsigned long long> sk_steps;
 };
 

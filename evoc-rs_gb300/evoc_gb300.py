@@ -478,8 +478,8 @@ class Context:
         return g.value
 
     def smooth_knn_steps(self) -> int:
-        """Row-sum evaluations (bisection steps over all rows) of the most
-        recent smooth_knn_dist pass on this context."""
+        """Bisection steps over all rows of the most recent smooth_knn_dist pass
+        on this context (most are decided without evaluating their sum)."""
         v = C.c_int64()
         self._check(self.lib.evoc_ctx_smooth_knn_steps(self.handle, C.byref(v)))
         return v.value

@@ -115,9 +115,10 @@ EVOC_API const char* evoc_last_error(const evoc_ctx_t* ctx);
 EVOC_API void* evoc_ctx_stream(const evoc_ctx_t* ctx);
 
 /* Bisection steps of the most recent smooth_knn_dist pass on ctx (by
- * evoc_smooth_knn_dist or a fuzzy set): the number of row-sum evaluations
- * over all rows, each of which evaluates one exp per row entry. A work
- * count for measurement (no counterpart). */
+ * evoc_smooth_knn_dist or a fuzzy set), over all rows: the steps that a serial
+ * evaluation of the reference takes, a row sum each. The kernel decides most of
+ * them without forming the sum, so this is not a count of sums or of exps
+ * evaluated (no counterpart). */
 EVOC_API int evoc_ctx_smooth_knn_steps(evoc_ctx_t* ctx, int64_t* steps);
 
 /* ---- fuzzy simplicial set ------------------------------------------------ */
