@@ -512,8 +512,9 @@ __device__ __forceinline__ void stcs8(float* p, const float* r) {
 
 // A row of DIMP floats (DIMP a multiple of 8: 32-byte aligned, else 16).
 // COH: the row may have been written earlier in the same launch (the
-// persistent all-epochs kernel), so it is read through L2 (ld.global.cg)
-// rather than the non-coherent read-only path.
+// persistent all-epochs kernel) or by the launch that this one overlaps, so it
+// is read through L2 in program order (volatile ld.global.cg) rather than by the
+// non-coherent read-only path.
 template <int DIMP, bool COH = false>
 __device__ __forceinline__ void load_row(const float* __restrict__ p, float (&r)[DIMP]) {
   if constexpr (DIMP % 8 == 0) {
@@ -528,7 +529,7 @@ __device__ __forceinline__ void load_row(const float* __restrict__ p, float (&r)
     const float4* p4 = reinterpret_cast<const float4*>(p);
 #pragma unroll
     for (int i = 0; i < DIMP / 4; ++i) {
-      const float4 x = COH ? __ldcg(p4 + i) : __ldg(p4 + i);
+      const float4 x = COH ? load_l2(p4 + i) : __ldg(p4 + i);
       r[4 * i + 0] = x.x;
       r[4 * i + 1] = x.y;
       r[4 * i + 2] = x.z;
@@ -1560,7 +1561,7 @@ __device__ __forceinline__ void slot_tile(const Epoch& ep, SlotSmem<DIMP, WIN>& 
   {
     const float4* src = reinterpret_cast<const float4*>(ep.e_cur() + (size_t)v0 * DIMP);
     float4* dst = reinterpret_cast<float4*>(&sm.rows[0][0]);
-    for (int i = lane; i < nt * (DIMP / 4); i += 32) dst[i] = __ldcg(src + i);
+    for (int i = lane; i < nt * (DIMP / 4); i += 32) dst[i] = load_l2(src + i);
     float4* sz = reinterpret_cast<float4*>(&sm.S[0][0]);
     for (int i = lane; i < nt * (DIMP / 4); i += 32) sz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }

@@ -72,6 +72,14 @@ __device__ __forceinline__ uint8_t load_l2(const uint8_t* p) {
   asm volatile("ld.global.cg.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return (uint8_t)v;
 }
+__device__ __forceinline__ float4 load_l2(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
 
 // max(a, 0) with NaN -> 0, the result of Rust's f32::max(a, 0.0).
 __device__ __forceinline__ float max0(float a) { return (a > 0.0f) ? a : 0.0f; }

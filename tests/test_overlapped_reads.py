@@ -38,6 +38,17 @@ def test_nothing_handed_on_is_read_as_constant():
             assert not plain, (name, p, plain)
 
 
+def test_epochs_read_rows_in_program_order():
+    """Rows and moments go from epoch to epoch, by launches that overlap or across the
+    barrier of one: read by load_l2 or ldcg8 (volatile, after the wait), not by an
+    intrinsic that the compiler may treat as a function of its address."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "embed.cu").read_text())
+    assert "__ldcg(" not in text
+    device = (CSRC / "evoc_device.cuh").read_text()
+    for body in re.findall(r"load_l2\(const [^{]*\{(.*?)\n\}", device, re.S):
+        assert "asm volatile" in body and '"memory"' in body and "ld.global.cg" in body
+
+
 @pytest.mark.gpu
 def test_rounds_with_hubs_repeat(ctx, oracle):
     """Short and long rows, labels spreading over many rounds, again and again."""
