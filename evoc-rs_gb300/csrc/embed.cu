@@ -2070,7 +2070,12 @@ static bool build_slots(evoc_plan* pl, const IncView& iv, const int64_t* eidx_ba
     EVOC_CUDA(cudaMemcpyAsync(htot.data(), tot.get(), tot.bytes(), cudaMemcpyDeviceToHost, s));
     EVOC_CUDA(cudaStreamSynchronize(s));
   };
-  bool use_planes = ne <= MASK_EPOCHS;
+  // An edge draws one negative per 1.5 ps / r epochs since it last fired, at most 2 ps
+  // before (epochs are whole), and what was left over then: fewer than 2 r / 1.5 + 1.
+  // Below a rate of 11.25 these fit four bits; from there on the planes' pass is for
+  // nothing as soon as one edge is near the largest weight (plans of 300k nodes, 100
+  // epochs, rates 12 to 30: 5 to 7 %).
+  bool use_planes = ne <= MASK_EPOCHS && pl->params.negative_sample_rate < 11.25f;
   // at a rate r an edge draws about r / 1.5 negatives when it fires, one more at times
   const bool wide_neg = pl->params.negative_sample_rate > 2.5f, wide_ep = ne > 64;
   bool mask_neg4 = wide_neg;
