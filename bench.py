@@ -193,7 +193,8 @@ def profiled_traffic() -> tuple[float | None, str | None]:
 def algorithmic_hbm_bytes(n: int, info: dict, dimp: int, stats: np.ndarray) -> np.ndarray:
     """Per-epoch bytes the epoch kernel must move to/from HBM (the partner and
     negative row gathers are served by L2 and counted separately).
-    Slots path (32-node tiles): tile offsets 8 (n/32 + 1), tile order 4 n/32, slots 4 per
+    Slots path (tiles of 32 nodes, the size of these workloads from 200k points
+    on): tile offsets 8 (n/32 + 1), tile order 4 n/32, slots 4 per
     fired directed entry (2 F_t) and per negative sample (N_t), own rows read +
     next rows written 2 * 4 dimp n, Adam moments read + written 4 * 4 dimp A_t.
     Bit-plane path: incidence offsets 8 (n + 1), fire + negative-count planes

@@ -238,7 +238,7 @@ int evoc_smooth_knn_dist(evoc_ctx_t* ctx, const float* dists,
   }
   evoc::smooth_knn_device(ctx, d.get(), rl.get(), n, k, k_target,
                           local_connectivity, n_iter, sg.get(), rh.get(),
-                          nullptr, nullptr);
+                          nullptr);
   EVOC_CUDA(cudaMemcpyAsync(sigmas, sg.get(), sg.bytes(), cudaMemcpyDeviceToHost, s));
   EVOC_CUDA(cudaMemcpyAsync(rhos, rh.get(), rh.bytes(), cudaMemcpyDeviceToHost, s));
   evoc::check_status(ctx, "smooth_knn_dist");

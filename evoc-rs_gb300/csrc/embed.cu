@@ -52,7 +52,7 @@ struct evoc_plan {
   int64_t n = 0;          // nodes over all problems
   int32_t dim = 0;        // n_components
   int32_t dimp = 0;       // padded row width (4, 8 or 16)
-  int32_t lanes = 0;      // warps (32-node tiles) per thread block of k_epoch
+  int32_t lanes = 0;      // warps (node tiles) per thread block of the epoch kernels
   evoc_embed_params_t params{};
   int32_t n_problems = 0;
   std::vector<int64_t> node_base;  // per problem, host
@@ -893,8 +893,8 @@ __global__ void k_tile_words(const int64_t* __restrict__ ptr, int64_t n, int64_t
 // entries in hand are first grouped by kind and by about how often they fire, so
 // that the lanes of a warp run out of epochs together. Stepping all entries
 // through all epochs took 2.95 ms for the edges of the 2M graph alone, and their
-// planes, twin recurrences, lists and counts 7 ms more (3.7 ms here, bound by
-// instruction issue). The masks are turned from entry-major to epoch-major by a
+// planes, twin recurrences, lists and counts 7 ms more (3.7 ms here; 0.66 instructions
+// a cycle and scheduler, the rest fixed latencies, shared memory and block barriers). The masks are turned from entry-major to epoch-major by a
 // 32 x 32 bit transpose. NW 32-epoch words, NB count bits; counts above
 // 2^NB - 1 are caught through max_neg by the host.
 constexpr int MASK_THREADS = 128;
@@ -1134,7 +1134,7 @@ __device__ __forceinline__ uint32_t negative_slot(uint64_t seed, uint32_t j, int
 // at 2M points (1.29 G slots): lane per fire word writing as it walks, 8 epochs to a
 // block, 7.3 ms; lane per epoch with shuffled slot words, 9.2 ms (each of its
 // stores went to 32 sectors, one per cycle and SM); this one 4.9 ms, bound by
-// instruction issue, the draws being a third of it.
+// instruction issue (0.85 a cycle and scheduler), the draws being a third of it.
 constexpr int FILL_WARPS = 8;
 struct FillJob {
   int64_t q;       // slot index

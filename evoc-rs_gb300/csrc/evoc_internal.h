@@ -198,7 +198,7 @@ void smooth_knn_device(evoc_ctx* ctx, const float* d_dist,
                        const int32_t* d_row_len, int64_t n, int32_t k,
                        uint64_t k_target, float local_connectivity,
                        int32_t n_iter, float* d_sigma, float* d_rho,
-                       float* d_weights_out, const uint32_t* d_idx_for_len);
+                       float* d_weights_out);
 void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
                       const float* d_dist, int64_t n, int32_t k,
                       float effective_n_neighbours, bool symmetrise,

@@ -23,7 +23,8 @@
 //                    which is the backward map of fuzzy_graph.rs:190.
 //   k_union          warp per row: merge the sorted forward and backward
 //                    lists, w = w_ij + w_ji - w_ij * w_ji, keep w > 0
-//                    (fuzzy_graph.rs:196-204); once to count, once to write.
+//                    (fuzzy_graph.rs:196-204), into per-row scratch;
+//                    k_union_compact copies the kept pairs into the CSR.
 #include "evoc_device.cuh"
 #include "evoc_internal.h"
 
@@ -84,8 +85,12 @@ __global__ void k_knn_rowlen(const uint32_t* __restrict__ idx, int64_t n,
 // M, for len terms of at most 1 each: the exact terms are off by at most 1.5e-7
 // (quotient, own exp at 1.2 ulp), the approximate ones by 2.4e-7 (ex2.approx
 // 2^-22.5, argument 3 roundings), either sum by len * sum * 2^-24, the target's
-// rounding by 5e-7. 2M rows of 30: 3.3 ms when every step was
-// evaluated, 0.90 now; it is bound by instruction issue.
+// rounding by 5e-7. 2M rows of 30: 3.3 ms when every step was evaluated, 0.90 now;
+// bound by instruction issue (0.87 a cycle and scheduler at 500k rows). Rows that cannot
+// be certified cost the Newton steps on top and hold their warp: 1M rows of 16, every
+// step evaluated in pools of rows / now: exactly 4 zeros in each row 0.43 / 0.43 ms, in
+// one of 32 0.79 / 0.43, an infinity in one of 32 0.79 / 0.70, distances of 3e38 in
+// each row 1.14 / 0.97, in one of 32 1.17 / 1.09.
 // ---------------------------------------------------------------------------
 struct RowState {
   int32_t len;
@@ -583,7 +588,7 @@ void smooth_knn_device(evoc_ctx* ctx, const float* d_dist,
                        const int32_t* d_row_len, int64_t n, int32_t k,
                        uint64_t k_target, float local_connectivity,
                        int32_t n_iter, float* d_sigma, float* d_rho,
-                       float* d_weights_out, const uint32_t* /*unused*/) {
+                       float* d_weights_out) {
   if (n == 0) return;
   const int32_t kp = k | 1;
   // four warps per block, one where that leaves SMs idle or the rows are long
@@ -647,7 +652,7 @@ void fuzzy_set_device(evoc_ctx* ctx, const uint32_t* d_idx,
   if (!d_rho) { rho_local.alloc(n, s); d_rho = rho_local.get(); }
   DevBuf<float> wts(n * (int64_t)k, s);
   smooth_knn_device(ctx, d_dist, row_len.get(), n, k, kk, 1.0f, 64, d_sig,
-                    d_rho, wts.get(), nullptr);
+                    d_rho, wts.get());
   check_status(ctx, "fuzzy set");
   trace.mark("smooth knn + weights");
 

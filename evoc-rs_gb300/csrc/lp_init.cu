@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_reduce_data(
 // ---------------------------------------------------------------------------
 // Products of the symmetric part G o G^T (rows merged with the transpose's,
 // both sorted) times N: key Q = part(j), value (i, s_ij * inv_Q), in
-// row-major order. With `same` the transpose is G itself (canonical graphs).
+// row-major order (canonical graphs pass themselves as the transpose).
 __global__ void k_sym_count(const int64_t* __restrict__ ap, const uint32_t* __restrict__ ai,
                             const int64_t* __restrict__ bp, const uint32_t* __restrict__ bi,
                             int64_t n, int32_t* __restrict__ cnt) {

@@ -360,8 +360,8 @@ __global__ void __launch_bounds__(UP_NODES / 2) k_mst_boxes_up(float* __restrict
 // busy in a leaf and left single warps with thousands of serial steps (1M points,
 // 8-d blobs, the same tree: core distances 26.8 ms against 7.3 here, and 8 to 13 ms
 // in each early round for one straggling warp against 0.8 to 1.1). The instruction
-// count bounds it: about 20 leaves and 10 groups per point, and 12 blocks per SM
-// (40 registers) gain only a tenth over 8.
+// count bounds it (0.88 issued a cycle and scheduler, 400k points): about 20 leaves
+// and 10 groups per point, and 12 blocks per SM (40 registers) gain only a tenth over 8.
 constexpr int MST_WARPS = 4;   // warps per block
 template <int DIMP>
 constexpr int mst_blocks() { return DIMP <= 8 ? 12 : 8; }  // blocks per SM (registers)
@@ -907,9 +907,9 @@ __global__ void __launch_bounds__(32 * MST_WARPS, mst_blocks<DIMP>()) k_mst_noc(
 // nodes. The walk tests nodes against the box of the group's points, so a node is
 // met once for all of them; at a leaf each lane tests its own point against the
 // leaf's box, and the leaf's foreign points (one per lane) are measured against
-// each point that it may still matter to. Bound by instructions, about 35 for a
-// point and leaf and 100 for a node group, as the walk by points. The last four rounds
-// 26.7 -> 9.5 ms (the test of the points before a group of nodes is entered: 24.6 ->
+// each point that it may still matter to. Bound by instructions (0.70 issued a cycle and
+// scheduler with 27 warps an SM, 400k points), about 35 for a point and leaf and 100 for
+// a node group, as the walk by points. The last four rounds 26.7 -> 9.5 ms (the test of the points before a group of nodes is entered: 24.6 ->
 // 22.5 of the whole tree, in the middle rounds, whose groups' boxes are loose).
 constexpr int MST_GROUP_BLOCKS = 8;  // per SM (registers)
 template <int DIMP>
